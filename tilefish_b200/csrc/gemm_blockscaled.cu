@@ -37,7 +37,6 @@ constexpr int kBlockM = 128;
 constexpr int kStageKBytes = 128;  // bytes of K per row per stage: one 128-byte swizzle atom
 constexpr int kAStageBytes = kBlockM * kStageKBytes;
 constexpr int kGemmThreads = 352;  // 11 warps: operand loads, MMA issue, epilogue group 0 (4), scale loads, epilogue group 1 (4)
-constexpr int kPairThreads = 192;  // the CTA-pair kernel keeps one load warp
 constexpr int kSmemLimit = 227 * 1024;
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 
@@ -194,6 +193,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
                "r"(x), "r"(y), "r"(bar)
                : "memory");
 }
+// TMA store of a shared-memory box (box row 0 = matrix row y), tracked by this thread's bulk groups.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void sts_128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
@@ -316,14 +325,16 @@ __device__ __forceinline__ void store_256(void* dst, uint32_t a, uint32_t b, uin
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
 }
 
-template <int EPI, int FMT>
+// Stores the chunk's bf16 outputs where STORE_OUT (the CTA-pair kernel stages them in shared memory instead) and applies the
+// quantized copy, the residual add and the running amax.
+template <int EPI, int FMT, bool STORE_OUT = true>
 __device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t (&packed)[16], int row, int col, uint32_t& amax2) {
   if (row >= p.m) return;
   if (p.q_codes && col + 32 <= p.n) store_chunk_quantized<FMT>(p, packed, row, col);
   if (!p.out) return;
-  uint16_t* orow = out_row_ptr(p, row) + col;
+  uint16_t* orow = STORE_OUT ? out_row_ptr(p, row) + col : nullptr;
   // 32-byte stores (whole L2 sectors, half as many store transactions per row) where the row's chunk is whole and 32-byte aligned
-  const bool wide = col + 32 <= p.n && (reinterpret_cast<uintptr_t>(orow) & 31u) == 0;
+  const bool wide = STORE_OUT && col + 32 <= p.n && (reinterpret_cast<uintptr_t>(orow) & 31u) == 0;
   if (wide) {
     store_256(orow, packed[0], packed[1], packed[2], packed[3], packed[4], packed[5], packed[6], packed[7]);
     store_256(orow + 16, packed[8], packed[9], packed[10], packed[11], packed[12], packed[13], packed[14], packed[15]);
@@ -331,7 +342,7 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t 
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     if (col + g * 8 + 8 <= p.n) {
-      if (!wide) *reinterpret_cast<uint4*>(orow + g * 8) = make_uint4(packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
+      if (STORE_OUT && !wide) *reinterpret_cast<uint4*>(orow + g * 8) = make_uint4(packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
       if (p.out_amax) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) amax2 = __vmaxu2(amax2, packed[4 * g + e] & 0x7FFF7FFFu);
@@ -354,23 +365,24 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t 
   }
 }
 
-// Which epilogue warps read chunk `c` (32 accumulator columns): GRP < 0: this warp reads all of them (the CTA-pair kernel has four
-// epilogue warps); GRP 0 / 1: the one-CTA kernel's two groups of four warps share the columns, alternating between the groups (with the
-// SiLU gate: by the gate chunk; its up chunk goes with it).
+// Which epilogue warps read chunk `c` (32 accumulator columns): the two groups of four warps (GRP 0 / 1) share the columns, alternating
+// between the groups (with the SiLU gate: by the gate chunk; its up chunk goes with it).
 template <int GRP, int EPI, int BLOCK_N>
 __device__ __forceinline__ constexpr bool chunk_is_mine(int c) {
   // the unit a group owns is a PAIR of adjacent chunks where there are at least four (a thread then writes 128 contiguous bytes of its
   // output row, a whole line), else single chunks
   constexpr int kUnits = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 64 : BLOCK_N / 32;
   const int u = (EPI == TF_EPI_SILU_GATE) ? (c % (BLOCK_N / 64)) : c;
-  return GRP < 0 || ((kUnits >= 4 ? (u >> 1) : u) & 1) == GRP;
+  return ((kUnits >= 4 ? (u >> 1) : u) & 1) == GRP;
 }
 
 // One tile's epilogue for accumulator BUF (compile time, so that the chunks held in registers are indexed statically).
 // t_acc: tensor-memory address of the accumulator for this warp's 32 lanes. Returns after the last store.
-template <int FMT, int BLOCK_N, int EPI, int BUF, int GRP, bool CLUSTER_BAR = false>
+// PAIR (the CTA-pair kernel): the release goes to the leader's barrier, and the bf16 outputs leave through `stage_smem`, this warp's
+// 4 KB staging box of 32 rows x 64 columns (128-byte swizzle), as one TMA store per pair of chunks.
+template <int FMT, int BLOCK_N, int EPI, int BUF, int GRP, bool PAIR = false>
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_acc, uint32_t bar_release, int lane, int row, int col0, float alpha,
-                                              uint32_t& amax2) {
+                                              uint32_t& amax2, const CUtensorMap* tma_out = nullptr, uint32_t stage_smem = 0) {
   using Cfg = TileCfg<FMT, BLOCK_N>;
   constexpr int kOutCols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;
   constexpr int kOv = Cfg::kOverlapChunks;
@@ -389,7 +401,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
   tc_fence_before();
   __syncwarp();
   if (lane == 0) {
-    if (CLUSTER_BAR) mbar_arrive_cluster(bar_release);
+    if (PAIR) mbar_arrive_cluster(bar_release);
     else mbar_arrive(bar_release);
   }
 
@@ -430,7 +442,27 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
       for (int j = 0; j < 16; ++j)
         packed[j] = pack_bf16x2(__fmul_rn(__uint_as_float(v[2 * j]), alpha), __fmul_rn(__uint_as_float(v[2 * j + 1]), alpha));
     }
-    store_chunk<EPI, FMT>(p, packed, row, col0 + c * 32, amax2);
+    if (!PAIR) {
+      store_chunk<EPI, FMT>(p, packed, row, col0 + c * 32, amax2);
+      continue;
+    }
+    store_chunk<EPI, FMT, false>(p, packed, row, col0 + c * 32, amax2);
+    if (!p.out) continue;
+    if ((c & 1) == 0) {  // the box is free once the previous store has read it
+      if (lane == 0) bulk_wait_read();
+      __syncwarp();
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+      sts_128(stage_smem + (uint32_t)lane * 128u + ((uint32_t)(((c & 1) * 4 + g) ^ (lane & 7)) << 4), packed[4 * g], packed[4 * g + 1], packed[4 * g + 2],
+              packed[4 * g + 3]);
+    if (c & 1) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      // a box that starts inside the matrix is clipped at its edges; one that starts outside is not stored
+      if (lane == 0 && row < p.m && col0 + (c - 1) * 32 < p.n) tma_store_2d(tma_out, stage_smem, col0 + (c - 1) * 32, row);
+      if (lane == 0) bulk_commit();
+    }
   }
 }
 
@@ -802,12 +834,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
 // ---- the 2-CTA kernel ------------------------------------------------------------------------------------------------------
 // Two CTAs of a cluster (a pair of SMs) compute one 256 x 256 tile with tcgen05.mma.cta_group::2: CTA r of the pair holds rows
 // [128 r, 128 r + 128) of the A tile and of the B tile in its own shared memory and the accumulator of its 128 rows in its own
-// tensor memory. Per 32 K MACs per K-byte each SM now fills 256 operand rows instead of 384, which is what the one-CTA kernel
-// is bound by. Each CTA loads its own halves with plain (non-multicast) TMA; the scale tiles of all 256 B rows are loaded by
-// both CTAs (4 KB per stage). The leader (rank 0) issues the scale copies and MMAs for both; barriers that both CTAs wait on
-// are signalled with tcgen05.commit's multicast arrive; the peer's producer and epilogue signal the leader through
-// cluster-mapped mbarrier addresses. Same bounded waits and teardown as the one-CTA kernel, plus a cluster barrier at both ends.
-template <int FMT, int EPI>
+// tensor memory. Per stage each SM fills 256 operand rows instead of the 384 that bound the one-CTA kernel (38 KB instead of 54
+// for nvfp4). Each CTA loads its own halves with plain (non-multicast) TMA; the scale tiles of all 256 B rows are loaded by
+// both CTAs (4 KB per stage). The warp roles are the one-CTA kernel's: operand loads (warp 0) and scale loads (warp 6), one
+// multi-lane instruction per stage each; the MMA issuer (warp 1, leader CTA only: it issues the scale copies and MMAs for both);
+// two groups of four epilogue warps. Barriers that both CTAs wait on are signalled with tcgen05.commit's multicast arrive; the
+// peer's load and epilogue warps signal the leader through cluster-mapped mbarrier addresses. The bf16 outputs are staged in
+// shared memory (a 4 KB box per epilogue warp) and leave as TMA stores: whole 128-byte lines instead of 32 partial lines per
+// warp instruction. Same bounded waits and teardown as the one-CTA kernel, plus a cluster barrier at both ends.
+template <int FMT>
 struct PairCfg {
   static constexpr int kST = FmtTraits<FMT>::kSfTiles;
   static constexpr int kBHalfBytes = 128 * kStageKBytes;
@@ -815,19 +850,22 @@ struct PairCfg {
   static constexpr int kSfbStageBytes = kST * 512 * 2;
   static constexpr int kStageBytes = kAStageBytes + kBHalfBytes + kSfaStageBytes + kSfbStageBytes;
   static constexpr int kBarrierBytes = 256;
-  static constexpr int kStagesRaw = (kSmemLimit - 1024 - kBarrierBytes) / kStageBytes;
+  static constexpr int kOutBoxBytes = 32 * 128;            // one epilogue warp's staging box
+  static constexpr int kOutStageBytes = 8 * kOutBoxBytes;
+  static constexpr int kStagesRaw = (kSmemLimit - 1024 - kBarrierBytes - kOutStageBytes) / kStageBytes;
   static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kOutStageBytes + kBarrierBytes + 1024;
 };
 
 template <int FMT, int EPI>
-__global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tma_a,
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                                  const __grid_constant__ CUtensorMap tma_b,
                                                                                  const __grid_constant__ CUtensorMap tma_sfa,
-                                                                                 const __grid_constant__ CUtensorMap tma_sfb, const GemmParams p) {
+                                                                                 const __grid_constant__ CUtensorMap tma_sfb,
+                                                                                 const __grid_constant__ CUtensorMap tma_out, const GemmParams p) {
   constexpr int BLOCK_N = 256;
   using Cfg = TileCfg<FMT, BLOCK_N>;  // tensor-memory layout (per CTA: 128 lanes x 256 columns) is the one-CTA kernel's
-  using PC = PairCfg<FMT, EPI>;
+  using PC = PairCfg<FMT>;
   constexpr int kStages = PC::kStages;
   constexpr int kST = PC::kST;
   constexpr int kNB = 2;
@@ -837,7 +875,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a = smem_base;
   const uint32_t smem_b = smem_a + kStages * kAStageBytes;
-  const uint32_t smem_sfa = smem_b + kStages * PC::kBHalfBytes;
+  const uint32_t smem_out = smem_b + kStages * PC::kBHalfBytes;  // 1024-byte aligned like the operand stages (the store's swizzle atom)
+  const uint32_t smem_sfa = smem_out + PC::kOutStageBytes;
   const uint32_t smem_sfb = smem_sfa + kStages * PC::kSfaStageBytes;
   const uint32_t bars = smem_sfb + kStages * PC::kSfbStageBytes;
   const uint32_t bar_full = bars, bar_empty = bars + 8 * kStages, bar_tmem_full = bars + 16 * kStages, bar_tmem_empty = bar_tmem_full + 8;
@@ -850,14 +889,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  griddep_launch_dependents();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(bar_full + 8 * s, 2);   // one arrive.expect_tx from each CTA's producer (used in the leader only)
+      mbar_init(bar_full + 8 * s, 4);   // one arrive.expect_tx from each load warp of each CTA (used in the leader only)
       mbar_init(bar_empty + 8 * s, 1);  // the leader's commit arrives in both CTAs
     }
     mbar_init(bar_tmem_full, 1);
-    mbar_init(bar_tmem_empty, 8);  // 4 epilogue warps of each CTA (used in the leader only)
+    mbar_init(bar_tmem_empty, 16);  // 8 epilogue warps of each CTA (used in the leader only)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -870,59 +910,48 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(
   cluster_sync_all();  // both CTAs' barriers are initialised before anything crosses
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  griddep_wait();
 
-  if (warp == 0) {
-    // ---------------- producer (each CTA loads its own halves; completion is counted on the leader's barrier) ----------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = pair; tile < p.num_tiles && ok; tile += num_pairs) {
-        const int m_blk = tile % p.m_blocks, n_blk = tile / p.m_blocks;
-        int b_row[kNB], b_rt[kNB];
-        bool b_ok[kNB];
-#pragma unroll
-        for (int nb = 0; nb < kNB; ++nb) {
-          b_row[nb] = (EPI == TF_EPI_SILU_GATE) ? nb * p.n + n_blk * 128 : n_blk * BLOCK_N + nb * 128;
-          b_rt[nb] = b_row[nb] >> 7;
-          b_ok[nb] = b_row[nb] < p.n_rows_b;
-        }
-        const int a_row = m_blk * 256 + (int)rank * 128;
-        const bool a_ok = a_row < p.m;
-        for (int ks = 0; ks < p.num_k_stages; ++ks) {
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, 1)) {
-            ok = false;
-            break;
-          }
-          // scale tiles come through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows
-          // past the end read as zero), because only the tensor form of the copy may signal the peer's barrier
-          constexpr uint32_t sf_bytes = (uint32_t)kST * 512u;
-          uint32_t tx = 0;
-          if (a_ok) tx += kAStageBytes + sf_bytes;
-          if (b_ok[rank]) tx += PC::kBHalfBytes;
-#pragma unroll
-          for (int nb = 0; nb < kNB; ++nb)
-            if (b_ok[nb]) tx += sf_bytes;
-          const uint32_t full = mapa_shared(bar_full + 8 * stage, 0);  // the leader's barrier
-          mbar_expect_tx_cluster(full, tx);
-          if (a_ok) {
-            tma_load_2d_pair(smem_a + stage * kAStageBytes, &tma_a, ks * kStageKBytes, a_row, full);
-            tma_load_2d_pair(smem_sfa + stage * PC::kSfaStageBytes, &tma_sfa, 0, (a_row >> 7) * p.sf_col_tiles + ks * kST, full);
-          }
-          if (b_ok[rank]) tma_load_2d_pair(smem_b + stage * PC::kBHalfBytes, &tma_b, ks * kStageKBytes, b_row[rank], full);
-#pragma unroll
-          for (int nb = 0; nb < kNB; ++nb)
-            if (b_ok[nb]) tma_load_2d_pair(smem_sfb + stage * PC::kSfbStageBytes + nb * kST * 512, &tma_sfb, 0, b_rt[nb] * p.sf_col_tiles + ks * kST, full);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1;
-          }
+  if (warp == 0 || warp == 6) {
+    // ---------------- load warps (each CTA loads its own halves; completion is counted on the leader's barrier) ----------------
+    // warp 0: lane 0 the A rows, lane 1 the B rows of this CTA. warp 6: lane 0 the A scales, lanes 1-2 the scales of the two B
+    // halves, through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows past the end read as
+    // zero), because only the tensor form of the copy may signal the peer's barrier.
+    const bool scales = warp == 6;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = pair; tile < p.num_tiles && ok; tile += num_pairs) {
+      const int m_blk = tile % p.m_blocks, n_blk = tile / p.m_blocks;
+      const int a_row = m_blk * 256 + (int)rank * 128;
+      const int half = scales ? (lane == 2 ? 1 : 0) : (int)rank;  // the B half a lane other than 0 serves
+      const int b_row = (EPI == TF_EPI_SILU_GATE) ? half * p.n + n_blk * 128 : n_blk * BLOCK_N + half * 128;
+      const int my_row = lane == 0 ? a_row : b_row;
+      const bool mine = lane == 0 ? a_row < p.m : (lane <= (scales ? 2 : 1) && b_row < p.n_rows_b);
+      const uint32_t copies = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine));
+      const CUtensorMap* my_map = scales ? (lane == 0 ? &tma_sfa : &tma_sfb) : (lane == 0 ? &tma_a : &tma_b);
+      const uint32_t my_dst = scales ? (lane == 0 ? smem_sfa : smem_sfb + (uint32_t)half * kST * 512) : (lane == 0 ? smem_a : smem_b);
+      const uint32_t my_stage_bytes = scales ? (lane == 0 ? PC::kSfaStageBytes : PC::kSfbStageBytes) : kAStageBytes;
+      const uint32_t tx = copies * (scales ? (uint32_t)kST * 512u : (uint32_t)kAStageBytes);
+      const int y_base = scales ? (my_row >> 7) * p.sf_col_tiles : my_row;
+      for (int ks = 0; ks < p.num_k_stages; ++ks) {
+        ok = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, 1);
+        ok = __all_sync(0xFFFFFFFFu, ok);
+        if (!ok) break;
+        const uint32_t full = mapa_shared(bar_full + 8 * stage, 0);  // the leader's barrier
+        if (lane == 0) mbar_expect_tx_cluster(full, tx);
+        __syncwarp();
+        if (mine) tma_load_2d_pair(my_dst + stage * my_stage_bytes, my_map, scales ? 0 : ks * kStageKBytes, scales ? y_base + ks * kST : y_base, full);
+        __syncwarp();
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1;
         }
       }
-      if (!ok) {
-        const unsigned long long t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-      }
+    }
+    if (!ok && lane == 0) {
+      const unsigned long long t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -957,24 +986,35 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(
           const uint32_t b_lo = (((smem_b + stage * PC::kBHalfBytes) & 0x3FFFFu) >> 4) | (1u << 16);
           const int sf_left = p.sf_col_tiles - ks * kST;
           const int k_left = p.k_bytes - ks * kStageKBytes;
-          const int sf_tiles = sf_left > kST ? kST : sf_left;
-          const int n_mma = k_left >= kStageKBytes ? 4 : (k_left + 31) >> 5;
+          const uint32_t first = ks > 0 ? 1u : 0u;
           if (elected) {
+            if (sf_left >= kST && k_left >= kStageKBytes) {
 #pragma unroll
-            for (int t = 0; t < kST; ++t) {
-              if (t < sf_tiles) {
+              for (int t = 0; t < kST; ++t) {
                 tc_cp_sf_pair(tmem_sfa + t * 4, make_desc(sfa_lo + t * 32, kDescHiSf));
 #pragma unroll
                 for (int nb = 0; nb < kNB; ++nb) tc_cp_sf_pair(tmem_sfb + (t * kNB + nb) * 4, make_desc(sfb_lo + (nb * kST + t) * 32, kDescHiSf));
               }
-            }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (j < n_mma) {
+              for (int j = 0; j < 4; ++j) {
                 const int t = (FMT == TF_FMT_MXFP8) ? 0 : (FMT == TF_FMT_MXFP4) ? (j >> 1) : j;
                 const uint32_t sf_id = (FMT == TF_FMT_MXFP8) ? (uint32_t)j : (FMT == TF_FMT_MXFP4) ? (uint32_t)((j & 1) * 2) : 0u;
                 tc_mma_pair<FMT>(tmem_acc, make_desc(a_lo + j * 2, kDescHiSw128), make_desc(b_lo + j * 2, kDescHiSw128),
-                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4, (j > 0 || ks > 0) ? 1u : 0u);
+                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4, j > 0 ? 1u : first);
+              }
+            } else {  // last, ragged stage: fewer scale tiles, fewer MMAs
+              const int sf_tiles = sf_left > kST ? kST : sf_left;
+              for (int t = 0; t < sf_tiles; ++t) {
+                tc_cp_sf_pair(tmem_sfa + t * 4, make_desc(sfa_lo + t * 32, kDescHiSf));
+#pragma unroll
+                for (int nb = 0; nb < kNB; ++nb) tc_cp_sf_pair(tmem_sfb + (t * kNB + nb) * 4, make_desc(sfb_lo + (nb * kST + t) * 32, kDescHiSf));
+              }
+              const int n_mma = k_left >= kStageKBytes ? 4 : (k_left + 31) >> 5;
+              for (int j = 0; j < n_mma; ++j) {
+                const int t = (FMT == TF_FMT_MXFP8) ? 0 : (FMT == TF_FMT_MXFP4) ? (j >> 1) : j;
+                const uint32_t sf_id = (FMT == TF_FMT_MXFP8) ? (uint32_t)j : (FMT == TF_FMT_MXFP4) ? (uint32_t)((j & 1) * 2) : 0u;
+                tc_mma_pair<FMT>(tmem_acc, make_desc(a_lo + j * 2, kDescHiSw128), make_desc(b_lo + j * 2, kDescHiSw128),
+                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4, j > 0 ? 1u : first);
               }
             }
             tc_commit_pair(bar_empty + 8 * stage);  // frees the stage in both CTAs
@@ -995,8 +1035,10 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(
   } else {
     // ---------------- epilogue: each CTA drains its own 128 rows; the release goes to the leader's barrier ----------------
     const int q = warp & 3;
+    const int grp = warp >= 7 ? 1 : 0;
     const float alpha = (FMT == TF_FMT_NVFP4) ? __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs)) : 1.0f;
     const uint32_t release = mapa_shared(bar_tmem_empty, 0);
+    const uint32_t stage_smem = smem_out + (uint32_t)(grp * 4 + q) * PC::kOutBoxBytes;
     uint32_t tile_phase = 0, acc_buf = 0;
     uint32_t amax2 = 0;
     for (int tile = pair; tile < p.num_tiles; tile += num_pairs) {
@@ -1009,13 +1051,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) gemm_blockscaled_pair_kernel(
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const int col0 = n_blk * kOutCols;
       const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(__ldg(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), __ldg(p.b_gs)) : alpha;
-      if (acc_buf == 0)
-        epilogue_tile<FMT, BLOCK_N, EPI, 0, -1, true>(p, t_row, release, lane, row, col0, alpha_t, amax2);
-      else
-        epilogue_tile<FMT, BLOCK_N, EPI, 1, -1, true>(p, t_row + Cfg::kAccStride, release, lane, row, col0, alpha_t, amax2);
+      if (acc_buf == 0) {
+        if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 0, 0, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+        else epilogue_tile<FMT, BLOCK_N, EPI, 0, 1, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+      } else {
+        if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 1, 0, true>(p, t_row + Cfg::kAccStride, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+        else epilogue_tile<FMT, BLOCK_N, EPI, 1, 1, true>(p, t_row + Cfg::kAccStride, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+      }
       acc_buf ^= 1;
       tile_phase ^= 1;
     }
+    if (lane == 0) bulk_wait_all();  // the stores have read their boxes and are written
+    __syncwarp();
     if (p.out_amax) {
       uint32_t mx = max(amax2 & 0xFFFFu, amax2 >> 16);
       for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
@@ -1149,10 +1196,28 @@ static tf_status make_scale_map(CUtensorMap* map, const void* base, int64_t tile
   return TF_OK;
 }
 
+// The bf16 output as [m, n] with leading dimension ldo: boxes of 32 rows x 64 columns (128 bytes), 128-byte swizzle.
+static tf_status make_output_map(CUtensorMap* map, const GemmParams& p) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(TF_ERR_CUDA, "tf_gemm_blockscaled: cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t dims[2] = {(cuuint64_t)p.n, (cuuint64_t)p.m};
+  const cuuint64_t strides[1] = {(cuuint64_t)p.ldo * 2u};
+  const cuuint32_t box[2] = {64u, 32u};
+  const cuuint32_t estr[2] = {1u, 1u};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(TF_ERR_CUDA, "tf_gemm_blockscaled: cuTensorMapEncodeTiled (output) failed with CUresult %d", (int)r);
+  return TF_OK;
+}
+
 template <int FMT, int EPI>
 static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
-  using PC = PairCfg<FMT, EPI>;
-  CUtensorMap tsa, tsb;
+  using PC = PairCfg<FMT>;
+  CUtensorMap tsa, tsb, to = {};
+  if (p.out) {
+    const tf_status so = make_output_map(&to, p);
+    if (so != TF_OK) return so;
+  }
   tf_status st = make_scale_map(&tsa, p.sfa, (int64_t)((p.m + 127) / 128) * p.sf_col_tiles, PC::kST);
   if (st != TF_OK) return st;
   st = make_scale_map(&tsb, p.sfb, (int64_t)p.sfb_row_tiles * p.sf_col_tiles, PC::kST);
@@ -1173,25 +1238,33 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   if (p.num_tiles < pairs) pairs = p.num_tiles;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(kPairThreads);
+  cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = PC::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tsa, tsb, p));
+  cfg.numAttrs = programmatic_launch_enabled() ? 2 : 1;
+  TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tsa, tsb, to, p));
   return TF_OK;
 }
 
-// Whether the 2-CTA kernel serves this problem: asked for (TF_GEMM_TWO_CTA=1 in the environment; the one-CTA kernel measured
-// faster on B200 under its power cap and is the default), more than one 128-row block, a full pair tile wide, no split-K.
-static bool use_pair_kernel(const GemmParams& p, const SplitPlan& sp) {
-  static const int enabled = getenv("TF_GEMM_TWO_CTA") ? atoi(getenv("TF_GEMM_TWO_CTA")) : 0;
-  return enabled && sp.splits == 1 && p.m > 128 && p.n_rows_b >= 256;
+// Whether the 2-CTA kernel serves this problem (TF_GEMM_TWO_CTA in the environment: 0 never, 1 wherever it can, unset this rule).
+// Per wave of tiles the pair is 5-13 % faster than the one-CTA kernel (measured on B200, one-CTA -> pair: nvfp4 4096 x 8192 x 28672
+// 385 -> 336 us, 4096 x 28672 x 8192 + gate 713 -> 666, 4096 x 6144 x 2560 35.1 -> 33.2; mxfp8 8192 x 6144 x 2560 106 -> 98.8;
+// mxfp4 300 x 8192 x 4096 12.8 -> 12.1), but its row blocks are 256 high: it is left where that costs a tenth more waves.
+static bool use_pair_kernel(const GemmParams& p, const SplitPlan& sp, int out_cols) {
+  static const int forced = getenv("TF_GEMM_TWO_CTA") ? atoi(getenv("TF_GEMM_TWO_CTA")) : -1;
+  if (forced == 0 || sp.splits != 1 || p.scatter_rows || p.m <= kBlockM || p.n_rows_b < 256) return false;
+  if (forced == 1) return true;
+  const int64_t sms = gemm_sms(), pairs = sms / 2, n_blocks = (p.n + out_cols - 1) / out_cols;
+  const int64_t waves = (p.m_blocks * n_blocks + sms - 1) / sms, pair_waves = ((p.m + 255) / 256 * n_blocks + pairs - 1) / pairs;
+  return 10 * pair_waves <= 11 * waves;
 }
 
 template <int FMT>
@@ -1234,7 +1307,7 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     TF_LAUNCH_CHECK();
     return TF_OK;
   }
-  if (use_pair_kernel(p, sp)) {
+  if (use_pair_kernel(p, sp, epilogue == TF_EPI_SILU_GATE ? 128 : 256)) {
     if (epilogue == TF_EPI_SILU_GATE) return launch_gemm_pair<FMT, TF_EPI_SILU_GATE>(ta, tb, p, stream);
     if (epilogue == TF_EPI_RESIDUAL) return launch_gemm_pair<FMT, TF_EPI_RESIDUAL>(ta, tb, p, stream);
     return launch_gemm_pair<FMT, TF_EPI_NONE>(ta, tb, p, stream);
