@@ -30,6 +30,10 @@ int sm_count();
     cudaError_t e__ = (call);                                                                               \
     if (e__ != cudaSuccess) return tf::fail(TF_ERR_CUDA, "%s: %s failed: %s", __func__, #call, cudaGetErrorString(e__)); \
   } while (0)
+// What a kernel that writes swizzled scales does about their padding: nothing (there is none, or the layout is plain) or zero it itself.
+// A scale pointer that is not 16-byte aligned gets the memset instead (*pad = 0).
+tf_status scale_padding(void* scales, int32_t format, int64_t rows, int64_t k, int32_t layout, cudaStream_t stream, int* pad);
+
 #define TF_LAUNCH_CHECK() TF_CUDA(cudaGetLastError())
 
 // Programmatic dependent launch (tf_set_programmatic_launch): a kernel launched through launch_dependent() may be scheduled

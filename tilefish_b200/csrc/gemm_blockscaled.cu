@@ -103,6 +103,7 @@ struct GemmParams {
   float* ws;
   uint8_t* q_codes;   // optional MX-quantized copy of the output (same format as the operands), swizzled scales
   uint8_t* q_scales;
+  int q_pad;      // the scales have padding that this launch zeroes (by the epilogue warps, while they wait for the first tile)
   int a_gs_rows;  // 0: a has one global scale; else a_gs[row / a_gs_rows] (row blocks quantized separately, e.g. gathered from ranks)
   int a_box_bytes;  // bytes one A load brings per stage: 128 bytes x the rows of its box (fewer than 128 rows when M is small)
   // Scattered output (tf_gemm_blockscaled_scatter): rows [i * scatter_rows, (i + 1) * scatter_rows) go to scatter_out[i], a
@@ -514,9 +515,11 @@ template <int EPI, int QFMT>  // QFMT: -1, or the MX format of a quantized copy 
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ ws, int splits, int m, int n, int n_acc, const float* a_gs,
                                                             const float* b_gs, uint16_t* __restrict__ out, int64_t ldo, float* __restrict__ residual,
                                                             unsigned int* __restrict__ out_amax, uint8_t* __restrict__ q_codes,
-                                                            uint8_t* __restrict__ q_scales, int a_gs_rows) {
+                                                            uint8_t* __restrict__ q_scales, int q_pad, int a_gs_rows) {
   griddep_launch_dependents();
   griddep_wait();
+  if (QFMT >= 0 && q_pad)
+    zero_scale_padding(q_scales, m, n >> 5, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
   const float alpha0 = (a_gs && b_gs) ? __fmul_rn(__ldg(a_gs), __ldg(b_gs)) : 1.0f;
   const int nvec = n >> 3;
   const int64_t total = (int64_t)m * nvec;
@@ -784,6 +787,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     const float alpha = (FMT == TF_FMT_NVFP4) ? __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs)) : 1.0f;
     uint32_t tile_phase = 0, acc_buf = 0;
     uint32_t amax2 = 0;  // running max of |out| as two packed bf16 magnitudes
+    if (FMT != TF_FMT_NVFP4 && p.q_codes && p.q_pad)
+      zero_scale_padding(p.q_scales, p.m, p.n >> 5, (int64_t)blockIdx.x * 256 + (grp * 4 + q) * 32 + lane, (int64_t)gridDim.x * 256);
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) {
       const int split = SPLITK ? tile / (p.m_blocks * p.n_blocks) : 0;
       const int rest = SPLITK ? tile % (p.m_blocks * p.n_blocks) : tile;
@@ -1041,6 +1046,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
     const uint32_t stage_smem = smem_out + (uint32_t)(grp * 4 + q) * PC::kOutBoxBytes;
     uint32_t tile_phase = 0, acc_buf = 0;
     uint32_t amax2 = 0;
+    if (FMT != TF_FMT_NVFP4 && p.q_codes && p.q_pad)
+      zero_scale_padding(p.q_scales, p.m, p.n >> 5, (int64_t)blockIdx.x * 256 + (grp * 4 + q) * 32 + lane, (int64_t)gridDim.x * 256);
     for (int tile = pair; tile < p.num_tiles; tile += num_pairs) {
       const int m_blk = tile % p.m_blocks, n_blk = tile / p.m_blocks;
       bool ok = mbar_wait(bar_tmem_full, tile_phase, abort_flag, 4);
@@ -1285,12 +1292,13 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     p.q_codes = qc;
     const int64_t total = (int64_t)p.m * (n_out >> 3);
     const int64_t need = (total + 255) / 256, cap = (int64_t)sm_count() * 8;
-    const unsigned grid = (unsigned)(need < cap ? need : cap);
+    unsigned grid = (unsigned)(need < cap ? need : cap);
+    if (qc && p.q_pad && grid < kPadBlocks) grid = kPadBlocks;
     const float* ags = FMT == TF_FMT_NVFP4 ? p.a_gs : nullptr;
     const float* bgs = FMT == TF_FMT_NVFP4 ? p.b_gs : nullptr;
 #define TF_REDUCE(EPI_, Q_) \
   launch_dependent(splitk_reduce_kernel<EPI_, Q_>, dim3(grid), dim3(256), 0, stream, (const float*)p.ws, (int)sp.splits, (int)p.m, (int)n_out, (int)p.n_rows_b, ags, bgs, \
-                   p.out, p.ldo, residual, amax, p.q_codes, p.q_scales, (int)p.a_gs_rows)
+                   p.out, p.ldo, residual, amax, p.q_codes, p.q_scales, (int)p.q_pad, (int)p.a_gs_rows)
     const int qf = p.q_codes ? FMT : -1;
     if (epilogue == TF_EPI_SILU_GATE) {
       if (qf == TF_FMT_MXFP8) TF_REDUCE(TF_EPI_SILU_GATE, TF_FMT_MXFP8);
@@ -1447,8 +1455,6 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
     if (epilogue == TF_EPI_RESIDUAL) return fail(TF_ERR_UNSUPPORTED, "%s: the residual epilogue has no quantized output", fn);
     if (n % 32 != 0) return fail(TF_ERR_UNSUPPORTED, "%s: a quantized output needs n %% 32 == 0", fn);
     TF_CHECK_ALIGNED(q_codes, 16, "q_codes");
-    const int64_t cols = n / 32;
-    if ((m & 127) || (cols & 3)) TF_CUDA(cudaMemsetAsync(q_scales, 0, (size_t)tf_scale_bytes(format, m, n, TF_SCALES_SWIZZLED), stream));
   }
   TF_CHECK_ARG(epilogue != TF_EPI_RESIDUAL || out, "%s: the residual epilogue needs out", fn);
   TF_CHECK_ARG(a_global_scale_rows >= 0 && a_global_scale_rows % 128 == 0, "%s: a_global_scale_rows must be 0 or a multiple of 128", fn);
@@ -1499,6 +1505,7 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
   p.out_amax = reinterpret_cast<unsigned int*>(out_amax);
   p.q_codes = static_cast<uint8_t*>(q_codes);
   p.q_scales = static_cast<uint8_t*>(q_scales);
+  p.q_pad = 0;
   p.a_gs_rows = (int)a_global_scale_rows;
   p.a_box_bytes = a_box_rows * kStageKBytes;
   p.scatter_rows = 0;
@@ -1523,6 +1530,10 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
       return fail(TF_ERR_WORKSPACE, "%s: this problem is split %d ways along K and needs a %lld-byte workspace (tf_gemm_workspace_bytes)", fn,
                   sp.splits, (long long)need);
     TF_CHECK_ALIGNED(workspace, 256, "workspace");
+  }
+  if (q_codes) {  // after every refusal: the unaligned case enqueues a memset
+    st = scale_padding(q_scales, format, m, n, TF_SCALES_SWIZZLED, stream, &p.q_pad);
+    if (st != TF_OK) return st;
   }
   switch (format) {
     case TF_FMT_MXFP8: return dispatch_gemm<TF_FMT_MXFP8>(ta, tb, p, epilogue, sp, stream, partial_splits != nullptr);

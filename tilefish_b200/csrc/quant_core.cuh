@@ -143,6 +143,35 @@ __device__ __forceinline__ void store_quantized16(uint8_t* __restrict__ codes_ou
   }
 }
 
+// Zeroes the padding of a swizzled scale tensor: the rows past `rows` of the last row tile and the columns past `cols` of the last
+// column tile. Thread `first` of `stride` threads that share the work. The bytes are disjoint from the scales, so no ordering is
+// needed; a kernel that writes scales does this itself instead of a memset of the whole tensor in front of it (measured in captured
+// graphs: the README block at one row 26.1 -> 25.0 us, its NVFP4 form at 16 rows 28.7 -> 26.7). One item of the
+// row padding is 16 contiguous bytes (the four row groups of one tile row), so a tensor of one row and 2560 columns takes two stores
+// per thread of a single block. `scales` is 16-byte aligned.
+constexpr unsigned kPadBlocks = 8;  // a launch that pads has at least this many blocks to share the work
+__device__ __forceinline__ void zero_scale_padding(uint8_t* __restrict__ scales, int64_t rows, int64_t cols, int64_t first, int64_t stride) {
+  const int64_t n_ct = (cols + 3) >> 2;
+  const int used = (int)(rows & 127);  // rows of the last row tile that hold scales; 0: all of them
+  if (used) {
+    uint8_t* tiles = scales + (rows >> 7) * n_ct * 512;
+    for (int64_t i = first; i < n_ct * 32; i += stride) {
+      const int rr = (int)(i & 31);
+      uint32_t* p = reinterpret_cast<uint32_t*>(tiles + i * 16);
+      if (rr >= used) {
+        *reinterpret_cast<uint4*>(p) = make_uint4(0, 0, 0, 0);
+      } else {
+        for (int g = 1; g < 4; ++g)
+          if (g * 32 + rr >= used) p[g] = 0u;
+      }
+    }
+  }
+  if (cols & 3) {
+    for (int64_t r = first; r < rows; r += stride)
+      for (int64_t c = cols; c < n_ct * 4; ++c) scales[swizzled_scale_offset(r, c, n_ct)] = 0;
+  }
+}
+
 // Stores one thread's codes (8 elements starting at element column `col` of row `row`) and, from the first lane of each
 // block, the scale byte. `vec` is the index of the 8-element vector inside the row.
 template <int FMT>

@@ -23,11 +23,15 @@ __device__ __forceinline__ void load_256(const void* p, uint32_t (&w)[8]) {
 template <int FMT>
 __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint8_t* __restrict__ x, int64_t m, int64_t k, int64_t ldx,
                                                                       uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
-                                                                      int swizzled, const float* __restrict__ gs_ptr, float* __restrict__ gs_out) {
+                                                                      int swizzled, int pad, const float* __restrict__ gs_ptr, float* __restrict__ gs_out) {
   const int tpr = blockDim.x;
   const int nvec = (int)(k >> 4);
   griddep_launch_dependents();
   griddep_wait();
+  if (pad)
+    zero_scale_padding(scales, m, k / (FMT == TF_FMT_NVFP4 ? 16 : 32),
+                       ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuantThreads + threadIdx.y * tpr + threadIdx.x,
+                       (int64_t)gridDim.x * gridDim.y * kQuantThreads);
   float gs = (FMT == TF_FMT_NVFP4) ? __ldg(gs_ptr) : 0.0f;
   if (FMT == TF_FMT_NVFP4 && gs_out != nullptr) {
     gs = __fdiv_rn(gs, 2688.0f);
@@ -95,7 +99,7 @@ __device__ __forceinline__ void lds_256(uint32_t addr, uint32_t (&w)[8]) {
 // Dynamic shared memory: `stages` chunk buffers of 4 KB, then one mbarrier per stage.
 template <int MODE>
 __global__ void __launch_bounds__(kRingThreads) ring_rows_kernel(const uint8_t* __restrict__ x, int64_t m, int64_t k, int64_t ldx,
-                                                                 uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int swizzled,
+                                                                 uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int swizzled, int pad,
                                                                  const float* __restrict__ gs_ptr, float* __restrict__ gs_out,
                                                                  unsigned int* __restrict__ amax_bits_out, int* __restrict__ status, int stages) {
   extern __shared__ __align__(128) uint8_t ring_smem[];
@@ -126,6 +130,9 @@ __global__ void __launch_bounds__(kRingThreads) ring_rows_kernel(const uint8_t* 
     }
     inv_t = gs != 0.0f ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
   }
+
+  if (MODE != kModeAmax && pad)
+    zero_scale_padding(scales, m, k / (MODE == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * kRingThreads + t, (int64_t)gridDim.x * kRingThreads);
 
   // thread 0: one bulk copy per chunk; a chunk is vectors [c * 128, min(nvec, c * 128 + 128)) of its row
   auto issue = [&](int64_t chunk, int stage) {
@@ -295,6 +302,15 @@ __global__ void __launch_bounds__(256) swizzle_kernel(const uint8_t* __restrict_
 
 static int block_of(int format) { return format == TF_FMT_NVFP4 ? 16 : 32; }
 
+tf_status scale_padding(void* scales, int32_t format, int64_t rows, int64_t k, int32_t layout, cudaStream_t stream, int* pad) {
+  *pad = layout == TF_SCALES_SWIZZLED && ((rows & 127) || ((k / block_of(format)) & 3));
+  if (*pad && reinterpret_cast<uintptr_t>(scales) % 16) {
+    *pad = 0;
+    TF_CUDA(cudaMemsetAsync(scales, 0, (size_t)tf_scale_bytes(format, rows, k, layout), stream));
+  }
+  return TF_OK;
+}
+
 static tf_status check_quant_args(const char* fn, const void* x, int64_t m, int64_t k, int64_t ldx, const void* codes, const void* scales,
                                   int layout) {
   if (!x || !codes || !scales) return fail(TF_ERR_INVALID_ARGUMENT, "%s: null pointer", fn);
@@ -315,16 +331,16 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   if (st != TF_OK) return st;
   if (FMT == TF_FMT_NVFP4 && !gs) return fail(TF_ERR_INVALID_ARGUMENT, "%s: nvfp4 needs a global scale", fn);
   if (m == 0) return TF_OK;
-  const int64_t cols = k / block_of(FMT);
-  if (layout == TF_SCALES_SWIZZLED && ((m & 127) || (cols & 3)))
-    TF_CUDA(cudaMemsetAsync(scales, 0, (size_t)tf_scale_bytes(FMT, m, k, layout), stream));
+  int pad = 0;
+  st = scale_padding(scales, FMT, m, k, layout, stream, &pad);
+  if (st != TF_OK) return st;
   if (use_ring(FMT, m, k)) {
     int* status = device_status_words();
     if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
     TF_CUDA(ring_configure<FMT>());
     const RingLaunch rl = ring_launch(FMT, m, k);
     TF_CUDA(launch_dependent(ring_rows_kernel<FMT>, dim3(rl.grid), dim3(kRingThreads), rl.smem, stream, static_cast<const uint8_t*>(x), m, k, ldx,
-                             static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), gs, gs_out,
+                             static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out,
                              (unsigned int*)nullptr, status, rl.stages));
     return TF_OK;
   }
@@ -340,8 +356,9 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
     const int64_t want = (2 * sm_count() + blocks_needed - 1) / blocks_needed;
     grid.y = (unsigned)(want < rounds ? want : rounds);
   }
+  if (pad && grid.x * grid.y < kPadBlocks) grid.x = kPadBlocks;
   TF_CUDA(launch_dependent(quantize_rows_kernel<FMT>, grid, block, 0, stream, static_cast<const uint8_t*>(x), m, k, ldx, static_cast<uint8_t*>(codes),
-                           static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), gs, gs_out));
+                           static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out));
   return TF_OK;
 }
 
@@ -401,7 +418,7 @@ tf_status tf_nvfp4_global_scale(const void* x, int64_t m, int64_t k, int64_t ldx
       if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", __func__);
       TF_CUDA(ring_configure<kModeAmax>());
       const RingLaunch rl = ring_launch(kModeAmax, m, k);
-      ring_rows_kernel<kModeAmax><<<rl.grid, kRingThreads, rl.smem, stream>>>(static_cast<const uint8_t*>(x), m, k, ldx, nullptr, nullptr, 0, nullptr, nullptr,
+      ring_rows_kernel<kModeAmax><<<rl.grid, kRingThreads, rl.smem, stream>>>(static_cast<const uint8_t*>(x), m, k, ldx, nullptr, nullptr, 0, 0, nullptr, nullptr,
                                                                               reinterpret_cast<unsigned int*>(out), status, rl.stages);
       TF_LAUNCH_CHECK();
       finalize_global_scale_kernel<<<1, 1, 0, stream>>>(out);

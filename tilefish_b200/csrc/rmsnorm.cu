@@ -15,7 +15,7 @@ template <int VPT, int QFMT>  // VPT: 8-element vectors per thread; QFMT: -1 non
 __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* __restrict__ x, float4* __restrict__ residual,
                                                                    const uint4* __restrict__ w, uint4* __restrict__ out, int64_t m, int d,
                                                                    float eps, float inv_d, uint8_t* __restrict__ q_codes,
-                                                                   uint8_t* __restrict__ q_scales, int q_swizzled,
+                                                                   uint8_t* __restrict__ q_scales, int q_swizzled, int q_pad,
                                                                    const float* __restrict__ q_gs_ptr, unsigned int* __restrict__ out_amax) {
   __shared__ float warp_sums[16];
   __shared__ unsigned int warp_amax[16];
@@ -27,6 +27,8 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
   griddep_wait();
   const float gs = (QFMT == TF_FMT_NVFP4) ? __ldg(q_gs_ptr) : 0.0f;
   const float inv_t = (QFMT == TF_FMT_NVFP4 && gs != 0.0f) ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
+  if (QFMT >= 0 && q_pad)
+    zero_scale_padding(q_scales, m, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * nthreads + tid, (int64_t)gridDim.x * nthreads);
 
   for (int64_t row = blockIdx.x; row < m; row += gridDim.x) {
     const uint4* xr = x + row * nvec;
@@ -105,12 +107,12 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
 
 template <int VPT>
 static void launch_vpt(int qfmt, dim3 grid, dim3 block, cudaStream_t s, const uint4* x, float4* res, const uint4* w, uint4* out, int64_t m, int d,
-                       float eps, float inv_d, uint8_t* qc, uint8_t* qs, int qsw, const float* qgs, unsigned int* amax) {
+                       float eps, float inv_d, uint8_t* qc, uint8_t* qs, int qsw, int qpad, const float* qgs, unsigned int* amax) {
   switch (qfmt) {
-    case TF_FMT_MXFP8: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qgs, amax); break;
-    case TF_FMT_MXFP4: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qgs, amax); break;
-    case TF_FMT_NVFP4: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qgs, amax); break;
-    default: launch_dependent(residual_add_rmsnorm_kernel<VPT, -1>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qgs, amax); break;
+    case TF_FMT_MXFP8: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    case TF_FMT_MXFP4: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    case TF_FMT_NVFP4: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    default: launch_dependent(residual_add_rmsnorm_kernel<VPT, -1>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
   }
 }
 
@@ -289,15 +291,17 @@ extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, cons
   TF_CHECK_ALIGNED(residual, 16, "residual");
   TF_CHECK_ALIGNED(w, 16, "w");
   if (out) TF_CHECK_ALIGNED(out, 16, "out");
+  int pad = 0;  // the kernel zeroes the padding of the scales
   if (q_format >= 0) {
     TF_CHECK_ARG(q_codes && q_scales, "%s: q_codes/q_scales missing", __func__);
     TF_CHECK_ARG(q_layout == TF_SCALES_PLAIN || q_layout == TF_SCALES_SWIZZLED, "%s: unknown scale layout %d", __func__, q_layout);
     TF_CHECK_ARG(q_format != TF_FMT_NVFP4 || q_global_scale, "%s: nvfp4 needs a global scale", __func__);
     if (d % 32 != 0) return fail(TF_ERR_UNSUPPORTED, "%s: quantized output needs d %% 32 == 0", __func__);
     TF_CHECK_ALIGNED(q_codes, 16, "q_codes");
-    const int64_t cols = d / (q_format == TF_FMT_NVFP4 ? 16 : 32);
-    if (q_layout == TF_SCALES_SWIZZLED && m > 0 && ((m & 127) || (cols & 3)))
-      TF_CUDA(cudaMemsetAsync(q_scales, 0, (size_t)tf_scale_bytes(q_format, m, d, q_layout), stream));
+    if (m > 0) {
+      const tf_status st = scale_padding(q_scales, q_format, m, d, q_layout, stream, &pad);
+      if (st != TF_OK) return st;
+    }
   }
   if (m == 0) return TF_OK;
 
@@ -308,6 +312,7 @@ extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, cons
   threads = (threads + 31) / 32 * 32;
   const int64_t cap = (int64_t)sm_count() * (2048 / threads);
   dim3 grid((unsigned)(m < cap ? m : cap)), block(threads);
+  if (pad && grid.x < kPadBlocks) grid.x = kPadBlocks;  // one to seven rows: blocks without a row share the padding (0.6 us at one row)
   const float inv_d = 1.0f / (float)d;  // correctly rounded f32 reciprocal of D (IEEE division on the host)
   const uint4* xp = static_cast<const uint4*>(x);
   float4* rp = static_cast<float4*>(residual);
@@ -317,10 +322,10 @@ extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, cons
   uint8_t* qs = static_cast<uint8_t*>(q_scales);
   const int qsw = q_layout == TF_SCALES_SWIZZLED;
   switch (vpt) {
-    case 1: launch_vpt<1>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
-    case 2: launch_vpt<2>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
-    case 4: launch_vpt<4>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
-    default: launch_vpt<8>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    case 1: launch_vpt<1>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    case 2: launch_vpt<2>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    case 4: launch_vpt<4>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    default: launch_vpt<8>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
   }
   TF_LAUNCH_CHECK();
   return TF_OK;
