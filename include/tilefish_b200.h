@@ -203,7 +203,9 @@ TF_API tf_status tf_gemm_blockscaled_static(const void* a_codes, const void* a_s
 /* The first pass of a split-K problem only (epilogue TF_EPI_NONE): the f32 partial sums stay in the workspace as `*splits` planes
  * [splits][m][n] for a consumer that sums them itself (tf_rmsnorm_quantize_rows: the few-rows step between two blocks, where a separate
  * reduction launch costs as much as the arithmetic). No counterpart in the reference. Shapes that are not split along K
- * (tf_gemm_splits == 1) are refused with TF_ERR_UNSUPPORTED. Other arguments as tf_gemm_blockscaled (one global scale for `a`). */
+ * (tf_gemm_splits == 1) are refused with TF_ERR_UNSUPPORTED. Other arguments as tf_gemm_blockscaled (one global scale for `a`).
+ * tf_gemm_splits is the number of planes this call leaves. tf_gemm_blockscaled sums the same K ranges where there are planes; where
+ * there are none it may still cut K over a cluster of CTAs, which needs no workspace. */
 TF_API int32_t tf_gemm_splits(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue);
 TF_API tf_status tf_gemm_blockscaled_partials(const void* a_codes, const void* a_scales, const float* a_global_scale, const void* b_codes,
                                               const void* b_scales, const float* b_global_scale, int64_t m, int64_t n, int64_t k, int32_t format,

@@ -1,0 +1,59 @@
+"""The forms one GEMM call can be launched in (128-column tiles, K ranges over a cluster of CTAs, the CTA pair) at the edges of their tiles.
+
+Bound against the oracle: both sides round one f32 sum to bf16 and differ by the order of the sum, 2**-8 of the largest result (the
+GEMM tests' own bound). Residual, amax and the quantized copy follow from the bf16 result exactly."""
+
+import pytest
+import torch
+
+from oracle import blockscaled as O
+
+pytestmark = pytest.mark.gpu
+TOL = 2.0**-8 * 1.01
+
+
+@pytest.fixture(scope="module")
+def K():
+    from tilefish_b200 import kernels
+
+    kernels.require_cuda()
+    return kernels
+
+
+SHAPES = [(1, 2560, 3072), (33, 264, 4096), (128, 136, 2080), (129, 1000, 1024), (300, 1024, 4128), (257, 392, 8192), (700, 520, 2048), (1024, 1024, 512),
+          (200, 2048, 1024), (513, 4104, 288), (1100, 3104, 544)]
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_every_form_meets_the_oracle(K, fmt, m, n, k):
+    a, w = O.randn((m, k), m, torch.bfloat16), O.randn((n, k), n, torch.bfloat16, scale=k**-0.5)
+    qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)
+    amax, res = torch.zeros(1, device="cuda"), O.randn((m, n), 7)
+    wide = torch.full((m, n + 16), -7.0, dtype=torch.bfloat16, device="cuda")
+    out = K.gemm_blockscaled(qa, qb, out=wide[:, :n], amax_out=amax)
+    oa, ob = O.quantize(a, fmt), O.quantize(w, fmt)
+    ref = O.dequantize(oa[0], oa[1], fmt, oa[2]) @ O.dequantize(ob[0], ob[1], fmt, ob[2]).t()
+    assert float((out.cpu().float() - ref).abs().max()) <= TOL * float(ref.abs().max())
+    assert bool((wide[:, n:] == -7.0).all()) and float(amax) == float(out.float().abs().max())
+    r = res.cuda()
+    again = K.gemm_blockscaled(qa, qb, epilogue="residual", residual=r)
+    assert torch.equal(again, K.gemm_blockscaled(qa, qb, epilogue="residual", residual=res.cuda())), "deterministic"
+    assert torch.equal(r.cpu(), res + again.cpu().float())
+    if fmt != "nvfp4" and n % 32 == 0:
+        o, q = K.gemm_blockscaled(qa, qb, quantize_out=True)
+        ref_q = K.quantize(o, fmt)
+        assert torch.equal(q.codes, ref_q.codes) and torch.equal(q.scales, ref_q.scales)
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "nvfp4"])
+@pytest.mark.parametrize("m,f,k", [(300, 128, 8192), (1317, 768, 4096), (257, 256, 2080), (1000, 640, 1024)])
+def test_gate_over_a_cluster_and_a_pair(K, fmt, m, f, k):
+    a, w = O.randn((m, k), m, torch.bfloat16), O.randn((2 * f, k), f, torch.bfloat16, scale=k**-0.5)
+    qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)
+    out = K.gemm_blockscaled(qa, qb, epilogue="silu_gate")
+    t = K.gemm_blockscaled(qa, qb).float()
+    ref = K.silu_gate(t.to(torch.bfloat16)).float()
+    # the gate reads two bf16 results that may differ by one rounding (2**-8 of the largest): |silu'| < 1.1, times the other factor
+    bound = 2 * TOL * float(t.abs().max()) * (float(t.abs().max()) + 1.0)
+    assert float((out.float() - ref).abs().max()) <= bound

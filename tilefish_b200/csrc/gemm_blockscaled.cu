@@ -140,6 +140,11 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -583,8 +588,125 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
   }
 }
 
+// ---- split-K inside a cluster -----------------------------------------------------------------------------------------------
+// The CTAs of a cluster hold one K range each of the same output tile. Every CTA leaves its f32 accumulator rows in its own shared
+// memory (the operand ring is free by then), the cluster meets, and each CTA sums its share of the tile over the ranges, read
+// from its peers' shared memory, in split order: the arithmetic, and so the bytes, of epilogue_partial + splitk_reduce_kernel
+// without the second launch and without the trip of the partial sums through the workspace.
+template <int BLOCK_N>
+struct DumpCfg {
+  static constexpr int kPitch = (BLOCK_N + 4) * 4;  // bytes per row; the 16 bytes of padding spread a warp's rows over the banks
+  static constexpr int kBytes = kBlockM * kPitch;
+};
+
+template <int FMT, int BLOCK_N, int GRP>
+__device__ __forceinline__ void epilogue_dump(uint32_t t_acc, uint32_t smem_row) {
+#pragma unroll
+  for (int c = 0; c < BLOCK_N / 32; ++c) {
+    if (!chunk_is_mine<GRP, TF_EPI_NONE, BLOCK_N>(c)) continue;
+    uint32_t v[32];
+    tc_ld32(t_acc + c * 32, v);
+    tc_wait_ld();
+#pragma unroll
+    for (int g = 0; g < 8; ++g) sts_128(smem_row + c * 128 + g * 16, v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+  }
+}
+
+// All threads of the CTA; `dump` is the shared address of the dumped rows (the same in every CTA of the cluster).
+template <int FMT, int BLOCK_N, int EPI>
+__device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dump, int rank, int m_blk, int n_blk) {
+  constexpr int kOutCols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;
+  constexpr int kVecs = kOutCols / 8;
+  const int rows = min(kBlockM, p.m - m_blk * kBlockM);
+  const int total = rows * kVecs;
+  const bool quantize = FMT != TF_FMT_NVFP4 && p.q_codes != nullptr;
+  uint32_t amax2 = 0;
+  // whole warps run every round (the quantizer's shuffles); the 4 lanes of one MX block always have data together
+  for (int i0 = rank * kGemmThreads; i0 < total; i0 += p.splits * kGemmThreads) {
+    const int i = i0 + (int)threadIdx.x;
+    const int r = i / kVecs, cv = i - r * kVecs;
+    const int row = m_blk * kBlockM + r, col = n_blk * kOutCols + cv * 8;
+    const bool live = i < total && col < p.n;
+    float acc[8], up[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = up[j] = 0.0f;
+    const uint32_t local = dump + (uint32_t)(live ? r : 0) * DumpCfg<BLOCK_N>::kPitch + (uint32_t)(live ? cv : 0) * 32u;
+    // four ranges' loads in flight (a remote read takes about 0.4 us); the second four lanes of every eight take their two halves in
+    // the other order, so that the eight lanes a read serves together touch different banks
+    const uint32_t swap = (threadIdx.x >> 2) & 1u;
+    for (int sp = 0; sp < p.splits; sp += 4) {
+      float4 x[4][2], u[4][2];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (sp + j < p.splits) {
+          const uint32_t src = mapa_shared(local, (uint32_t)(sp + j));
+          x[j][0] = ld_cluster_f4(src + 16 * swap);
+          x[j][1] = ld_cluster_f4(src + 16 - 16 * swap);
+          if (EPI == TF_EPI_SILU_GATE) {
+            u[j][0] = ld_cluster_f4(src + BLOCK_N * 2 + 16 * swap);
+            u[j][1] = ld_cluster_f4(src + BLOCK_N * 2 + 16 - 16 * swap);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (sp + j < p.splits) {
+          const float4 x0 = swap ? x[j][1] : x[j][0], x1 = swap ? x[j][0] : x[j][1];
+          acc[0] += x0.x; acc[1] += x0.y; acc[2] += x0.z; acc[3] += x0.w; acc[4] += x1.x; acc[5] += x1.y; acc[6] += x1.z; acc[7] += x1.w;
+          if (EPI == TF_EPI_SILU_GATE) {
+            const float4 u0 = swap ? u[j][1] : u[j][0], u1 = swap ? u[j][0] : u[j][1];
+            up[0] += u0.x; up[1] += u0.y; up[2] += u0.z; up[3] += u0.w; up[4] += u1.x; up[5] += u1.y; up[6] += u1.z; up[7] += u1.w;
+          }
+        }
+      }
+    }
+    float alpha = 1.0f;
+    if (FMT == TF_FMT_NVFP4 && live) alpha = __fmul_rn(__ldg(p.a_gs + (p.a_gs_rows > 0 ? row / p.a_gs_rows : 0)), __ldg(p.b_gs));
+    uint32_t packed[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t g2 = pack_bf16x2(__fmul_rn(acc[2 * j], alpha), __fmul_rn(acc[2 * j + 1], alpha));
+      if (EPI == TF_EPI_SILU_GATE) {
+        const uint32_t u2 = pack_bf16x2(__fmul_rn(up[2 * j], alpha), __fmul_rn(up[2 * j + 1], alpha));
+        packed[j] = pack_bf16x2(__fmul_rn(silu_f32(bf16lo_to_f32(g2)), bf16lo_to_f32(u2)), __fmul_rn(silu_f32(bf16hi_to_f32(g2)), bf16hi_to_f32(u2)));
+      } else {
+        packed[j] = g2;
+      }
+    }
+    if (quantize) {
+      uint32_t c0, c1, sc;
+      constexpr int kQ = FMT == TF_FMT_NVFP4 ? TF_FMT_MXFP8 : FMT;
+      quantize_vec8<kQ>(make_uint4(packed[0], packed[1], packed[2], packed[3]), 0.0f, 0.0f, c0, c1, sc);
+      if (live) store_quantized<kQ>(p.q_codes, p.q_scales, 1, row, col >> 3, p.n, c0, c1, sc);
+    }
+    if (!live) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) amax2 = __vmaxu2(amax2, packed[j] & 0x7FFF7FFFu);
+    if (p.out) *reinterpret_cast<uint4*>(out_row_ptr(p, row) + col) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    if (EPI == TF_EPI_RESIDUAL) {
+      float4* rp = reinterpret_cast<float4*>(p.residual + (int64_t)row * p.n + col);
+      float4 r0 = rp[0], r1 = rp[1];
+      r0.x = __fadd_rn(r0.x, bf16lo_to_f32(packed[0])); r0.y = __fadd_rn(r0.y, bf16hi_to_f32(packed[0]));
+      r0.z = __fadd_rn(r0.z, bf16lo_to_f32(packed[1])); r0.w = __fadd_rn(r0.w, bf16hi_to_f32(packed[1]));
+      r1.x = __fadd_rn(r1.x, bf16lo_to_f32(packed[2])); r1.y = __fadd_rn(r1.y, bf16hi_to_f32(packed[2]));
+      r1.z = __fadd_rn(r1.z, bf16lo_to_f32(packed[3])); r1.w = __fadd_rn(r1.w, bf16hi_to_f32(packed[3]));
+      rp[0] = r0;
+      rp[1] = r1;
+    }
+  }
+  if (p.out_amax) {
+    uint32_t mx = max(amax2 & 0xFFFFu, amax2 >> 16);
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    if ((threadIdx.x & 31) == 0 && mx) atomicMax(p.out_amax, mx << 16);
+  }
+}
+
 // ---- the kernel ------------------------------------------------------------------------------------------------------------
-template <int FMT, int BLOCK_N, int EPI, bool SPLITK>
+// SPLITK: kSplitNone; kSplitPlanes: every (tile, K range) is a unit of its own and leaves its accumulator in the workspace;
+// kSplitCluster: a cluster of `splits` CTAs per tile, launched with exactly one tile per cluster.
+constexpr int kSplitNone = 0, kSplitPlanes = 1, kSplitCluster = 2;
+constexpr int kMaxClusterSplits = 8;  // the portable cluster size
+template <int FMT, int BLOCK_N, int EPI, int SPLITK>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                             const __grid_constant__ CUtensorMap tma_b, const GemmParams p) {
   using Cfg = TileCfg<FMT, BLOCK_N>;
@@ -592,6 +714,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
   constexpr int kNB = Cfg::kNB;
   constexpr int kST = Cfg::kST;
   constexpr int kOutCols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;  // output columns per tile
+  constexpr bool kCluster = SPLITK == kSplitCluster;
+  static_assert(!kCluster || DumpCfg<BLOCK_N>::kBytes <= kStages * Cfg::kStageBytes, "the dumped accumulator must fit in the operand ring");
   static_assert(EPI != TF_EPI_SILU_GATE || BLOCK_N == 256, "the SiLU-gate epilogue pairs a 128-column gate tile with its up tile");
 
   extern __shared__ uint8_t smem_raw[];
@@ -641,8 +765,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
-      const int split = SPLITK ? tile / (p.m_blocks * p.n_blocks) : 0;
-      const int rest = SPLITK ? tile % (p.m_blocks * p.n_blocks) : tile;
+      const int split = SPLITK == kSplitPlanes ? tile / (p.m_blocks * p.n_blocks) : kCluster ? tile % p.splits : 0;
+      const int rest = SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile;
       const int m_blk = rest % p.m_blocks, n_blk = rest / p.m_blocks;
       const int ks_begin = split * p.k_stages_per_split;
       const int ks_end = min(ks_begin + p.k_stages_per_split, p.num_k_stages);
@@ -708,8 +832,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
       tc_fence_after();
       const uint32_t tmem_acc = tmem_base + acc_buf * Cfg::kAccStride;
       acc_buf ^= 1;
-      const int split = SPLITK ? tile / (p.m_blocks * p.n_blocks) : 0;
-      const int n_blk = (SPLITK ? tile % (p.m_blocks * p.n_blocks) : tile) / p.m_blocks;
+      const int split = SPLITK == kSplitPlanes ? tile / (p.m_blocks * p.n_blocks) : kCluster ? tile % p.splits : 0;
+      const int n_blk = (SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile) / p.m_blocks;
       const int ks_begin = split * p.k_stages_per_split;
       const int ks_end = min(ks_begin + p.k_stages_per_split, p.num_k_stages);
       bool all_b = true;
@@ -790,8 +914,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     if (FMT != TF_FMT_NVFP4 && p.q_codes && p.q_pad)
       zero_scale_padding(p.q_scales, p.m, p.n >> 5, (int64_t)blockIdx.x * 256 + (grp * 4 + q) * 32 + lane, (int64_t)gridDim.x * 256);
     for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x) {
-      const int split = SPLITK ? tile / (p.m_blocks * p.n_blocks) : 0;
-      const int rest = SPLITK ? tile % (p.m_blocks * p.n_blocks) : tile;
+      const int split = SPLITK == kSplitPlanes ? tile / (p.m_blocks * p.n_blocks) : kCluster ? tile % p.splits : 0;
+      const int rest = SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile;
       const int m_blk = rest % p.m_blocks, n_blk = rest / p.m_blocks;
       bool ok = mbar_wait(bar_tmem_full, tile_phase, abort_flag, 4);
       ok = __all_sync(0xFFFFFFFFu, ok);
@@ -801,7 +925,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const int col0 = n_blk * kOutCols;
       const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(__ldg(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), __ldg(p.b_gs)) : alpha;
-      if (SPLITK) {
+      if (kCluster) {
+        if (m_blk * kBlockM + q * 32 < p.m) {
+          const uint32_t smem_row = smem_a + (uint32_t)(q * 32 + lane) * DumpCfg<BLOCK_N>::kPitch;
+          if (grp == 0) epilogue_dump<FMT, BLOCK_N, 0>(t_row, smem_row);
+          else epilogue_dump<FMT, BLOCK_N, 1>(t_row, smem_row);
+        }
+      } else if (SPLITK == kSplitPlanes) {
         float* ws_row = p.ws + ((int64_t)split * p.m + row) * p.n;
         if (acc_buf == 0) {
           if (grp == 0) epilogue_partial<FMT, BLOCK_N, 0, 0>(p, t_row, bar_tmem_empty, lane, row, col0, ws_row);
@@ -820,7 +950,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
       acc_buf ^= 1;
       tile_phase ^= 1;
     }
-    if (!SPLITK && p.out_amax) {  // one atomic per warp
+    if (SPLITK == kSplitNone && p.out_amax) {  // one atomic per warp
       uint32_t mx = max(amax2 & 0xFFFFu, amax2 >> 16);
       for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
       if (lane == 0 && mx) atomicMax(p.out_amax, mx << 16);
@@ -830,6 +960,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
   // ---------------- teardown: every thread arrives, then the allocating warp frees tensor memory ----------------
   tc_fence_before();
   __syncthreads();
+  if (kCluster) {
+    cluster_sync_all();  // every CTA's rows are dumped
+    const int rest = (int)blockIdx.x / p.splits;
+    cluster_reduce<FMT, BLOCK_N, EPI>(p, smem_a, (int)blockIdx.x % p.splits, rest % p.m_blocks, rest / p.m_blocks);
+    cluster_sync_all();  // nobody leaves while a peer may still read this CTA's shared memory
+  }
   if (warp == 1) {
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)Cfg::kTmemCols) : "memory");
@@ -1170,7 +1306,7 @@ static SplitPlan split_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogue)
   return sp;
 }
 
-template <int FMT, int BLOCK_N, int EPI, bool SPLITK>
+template <int FMT, int BLOCK_N, int EPI, int SPLITK>
 static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
   using Cfg = TileCfg<FMT, BLOCK_N>;
   auto kernel = gemm_blockscaled_kernel<FMT, BLOCK_N, EPI, SPLITK>;
@@ -1184,6 +1320,24 @@ static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmP
   constexpr int out_cols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;
   p.n_blocks = (p.n + out_cols - 1) / out_cols;
   p.num_tiles = p.m_blocks * p.n_blocks * p.splits;
+  if (SPLITK == kSplitCluster) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.num_tiles);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic_launch_enabled() ? 2 : 1;
+    TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
+    return TF_OK;
+  }
   const int grid = p.num_tiles < gemm_sms() ? p.num_tiles : gemm_sms();
   TF_CUDA(launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, ta, tb, p));
   return TF_OK;
@@ -1261,23 +1415,112 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   return TF_OK;
 }
 
+// How one call is launched: the form of the split along K (kSplit...), the tile width, the K ranges and the stages of each.
+struct LaunchPlan {
+  int form, block_n, splits, k_stages_per_split;
+};
+
+static int two_cta_forced() {
+  static const int forced = getenv("TF_GEMM_TWO_CTA") ? atoi(getenv("TF_GEMM_TWO_CTA")) : -1;
+  return forced;
+}
+
 // Whether the 2-CTA kernel serves this problem (TF_GEMM_TWO_CTA in the environment: 0 never, 1 wherever it can, unset this rule).
 // Per wave of tiles the pair is 5-13 % faster than the one-CTA kernel (measured on B200, one-CTA -> pair: nvfp4 4096 x 8192 x 28672
 // 385 -> 336 us, 4096 x 28672 x 8192 + gate 713 -> 666, 4096 x 6144 x 2560 35.1 -> 33.2; mxfp8 8192 x 6144 x 2560 106 -> 98.8;
 // mxfp4 300 x 8192 x 4096 12.8 -> 12.1), but its row blocks are 256 high: it is left where that costs a tenth more waves.
-static bool use_pair_kernel(const GemmParams& p, const SplitPlan& sp, int out_cols) {
-  static const int forced = getenv("TF_GEMM_TWO_CTA") ? atoi(getenv("TF_GEMM_TWO_CTA")) : -1;
-  if (forced == 0 || sp.splits != 1 || p.scatter_rows || p.m <= kBlockM || p.n_rows_b < 256) return false;
+static bool use_pair_kernel(const GemmParams& p, const LaunchPlan& lp, int out_cols) {
+  const int forced = two_cta_forced();
+  if (forced == 0 || lp.form != kSplitNone || lp.block_n != 256 || p.scatter_rows || p.m <= kBlockM || p.n_rows_b < 256) return false;
   if (forced == 1) return true;
   const int64_t sms = gemm_sms(), pairs = sms / 2, n_blocks = (p.n + out_cols - 1) / out_cols;
   const int64_t waves = (p.m_blocks * n_blocks + sms - 1) / sms, pair_waves = ((p.m + 255) / 256 * n_blocks + pairs - 1) / pairs;
   return 10 * pair_waves <= 11 * waves;
 }
 
+// How many clusters of `splits` GEMM CTAs (one CTA fills an SM) the current device runs at once: a cluster lives inside one GPC, so
+// this is less than SMs / splits (measured on B200: 47 clusters of 3 or fewer, where 48 would need 144 of the 148 SMs). Asked once.
+static int cluster_capacity(int splits) {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> cached[kMaxDevices][kMaxClusterSplits + 1];  // 0: not asked yet; else capacity + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  int c = cached[dev][splits].load(std::memory_order_relaxed);
+  if (c == 0) {
+    using Cfg = TileCfg<TF_FMT_MXFP8, 128>;
+    auto kernel = gemm_blockscaled_kernel<TF_FMT_MXFP8, 128, TF_EPI_NONE, kSplitCluster>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)splits);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+    c = n + 1;
+    cached[dev][splits].store(c, std::memory_order_relaxed);
+  }
+  return c - 1;
+}
+
+// The launch plan: `sp` as it stands, or 128-column tiles, or (kSplitCluster) each tile cut over a cluster of CTAs, whichever the model
+// below says is shortest. Microseconds beyond a launch's fixed 4.4, fitted to B200 measurements of graphs of 24 launches:
+//   a K stage takes 0.235 with 128-column tiles and 0.38 with 256 (bound by shared-memory reads and fills), a tile's epilogue 0.5 / 1.0;
+//   planes and a reduction launch 2.0 + 8 bytes per partial sum at 3 TB/s; a cluster 1.6 + its remote reads at 26.6 GB/s per SM.
+// before -> after: mxfp8 512 x 2560 x 3072 13.5 -> 11.2 us (128-column tiles), 128 x 2560 x 3072 12.4 -> 10.2 (4 ranges), 1 x 2560 x 3072
+// 7.3 -> 6.2 (6), 700 x 1024 x 16384 43.0 -> 23.2 (2), mxfp4 300 x 1024 x 8192 residual 27.0 -> 11.0 (3).
+// A problem with a planes plan keeps that plan's K ranges in every form, so that its result is the sum of the planes bit for bit.
+// The SiLU gate pairs 128 + 128 columns, so its tiles stay 256 wide; with planes available (m <= 256) those measured faster (9.2 against
+// 9.5 us at 1 x 3072 x 2560), so a cluster takes it only above that.
+static LaunchPlan launch_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogue, const SplitPlan& sp) {
+  LaunchPlan best = {sp.splits > 1 ? kSplitPlanes : kSplitNone, sp.block_n, sp.splits, sp.k_stages_per_split};
+  if (two_cta_forced() == 1) return best;
+  const bool gate = epilogue == TF_EPI_SILU_GATE;
+  const int64_t sms = gemm_sms(), m_blocks = (m + kBlockM - 1) / kBlockM, n_acc = gate ? 2 * n : n;
+  const int64_t stages = (k_bytes + kStageKBytes - 1) / kStageKBytes, rows = m < kBlockM ? m : kBlockM;
+  auto tiles = [&](int bn) { return m_blocks * ((n_acc + bn - 1) / bn); };
+  auto stage_us = [](int bn) { return bn == 128 ? 0.235 : 0.38; };
+  auto tile_us = [&](int bn, int64_t kps) { return (double)kps * stage_us(bn) + (bn == 128 ? 0.5 : 1.0); };
+  if (tiles(128) > 2 * sms) return best;  // at least one full wave of 256-column tiles
+  double cost = (double)((tiles(sp.block_n) * sp.splits + sms - 1) / sms) * tile_us(sp.block_n, sp.k_stages_per_split);
+  if (sp.splits > 1) cost += 2.0 + (double)sp.splits * (double)m * (double)n_acc * 8.0 / 3.0e6;
+  if (!gate && sp.splits == 1 && tiles(128) <= sms && tile_us(128, stages) < cost) {
+    cost = tile_us(128, stages);
+    best = {kSplitNone, 128, 1, (int)stages};
+  }
+  if (gate && m <= 256) return best;
+  const int bn = gate ? 256 : 128;
+  for (int64_t want = 2; want <= kMaxClusterSplits && stages / want >= 2; ++want) {
+    const int64_t kps = (stages + want - 1) / want, splits = (stages + kps - 1) / kps;
+    if (splits < 2 || tiles(bn) * splits > sms || tiles(bn) > cluster_capacity((int)splits)) continue;
+    if (sp.splits > 1 && (splits != sp.splits || kps != sp.k_stages_per_split)) continue;  // the sums tf_gemm_blockscaled_partials leaves
+    const double c = tile_us(bn, kps) + 1.6 + (double)rows * bn * 4.0 * (double)(splits - 1) / (double)splits / 26600.0;
+    if (c < cost) {
+      cost = c;
+      best = {kSplitCluster, bn, (int)splits, (int)kps};
+    }
+  }
+  return best;
+}
+
 template <int FMT>
-static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int epilogue, const SplitPlan& sp, cudaStream_t stream,
+static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int epilogue, const LaunchPlan& lp, cudaStream_t stream,
                                bool partials_only = false) {
-  if (sp.splits > 1) {
+  if (lp.form == kSplitCluster) {
+    if (epilogue == TF_EPI_SILU_GATE) return launch_gemm<FMT, 256, TF_EPI_SILU_GATE, kSplitCluster>(ta, tb, p, stream);
+    if (epilogue == TF_EPI_RESIDUAL) return launch_gemm<FMT, 128, TF_EPI_RESIDUAL, kSplitCluster>(ta, tb, p, stream);
+    return launch_gemm<FMT, 128, TF_EPI_NONE, kSplitCluster>(ta, tb, p, stream);
+  }
+  if (lp.form == kSplitPlanes) {
     // first pass: plain accumulation over all accumulator columns into the workspace; second pass: reduce + epilogue
     const int n_out = p.n;
     float* residual = p.residual;
@@ -1286,7 +1529,7 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     p.out_amax = nullptr;
     uint8_t* qc = p.q_codes;
     p.q_codes = nullptr;  // the quantized copy is produced by the second pass
-    tf_status st = sp.block_n == 128 ? launch_gemm<FMT, 128, TF_EPI_NONE, true>(ta, tb, p, stream) : launch_gemm<FMT, 256, TF_EPI_NONE, true>(ta, tb, p, stream);
+    tf_status st = lp.block_n == 128 ? launch_gemm<FMT, 128, TF_EPI_NONE, kSplitPlanes>(ta, tb, p, stream) : launch_gemm<FMT, 256, TF_EPI_NONE, kSplitPlanes>(ta, tb, p, stream);
     if (st != TF_OK) return st;
     if (partials_only) return TF_OK;  // the caller's next kernel sums the planes (tf_gemm_blockscaled_partials)
     p.q_codes = qc;
@@ -1297,7 +1540,7 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     const float* ags = FMT == TF_FMT_NVFP4 ? p.a_gs : nullptr;
     const float* bgs = FMT == TF_FMT_NVFP4 ? p.b_gs : nullptr;
 #define TF_REDUCE(EPI_, Q_) \
-  launch_dependent(splitk_reduce_kernel<EPI_, Q_>, dim3(grid), dim3(256), 0, stream, (const float*)p.ws, (int)sp.splits, (int)p.m, (int)n_out, (int)p.n_rows_b, ags, bgs, \
+  launch_dependent(splitk_reduce_kernel<EPI_, Q_>, dim3(grid), dim3(256), 0, stream, (const float*)p.ws, (int)lp.splits, (int)p.m, (int)n_out, (int)p.n_rows_b, ags, bgs, \
                    p.out, p.ldo, residual, amax, p.q_codes, p.q_scales, (int)p.q_pad, (int)p.a_gs_rows)
     const int qf = p.q_codes ? FMT : -1;
     if (epilogue == TF_EPI_SILU_GATE) {
@@ -1315,15 +1558,15 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     TF_LAUNCH_CHECK();
     return TF_OK;
   }
-  if (use_pair_kernel(p, sp, epilogue == TF_EPI_SILU_GATE ? 128 : 256)) {
+  if (use_pair_kernel(p, lp, epilogue == TF_EPI_SILU_GATE ? 128 : 256)) {
     if (epilogue == TF_EPI_SILU_GATE) return launch_gemm_pair<FMT, TF_EPI_SILU_GATE>(ta, tb, p, stream);
     if (epilogue == TF_EPI_RESIDUAL) return launch_gemm_pair<FMT, TF_EPI_RESIDUAL>(ta, tb, p, stream);
     return launch_gemm_pair<FMT, TF_EPI_NONE>(ta, tb, p, stream);
   }
-  if (epilogue == TF_EPI_SILU_GATE) return launch_gemm<FMT, 256, TF_EPI_SILU_GATE, false>(ta, tb, p, stream);
+  if (epilogue == TF_EPI_SILU_GATE) return launch_gemm<FMT, 256, TF_EPI_SILU_GATE, kSplitNone>(ta, tb, p, stream);
   if (epilogue == TF_EPI_RESIDUAL)
-    return sp.block_n == 256 ? launch_gemm<FMT, 256, TF_EPI_RESIDUAL, false>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_RESIDUAL, false>(ta, tb, p, stream);
-  return sp.block_n == 256 ? launch_gemm<FMT, 256, TF_EPI_NONE, false>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_NONE, false>(ta, tb, p, stream);
+    return lp.block_n == 256 ? launch_gemm<FMT, 256, TF_EPI_RESIDUAL, kSplitNone>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_RESIDUAL, kSplitNone>(ta, tb, p, stream);
+  return lp.block_n == 256 ? launch_gemm<FMT, 256, TF_EPI_NONE, kSplitNone>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_NONE, kSplitNone>(ta, tb, p, stream);
 }
 
 // Scratch of tf_gemm_blockscaled_static: lives in the library's device image, one copy per GPU that loads the library,
@@ -1511,6 +1754,8 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
   p.scatter_rows = 0;
   for (int i = 0; i < 8; ++i) p.scatter_out[i] = nullptr;
   const SplitPlan sp = split_plan(m, n, k_bytes, epilogue);
+  LaunchPlan lp = {kSplitPlanes, sp.block_n, sp.splits, sp.k_stages_per_split};
+  if (!partial_splits) lp = launch_plan(m, n, k_bytes, epilogue, sp);
   if (scatter_ptrs) {
     if (sp.splits > 1)
       return fail(TF_ERR_UNSUPPORTED, "%s: this shape is split along K (tf_gemm_workspace_bytes > 0), which has no scattered output", fn);
@@ -1521,8 +1766,8 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
     if (sp.splits <= 1) return fail(TF_ERR_UNSUPPORTED, "%s: this shape is not split along K (tf_gemm_splits == 1): there are no partial sums to leave", fn);
     *partial_splits = sp.splits;
   }
-  p.splits = sp.splits;
-  p.k_stages_per_split = sp.k_stages_per_split;
+  p.splits = lp.splits;
+  p.k_stages_per_split = lp.k_stages_per_split;
   p.ws = static_cast<float*>(workspace);
   if (sp.splits > 1) {
     const int64_t need = (int64_t)sp.splits * m * n_rows_b * 4;
@@ -1536,9 +1781,9 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
     if (st != TF_OK) return st;
   }
   switch (format) {
-    case TF_FMT_MXFP8: return dispatch_gemm<TF_FMT_MXFP8>(ta, tb, p, epilogue, sp, stream, partial_splits != nullptr);
-    case TF_FMT_MXFP4: return dispatch_gemm<TF_FMT_MXFP4>(ta, tb, p, epilogue, sp, stream, partial_splits != nullptr);
-    default: return dispatch_gemm<TF_FMT_NVFP4>(ta, tb, p, epilogue, sp, stream, partial_splits != nullptr);
+    case TF_FMT_MXFP8: return dispatch_gemm<TF_FMT_MXFP8>(ta, tb, p, epilogue, lp, stream, partial_splits != nullptr);
+    case TF_FMT_MXFP4: return dispatch_gemm<TF_FMT_MXFP4>(ta, tb, p, epilogue, lp, stream, partial_splits != nullptr);
+    default: return dispatch_gemm<TF_FMT_NVFP4>(ta, tb, p, epilogue, lp, stream, partial_splits != nullptr);
   }
 }
 
