@@ -77,8 +77,9 @@ TF_API tf_status tf_device_status(int32_t* status, int32_t* detail);
  * 0 restores the default. No counterpart in the reference (its GEMM is cuBLASLt's `sm_count_target`, python/src/tilefish/_cublaslt.py). */
 TF_API tf_status tf_set_sm_margin(int32_t sms);
 
-/* Programmatic dependent launch for this library's kernels (off by default; PROCESS-WIDE, as tf_set_sm_margin). On: the quantize, rmsnorm, GEMM and
- * split-K reduction kernels are launched so that each may be scheduled while the kernel before it on the stream is still
+/* Programmatic dependent launch for all of this library's kernels (off by default: then only GEMMs of at most 256 rows and
+ * row kernels of at most 4 rows use it; PROCESS-WIDE, as tf_set_sm_margin). On: the quantize, rmsnorm, GEMM and split-K
+ * reduction kernels are launched so that each may be scheduled while the kernel before it on the stream is still
  * draining; each waits (griddepcontrol.wait) for that kernel to complete before its first access to global memory, so results
  * are unchanged. It hides launch latency and kernel set-up in chains of short kernels (small M, decode, many GPUs). No
  * counterpart in the reference. */

@@ -39,13 +39,24 @@ tf_status scale_padding(void* scales, int32_t format, int64_t rows, int64_t k, i
 // Programmatic dependent launch (tf_set_programmatic_launch): a kernel launched through launch_dependent() may be scheduled
 // while the kernel before it on the stream is still draining, so that its launch latency and set-up overlap that tail. Every
 // kernel launched this way executes griddep_wait() before its first access to global memory, which blocks until the previous
-// kernel has completed and its writes are visible. Off: a plain stream-ordered launch.
+// kernel has completed and its writes are visible. Off: a plain stream-ordered launch, but for chains of short kernels (`chain`, see
+// chain_gemm_launch), where the overlap is worth more than it costs.
 bool programmatic_launch_enabled();
 void set_programmatic_launch(bool on);
 
 #ifdef __CUDACC__
+// Launched as programmatic dependents whatever the switch says: GEMMs of one wave and at most 256 rows, and the row kernels of at most
+// four rows. A GEMM's CTAs take a whole SM each, so starting early only hides their set-up. A row kernel's CTAs are small: started
+// early they all pile onto the few SMs that the GEMM in front leaves free and then share those (70B-shaped decode at 64 rows: its
+// rmsnorm launch went from 9.8 to 14.7 us; two blocks at 16 rows 184.6 us without, 190.4 with). Above 256 rows the waiting CTAs
+// take the registers that the rest of the row kernel in front needs (README block at 8192 rows 189.5 -> 196.2 us).
+// Captured graphs, before -> after: README block at one row 20.5 -> 18.4 us, 70B-shaped decode at 64 rows 402 -> 389, two
+// 4096 x 8192 blocks at 200 rows 93 -> 85.
+inline bool chain_gemm_launch(int64_t rows) { return rows <= 256; }
+inline bool chain_rows_launch(int64_t rows) { return rows <= 4; }
+
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_dependent(bool chain, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -55,7 +66,7 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = programmatic_launch_enabled() ? 1 : 0;
+  cfg.numAttrs = chain || programmatic_launch_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 #endif

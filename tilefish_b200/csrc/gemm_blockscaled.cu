@@ -1334,12 +1334,12 @@ static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmP
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = programmatic_launch_enabled() ? 2 : 1;
+    cfg.numAttrs = chain_gemm_launch(p.m) || programmatic_launch_enabled() ? 2 : 1;
     TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
     return TF_OK;
   }
   const int grid = p.num_tiles < gemm_sms() ? p.num_tiles : gemm_sms();
-  TF_CUDA(launch_dependent(kernel, dim3(grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, ta, tb, p));
+  TF_CUDA(launch_dependent(chain_gemm_launch(p.m) && p.num_tiles <= grid, kernel, dim3(grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, ta, tb, p));
   return TF_OK;
 }
 
@@ -1410,7 +1410,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = programmatic_launch_enabled() ? 2 : 1;
+  cfg.numAttrs = chain_gemm_launch(p.m) || programmatic_launch_enabled() ? 2 : 1;
   TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tsa, tsb, to, p));
   return TF_OK;
 }
@@ -1540,7 +1540,7 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     const float* ags = FMT == TF_FMT_NVFP4 ? p.a_gs : nullptr;
     const float* bgs = FMT == TF_FMT_NVFP4 ? p.b_gs : nullptr;
 #define TF_REDUCE(EPI_, Q_) \
-  launch_dependent(splitk_reduce_kernel<EPI_, Q_>, dim3(grid), dim3(256), 0, stream, (const float*)p.ws, (int)lp.splits, (int)p.m, (int)n_out, (int)p.n_rows_b, ags, bgs, \
+  launch_dependent(chain_rows_launch(p.m), splitk_reduce_kernel<EPI_, Q_>, dim3(grid), dim3(256), 0, stream, (const float*)p.ws, (int)lp.splits, (int)p.m, (int)n_out, (int)p.n_rows_b, ags, bgs, \
                    p.out, p.ldo, residual, amax, p.q_codes, p.q_scales, (int)p.q_pad, (int)p.a_gs_rows)
     const int qf = p.q_codes ? FMT : -1;
     if (epilogue == TF_EPI_SILU_GATE) {

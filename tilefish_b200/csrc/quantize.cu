@@ -339,7 +339,7 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
     if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
     TF_CUDA(ring_configure<FMT>());
     const RingLaunch rl = ring_launch(FMT, m, k);
-    TF_CUDA(launch_dependent(ring_rows_kernel<FMT>, dim3(rl.grid), dim3(kRingThreads), rl.smem, stream, static_cast<const uint8_t*>(x), m, k, ldx,
+    TF_CUDA(launch_dependent(chain_rows_launch(m), ring_rows_kernel<FMT>, dim3(rl.grid), dim3(kRingThreads), rl.smem, stream, static_cast<const uint8_t*>(x), m, k, ldx,
                              static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out,
                              (unsigned int*)nullptr, status, rl.stages));
     return TF_OK;
@@ -357,7 +357,7 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
     grid.y = (unsigned)(want < rounds ? want : rounds);
   }
   if (pad && grid.x * grid.y < kPadBlocks) grid.x = kPadBlocks;
-  TF_CUDA(launch_dependent(quantize_rows_kernel<FMT>, grid, block, 0, stream, static_cast<const uint8_t*>(x), m, k, ldx, static_cast<uint8_t*>(codes),
+  TF_CUDA(launch_dependent(chain_rows_launch(m), quantize_rows_kernel<FMT>, grid, block, 0, stream, static_cast<const uint8_t*>(x), m, k, ldx, static_cast<uint8_t*>(codes),
                            static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out));
   return TF_OK;
 }

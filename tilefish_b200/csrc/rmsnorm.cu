@@ -109,10 +109,10 @@ template <int VPT>
 static void launch_vpt(int qfmt, dim3 grid, dim3 block, cudaStream_t s, const uint4* x, float4* res, const uint4* w, uint4* out, int64_t m, int d,
                        float eps, float inv_d, uint8_t* qc, uint8_t* qs, int qsw, int qpad, const float* qgs, unsigned int* amax) {
   switch (qfmt) {
-    case TF_FMT_MXFP8: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
-    case TF_FMT_MXFP4: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
-    case TF_FMT_NVFP4: launch_dependent(residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
-    default: launch_dependent(residual_add_rmsnorm_kernel<VPT, -1>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    case TF_FMT_MXFP8: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    case TF_FMT_MXFP4: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    case TF_FMT_NVFP4: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    default: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, -1>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
   }
 }
 
@@ -266,9 +266,9 @@ static void launch_rows_vpt(int qfmt, dim3 grid, dim3 block, cudaStream_t s, con
                             const float* b_gs, int a_gs_rows, float4* res, const uint4* w, uint4* out, int m, int d, float eps, float inv_d, uint8_t* qc,
                             uint8_t* qs, float* qgs, unsigned int* sync, int* status) {
   switch (qfmt) {
-    case TF_FMT_MXFP8: launch_dependent(rmsnorm_quantize_rows_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, partials, splits, a_gs, b_gs, a_gs_rows, res, w, out, m, d, eps, inv_d, qc, qs, qgs, sync, status); break;
-    case TF_FMT_MXFP4: launch_dependent(rmsnorm_quantize_rows_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, partials, splits, a_gs, b_gs, a_gs_rows, res, w, out, m, d, eps, inv_d, qc, qs, qgs, sync, status); break;
-    default: launch_dependent(rmsnorm_quantize_rows_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, partials, splits, a_gs, b_gs, a_gs_rows, res, w, out, m, d, eps, inv_d, qc, qs, qgs, sync, status); break;
+    case TF_FMT_MXFP8: launch_dependent(chain_rows_launch(m), rmsnorm_quantize_rows_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, partials, splits, a_gs, b_gs, a_gs_rows, res, w, out, m, d, eps, inv_d, qc, qs, qgs, sync, status); break;
+    case TF_FMT_MXFP4: launch_dependent(chain_rows_launch(m), rmsnorm_quantize_rows_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, partials, splits, a_gs, b_gs, a_gs_rows, res, w, out, m, d, eps, inv_d, qc, qs, qgs, sync, status); break;
+    default: launch_dependent(chain_rows_launch(m), rmsnorm_quantize_rows_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, partials, splits, a_gs, b_gs, a_gs_rows, res, w, out, m, d, eps, inv_d, qc, qs, qgs, sync, status); break;
   }
 }
 
