@@ -99,10 +99,22 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
   asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
   return r;
 }
-// two f32 -> two e2m1 nibbles in one byte (lo in bits 0-3), RNE ties-to-even, saturating to +-6.
-__device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi) {
-  uint16_t r;
-  asm("{ .reg .b8 t;\n cvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n mov.b16 %0, {t, 0}; }" : "=h"(r) : "f"(hi), "f"(lo));
+// eight f32 -> eight e2m1 nibbles in one word (element i in bits 4i .. 4i+3), RNE ties-to-even, saturating to +-6. The four bytes are
+// packed as registers, without a shift and an OR for each.
+__device__ __forceinline__ uint32_t cvt_e2m1x8(float a0, float a1, float a2, float a3, float a4, float a5, float a6, float a7) {
+  uint32_t r;
+  asm("{ .reg .b8 b0, b1, b2, b3;\n cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n"
+      " cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n mov.b32 %0, {b0, b1, b2, b3}; }"
+      : "=r"(r)
+      : "f"(a0), "f"(a1), "f"(a2), "f"(a3), "f"(a4), "f"(a5), "f"(a6), "f"(a7));
+  return r;
+}
+// four f32 -> four e4m3 bytes in one word.
+__device__ __forceinline__ uint32_t cvt_e4m3x4(float a0, float a1, float a2, float a3) {
+  uint32_t r;
+  asm("{ .reg .b16 h0, h1;\n cvt.rn.satfinite.e4m3x2.f32 h0, %2, %1;\n cvt.rn.satfinite.e4m3x2.f32 h1, %4, %3;\n mov.b32 %0, {h0, h1}; }"
+      : "=r"(r)
+      : "f"(a0), "f"(a1), "f"(a2), "f"(a3));
   return r;
 }
 // one e4m3 byte -> f32 (exact).

@@ -309,19 +309,16 @@ __device__ __forceinline__ void store_chunk_quantized(const GemmParams& p, const
     uint32_t c[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      c[j] = cvt_e4m3x2(bf16lo_to_f32(q[2 * j]), bf16hi_to_f32(q[2 * j])) | (cvt_e4m3x2(bf16lo_to_f32(q[2 * j + 1]), bf16hi_to_f32(q[2 * j + 1])) << 16);
+      c[j] = cvt_e4m3x4(bf16lo_to_f32(q[2 * j]), bf16hi_to_f32(q[2 * j]), bf16lo_to_f32(q[2 * j + 1]), bf16hi_to_f32(q[2 * j + 1]));
     uint4* dst = reinterpret_cast<uint4*>(p.q_codes + (int64_t)row * p.n + col);
     dst[0] = make_uint4(c[0], c[1], c[2], c[3]);
     dst[1] = make_uint4(c[4], c[5], c[6], c[7]);
   } else {
     uint32_t c[4];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      uint32_t w = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w |= cvt_e2m1x2(bf16lo_to_f32(q[4 * h + j]), bf16hi_to_f32(q[4 * h + j])) << (8 * j);
-      c[h] = w;
-    }
+    for (int h = 0; h < 4; ++h)
+      c[h] = cvt_e2m1x8(bf16lo_to_f32(q[4 * h]), bf16hi_to_f32(q[4 * h]), bf16lo_to_f32(q[4 * h + 1]), bf16hi_to_f32(q[4 * h + 1]),
+                        bf16lo_to_f32(q[4 * h + 2]), bf16hi_to_f32(q[4 * h + 2]), bf16lo_to_f32(q[4 * h + 3]), bf16hi_to_f32(q[4 * h + 3]));
     *reinterpret_cast<uint4*>(p.q_codes + (int64_t)row * (p.n >> 1) + (col >> 1)) = make_uint4(c[0], c[1], c[2], c[3]);
   }
   p.q_scales[swizzled_scale_offset(row, col >> 5, ((p.n >> 5) + 3) >> 2)] = (uint8_t)scale;

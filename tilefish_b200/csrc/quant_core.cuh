@@ -43,10 +43,9 @@ __device__ __forceinline__ void quantize_vec8(const uint4& v, float gs, float in
     const bool zero = (d == 0.0f);
     const float inv = zero ? 0.0f : __frcp_rn(d);
     scale = s8;
-    c0 = cvt_e2m1x2(__fmul_rn(bf16lo_to_f32(v.x), inv), __fmul_rn(bf16hi_to_f32(v.x), inv)) |
-         (cvt_e2m1x2(__fmul_rn(bf16lo_to_f32(v.y), inv), __fmul_rn(bf16hi_to_f32(v.y), inv)) << 8) |
-         (cvt_e2m1x2(__fmul_rn(bf16lo_to_f32(v.z), inv), __fmul_rn(bf16hi_to_f32(v.z), inv)) << 16) |
-         (cvt_e2m1x2(__fmul_rn(bf16lo_to_f32(v.w), inv), __fmul_rn(bf16hi_to_f32(v.w), inv)) << 24);
+    c0 = cvt_e2m1x8(__fmul_rn(bf16lo_to_f32(v.x), inv), __fmul_rn(bf16hi_to_f32(v.x), inv), __fmul_rn(bf16lo_to_f32(v.y), inv),
+                    __fmul_rn(bf16hi_to_f32(v.y), inv), __fmul_rn(bf16lo_to_f32(v.z), inv), __fmul_rn(bf16hi_to_f32(v.z), inv),
+                    __fmul_rn(bf16lo_to_f32(v.w), inv), __fmul_rn(bf16hi_to_f32(v.w), inv));
     if (zero) c0 = 0;
     c1 = 0;
     return;
@@ -61,11 +60,11 @@ __device__ __forceinline__ void quantize_vec8(const uint4& v, float gs, float in
   const uint32_t inv2 = inv1 | (inv1 << 16);
   const uint32_t q0 = mul_bf16x2(v.x, inv2), q1 = mul_bf16x2(v.y, inv2), q2 = mul_bf16x2(v.z, inv2), q3 = mul_bf16x2(v.w, inv2);
   if (FMT == TF_FMT_MXFP8) {
-    c0 = cvt_e4m3x2(bf16lo_to_f32(q0), bf16hi_to_f32(q0)) | (cvt_e4m3x2(bf16lo_to_f32(q1), bf16hi_to_f32(q1)) << 16);
-    c1 = cvt_e4m3x2(bf16lo_to_f32(q2), bf16hi_to_f32(q2)) | (cvt_e4m3x2(bf16lo_to_f32(q3), bf16hi_to_f32(q3)) << 16);
+    c0 = cvt_e4m3x4(bf16lo_to_f32(q0), bf16hi_to_f32(q0), bf16lo_to_f32(q1), bf16hi_to_f32(q1));
+    c1 = cvt_e4m3x4(bf16lo_to_f32(q2), bf16hi_to_f32(q2), bf16lo_to_f32(q3), bf16hi_to_f32(q3));
   } else {
-    c0 = cvt_e2m1x2(bf16lo_to_f32(q0), bf16hi_to_f32(q0)) | (cvt_e2m1x2(bf16lo_to_f32(q1), bf16hi_to_f32(q1)) << 8) |
-         (cvt_e2m1x2(bf16lo_to_f32(q2), bf16hi_to_f32(q2)) << 16) | (cvt_e2m1x2(bf16lo_to_f32(q3), bf16hi_to_f32(q3)) << 24);
+    c0 = cvt_e2m1x8(bf16lo_to_f32(q0), bf16hi_to_f32(q0), bf16lo_to_f32(q1), bf16hi_to_f32(q1), bf16lo_to_f32(q2), bf16hi_to_f32(q2),
+                    bf16lo_to_f32(q3), bf16hi_to_f32(q3));
     c1 = 0;
   }
 }
@@ -93,11 +92,13 @@ __device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs,
     scale = s8;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      uint32_t c = 0;
+      float f[8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        c |= cvt_e2m1x2(__fmul_rn(bf16lo_to_f32(w[4 * h + j]), inv), __fmul_rn(bf16hi_to_f32(w[4 * h + j]), inv)) << (8 * j);
-      codes[h] = zero ? 0u : c;
+      for (int j = 0; j < 4; ++j) {
+        f[2 * j] = __fmul_rn(bf16lo_to_f32(w[4 * h + j]), inv);
+        f[2 * j + 1] = __fmul_rn(bf16hi_to_f32(w[4 * h + j]), inv);
+      }
+      codes[h] = zero ? 0u : cvt_e2m1x8(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
     }
     codes[2] = codes[3] = 0;
     return;
@@ -113,15 +114,12 @@ __device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs,
   if (FMT == TF_FMT_MXFP8) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      codes[j] = cvt_e4m3x2(bf16lo_to_f32(q[2 * j]), bf16hi_to_f32(q[2 * j])) | (cvt_e4m3x2(bf16lo_to_f32(q[2 * j + 1]), bf16hi_to_f32(q[2 * j + 1])) << 16);
+      codes[j] = cvt_e4m3x4(bf16lo_to_f32(q[2 * j]), bf16hi_to_f32(q[2 * j]), bf16lo_to_f32(q[2 * j + 1]), bf16hi_to_f32(q[2 * j + 1]));
   } else {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint32_t c = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) c |= cvt_e2m1x2(bf16lo_to_f32(q[4 * h + j]), bf16hi_to_f32(q[4 * h + j])) << (8 * j);
-      codes[h] = c;
-    }
+    for (int h = 0; h < 2; ++h)
+      codes[h] = cvt_e2m1x8(bf16lo_to_f32(q[4 * h]), bf16hi_to_f32(q[4 * h]), bf16lo_to_f32(q[4 * h + 1]), bf16hi_to_f32(q[4 * h + 1]),
+                            bf16lo_to_f32(q[4 * h + 2]), bf16hi_to_f32(q[4 * h + 2]), bf16lo_to_f32(q[4 * h + 3]), bf16hi_to_f32(q[4 * h + 3]));
     codes[2] = codes[3] = 0;
   }
 }

@@ -1,15 +1,19 @@
 // BlockScaled quantization row kernels (bf16 -> MXFP8 / MXFP4 / NVFP4) and the scale-layout helpers.
 //
-// HBM-bound: every thread moves one 256-bit vector of 16 bf16 per step (coalesced: consecutive lanes, consecutive
+// HBM-bound: every thread moves four 256-bit vectors of 16 bf16 per step (coalesced: consecutive lanes, consecutive
 // vectors), block maxima are combined with at most one warp shuffle, codes leave as 16-byte (e4m3) or 8-byte (e2m1)
 // coalesced stores. Algorithmic bytes per element: 2 + 1 + 1/32 (mxfp8), 2 + 0.5 + 1/32 (mxfp4), 2 + 0.5 + 1/16 (nvfp4).
+// Four loads in flight per thread, two before, and a shared-memory ring fed by bulk copies for mxfp8 (graphs of 12 launches, ring or
+// two -> four): 65536 x 4096 mxfp8 135.2 -> 132.9 us (6.1 TB/s), mxfp4 111.7 -> 102.5 (6.6 TB/s), nvfp4 112.3 -> 104.2 (6.6 TB/s);
+// 8192 x 4096 nvfp4 17.9 -> 16.8; 16384 x 2080 mxfp8 37.5 -> 20.7. Eight loads, 64, 128 or 512 threads and streaming (evict-first)
+// stores were no better over that range.
 #include "async_copy.cuh"
 #include "quant_core.cuh"
 
 namespace tf {
 
 constexpr int kQuantThreads = 256;
-constexpr int kQuantUnroll = 2;
+constexpr int kQuantUnroll = 4;
 
 // Block = (TPR threads along the row) x (256 / TPR rows); rows are taken grid-stride.
 __device__ __forceinline__ void load_256(const void* p, uint32_t (&w)[8]) {
@@ -77,169 +81,123 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint
   }
 }
 
-// ---- the streaming form: rows staged through a shared-memory ring by bulk copies -------------------------------------------
-// Used by the mxfp8 quantizer and the amax pass (see use_ring). For long rows (k >= 2048) the input is cut into chunks of up to 2048 consecutive bf16 of one row (4 KB). Every CTA owns a ring
-// of kRingStages chunk buffers; thread 0 keeps the ring full with cp.async.bulk (one 4 KB request per chunk, completion counted
-// on an mbarrier), so each CTA has (kRingStages - 1) x 4 KB in flight whatever its threads are doing, and eight CTAs fit on an
-// SM: the loads no longer wait for registers. The 128 threads then take 32 bytes each from the stage (16 consecutive bf16,
-// the same thread <-> element mapping and the same arithmetic as quantize_rows_kernel, hence the same bytes), hand the stage
-// back, and quantize and store while the next copies are in flight. Waits are bounded (async_copy.cuh).
-constexpr int kRingThreads = 128;
-constexpr int kRingChunkVecs = kRingThreads;        // 16-element vectors per chunk
-constexpr int kRingChunkBytes = kRingChunkVecs * 32;
-constexpr int kRingMaxStages = 8;
-constexpr unsigned long long kRingWaitLimitNs = 1000000000ull;
-constexpr int kModeAmax = 3;  // MODE of ring_rows_kernel beyond the three formats: only the tensor's amax
+// ---- the amax pass of a dense tensor: one run of bytes staged through a shared-memory ring by bulk copies ------------------------
+// The tensor is cut into 8 KB chunks that the CTAs take in turn. Every CTA owns a ring of chunk buffers; thread 0 keeps it full with
+// cp.async.bulk (completion counted on an mbarrier), so the loads wait for neither registers nor arithmetic. 96 % of the copy rate at
+// 65536 x 4096 (84.5 us). Chunks are cut across rows, so widths that are no multiple of a chunk cost nothing: against a ring of row
+// chunks 16384 x 2080 24.9 -> 18.3 us with its two small launches, 4096 x 2560 11.8 -> 8.4. Waits are bounded (async_copy.cuh).
+constexpr int kStreamThreads = 128;
+constexpr int kStreamVpt = 2;
+constexpr int kStreamChunkVecs = kStreamThreads * kStreamVpt;
+constexpr int kStreamChunkBytes = kStreamChunkVecs * 32;
+constexpr int kStreamStages = 4;
+constexpr int kStreamCtasPerSm = 6;
+constexpr size_t kStreamSmem = (size_t)kStreamStages * (kStreamChunkBytes + 8);
+constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 
 __device__ __forceinline__ void lds_256(uint32_t addr, uint32_t (&w)[8]) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(addr + 16));
 }
 
-// Dynamic shared memory: `stages` chunk buffers of 4 KB, then one mbarrier per stage.
-template <int MODE>
-__global__ void __launch_bounds__(kRingThreads) ring_rows_kernel(const uint8_t* __restrict__ x, int64_t m, int64_t k, int64_t ldx,
-                                                                 uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int swizzled, int pad,
-                                                                 const float* __restrict__ gs_ptr, float* __restrict__ gs_out,
-                                                                 unsigned int* __restrict__ amax_bits_out, int* __restrict__ status, int stages) {
+// Two packed 16-bit maxima of the magnitudes of 16 bf16, joined with `acc`.
+__device__ __forceinline__ uint32_t amax16(const uint32_t (&w)[8], uint32_t acc) {
+  const uint32_t km = 0x7FFF7FFFu;
+  uint32_t t0 = __vimax3_u16x2(w[0] & km, w[1] & km, w[2] & km);
+  uint32_t t1 = __vimax3_u16x2(w[3] & km, w[4] & km, w[5] & km);
+  t0 = __vimax3_u16x2(t0, w[6] & km, w[7] & km);
+  return __vimax3_u16x2(acc, t0, t1);
+}
+
+// The block's maximum of two packed maxima per thread, in thread 0. Every thread of the block calls it.
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_amax(uint32_t acc, int tid) {
+  __shared__ uint32_t warp_max[THREADS / 32];
+  uint32_t mx = max(acc & 0xFFFFu, acc >> 16);
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+  if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
+  __syncthreads();
+  if (tid == 0)
+    for (int wi = 1; wi < THREADS / 32; ++wi) mx = max(mx, warp_max[wi]);
+  return mx;
+}
+
+// Dynamic shared memory: kStreamStages chunk buffers, then one mbarrier per stage. total: 16-element vectors of the tensor.
+__global__ void __launch_bounds__(kStreamThreads) stream_amax_kernel(const uint8_t* __restrict__ x, int64_t total, unsigned int* __restrict__ out_bits,
+                                                                     int* __restrict__ status) {
   extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ int abort_flag;
-  constexpr int FMT = MODE == kModeAmax ? TF_FMT_MXFP8 : MODE;
   const uint32_t ring = smem_u32(ring_smem);
-  const uint32_t bars = ring + (uint32_t)stages * kRingChunkBytes;
+  const uint32_t bars = ring + (uint32_t)kStreamStages * kStreamChunkBytes;
   const int t = threadIdx.x;
-  const int nvec = (int)(k >> 4);
-  const int cpr = (nvec + kRingChunkVecs - 1) / kRingChunkVecs;  // chunks per row
-  const int64_t total = m * cpr;
-  const int64_t stride = gridDim.x;
   if (t == 0) {
-    for (int s = 0; s < stages; ++s) mbar_init(bars + 8 * s, 1);
+    for (int s = 0; s < kStreamStages; ++s) mbar_init(bars + 8 * s, 1);
     abort_flag = 0;
     mbar_fence_init();
   }
   __syncthreads();
-  griddep_launch_dependents();
-  griddep_wait();
-
-  float gs = 0.0f, inv_t = 0.0f;
-  if (MODE == TF_FMT_NVFP4) {
-    gs = __ldg(gs_ptr);
-    if (gs_out != nullptr) {
-      gs = __fdiv_rn(gs, 2688.0f);
-      if (blockIdx.x == 0 && t == 0) gs_out[0] = gs;
-    }
-    inv_t = gs != 0.0f ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
-  }
-
-  if (MODE != kModeAmax && pad)
-    zero_scale_padding(scales, m, k / (MODE == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * kRingThreads + t, (int64_t)gridDim.x * kRingThreads);
-
-  // thread 0: one bulk copy per chunk; a chunk is vectors [c * 128, min(nvec, c * 128 + 128)) of its row
-  auto issue = [&](int64_t chunk, int stage) {
-    const int64_t row = chunk / cpr;
-    const int v0 = (int)(chunk - row * cpr) * kRingChunkVecs;
-    const int nv = min(kRingChunkVecs, nvec - v0);
+  // thread 0: one bulk copy per chunk, the last one possibly short
+  const int64_t stride = (int64_t)gridDim.x * kStreamChunkVecs;
+  auto issue = [&](int64_t base, int stage) {
+    const uint32_t bytes = (uint32_t)min((int64_t)kStreamChunkVecs, total - base) * 32u;
     const uint32_t bar = bars + 8 * stage;
-    mbar_expect_tx(bar, (uint32_t)nv * 32u);
-    bulk_load(ring + (uint32_t)stage * kRingChunkBytes, x + (row * ldx + (int64_t)v0 * 16) * 2, (uint32_t)nv * 32u, bar);
+    mbar_expect_tx(bar, bytes);
+    bulk_load(ring + (uint32_t)stage * kStreamChunkBytes, x + base * 32, bytes, bar);
   };
-  int64_t chunk = blockIdx.x;
+  int64_t base = (int64_t)blockIdx.x * kStreamChunkVecs;
   if (t == 0) {
-    for (int s = 0; s < stages; ++s)
-      if (chunk + s * stride < total) issue(chunk + s * stride, s);
+    for (int s = 0; s < kStreamStages; ++s)
+      if (base + s * stride < total) issue(base + s * stride, s);
   }
-  uint32_t acc = 0;  // MODE == kModeAmax: two packed 16-bit maxima
+  uint32_t acc = 0;  // two packed 16-bit maxima
   int stage = 0;
   uint32_t phase = 0;
-  for (; chunk < total; chunk += stride) {
-    const int64_t row = chunk / cpr;
-    const int v0 = (int)(chunk - row * cpr) * kRingChunkVecs;
-    const bool has = v0 + t < nvec;
-    bool ok = mbar_wait_bounded(bars + 8 * stage, phase, &abort_flag, status, 10, kRingWaitLimitNs);
-    uint32_t w[8];
-    if (ok && has) {
-      lds_256(ring + (uint32_t)stage * kRingChunkBytes + t * 32, w);
-    } else {
+  for (; base < total; base += stride) {
+    const bool ok = mbar_wait_bounded(bars + 8 * stage, phase, &abort_flag, status, 10, kWaitLimitNs);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) w[e] = 0;
+    for (int j = 0; j < kStreamVpt; ++j) {
+      if (ok && base + t + j * kStreamThreads < total) {
+        uint32_t w[8];
+        lds_256(ring + (uint32_t)stage * kStreamChunkBytes + (t + j * kStreamThreads) * 32, w);
+        acc = amax16(w, acc);
+      }
     }
-    // every thread has taken its bytes (or the wait ran out somewhere: then all leave together)
+    // every thread has read its bytes (or the wait ran out somewhere: then all leave together)
     if (!__syncthreads_and(ok)) break;
-    if (t == 0 && chunk + stages * stride < total) issue(chunk + stages * stride, stage);
-    if (MODE == kModeAmax) {
-      const uint32_t km = 0x7FFF7FFFu;
-      uint32_t t0 = __vimax3_u16x2(w[0] & km, w[1] & km, w[2] & km);
-      uint32_t t1 = __vimax3_u16x2(w[3] & km, w[4] & km, w[5] & km);
-      t0 = __vimax3_u16x2(t0, w[6] & km, w[7] & km);
-      acc = __vimax3_u16x2(acc, t0, t1);
-    } else {
-      uint32_t c[4], sc;
-      quantize_vec16<FMT>(w, gs, inv_t, c, sc);  // whole warps: lanes without data quantize zeros
-      if (has) store_quantized16<FMT>(codes, scales, swizzled, row, v0 + t, k, c, sc);
-    }
-    if (++stage == stages) {
+    if (t == 0 && base + kStreamStages * stride < total) issue(base + kStreamStages * stride, stage);
+    if (++stage == kStreamStages) {
       stage = 0;
       phase ^= 1;
     }
   }
-  if (MODE == kModeAmax) {
-    uint32_t mx = max(acc & 0xFFFFu, acc >> 16);
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-    __shared__ uint32_t warp_max[kRingThreads / 32];
-    if ((t & 31) == 0) warp_max[t >> 5] = mx;
-    __syncthreads();
-    if (t == 0) {
-      for (int wi = 1; wi < kRingThreads / 32; ++wi) mx = max(mx, warp_max[wi]);
-      if (mx) atomicMax(amax_bits_out, mx << 16);
-    }
-  }
+  const uint32_t mx = block_amax<kStreamThreads>(acc, t);
+  if (t == 0 && mx) atomicMax(out_bits, mx << 16);  // the f32 bit pattern of a non-negative bf16 orders like the integer
   if (t == 0 && abort_flag) {  // a wait ran out: give copies still in flight time to land before shared memory is released
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
 }
 
-// Whether the streaming form serves this shape: rows of at least one full chunk, enough chunks to fill the GPU once. Measured on
-// B200 (65536 x 4096, back-to-back launches): the amax pass gains 10 % (96 % of the copy rate) and mxfp8 9 % (90 %); the
-// e2m1 formats are issue-bound rather than load-bound and lose, so they keep the register form.
-static bool use_ring(int mode, int64_t m, int64_t k) {
-  if (mode != TF_FMT_MXFP8 && mode != kModeAmax) return false;
-  const int64_t cpr = ((k >> 4) + kRingChunkVecs - 1) / kRingChunkVecs;
-  return k >= 2048 && m * cpr >= 2 * (int64_t)sm_count();
+// Whether the streaming form serves this tensor: dense, and at least two chunks per SM.
+static bool use_stream(int64_t m, int64_t k, int64_t ldx) {
+  return (ldx == k || m == 1) && m * (k >> 4) >= 2 * (int64_t)sm_count() * kStreamChunkVecs;
 }
 
-struct RingLaunch {
-  unsigned grid;
-  int stages;
-  size_t smem;
-};
-
-// Ring depth and CTAs per SM: stages x 4 KB per CTA, CTAs x that per SM in flight.
-static RingLaunch ring_launch(int mode, int64_t m, int64_t k) {
-  RingLaunch r;
-  r.stages = 4;
-  const int ctas_per_sm = mode == kModeAmax ? 8 : 6;
-  r.smem = (size_t)r.stages * kRingChunkBytes + 8 * (size_t)r.stages;
-  const int64_t cpr = ((k >> 4) + kRingChunkVecs - 1) / kRingChunkVecs;
-  const int64_t total = m * cpr, cap = (int64_t)sm_count() * ctas_per_sm;
-  r.grid = (unsigned)(total < cap ? total : cap);
-  return r;
-}
-
-template <int MODE>
-static cudaError_t ring_configure() {
+static tf_status launch_stream_amax(const char* fn, const void* x, int64_t total, unsigned int* out_bits, cudaStream_t stream) {
+  int* status = device_status_words();
+  if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
   static thread_local int configured_dev = -1;
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (configured_dev == dev) return cudaSuccess;
-  e = cudaFuncSetAttribute(ring_rows_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRingMaxStages * (kRingChunkBytes + 8));
-  if (e != cudaSuccess) return e;
-  // the ring is all these kernels use of the SM's memory: let the carve-out hold as many CTAs' rings as possible
-  e = cudaFuncSetAttribute(ring_rows_kernel<MODE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return e;
-  configured_dev = dev;
-  return cudaSuccess;
+  TF_CUDA(cudaGetDevice(&dev));
+  if (configured_dev != dev) {
+    // the ring is all this kernel uses of the SM's memory: let the carve-out hold as many CTAs' rings as possible
+    TF_CUDA(cudaFuncSetAttribute(stream_amax_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    configured_dev = dev;
+  }
+  const int64_t chunks = (total + kStreamChunkVecs - 1) / kStreamChunkVecs, cap = (int64_t)sm_count() * kStreamCtasPerSm;
+  stream_amax_kernel<<<(unsigned)(chunks < cap ? chunks : cap), kStreamThreads, kStreamSmem, stream>>>(static_cast<const uint8_t*>(x), total, out_bits, status);
+  TF_LAUNCH_CHECK();
+  return TF_OK;
 }
 
 // max |x| over the tensor as the f32 bit pattern of a bf16 magnitude: 256-bit loads, four in flight per thread.
@@ -334,16 +292,6 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   int pad = 0;
   st = scale_padding(scales, FMT, m, k, layout, stream, &pad);
   if (st != TF_OK) return st;
-  if (use_ring(FMT, m, k)) {
-    int* status = device_status_words();
-    if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
-    TF_CUDA(ring_configure<FMT>());
-    const RingLaunch rl = ring_launch(FMT, m, k);
-    TF_CUDA(launch_dependent(chain_rows_launch(m), ring_rows_kernel<FMT>, dim3(rl.grid), dim3(kRingThreads), rl.smem, stream, static_cast<const uint8_t*>(x), m, k, ldx,
-                             static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out,
-                             (unsigned int*)nullptr, status, rl.stages));
-    return TF_OK;
-  }
   int tpr = 2;
   while (tpr < kQuantThreads && tpr * kQuantUnroll < (k >> 4)) tpr <<= 1;
   const int rpb = kQuantThreads / tpr;
@@ -413,14 +361,9 @@ tf_status tf_nvfp4_global_scale(const void* x, int64_t m, int64_t k, int64_t ldx
   TF_CHECK_ALIGNED(x, 32, "x");
   TF_CUDA(cudaMemsetAsync(out, 0, sizeof(float), stream));
   if (m > 0) {
-    if (use_ring(kModeAmax, m, k)) {
-      int* status = device_status_words();
-      if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", __func__);
-      TF_CUDA(ring_configure<kModeAmax>());
-      const RingLaunch rl = ring_launch(kModeAmax, m, k);
-      ring_rows_kernel<kModeAmax><<<rl.grid, kRingThreads, rl.smem, stream>>>(static_cast<const uint8_t*>(x), m, k, ldx, nullptr, nullptr, 0, 0, nullptr, nullptr,
-                                                                              reinterpret_cast<unsigned int*>(out), status, rl.stages);
-      TF_LAUNCH_CHECK();
+    if (use_stream(m, k, ldx)) {
+      const tf_status st = launch_stream_amax(__func__, x, m * (k >> 4), reinterpret_cast<unsigned int*>(out), stream);
+      if (st != TF_OK) return st;
       finalize_global_scale_kernel<<<1, 1, 0, stream>>>(out);
       TF_LAUNCH_CHECK();
       return TF_OK;
