@@ -93,6 +93,14 @@ TF_API tf_status tf_selftest_bounded_wait(int32_t limit_ms, void* stream);
 /* Bytes of the scale tensor of a [rows, k] operand in `format`, in `layout`. Returns -1 on a bad argument. */
 TF_API int64_t tf_scale_bytes(int32_t format, int64_t rows, int64_t k, int32_t layout);
 
+/* nvfp4 from the tensor alone: an amax launch, then the quantizer, which derives the scale. The bytes of
+ * tf_nvfp4_global_scale followed by tf_quantize_nvfp4.
+ *   global_scale_out   f32 [1], receives max|x| / 2688
+ *   scratch            tf_quantize_nvfp4_dynamic_scratch_bytes() bytes, 4-byte aligned, whose content does not matter */
+TF_API int64_t tf_quantize_nvfp4_dynamic_scratch_bytes(void);
+TF_API tf_status tf_quantize_nvfp4_dynamic(const void* x, int64_t m, int64_t k, int64_t ldx, void* codes, void* scales, int32_t layout,
+                                           float* global_scale_out, float* scratch, void* stream);
+
 /* BlockScaled quantization of a bf16 matrix along its last axis. The reference types this operation but refuses to run
  * it (python/src/tilefish/ops.py:556-559); these entry points are what `x.to(mxfp8)` lowers to here.
  *   x        bf16 [m, k], row stride ldx elements (ldx >= k, ldx % 16 == 0), 32-byte aligned (256-bit loads)

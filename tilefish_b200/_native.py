@@ -42,6 +42,8 @@ SIGNATURES = {
     "tf_quantize_mxfp4": (c_int32, [_P, c_int64, c_int64, c_int64, _P, _P, c_int32, _P]),
     "tf_quantize_nvfp4": (c_int32, [_P, c_int64, c_int64, c_int64, _P, _P, c_int32, _P, _P]),
     "tf_quantize_nvfp4_from_amax": (c_int32, [_P, c_int64, c_int64, c_int64, _P, _P, c_int32, _P, _P, _P]),
+    "tf_quantize_nvfp4_dynamic_scratch_bytes": (c_int64, []),
+    "tf_quantize_nvfp4_dynamic": (c_int32, [_P, c_int64, c_int64, c_int64, _P, _P, c_int32, _P, _P, _P]),
     "tf_nvfp4_global_scale": (c_int32, [_P, c_int64, c_int64, c_int64, _P, _P]),
     "tf_swizzle_scales": (c_int32, [_P, c_int64, c_int64, _P, _P]),
     "tf_unswizzle_scales": (c_int32, [_P, c_int64, c_int64, _P, _P]),

@@ -22,61 +22,97 @@ __device__ __forceinline__ void load_256(const void* p, uint32_t (&w)[8]) {
                : "l"(p));
 }
 
-// gs_ptr holds the nvfp4 global scale, or (gs_out != nullptr) the tensor's amax from which it is derived here.
+// One round of a row: vectors base + threadIdx.x + j * blockDim.x, kQuantUnroll 256-bit loads in flight per thread. Threads without
+// data (no such row, or past its end) get zeros.
+__device__ __forceinline__ void load_round(const uint8_t* __restrict__ xr, bool row_ok, int base, int nvec, uint32_t (&v)[kQuantUnroll][8],
+                                           bool (&has)[kQuantUnroll]) {
+#pragma unroll
+  for (int j = 0; j < kQuantUnroll; ++j) {
+    const int vj = base + threadIdx.x + j * (int)blockDim.x;
+    has[j] = row_ok && vj < nvec;
+    if (has[j]) {
+      load_256(xr + (int64_t)vj * 32, v[j]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[j][e] = 0;
+    }
+  }
+}
+
+// Quantizes and stores one round. All threads of the block call it with the same `base`, so the warp shuffle inside quantize_vec16
+// always sees whole warps; threads without data quantize zeros and store nothing. nvec is even and blockDim.x a power of two >= 2,
+// so the two lanes of one 32-element block have data together.
+template <int FMT>
+__device__ __forceinline__ void store_round(const uint32_t (&v)[kQuantUnroll][8], const bool (&has)[kQuantUnroll], int64_t row, int base, int nvec,
+                                            int64_t k, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int swizzled, float gs, float inv_t) {
+#pragma unroll
+  for (int j = 0; j < kQuantUnroll; ++j) {
+    if (base + j * (int)blockDim.x < nvec) {  // uniform over the block
+      uint32_t c[4], sc;
+      quantize_vec16<FMT>(v[j], gs, inv_t, c, sc);
+      if (has[j]) store_quantized16<FMT>(codes, scales, swizzled, row, base + threadIdx.x + j * (int)blockDim.x, k, c, sc);
+    }
+  }
+}
+
+// gridDim.y cuts the rows into segments of whole rounds (few, long rows: more CTAs than row blocks). The segment of this block.
+__device__ __forceinline__ void row_segment(int nvec, int& begin, int& end) {
+  const int step = kQuantUnroll * (int)blockDim.x;
+  const int rounds = (nvec + step - 1) / step;
+  const int per_seg = (rounds + (int)gridDim.y - 1) / (int)gridDim.y;
+  begin = (int)blockIdx.y * per_seg * step;
+  end = min(nvec, begin + per_seg * step);
+}
+
+// gs_ptr holds the nvfp4 global scale, or (gs_out != nullptr) the tensor's amax from which it is derived here: one value, or the
+// `n_partials` maxima that the blocks of an amax launch left (every block of this kernel takes their maximum again: at most 1024 words).
 // One thread = 16 consecutive bf16 (one 256-bit load); block = (TPR threads along the row) x (256 / TPR rows).
 template <int FMT>
 __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint8_t* __restrict__ x, int64_t m, int64_t k, int64_t ldx,
                                                                       uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
-                                                                      int swizzled, int pad, const float* __restrict__ gs_ptr, float* __restrict__ gs_out) {
-  const int tpr = blockDim.x;
+                                                                      int swizzled, int pad, const float* __restrict__ gs_ptr, float* __restrict__ gs_out,
+                                                                      int n_partials, int backwards) {
   const int nvec = (int)(k >> 4);
   griddep_launch_dependents();
   griddep_wait();
   if (pad)
     zero_scale_padding(scales, m, k / (FMT == TF_FMT_NVFP4 ? 16 : 32),
-                       ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuantThreads + threadIdx.y * tpr + threadIdx.x,
+                       ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuantThreads + threadIdx.y * blockDim.x + threadIdx.x,
                        (int64_t)gridDim.x * gridDim.y * kQuantThreads);
-  float gs = (FMT == TF_FMT_NVFP4) ? __ldg(gs_ptr) : 0.0f;
+  float gs = 0.0f;
+  if (FMT == TF_FMT_NVFP4 && n_partials > 0) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    uint32_t mx = 0;  // non-negative floats order like their bits
+    for (int i = tid; i < n_partials; i += kQuantThreads) mx = max(mx, __float_as_uint(__ldg(gs_ptr + i)));
+    __shared__ uint32_t warp_max[kQuantThreads / 32];
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kQuantThreads / 32; ++i) mx = max(mx, warp_max[i]);
+    gs = __uint_as_float(mx);
+  } else if (FMT == TF_FMT_NVFP4) {
+    gs = __ldg(gs_ptr);
+  }
   if (FMT == TF_FMT_NVFP4 && gs_out != nullptr) {
     gs = __fdiv_rn(gs, 2688.0f);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) gs_out[0] = gs;
   }
   const float inv_t = (FMT == TF_FMT_NVFP4 && gs != 0.0f) ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
   const int64_t row_stride = (int64_t)gridDim.x * blockDim.y;
-  // Both loops run the same number of times for every thread of the block, so the warp shuffle inside quantize_vec16 always
-  // sees whole warps; threads without data (row >= m or vector >= nvec) quantize zeros and store nothing. nvec is even and
-  // tpr a power of two >= 2, so the two lanes of one 32-element block have data together.
-  for (int64_t row_base = (int64_t)blockIdx.x * blockDim.y; row_base < m; row_base += row_stride) {
-    const int64_t row = row_base + threadIdx.y;
+  int begin, end;
+  row_segment(nvec, begin, end);
+  // backwards: the last rows first, which the amax launch in front read last and left in L2
+  const int64_t last = (m - 1) / blockDim.y * blockDim.y;
+  for (int64_t row_it = (int64_t)blockIdx.x * blockDim.y; row_it < m; row_it += row_stride) {
+    const int64_t row = (backwards ? last - row_it : row_it) + threadIdx.y;
     const bool row_ok = row < m;
     const uint8_t* xr = x + (row_ok ? row : 0) * ldx * 2;
-    // gridDim.y cuts the row into segments of whole rounds (few, long rows: more CTAs than row blocks)
-    const int rounds = (nvec + kQuantUnroll * tpr - 1) / (kQuantUnroll * tpr);
-    const int rounds_per_seg = (rounds + (int)gridDim.y - 1) / (int)gridDim.y;
-    const int base_begin = (int)blockIdx.y * rounds_per_seg * kQuantUnroll * tpr;
-    const int base_end = min(nvec, base_begin + rounds_per_seg * kQuantUnroll * tpr);
-    for (int base = base_begin; base < base_end; base += kQuantUnroll * tpr) {  // kQuantUnroll 256-bit loads in flight per thread
+    for (int base = begin; base < end; base += kQuantUnroll * (int)blockDim.x) {
       uint32_t v[kQuantUnroll][8];
       bool has[kQuantUnroll];
-#pragma unroll
-      for (int j = 0; j < kQuantUnroll; ++j) {
-        const int vj = base + threadIdx.x + j * tpr;
-        has[j] = row_ok && vj < nvec;
-        if (has[j]) {
-          load_256(xr + (int64_t)vj * 32, v[j]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[j][e] = 0;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kQuantUnroll; ++j) {
-        if (base + j * tpr < nvec) {  // uniform over the block
-          uint32_t c[4], sc;
-          quantize_vec16<FMT>(v[j], gs, inv_t, c, sc);
-          if (has[j]) store_quantized16<FMT>(codes, scales, swizzled, row, base + threadIdx.x + j * tpr, k, c, sc);
-        }
-      }
+      load_round(xr, row_ok, base, nvec, v, has);
+      store_round<FMT>(v, has, row, base, nvec, k, codes, scales, swizzled, gs, inv_t);
     }
   }
 }
@@ -123,8 +159,10 @@ __device__ __forceinline__ uint32_t block_amax(uint32_t acc, int tid) {
 }
 
 // Dynamic shared memory: kStreamStages chunk buffers, then one mbarrier per stage. total: 16-element vectors of the tensor.
+// The maximum goes to *out_bits (an atomic max), or as this block's own word to partials[blockIdx.x].
 __global__ void __launch_bounds__(kStreamThreads) stream_amax_kernel(const uint8_t* __restrict__ x, int64_t total, unsigned int* __restrict__ out_bits,
-                                                                     int* __restrict__ status) {
+                                                                     unsigned int* __restrict__ partials, int* __restrict__ status) {
+  griddep_launch_dependents();
   extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ int abort_flag;
   const uint32_t ring = smem_u32(ring_smem);
@@ -171,7 +209,8 @@ __global__ void __launch_bounds__(kStreamThreads) stream_amax_kernel(const uint8
     }
   }
   const uint32_t mx = block_amax<kStreamThreads>(acc, t);
-  if (t == 0 && mx) atomicMax(out_bits, mx << 16);  // the f32 bit pattern of a non-negative bf16 orders like the integer
+  if (t == 0 && partials) partials[blockIdx.x] = mx << 16;
+  else if (t == 0 && mx) atomicMax(out_bits, mx << 16);  // the f32 bit pattern of a non-negative bf16 orders like the integer
   if (t == 0 && abort_flag) {  // a wait ran out: give copies still in flight time to land before shared memory is released
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -183,27 +222,10 @@ static bool use_stream(int64_t m, int64_t k, int64_t ldx) {
   return (ldx == k || m == 1) && m * (k >> 4) >= 2 * (int64_t)sm_count() * kStreamChunkVecs;
 }
 
-static tf_status launch_stream_amax(const char* fn, const void* x, int64_t total, unsigned int* out_bits, cudaStream_t stream) {
-  int* status = device_status_words();
-  if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
-  static thread_local int configured_dev = -1;
-  int dev = 0;
-  TF_CUDA(cudaGetDevice(&dev));
-  if (configured_dev != dev) {
-    // the ring is all this kernel uses of the SM's memory: let the carve-out hold as many CTAs' rings as possible
-    TF_CUDA(cudaFuncSetAttribute(stream_amax_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    configured_dev = dev;
-  }
-  const int64_t chunks = (total + kStreamChunkVecs - 1) / kStreamChunkVecs, cap = (int64_t)sm_count() * kStreamCtasPerSm;
-  stream_amax_kernel<<<(unsigned)(chunks < cap ? chunks : cap), kStreamThreads, kStreamSmem, stream>>>(static_cast<const uint8_t*>(x), total, out_bits, status);
-  TF_LAUNCH_CHECK();
-  return TF_OK;
-}
-
 // max |x| over the tensor as the f32 bit pattern of a bf16 magnitude: 256-bit loads, four in flight per thread.
 __global__ void __launch_bounds__(256) amax_bits_kernel(const uint8_t* __restrict__ x, int64_t m, int nvec, int64_t ldx,
-                                                        unsigned int* __restrict__ out_bits) {
-  const uint32_t k = 0x7FFF7FFFu;
+                                                        unsigned int* __restrict__ out_bits, unsigned int* __restrict__ partials) {
+  griddep_launch_dependents();
   uint32_t acc = 0;  // two packed 16-bit maxima
   const int64_t total = m * nvec;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -226,22 +248,47 @@ __global__ void __launch_bounds__(256) amax_bits_kernel(const uint8_t* __restric
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t t0 = __vimax3_u16x2(v[j][0] & k, v[j][1] & k, v[j][2] & k);
-      uint32_t t1 = __vimax3_u16x2(v[j][3] & k, v[j][4] & k, v[j][5] & k);
-      t0 = __vimax3_u16x2(t0, v[j][6] & k, v[j][7] & k);
-      acc = __vimax3_u16x2(acc, t0, t1);
+    for (int j = 0; j < 4; ++j) acc = amax16(v[j], acc);
+  }
+  const uint32_t mx = block_amax<256>(acc, threadIdx.x);
+  if (threadIdx.x == 0 && partials) partials[blockIdx.x] = mx << 16;
+  else if (threadIdx.x == 0 && mx) atomicMax(out_bits, mx << 16);
+}
+
+// nvfp4 without a given scale is two launches: an amax launch whose blocks leave their maxima, and the quantizer, which derives the scale
+// from them. Before: a memset, an amax launch with an atomic, a one-thread launch for the scale and the quantizer. Graphs of 12: 128 x
+// 4096 10.5 -> 5.7 us, 4096 x 2560 20.6 -> 14.1, 8192 x 4096 35.1 -> 30.0, 65536 x 4096 212 -> 194. One cooperative launch with a grid
+// barrier in place of the two took 10.5 us at 128 x 4096 and 201 at 65536 x 4096 (such launches start late).
+constexpr int kMaxAmaxBlocks = 1024;  // blocks of an amax launch, and words of its partial maxima
+
+// The amax launch: into *out_bits (zeroed by the caller), or a word per block into `partials`, whose number goes to *blocks.
+static tf_status launch_amax(const char* fn, const void* x, int64_t m, int64_t k, int64_t ldx, unsigned int* out_bits, unsigned int* partials, int* blocks,
+                             cudaStream_t stream) {
+  const uint8_t* xb = static_cast<const uint8_t*>(x);
+  const int64_t total = m * (k >> 4);
+  if (use_stream(m, k, ldx)) {
+    int* status = device_status_words();
+    if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
+    static thread_local int configured_dev = -1;
+    int dev = 0;
+    TF_CUDA(cudaGetDevice(&dev));
+    if (configured_dev != dev) {
+      // the ring is all this kernel uses of the SM's memory: let the carve-out hold as many CTAs' rings as possible
+      TF_CUDA(cudaFuncSetAttribute(stream_amax_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+      configured_dev = dev;
     }
+    const int64_t chunks = (total + kStreamChunkVecs - 1) / kStreamChunkVecs;
+    int64_t cap = (int64_t)sm_count() * kStreamCtasPerSm;
+    if (cap > kMaxAmaxBlocks) cap = kMaxAmaxBlocks;
+    *blocks = (int)(chunks < cap ? chunks : cap);
+    stream_amax_kernel<<<*blocks, kStreamThreads, kStreamSmem, stream>>>(xb, total, out_bits, partials, status);
+  } else {
+    const int64_t need = (total + 1023) / 1024;
+    *blocks = (int)(need < kMaxAmaxBlocks ? need : kMaxAmaxBlocks);
+    amax_bits_kernel<<<*blocks, 256, 0, stream>>>(xb, m, (int)(k >> 4), ldx, out_bits, partials);
   }
-  uint32_t mx = max(acc & 0xFFFFu, acc >> 16);
-  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-  __shared__ uint32_t warp_max[8];
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) mx = max(mx, warp_max[w]);
-    if (mx) atomicMax(out_bits, mx << 16);  // the f32 bit pattern of a non-negative bf16 orders like the integer
-  }
+  TF_LAUNCH_CHECK();
+  return TF_OK;
 }
 
 __global__ void finalize_global_scale_kernel(float* gs) { gs[0] = __fdiv_rn(gs[0], 2688.0f); }
@@ -282,9 +329,26 @@ static tf_status check_quant_args(const char* fn, const void* x, int64_t m, int6
   return TF_OK;
 }
 
+// Block and grid of the register form: a power of two of threads along the row, at most `per_sm` blocks per SM.
+static void quantize_shape(int64_t m, int64_t k, int pad, int per_sm, dim3& grid, dim3& block) {
+  int tpr = 2;
+  while (tpr < kQuantThreads && tpr * kQuantUnroll < (k >> 4)) tpr <<= 1;
+  const int rpb = kQuantThreads / tpr;
+  const int64_t blocks_needed = (m + rpb - 1) / rpb, cap = (int64_t)sm_count() * per_sm;
+  block = dim3(tpr, rpb);
+  grid = dim3((unsigned)(blocks_needed < cap ? blocks_needed : cap));
+  const int64_t rounds = ((k >> 4) + kQuantUnroll * tpr - 1) / (kQuantUnroll * tpr);
+  if (blocks_needed < 2 * sm_count() && rounds > 1) {  // few long rows: cut them into segments so that every SM gets work
+    int64_t want = (2 * sm_count() + blocks_needed - 1) / blocks_needed;
+    if (want * blocks_needed > cap) want = cap / blocks_needed;
+    grid.y = (unsigned)(want < 1 ? 1 : want < rounds ? want : rounds);
+  }
+  if (pad && grid.x * grid.y < kPadBlocks) grid.x = kPadBlocks;
+}
+
 template <int FMT>
 static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64_t k, int64_t ldx, void* codes, void* scales, int layout,
-                                 const float* gs, cudaStream_t stream, float* gs_out = nullptr) {
+                                 const float* gs, cudaStream_t stream, float* gs_out = nullptr, int n_partials = 0) {
   tf_status st = check_quant_args(fn, x, m, k, ldx, codes, scales, layout);
   if (st != TF_OK) return st;
   if (FMT == TF_FMT_NVFP4 && !gs) return fail(TF_ERR_INVALID_ARGUMENT, "%s: nvfp4 needs a global scale", fn);
@@ -292,21 +356,13 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   int pad = 0;
   st = scale_padding(scales, FMT, m, k, layout, stream, &pad);
   if (st != TF_OK) return st;
-  int tpr = 2;
-  while (tpr < kQuantThreads && tpr * kQuantUnroll < (k >> 4)) tpr <<= 1;
-  const int rpb = kQuantThreads / tpr;
-  const int64_t blocks_needed = (m + rpb - 1) / rpb;
-  const int64_t cap = (int64_t)sm_count() * 8;
-  dim3 block(tpr, rpb);
-  dim3 grid((unsigned)(blocks_needed < cap ? blocks_needed : cap));
-  const int64_t rounds = ((k >> 4) + kQuantUnroll * tpr - 1) / (kQuantUnroll * tpr);
-  if (blocks_needed < 2 * sm_count() && rounds > 1) {  // few long rows: cut them into segments so that every SM gets work
-    const int64_t want = (2 * sm_count() + blocks_needed - 1) / blocks_needed;
-    grid.y = (unsigned)(want < rounds ? want : rounds);
-  }
-  if (pad && grid.x * grid.y < kPadBlocks) grid.x = kPadBlocks;
-  TF_CUDA(launch_dependent(chain_rows_launch(m), quantize_rows_kernel<FMT>, grid, block, 0, stream, static_cast<const uint8_t*>(x), m, k, ldx, static_cast<uint8_t*>(codes),
-                           static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out));
+  dim3 grid, block;
+  quantize_shape(m, k, pad, 8, grid, block);
+  // After its own amax launch (n_partials > 0) a quantizer of at most 16 M elements starts as that launch's dependent (128 x 4096 6.3 ->
+  // 5.7 us, 4096 x 2560 14.4 -> 14.1); beyond that its waiting blocks cost the amax launch more (8192 x 4096 30.0 -> 31.6 us).
+  TF_CUDA(launch_dependent((n_partials > 0 && m * k <= (int64_t)1 << 24) || chain_rows_launch(m), quantize_rows_kernel<FMT>, grid, block, 0, stream, static_cast<const uint8_t*>(x), m, k,
+                           ldx, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out,
+                           n_partials, (int)(n_partials > 0)));
   return TF_OK;
 }
 
@@ -353,6 +409,27 @@ tf_status tf_quantize_nvfp4_from_amax(const void* x, int64_t m, int64_t k, int64
   return launch_quantize<TF_FMT_NVFP4>(__func__, x, m, k, ldx, codes, scales, layout, amax, (cudaStream_t)stream, global_scale_out);
 }
 
+int64_t tf_quantize_nvfp4_dynamic_scratch_bytes(void) { return kMaxAmaxBlocks * (int64_t)sizeof(float); }
+
+tf_status tf_quantize_nvfp4_dynamic(const void* x, int64_t m, int64_t k, int64_t ldx, void* codes, void* scales, int32_t layout,
+                                    float* global_scale_out, float* scratch, void* stream_) {
+  clear_error();
+  cudaStream_t stream = (cudaStream_t)stream_;
+  TF_CHECK_ARG(global_scale_out && scratch, "%s: null pointer", __func__);
+  TF_CHECK_ALIGNED(global_scale_out, 4, "global_scale_out");
+  TF_CHECK_ALIGNED(scratch, 4, "scratch");
+  tf_status st = check_quant_args(__func__, x, m, k, ldx, codes, scales, layout);
+  if (st != TF_OK) return st;
+  if (m == 0) {
+    TF_CUDA(cudaMemsetAsync(global_scale_out, 0, sizeof(float), stream));
+    return TF_OK;
+  }
+  int blocks = 0;
+  st = launch_amax(__func__, x, m, k, ldx, nullptr, reinterpret_cast<unsigned int*>(scratch), &blocks, stream);
+  if (st != TF_OK) return st;
+  return launch_quantize<TF_FMT_NVFP4>(__func__, x, m, k, ldx, codes, scales, layout, scratch, stream, global_scale_out, blocks);
+}
+
 tf_status tf_nvfp4_global_scale(const void* x, int64_t m, int64_t k, int64_t ldx, float* out, void* stream_) {
   clear_error();
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -361,18 +438,9 @@ tf_status tf_nvfp4_global_scale(const void* x, int64_t m, int64_t k, int64_t ldx
   TF_CHECK_ALIGNED(x, 32, "x");
   TF_CUDA(cudaMemsetAsync(out, 0, sizeof(float), stream));
   if (m > 0) {
-    if (use_stream(m, k, ldx)) {
-      const tf_status st = launch_stream_amax(__func__, x, m * (k >> 4), reinterpret_cast<unsigned int*>(out), stream);
-      if (st != TF_OK) return st;
-      finalize_global_scale_kernel<<<1, 1, 0, stream>>>(out);
-      TF_LAUNCH_CHECK();
-      return TF_OK;
-    }
-    const int64_t total = m * (k >> 4);
-    const int64_t need = (total + 1023) / 1024, cap = (int64_t)sm_count() * 8;
-    amax_bits_kernel<<<(unsigned)(need < cap ? need : cap), 256, 0, stream>>>(static_cast<const uint8_t*>(x), m, (int)(k >> 4), ldx,
-                                                                              reinterpret_cast<unsigned int*>(out));
-    TF_LAUNCH_CHECK();
+    int blocks = 0;
+    const tf_status st = launch_amax(__func__, x, m, k, ldx, reinterpret_cast<unsigned int*>(out), nullptr, &blocks, stream);
+    if (st != TF_OK) return st;
   }
   finalize_global_scale_kernel<<<1, 1, 0, stream>>>(out);
   TF_LAUNCH_CHECK();

@@ -161,13 +161,16 @@ def quantize(x, fmt: str, *, layout: str = "swizzled", global_scale=None, amax=N
         gs = out.global_scale if out is not None and out.global_scale is not None else torch.empty(1, dtype=torch.float32, device=x.device)
         N.check(lib.tf_quantize_nvfp4_from_amax(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, amax.data_ptr(), gs.data_ptr(), s),
                 "tf_quantize_nvfp4_from_amax")
+    elif fmt == "nvfp4" and global_scale is None:
+        _pre(x.stride(0) % 16 == 0, "x: rows must be dense, K and the row stride multiples of 16", "contiguous", "x")
+        gs = out.global_scale if out is not None and out.global_scale is not None else torch.empty(1, dtype=torch.float32, device=x.device)
+        scratch = torch.empty(lib.tf_quantize_nvfp4_dynamic_scratch_bytes(), dtype=torch.uint8, device=x.device)
+        N.check(lib.tf_quantize_nvfp4_dynamic(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), scratch.data_ptr(), s),
+                "tf_quantize_nvfp4_dynamic")
     elif fmt == "nvfp4":
-        if global_scale is None:
-            gs = nvfp4_global_scale(x, out=out.global_scale if out is not None else None, stream=stream)
-        else:
-            _check(global_scale, "global_scale", torch.float32, None, x.device, align=4)
-            _pre(global_scale.numel() == 1, "global_scale: expected one element", "shape", "global_scale")
-            gs = global_scale
+        _check(global_scale, "global_scale", torch.float32, None, x.device, align=4)
+        _pre(global_scale.numel() == 1, "global_scale: expected one element", "shape", "global_scale")
+        gs = global_scale
         N.check(lib.tf_quantize_nvfp4(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), s), "tf_quantize_nvfp4")
     elif fmt == "mxfp8":
         N.check(lib.tf_quantize_mxfp8(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, s), "tf_quantize_mxfp8")
