@@ -20,10 +20,21 @@ ELEMS_PER_BYTE = {"mxfp8": 1, "mxfp4": 2, "nvfp4": 2}
 EPILOGUES = {"none": N.EPI_NONE, "silu_gate": N.EPI_SILU_GATE, "residual": N.EPI_RESIDUAL}
 
 
-def _torch():
-    import torch
+_torch_module = None
 
-    return torch
+
+def _torch():
+    global _torch_module
+    if _torch_module is None:
+        import torch
+
+        _torch_module = torch
+    return _torch_module
+
+
+# The checks below run on every call, in front of launches that take a few microseconds: a check that holds must not format its message.
+# Eager messages (an f-string with a dtype, a device or strides for every check) were most of a call: ``gemm`` of 16 bf16 mxfp8 rows took
+# 63 us per call, 11 of them on the device; with lazy ones 30.
 
 
 def _pre(cond: bool, msg: str, kind: str, arg: Optional[str] = None) -> None:
@@ -32,6 +43,13 @@ def _pre(cond: bool, msg: str, kind: str, arg: Optional[str] = None) -> None:
 
 
 def _check(t, name: str, dtype, rank: Optional[int] = None, device=None, align: int = 16) -> None:
+    if (isinstance(t, _torch().Tensor) and t.is_cuda and t.dtype == dtype and (rank is None or t.dim() == rank) and (device is None or t.device == device)
+            and (t.data_ptr() % align == 0 or t.numel() == 0)):
+        return
+    _check_failed(t, name, dtype, rank, device, align)
+
+
+def _check_failed(t, name: str, dtype, rank: Optional[int], device, align: int) -> None:
     torch = _torch()
     _pre(isinstance(t, torch.Tensor), f"{name}: expected a torch tensor, got {type(t).__name__}", "dtype", name)
     _pre(t.is_cuda, f"{name}: the tensor is on {t.device}; this backend runs on CUDA only (no CPU fallback)", "device", name)
@@ -44,7 +62,8 @@ def _check(t, name: str, dtype, rank: Optional[int] = None, device=None, align: 
 
 
 def _dense(t, name: str) -> None:
-    _pre(t.is_contiguous(), f"{name}: must be contiguous (strides {tuple(t.stride())})", "contiguous", name)
+    if not t.is_contiguous():
+        _pre(False, f"{name}: must be contiguous (strides {tuple(t.stride())})", "contiguous", name)
 
 
 def _stream(stream) -> int:
@@ -53,7 +72,7 @@ def _stream(stream) -> int:
     ``stream=`` that is not the current one is refused unless it is a ``torch.cuda.Stream`` the caller made current
     (``with torch.cuda.stream(s): ...``) or the caller passes every output and workspace itself."""
     torch = _torch()
-    current = torch.cuda.current_stream().cuda_stream
+    current = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # torch.cuda.current_stream().cuda_stream without the object
     if stream is None:
         return current
     handle = getattr(stream, "cuda_stream", stream)
@@ -77,7 +96,7 @@ class BlockScaledTensor:
         if fmt not in FORMATS:
             raise TilefishPreconditionError(f"unknown block-scaled format {fmt!r}", kind="dtype")
         self.fmt = fmt
-        self.shape = tuple(int(s) for s in shape)
+        self.shape = (int(shape[0]), int(shape[1])) if len(shape) == 2 else tuple(int(s) for s in shape)
         self.codes = codes
         self.scales = scales
         self.global_scale = global_scale
@@ -108,6 +127,11 @@ class BlockScaledTensor:
         return f"BlockScaledTensor({self.fmt}, shape={self.shape}, scales={self.layout})"
 
 
+def _swizzled_bytes(fmt: str, rows: int, k: int) -> int:
+    """``scale_bytes`` of a shape that was checked already: whole tiles of 128 rows x 4 columns."""
+    return -(-rows // 128) * -(-k // (4 * BLOCK[fmt])) * 512
+
+
 def scale_bytes(fmt: str, rows: int, k: int, layout: str = "swizzled") -> int:
     return N.scale_bytes(FORMATS[fmt], rows, k, N.SCALES_SWIZZLED if layout == "swizzled" else N.SCALES_PLAIN)
 
@@ -133,21 +157,27 @@ def quantize(x, fmt: str, *, layout: str = "swizzled", global_scale=None, amax=N
     from ``amax`` (float32 [1] holding max|x|, e.g. the ``amax_out`` of the producing kernel), or computed by an extra pass.
     """
     torch = _torch()
-    _pre(fmt in FORMATS, f"unknown block-scaled format {fmt!r}", "dtype", "fmt")
-    _pre(layout in ("swizzled", "plain"), f"unknown scale layout {layout!r}", "argument", "layout")
+    if fmt not in FORMATS:
+        _pre(False, f"unknown block-scaled format {fmt!r}", "dtype", "fmt")
+    if layout != "swizzled" and layout != "plain":
+        _pre(False, f"unknown scale layout {layout!r}", "argument", "layout")
     _check(x, "x", torch.bfloat16, 2)
     m, k = x.shape
-    _pre(x.stride(1) == 1 and (m <= 1 or (x.stride(0) >= k and x.stride(0) % 16 == 0)), "x: rows must be dense with a row stride that is a multiple of 16", "contiguous", "x")
-    _pre(k % 32 == 0 and k > 0, f"x: K={k} is not a multiple of 32", "divisible", "x")
-    _pre(m == 0 or x.data_ptr() % 32 == 0, "x: the data pointer is not 32-byte aligned (the quantizer uses 256-bit loads)", "pointer_alignment", "x")
-    ldx = x.stride(0) if m > 1 else k
+    ld, inner = x.stride()
+    _pre(inner == 1 and (m <= 1 or (ld >= k and ld % 16 == 0)), "x: rows must be dense with a row stride that is a multiple of 16", "contiguous", "x")
+    if k % 32 != 0 or k <= 0:
+        _pre(False, f"x: K={k} is not a multiple of 32", "divisible", "x")
+    xp = x.data_ptr()
+    _pre(m == 0 or xp % 32 == 0, "x: the data pointer is not 32-byte aligned (the quantizer uses 256-bit loads)", "pointer_alignment", "x")
+    ldx = ld if m > 1 else k
     lay = N.SCALES_SWIZZLED if layout == "swizzled" else N.SCALES_PLAIN
     if out is not None:  # preallocated result (a plan's arena): same format, shape and layout
-        _pre(out.fmt == fmt and out.shape == (m, k) and out.layout == layout, f"out: expected a {fmt} {layout} tensor of shape {(m, k)}", "shape", "out")
+        if out.fmt != fmt or out.shape != (m, k) or out.layout != layout:
+            _pre(False, f"out: expected a {fmt} {layout} tensor of shape {(m, k)}", "shape", "out")
         codes, scales = out.codes, out.scales
     else:
         codes = torch.empty((m, k // ELEMS_PER_BYTE[fmt]), dtype=torch.uint8, device=x.device)
-        scales = torch.empty(N.scale_bytes(FORMATS[fmt], m, k, lay), dtype=torch.uint8, device=x.device)
+        scales = torch.empty(_swizzled_bytes(fmt, m, k) if layout == "swizzled" else m * (k // BLOCK[fmt]), dtype=torch.uint8, device=x.device)
     s = _stream(stream)
     lib = N.load()
     gs = None
@@ -159,23 +189,23 @@ def quantize(x, fmt: str, *, layout: str = "swizzled", global_scale=None, amax=N
         _check(amax, "amax", torch.float32, None, x.device, align=4)
         _pre(amax.numel() == 1 and global_scale is None, "amax: expected one element and no global_scale", "shape", "amax")
         gs = out.global_scale if out is not None and out.global_scale is not None else torch.empty(1, dtype=torch.float32, device=x.device)
-        N.check(lib.tf_quantize_nvfp4_from_amax(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, amax.data_ptr(), gs.data_ptr(), s),
+        N.check(lib.tf_quantize_nvfp4_from_amax(xp, m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, amax.data_ptr(), gs.data_ptr(), s),
                 "tf_quantize_nvfp4_from_amax")
     elif fmt == "nvfp4" and global_scale is None:
-        _pre(x.stride(0) % 16 == 0, "x: rows must be dense, K and the row stride multiples of 16", "contiguous", "x")
+        _pre(ld % 16 == 0, "x: rows must be dense, K and the row stride multiples of 16", "contiguous", "x")
         gs = out.global_scale if out is not None and out.global_scale is not None else torch.empty(1, dtype=torch.float32, device=x.device)
         scratch = torch.empty(lib.tf_quantize_nvfp4_dynamic_scratch_bytes(), dtype=torch.uint8, device=x.device)
-        N.check(lib.tf_quantize_nvfp4_dynamic(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), scratch.data_ptr(), s),
+        N.check(lib.tf_quantize_nvfp4_dynamic(xp, m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), scratch.data_ptr(), s),
                 "tf_quantize_nvfp4_dynamic")
     elif fmt == "nvfp4":
         _check(global_scale, "global_scale", torch.float32, None, x.device, align=4)
         _pre(global_scale.numel() == 1, "global_scale: expected one element", "shape", "global_scale")
         gs = global_scale
-        N.check(lib.tf_quantize_nvfp4(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), s), "tf_quantize_nvfp4")
+        N.check(lib.tf_quantize_nvfp4(xp, m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), s), "tf_quantize_nvfp4")
     elif fmt == "mxfp8":
-        N.check(lib.tf_quantize_mxfp8(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, s), "tf_quantize_mxfp8")
+        N.check(lib.tf_quantize_mxfp8(xp, m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, s), "tf_quantize_mxfp8")
     else:
-        N.check(lib.tf_quantize_mxfp4(x.data_ptr(), m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, s), "tf_quantize_mxfp4")
+        N.check(lib.tf_quantize_mxfp4(xp, m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, s), "tf_quantize_mxfp4")
     return BlockScaledTensor(fmt, (m, k), codes, scales, gs, layout)
 
 
@@ -213,9 +243,12 @@ def residual_add_rmsnorm(x, residual, w, eps: float = 1e-6, *, out=None, quantiz
     for t, n in ((x, "x"), (residual, "residual"), (w, "w")):
         _dense(t, n)
     m, d = x.shape
-    _pre(tuple(residual.shape) == (m, d), f"residual: shape {tuple(residual.shape)}, expected {(m, d)}", "shape", "residual")
-    _pre(tuple(w.shape) == (d,), f"w: shape {tuple(w.shape)}, expected {(d,)}", "shape", "w")
-    _pre(d % 8 == 0, f"x: D={d} is not a multiple of 8", "divisible", "x")
+    if residual.shape != x.shape:
+        _pre(False, f"residual: shape {tuple(residual.shape)}, expected {(m, d)}", "shape", "residual")
+    if w.shape[0] != d:
+        _pre(False, f"w: shape {tuple(w.shape)}, expected {(d,)}", "shape", "w")
+    if d % 8 != 0:
+        _pre(False, f"x: D={d} is not a multiple of 8", "divisible", "x")
     if want_bf16:
         if out is None:
             out = torch.empty((m, d), dtype=torch.bfloat16, device=x.device)
@@ -238,7 +271,7 @@ def residual_add_rmsnorm(x, residual, w, eps: float = 1e-6, *, out=None, quantiz
             codes, scales = q_out.codes, q_out.scales
         else:
             codes = torch.empty((m, d // ELEMS_PER_BYTE[quantize_to]), dtype=torch.uint8, device=x.device)
-            scales = torch.empty(N.scale_bytes(qfmt, m, d, N.SCALES_SWIZZLED), dtype=torch.uint8, device=x.device)
+            scales = torch.empty(_swizzled_bytes(quantize_to, m, d), dtype=torch.uint8, device=x.device)
         if quantize_to == "nvfp4":
             _pre(q_global_scale is not None, "nvfp4 output needs q_global_scale (a float32 [1] device tensor)", "argument", "q_global_scale")
             _check(q_global_scale, "q_global_scale", torch.float32, None, x.device, align=4)
@@ -316,18 +349,22 @@ def gemm_blockscaled(a: BlockScaledTensor, b: BlockScaledTensor, *, epilogue: st
     """
     torch = _torch()
     _pre(isinstance(a, BlockScaledTensor) and isinstance(b, BlockScaledTensor), "a and b must be BlockScaledTensor", "dtype")
-    _pre(a.fmt == b.fmt, f"a is {a.fmt} but b is {b.fmt}: block-scaled formats must match exactly", "dtype", "b")
+    if a.fmt != b.fmt:
+        _pre(False, f"a is {a.fmt} but b is {b.fmt}: block-scaled formats must match exactly", "dtype", "b")
     _pre(a.layout == "swizzled" and b.layout == "swizzled", "the GEMM consumes swizzled scales", "contiguous")
-    _pre(epilogue in EPILOGUES, f"unknown epilogue {epilogue!r}", "argument", "epilogue")
+    if epilogue not in EPILOGUES:
+        _pre(False, f"unknown epilogue {epilogue!r}", "argument", "epilogue")
     m, k = a.shape
     nb, kb = b.shape
-    _pre(k == kb, f"K differs: a is {a.shape}, b is {b.shape}", "shape", "b")
+    if k != kb:
+        _pre(False, f"K differs: a is {a.shape}, b is {b.shape}", "shape", "b")
     n = nb // 2 if epilogue == "silu_gate" else nb
-    if epilogue == "silu_gate":
-        _pre(nb % 256 == 0, f"silu_gate: b has {nb} rows; each half must be a multiple of 128", "divisible", "b")
-    _pre(a.device == b.device, "a and b are on different devices", "device", "b")
+    if epilogue == "silu_gate" and nb % 256 != 0:
+        _pre(False, f"silu_gate: b has {nb} rows; each half must be a multiple of 128", "divisible", "b")
+    device = a.device
+    _pre(device == b.device, "a and b are on different devices", "device", "b")
     for t, nm in ((a.codes, "a.codes"), (b.codes, "b.codes"), (a.scales, "a.scales"), (b.scales, "b.scales")):
-        _check(t, nm, torch.uint8, None, a.device)
+        _check(t, nm, torch.uint8, None, device)
         _dense(t, nm)
     if a.fmt == "nvfp4":
         _pre(a.global_scale is not None and b.global_scale is not None, "nvfp4 operands need their global scales", "argument")
@@ -347,7 +384,7 @@ def gemm_blockscaled(a: BlockScaledTensor, b: BlockScaledTensor, *, epilogue: st
     if not want_bf16:
         out = None
     elif out is None:
-        out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
+        out = torch.empty((m, n), dtype=torch.bfloat16, device=device)
     else:
         _check(out, "out", torch.bfloat16, 2, a.device)
         _pre(tuple(out.shape) == (m, n) and out.stride(1) == 1 and (m <= 1 or out.stride(0) % 8 == 0), "out: wrong shape or strides", "shape", "out")
@@ -359,18 +396,20 @@ def gemm_blockscaled(a: BlockScaledTensor, b: BlockScaledTensor, *, epilogue: st
         _dense(residual, "residual")
         _pre(tuple(residual.shape) == (m, n), "residual: wrong shape", "shape", "residual")
         res_ptr = residual.data_ptr()
-    need = gemm_workspace_bytes(m, n, k, a.fmt, epilogue)
+    lib, fmt_id, epi_id = N.load(), FORMATS[a.fmt], EPILOGUES[epilogue]
+    need = lib.tf_gemm_workspace_bytes(m, n, k, fmt_id, epi_id)
     ws_ptr, ws_bytes = None, 0
     if need > 0:
         if workspace is None:
             workspace = torch.empty(need, dtype=torch.uint8, device=a.device)
-        _pre(workspace.numel() * workspace.element_size() >= need, f"workspace: {need} bytes needed", "workspace", "workspace")
         ws_ptr, ws_bytes = workspace.data_ptr(), workspace.numel() * workspace.element_size()
+        if ws_bytes < need:
+            _pre(False, f"workspace: {need} bytes needed", "workspace", "workspace")
     N.check(
-        N.load().tf_gemm_blockscaled(
+        lib.tf_gemm_blockscaled(
             a.codes.data_ptr(), a.scales.data_ptr(), a.global_scale.data_ptr() if a.global_scale is not None else None,
             b.codes.data_ptr(), b.scales.data_ptr(), b.global_scale.data_ptr() if b.global_scale is not None else None,
-            out.data_ptr() if out is not None else None, ldo, m, n, k, FORMATS[a.fmt], EPILOGUES[epilogue], res_ptr, _amax_ptr(amax_out, a.device),
+            out.data_ptr() if out is not None else None, ldo, m, n, k, fmt_id, epi_id, res_ptr, _amax_ptr(amax_out, a.device),
             q.codes.data_ptr() if q is not None and m > 0 else None, q.scales.data_ptr() if q is not None and m > 0 else None, a.gs_rows, ws_ptr, ws_bytes,
             _stream(stream)),
         "tf_gemm_blockscaled",

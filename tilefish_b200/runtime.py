@@ -396,6 +396,7 @@ class PlanRunner:
         self._arenas: Dict[int, Tuple[Any, int]] = {}
         self._loaded: Dict[Tuple[str, int], Any] = {}
         self._checked: set = set()
+        self._resolved: Dict[int, Tuple[Dict[str, Tuple[str, Tuple[int, ...]]], List[Dict[str, _Bound]]]] = {}
         self._buffers = {b["name"]: b for b in doc["buffers"]}
         self._algo = (manifest.get("library_file") or {}).get("sha256") or ""
 
@@ -438,6 +439,16 @@ class PlanRunner:
             else:
                 out[a["name"]] = _Bound(a["name"], a["binding"], dtype, tuple(v["shape"]), tuple(v["strides"]), v["offset"] * P.ITEMSIZE[dtype])
         return out
+
+    def _bucket(self, bucket: int) -> Tuple[Dict[str, Tuple[str, Tuple[int, ...]]], List[Dict[str, _Bound]]]:
+        """Shapes of every buffer and the bound arguments of every step of a bucket: they depend on the document alone, so they are
+        worked out once per bucket."""
+        got = self._resolved.get(bucket)
+        if got is None:
+            bdoc = self.doc["buckets"][bucket]
+            shapes = P.buffer_shapes(self.doc, bdoc["values"])
+            got = self._resolved[bucket] = (shapes, [self._bind_args(st, shapes) for st in bdoc["steps"]])
+        return got
 
     # -- one step as backend calls
     def _calls(self, step: Dict[str, Any], bound: Dict[str, _Bound], addr: Dict[str, int], index: int) -> List[Tuple[str, Any]]:
@@ -516,15 +527,14 @@ class PlanRunner:
 
     def enqueue(self, bucket: int, addr: Dict[str, int], index: int, stream: int, taps: Optional[Dict[Any, Any]] = None, only_step: Optional[int] = None) -> None:
         """Checks every step of the bucket, then enqueues them (``only_step``: that one step) on ``stream``."""
-        bdoc = self.doc["buckets"][bucket]
-        shapes = P.buffer_shapes(self.doc, bdoc["values"])
-        steps = bdoc["steps"]
+        steps = self.doc["buckets"][bucket]["steps"]
+        shapes, bound_steps = self._bucket(bucket)
         plan_calls: List[List[Tuple[str, Any]]] = []
         for i, st in enumerate(steps):
             if only_step is not None and i != only_step:
                 plan_calls.append([])
                 continue
-            bound = self._bind_args(st, shapes)
+            bound = bound_steps[i]
             self._check_step(st, bound, addr)
             calls = self._calls(st, bound, addr, index)
             for what, payload in calls:
@@ -571,7 +581,7 @@ class PlanRunner:
     def run(self, values: Dict[str, int], tensors: Dict[str, Any], device, outputs: Any = None, taps: Optional[Dict[Any, Any]] = None):
         index = self.backend.device_index(device)
         bucket = self.bucket_index(values)
-        shapes = P.buffer_shapes(self.doc, self.doc["buckets"][bucket]["values"])
+        shapes, _ = self._bucket(bucket)
         results = []
         if outputs is not None and not isinstance(outputs, (dict, list, tuple)):
             outputs = [outputs]  # one tensor for the one returned value
