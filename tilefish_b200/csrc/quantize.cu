@@ -75,10 +75,11 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint
   const int nvec = (int)(k >> 4);
   griddep_launch_dependents();
   griddep_wait();
+  const int cols = nvec / (FMT == TF_FMT_NVFP4 ? 1 : 2);
   if (pad)
-    zero_scale_padding(scales, m, k / (FMT == TF_FMT_NVFP4 ? 16 : 32),
-                       ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuantThreads + threadIdx.y * blockDim.x + threadIdx.x,
-                       (int64_t)gridDim.x * gridDim.y * kQuantThreads);
+    zero_scale_padding<false>(scales, m, cols,
+                              ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuantThreads + threadIdx.y * blockDim.x + threadIdx.x,
+                              (int64_t)gridDim.x * gridDim.y * kQuantThreads);
   float gs = 0.0f;
   if (FMT == TF_FMT_NVFP4 && n_partials > 0) {
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint
       load_round(xr, row_ok, base, nvec, v, has);
       store_round<FMT>(v, has, row, base, nvec, k, codes, scales, swizzled, gs, inv_t);
     }
+    if (pad && row_ok && blockIdx.y == 0 && threadIdx.x < 2) zero_row_padding(scales, row, cols, threadIdx.x);
   }
 }
 

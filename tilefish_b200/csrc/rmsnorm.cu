@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
   const float gs = (QFMT == TF_FMT_NVFP4) ? __ldg(q_gs_ptr) : 0.0f;
   const float inv_t = (QFMT == TF_FMT_NVFP4 && gs != 0.0f) ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
   if (QFMT >= 0 && q_pad)
-    zero_scale_padding(q_scales, m, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * nthreads + tid, (int64_t)gridDim.x * nthreads);
+    zero_scale_padding<false>(q_scales, m, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * nthreads + tid, (int64_t)gridDim.x * nthreads);
 
   for (int64_t row = blockIdx.x; row < m; row += gridDim.x) {
     const uint4* xr = x + row * nvec;
@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
         }
       }
     }
+    if (QFMT >= 0 && q_pad && tid < 2) zero_row_padding(q_scales, row, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), tid);
     __syncthreads();  // warp_sums / row_rstd are reused by the next row
   }
   if (out_amax) {  // one atomic per block
