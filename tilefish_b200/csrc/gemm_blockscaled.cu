@@ -15,7 +15,8 @@
 //            stores. With short K (10-20 stages per tile) one group of four could not drain a tile as fast as the MMAs fill one
 // The accumulator is double-buffered in tensor memory (overlapped for 256-column tiles, see TileCfg), so a tile's epilogue
 // runs while the next tile's MMAs are issued.
-// No TMA multicast, no clusters. Every mbarrier wait is bounded (about one second): on a timeout the kernel records
+// Further forms, chosen by launch_plan and use_pair_kernel: a pair of CTAs per 256 x 256 tile, K ranges over a cluster of CTAs or over
+// planes of a workspace. No TMA multicast. Every mbarrier wait is bounded (about one second): on a timeout the kernel records
 // TF_ERR_DEVICE_TIMEOUT in a device status word, every role leaves its loop, tensor memory is freed and the kernel returns.
 //
 // Scale layout consumed: the 512-byte 128x4 tiles described in the header; one tile feeds 4 tensor-memory columns through
