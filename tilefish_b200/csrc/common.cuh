@@ -78,6 +78,15 @@ inline cudaError_t launch_dependent(bool chain, void (*kernel)(KArgs...), dim3 g
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// One f32 that a kernel in front may have written. A dependent can be resident while its predecessor still runs, so what that kernel may
+// write is read with ordinary loads that stay behind griddep_wait(): the non-coherent path (__ldg, ld.global.nc) holds only for memory
+// that nobody writes during the kernel's whole lifetime, and the compiler may move such loads. It is left to the norm weights.
+__device__ __forceinline__ float load_f32(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float bf16lo_to_f32(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi_to_f32(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 

@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
   griddep_wait();
   if (QFMT >= 0 && q_pad)
     zero_scale_padding(q_scales, m, n >> 5, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
-  const float alpha0 = (a_gs && b_gs) ? __fmul_rn(__ldg(a_gs), __ldg(b_gs)) : 1.0f;
+  const float alpha0 = (a_gs && b_gs) ? __fmul_rn(load_f32(a_gs), load_f32(b_gs)) : 1.0f;
   const int nvec = n >> 3;
   const int64_t total = (int64_t)m * nvec;
   const int64_t plane = (int64_t)m * n_acc;
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     float acc[8], up[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = up[j] = 0.0f;
-    const float alpha = (a_gs && b_gs && a_gs_rows > 0) ? __fmul_rn(__ldg(a_gs + row / a_gs_rows), __ldg(b_gs)) : alpha0;
+    const float alpha = (a_gs && b_gs && a_gs_rows > 0) ? __fmul_rn(load_f32(a_gs + row / a_gs_rows), load_f32(b_gs)) : alpha0;
     const float* base = ws + (int64_t)row * n_acc + col;
     for (int sp = 0; sp < (live ? splits : 0); ++sp) {
       const float4 x0 = __ldcs(reinterpret_cast<const float4*>(base + sp * plane)), x1 = __ldcs(reinterpret_cast<const float4*>(base + sp * plane) + 1);
@@ -676,6 +676,7 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
   const int rows = min(kBlockM, p.m - m_blk * kBlockM);
   const int total = rows * kVecs;
   const bool quantize = FMT != TF_FMT_NVFP4 && p.q_codes != nullptr;
+  const float alpha0 = (FMT == TF_FMT_NVFP4) ? __fmul_rn(load_f32(p.a_gs), load_f32(p.b_gs)) : 1.0f;
   uint32_t amax2 = 0;
   // whole warps run every round (the quantizer's shuffles); the 4 lanes of one MX block always have data together
   for (int i0 = rank * kGemmThreads; i0 < total; i0 += p.splits * kGemmThreads) {
@@ -716,8 +717,7 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
         }
       }
     }
-    float alpha = 1.0f;
-    if (FMT == TF_FMT_NVFP4 && live) alpha = __fmul_rn(__ldg(p.a_gs + (p.a_gs_rows > 0 ? row / p.a_gs_rows : 0)), __ldg(p.b_gs));
+    const float alpha = (FMT == TF_FMT_NVFP4 && live && p.a_gs_rows > 0) ? __fmul_rn(load_f32(p.a_gs + row / p.a_gs_rows), load_f32(p.b_gs)) : alpha0;
     uint32_t packed[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     // ---------------- epilogue (warps 2..5 = group 0, warps 7..10 = group 1; warp w reads lanes 32*(w%4) .. +31) ----------------
     const int q = warp & 3;
     const int grp = warp >= 7 ? 1 : 0;
-    const float alpha = (FMT == TF_FMT_NVFP4) ? __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs)) : 1.0f;
+    const float alpha = (FMT == TF_FMT_NVFP4 && SPLITK == kSplitNone) ? __fmul_rn(load_f32(p.a_gs), load_f32(p.b_gs)) : 1.0f;
     uint32_t tile_phase = 0, acc_buf = 0;
     uint32_t amax2 = 0;  // running max of |out| as two packed bf16 magnitudes
     if (FMT != TF_FMT_NVFP4 && p.q_codes && p.q_pad)
@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
       const int row = m_blk * kBlockM + q * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const int col0 = n_blk * kOutCols;
-      const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(__ldg(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), __ldg(p.b_gs)) : alpha;
+      const float alpha_t = (FMT == TF_FMT_NVFP4 && SPLITK == kSplitNone && p.a_gs_rows > 0) ? __fmul_rn(load_f32(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), load_f32(p.b_gs)) : alpha;
       if (kCluster) {
         if (m_blk * kBlockM + q * 32 < p.m) {
           const uint32_t smem_row = smem_a + (uint32_t)(q * 32 + lane) * DumpCfg<BLOCK_N>::kPitch;
@@ -1232,7 +1232,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
     // ---------------- epilogue: each CTA drains its own 128 rows; the release goes to the leader's barrier ----------------
     const int q = warp & 3;
     const int grp = warp >= 7 ? 1 : 0;
-    const float alpha = (FMT == TF_FMT_NVFP4) ? __fmul_rn(__ldg(p.a_gs), __ldg(p.b_gs)) : 1.0f;
+    const float alpha = (FMT == TF_FMT_NVFP4) ? __fmul_rn(load_f32(p.a_gs), load_f32(p.b_gs)) : 1.0f;
     const uint32_t release = mapa_shared(bar_tmem_empty, 0);
     const uint32_t stage_smem = smem_out + (uint32_t)(grp * 4 + q) * PC::kOutBoxBytes;
     uint32_t tile_phase = 0, acc_buf = 0;
@@ -1248,7 +1248,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
       const int row = m_blk * 256 + (int)rank * 128 + q * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const int col0 = n_blk * kOutCols;
-      const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(__ldg(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), __ldg(p.b_gs)) : alpha;
+      const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(load_f32(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), load_f32(p.b_gs)) : alpha;
       if (acc_buf == 0) {
         if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 0, 0, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
         else epilogue_tile<FMT, BLOCK_N, EPI, 0, 1, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);

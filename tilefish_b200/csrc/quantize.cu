@@ -17,7 +17,7 @@ constexpr int kQuantUnroll = 4;
 
 // Block = (TPR threads along the row) x (256 / TPR rows); rows are taken grid-stride.
 __device__ __forceinline__ void load_256(const void* p, uint32_t (&w)[8]) {
-  asm volatile("ld.global.nc.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm volatile("ld.global.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                : "l"(p));
 }
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint
   if (FMT == TF_FMT_NVFP4 && n_partials > 0) {
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     uint32_t mx = 0;  // non-negative floats order like their bits
-    for (int i = tid; i < n_partials; i += kQuantThreads) mx = max(mx, __float_as_uint(__ldg(gs_ptr + i)));
+    for (int i = tid; i < n_partials; i += kQuantThreads) mx = max(mx, __float_as_uint(load_f32(gs_ptr + i)));
     __shared__ uint32_t warp_max[kQuantThreads / 32];
     mx = __reduce_max_sync(0xFFFFFFFFu, mx);
     if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint
     for (int i = 0; i < kQuantThreads / 32; ++i) mx = max(mx, warp_max[i]);
     gs = __uint_as_float(mx);
   } else if (FMT == TF_FMT_NVFP4) {
-    gs = __ldg(gs_ptr);
+    gs = load_f32(gs_ptr);
   }
   if (FMT == TF_FMT_NVFP4 && gs_out != nullptr) {
     gs = __fdiv_rn(gs, 2688.0f);

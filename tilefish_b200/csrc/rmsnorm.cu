@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
   const int tid = threadIdx.x, nthreads = blockDim.x;
   griddep_launch_dependents();
   griddep_wait();
-  const float gs = (QFMT == TF_FMT_NVFP4) ? __ldg(q_gs_ptr) : 0.0f;
+  const float gs = (QFMT == TF_FMT_NVFP4) ? load_f32(q_gs_ptr) : 0.0f;
   const float inv_t = (QFMT == TF_FMT_NVFP4 && gs != 0.0f) ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
   if (QFMT >= 0 && q_pad)
     zero_scale_padding<false>(q_scales, m, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * nthreads + tid, (int64_t)gridDim.x * nthreads);
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(512) rmsnorm_quantize_rows_kernel(const uint4*
   griddep_launch_dependents();
   griddep_wait();
   float alpha = 1.0f;
-  if (splits > 0 && a_gs && b_gs) alpha = __fmul_rn(__ldg(a_gs + (a_gs_rows > 0 ? row / a_gs_rows : 0)), __ldg(b_gs));
+  if (splits > 0 && a_gs && b_gs) alpha = __fmul_rn(load_f32(a_gs + (a_gs_rows > 0 ? row / a_gs_rows : 0)), load_f32(b_gs));
   const int64_t plane = (int64_t)m * d;
   float4* rr = residual + (int64_t)row * (nvec * 2);
   float r[VPT][8];
