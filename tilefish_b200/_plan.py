@@ -68,36 +68,7 @@ def swizzled_scale_bytes(rows: int, k: int, fmt: str) -> int:
     return ((rows + 127) // 128) * ((cols + 3) // 4) * 512
 
 
-# ---- the kernel library's split-K rule, restated (csrc/gemm_blockscaled.cu ``split_plan`` and ``few_rows_plan``) -------------------
-def _few_rows_plan(m: int, n: int, k_bytes: int, sms: int) -> Tuple[int, int, int]:
-    """Up to 64 rows without a gate: stage, streaming and reduction times in microseconds, the library's operations in its order."""
-    stages = (k_bytes + 127) // 128
-    plan, best = (128, 1, stages), 1e30
-    for bn in (256, 128):
-        tiles = (n + bn - 1) // bn
-        for want in range(1, 17):
-            if want > 1 and stages // want < 4:
-                break
-            kps = (stages + want - 1) // want
-            splits = (stages + kps - 1) // kps
-            units = tiles * splits
-            unit_bytes = float(n) * float(k_bytes) / float(units)
-            rem = units % sms
-            stream = float(units // sms * sms) * unit_bytes / 5.5e6
-            if rem:
-                stream += float(rem) * unit_bytes / min(float(rem) * 7.0e4, 5.5e6)
-            cost = float((units + sms - 1) // sms) * (float(kps) * (0.235 if bn == 128 else 0.38) + (0.5 if bn == 128 else 1.0))
-            cost = max(cost, stream)
-            if splits > 1:
-                if bn == 128 and splits <= 8 and units <= 140:
-                    cost += 1.6 + float(m) * bn * 4.0 * float(splits - 1) / float(splits) / 26600.0
-                else:
-                    cost += 2.0 + float(splits) * float(m) * float(n) * 8.0 / 3.0e6
-            if cost < best - 1e-9:
-                best, plan = cost, (bn, splits, kps)
-    return plan
-
-
+# ---- the kernel library's split-K rule, restated (csrc/gemm_blockscaled.cu ``split_plan``) -------------------------------------
 def gemm_split_plan(m: int, n: int, k_bytes: int, epilogue: str, sms: int = PLANNED_SM_COUNT) -> Tuple[int, int, int]:
     """(tile width, K ranges, K stages per range) the GEMM uses for a problem on ``sms`` SMs."""
     m_blocks = (m + 127) // 128
@@ -108,8 +79,6 @@ def gemm_split_plan(m: int, n: int, k_bytes: int, epilogue: str, sms: int = PLAN
         block_n = 128
     if m > 256:
         return block_n, splits, kps
-    if m <= 64 and epilogue != "silu_gate":
-        return _few_rows_plan(m, n, k_bytes, sms)
     a_rows = min(m, 128)
     best = 1e30
     for bn in (256, 128):

@@ -761,6 +761,7 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
 // SPLITK: kSplitNone; kSplitPlanes: every (tile, K range) is a unit of its own and leaves its accumulator in the workspace;
 // kSplitCluster: a cluster of `splits` CTAs per tile, launched with exactly one tile per cluster.
 constexpr int kSplitNone = 0, kSplitPlanes = 1, kSplitCluster = 2;
+constexpr int kMaxClusterSplits = 8;  // the portable cluster size
 template <int FMT, int BLOCK_N, int EPI, int SPLITK>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                             const __grid_constant__ CUtensorMap tma_b, const GemmParams p) {
@@ -1321,44 +1322,6 @@ struct SplitPlan {
   int block_n, splits, k_stages_per_split;
 };
 
-// Microseconds beyond a launch's fixed part, fitted to B200 measurements of graphs of 24 launches: a K stage takes 0.235 with 128-column
-// tiles and 0.38 with 256 (bound by shared-memory reads and fills), a tile's epilogue 0.5 / 1.0; planes and a reduction launch cost 2.0 +
-// 8 bytes per partial sum at 3 TB/s, a cluster 1.6 + its remote reads at 26.6 GB/s per SM.
-static double stage_us(int bn) { return bn == 128 ? 0.235 : 0.38; }
-static double tile_us(int bn, int64_t kps) { return (double)kps * stage_us(bn) + (bn == 128 ? 0.5 : 1.0); }
-static double planes_us(int64_t splits, int64_t m, int64_t n_acc) { return 2.0 + (double)splits * (double)m * (double)n_acc * 8.0 / 3.0e6; }
-constexpr int kMaxClusterSplits = 8;  // the portable cluster size
-static double cluster_us(int bn, int64_t splits, int64_t rows) { return 1.6 + (double)rows * bn * 4.0 * (double)(splits - 1) / (double)splits / 26600.0; }
-
-// Up to 64 rows without a gate: 128-column tiles and the K ranges that finish first, the weights streamed at 5.5 TB/s but at no more than
-// 70 GB/s by one SM. A split of at most 8 ranges and 140 CTAs runs as clusters (it fits the GPCs whatever their sizes). Before (the row
-// segment model below) -> after, graphs of 24: nvfp4 64 x 8192 x 28672 30.6 -> 27.0 us, mxfp4 1 x 3240 x 8096 7.0 -> 6.6, the other 40 shapes of a random
-// sweep within 4 %.
-static SplitPlan few_rows_plan(int64_t m, int64_t n, int64_t k_bytes) {
-  const int64_t sms = sm_count(), stages = (k_bytes + kStageKBytes - 1) / kStageKBytes;
-  SplitPlan sp = {128, 1, (int)stages};
-  double best = 1e30;
-  for (int bn = 256; bn >= 128; bn -= 128) {
-    const int64_t tiles = (n + bn - 1) / bn;
-    for (int64_t want = 1; want <= 16; ++want) {
-      if (want > 1 && stages / want < 4) break;
-      const int64_t kps = (stages + want - 1) / want, splits = (stages + kps - 1) / kps, units = tiles * splits;
-      const double bytes = (double)n * (double)k_bytes / (double)units;  // of one unit
-      const int64_t rem = units % sms;
-      double stream = (double)(units / sms * sms) * bytes / 5.5e6;
-      if (rem) stream += (double)rem * bytes / ((double)rem * 7.0e4 < 5.5e6 ? (double)rem * 7.0e4 : 5.5e6);
-      double cost = (double)((units + sms - 1) / sms) * tile_us(bn, kps);
-      if (stream > cost) cost = stream;
-      if (splits > 1) cost += (bn == 128 && splits <= kMaxClusterSplits && units <= 140) ? cluster_us(bn, splits, m) : planes_us(splits, m, n);
-      if (cost < best - 1e-9) {
-        best = cost;
-        sp = {bn, (int)splits, (int)kps};
-      }
-    }
-  }
-  return sp;
-}
-
 // Small M (at most two row blocks): the GEMM streams the weights once and is bound by how evenly that stream is spread over
 // the SMs. Measured on B200: one CTA's TMA pipeline draws about one 128-byte row segment per 4 clocks from HBM (about
 // 60 GB/s), so the time of a launch is the largest number of row segments any CTA fetches. The plan minimises
@@ -1375,7 +1338,6 @@ static SplitPlan split_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogue)
   sp.k_stages_per_split = (int)stages;
   if (n <= 128 && epilogue != TF_EPI_SILU_GATE) sp.block_n = 128;
   if (m > 256) return sp;
-  if (m <= 64 && epilogue != TF_EPI_SILU_GATE) return few_rows_plan(m, n, k_bytes);
   const int64_t a_rows = m < kBlockM ? m : kBlockM;
   double best = 1e30;
   for (int bn = 256; bn >= 128; bn -= 128) {
@@ -1567,7 +1529,9 @@ static int cluster_capacity(int splits) {
 }
 
 // The launch plan: `sp` as it stands, or 128-column tiles, or (kSplitCluster) each tile cut over a cluster of CTAs, whichever the model
-// above says is shortest.
+// below says is shortest. Microseconds beyond a launch's fixed 4.4, fitted to B200 measurements of graphs of 24 launches:
+//   a K stage takes 0.235 with 128-column tiles and 0.38 with 256 (bound by shared-memory reads and fills), a tile's epilogue 0.5 / 1.0;
+//   planes and a reduction launch 2.0 + 8 bytes per partial sum at 3 TB/s; a cluster 1.6 + its remote reads at 26.6 GB/s per SM.
 // before -> after: mxfp8 512 x 2560 x 3072 13.5 -> 11.2 us (128-column tiles), 128 x 2560 x 3072 12.4 -> 10.2 (4 ranges), 1 x 2560 x 3072
 // 7.3 -> 6.2 (6), 700 x 1024 x 16384 43.0 -> 23.2 (2), mxfp4 300 x 1024 x 8192 residual 27.0 -> 11.0 (3).
 // A problem with a planes plan keeps that plan's K ranges in every form, so that its result is the sum of the planes bit for bit.
@@ -1580,9 +1544,11 @@ static LaunchPlan launch_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogu
   const int64_t sms = gemm_sms(), m_blocks = (m + kBlockM - 1) / kBlockM, n_acc = gate ? 2 * n : n;
   const int64_t stages = (k_bytes + kStageKBytes - 1) / kStageKBytes, rows = m < kBlockM ? m : kBlockM;
   auto tiles = [&](int bn) { return m_blocks * ((n_acc + bn - 1) / bn); };
+  auto stage_us = [](int bn) { return bn == 128 ? 0.235 : 0.38; };
+  auto tile_us = [&](int bn, int64_t kps) { return (double)kps * stage_us(bn) + (bn == 128 ? 0.5 : 1.0); };
   if (tiles(128) > 2 * sms) return best;  // at least one full wave of 256-column tiles
   double cost = (double)((tiles(sp.block_n) * sp.splits + sms - 1) / sms) * tile_us(sp.block_n, sp.k_stages_per_split);
-  if (sp.splits > 1) cost += planes_us(sp.splits, m, n_acc);
+  if (sp.splits > 1) cost += 2.0 + (double)sp.splits * (double)m * (double)n_acc * 8.0 / 3.0e6;
   if (!gate && sp.splits == 1 && tiles(128) <= sms && tile_us(128, stages) < cost) {
     cost = tile_us(128, stages);
     best = {kSplitNone, 128, 1, (int)stages};
@@ -1593,7 +1559,7 @@ static LaunchPlan launch_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogu
     const int64_t kps = (stages + want - 1) / want, splits = (stages + kps - 1) / kps;
     if (splits < 2 || tiles(bn) * splits > sms || tiles(bn) > cluster_capacity((int)splits)) continue;
     if (sp.splits > 1 && (splits != sp.splits || kps != sp.k_stages_per_split)) continue;  // the sums tf_gemm_blockscaled_partials leaves
-    const double c = tile_us(bn, kps) + cluster_us(bn, splits, rows);
+    const double c = tile_us(bn, kps) + 1.6 + (double)rows * bn * 4.0 * (double)(splits - 1) / (double)splits / 26600.0;
     if (c < cost) {
       cost = c;
       best = {kSplitCluster, bn, (int)splits, (int)kps};
