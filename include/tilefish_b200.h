@@ -72,7 +72,7 @@ TF_API tf_status tf_device_status(int32_t* status, int32_t* detail);
 
 /* PROCESS-WIDE and not synchronized with calls in flight on other threads (set it while no other thread launches): the persistent GEMM
  * launches on (SM count - sms) SMs from now on, for every caller in the process, tf_gemm_blockscaled_static included; a CUDA graph keeps
- * the grid that was in force when it was captured. Purpose: so that a collective running beside it in
+ * the grid that was in force when it was captured. Results do not depend on it, byte for byte. Purpose: so that a collective running beside it in
  * another stream (the tensor-parallel MLP overlaps one row chunk's all-reduce with the other chunk's GEMMs) finds free SMs.
  * 0 restores the default. No counterpart in the reference (its GEMM is cuBLASLt's `sm_count_target`, python/src/tilefish/_cublaslt.py). */
 TF_API tf_status tf_set_sm_margin(int32_t sms);
@@ -219,6 +219,11 @@ TF_API int32_t tf_gemm_splits(int64_t m, int64_t n, int64_t k, int32_t format, i
 TF_API tf_status tf_gemm_blockscaled_partials(const void* a_codes, const void* a_scales, const float* a_global_scale, const void* b_codes,
                                               const void* b_scales, const float* b_global_scale, int64_t m, int64_t n, int64_t k, int32_t format,
                                               void* workspace, int64_t workspace_bytes, int32_t* splits, void* stream);
+
+/* How tf_gemm_blockscaled launches a problem under the settings in force, for tests and profiles (no counterpart in the reference): form[0] = 0
+ * one CTA per tile, 1 K ranges as planes of the workspace and a reduction launch, 2 K ranges over a cluster of CTAs, 3 a pair of CTAs per
+ * 256 x 256 tile; form[1] = accumulator columns of a tile (of one CTA); form[2] = K ranges. */
+TF_API tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue, int32_t* form);
 
 /* The GEMM with a scattered output: the tensor-parallel second GEMM (w_d split along K) whose epilogue delivers each row block of
  * its partial result straight to the rank that will sum it, so that no separate kernel has to pull the partial results across

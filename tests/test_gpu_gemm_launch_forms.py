@@ -57,3 +57,32 @@ def test_gate_over_a_cluster_and_a_pair(K, fmt, m, f, k):
     # the gate reads two bf16 results that may differ by one rounding (2**-8 of the largest): |silu'| < 1.1, times the other factor
     bound = 2 * TOL * float(t.abs().max()) * (float(t.abs().max()) + 1.0)
     assert float((out.float() - ref).abs().max()) <= bound
+
+
+@pytest.fixture
+def margin():
+    """Sets the SM margin; 0 again afterwards."""
+    from tilefish_b200 import _native as N
+
+    def set_margin(sms):
+        N.check(N.load().tf_set_sm_margin(sms), "tf_set_sm_margin")
+
+    yield set_margin
+    set_margin(0)
+
+
+@pytest.mark.parametrize("m,n,k,epi", [(520, 1064, 4960, "none"), (520, 1064, 4960, "residual"), (1, 1568, 1408, "none"), (384, 640, 8192, "silu_gate"),
+                                       (700, 1024, 16384, "none"), (1024, 2304, 512, "none")])
+def test_the_margin_does_not_change_a_byte(K, margin, m, n, k, epi):
+    """The SM margin is a matter of occupancy: K is cut into the same ranges, so the sums are the same (MXFP8: the sums round)."""
+    qa = K.quantize(O.randn((m, k), m, torch.bfloat16).cuda(), "mxfp8")
+    qb = K.quantize(O.randn((2 * n if epi == "silu_gate" else n, k), n, torch.bfloat16, scale=k**-0.5).cuda(), "mxfp8")
+    results = []
+    for sms in (0, 16, 32, 64):
+        margin(sms)
+        res = O.randn((m, n), 7).cuda() if epi == "residual" else None
+        results.append((K.gemm_launch_form(m, n, k, "mxfp8", epi)[2], K.gemm_blockscaled(qa, qb, epilogue=epi, residual=res), res))
+    assert results[0][0] > 1 or k == 512
+    for ranges, out, res in results[1:]:
+        assert ranges == results[0][0] and torch.equal(out, results[0][1])
+        assert res is None or torch.equal(res, results[0][2])

@@ -761,6 +761,7 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
 // SPLITK: kSplitNone; kSplitPlanes: every (tile, K range) is a unit of its own and leaves its accumulator in the workspace;
 // kSplitCluster: a cluster of `splits` CTAs per tile, launched with exactly one tile per cluster.
 constexpr int kSplitNone = 0, kSplitPlanes = 1, kSplitCluster = 2;
+constexpr int kFormPair = 3;  // what tf_gemm_launch_form calls the CTA pair
 constexpr int kMaxClusterSplits = 8;  // the portable cluster size
 template <int FMT, int BLOCK_N, int EPI, int SPLITK>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tma_a,
@@ -1485,12 +1486,13 @@ static int two_cta_forced() {
 // Per wave of tiles the pair is 5-13 % faster than the one-CTA kernel (measured on B200, one-CTA -> pair: nvfp4 4096 x 8192 x 28672
 // 385 -> 336 us, 4096 x 28672 x 8192 + gate 713 -> 666, 4096 x 6144 x 2560 35.1 -> 33.2; mxfp8 8192 x 6144 x 2560 106 -> 98.8;
 // mxfp4 300 x 8192 x 4096 12.8 -> 12.1), but its row blocks are 256 high: it is left where that costs a tenth more waves.
-static bool use_pair_kernel(const GemmParams& p, const LaunchPlan& lp, int out_cols) {
+static bool use_pair_kernel(int64_t m, int64_t n, int epilogue, const LaunchPlan& lp) {
   const int forced = two_cta_forced();
-  if (forced == 0 || lp.form != kSplitNone || lp.block_n != 256 || p.scatter_rows || p.m <= kBlockM || p.n_rows_b < 256) return false;
+  const bool gate = epilogue == TF_EPI_SILU_GATE;
+  if (forced == 0 || lp.form != kSplitNone || lp.block_n != 256 || m <= kBlockM || (gate ? 2 * n : n) < 256) return false;
   if (forced == 1) return true;
-  const int64_t sms = gemm_sms(), pairs = sms / 2, n_blocks = (p.n + out_cols - 1) / out_cols;
-  const int64_t waves = (p.m_blocks * n_blocks + sms - 1) / sms, pair_waves = ((p.m + 255) / 256 * n_blocks + pairs - 1) / pairs;
+  const int64_t sms = gemm_sms(), pairs = sms / 2, n_blocks = gate ? (n + 127) / 128 : (n + 255) / 256;
+  const int64_t waves = ((m + kBlockM - 1) / kBlockM * n_blocks + sms - 1) / sms, pair_waves = ((m + 255) / 256 * n_blocks + pairs - 1) / pairs;
   return 10 * pair_waves <= 11 * waves;
 }
 
@@ -1535,13 +1537,15 @@ static int cluster_capacity(int splits) {
 // before -> after: mxfp8 512 x 2560 x 3072 13.5 -> 11.2 us (128-column tiles), 128 x 2560 x 3072 12.4 -> 10.2 (4 ranges), 1 x 2560 x 3072
 // 7.3 -> 6.2 (6), 700 x 1024 x 16384 43.0 -> 23.2 (2), mxfp4 300 x 1024 x 8192 residual 27.0 -> 11.0 (3).
 // A problem with a planes plan keeps that plan's K ranges in every form, so that its result is the sum of the planes bit for bit.
+// The plan is made for the whole device, whatever margin is set (tf_set_sm_margin): K ranges are part of a result, so they may not depend on
+// it. Beside a margin a cluster launch takes the SMs it was planned for; the tile width, which no sum depends on, follows the free SMs.
 // The SiLU gate pairs 128 + 128 columns, so its tiles stay 256 wide; with planes available (m <= 256) those measured faster (9.2 against
 // 9.5 us at 1 x 3072 x 2560), so a cluster takes it only above that.
 static LaunchPlan launch_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogue, const SplitPlan& sp) {
   LaunchPlan best = {sp.splits > 1 ? kSplitPlanes : kSplitNone, sp.block_n, sp.splits, sp.k_stages_per_split};
   if (two_cta_forced() == 1) return best;
   const bool gate = epilogue == TF_EPI_SILU_GATE;
-  const int64_t sms = gemm_sms(), m_blocks = (m + kBlockM - 1) / kBlockM, n_acc = gate ? 2 * n : n;
+  const int64_t sms = sm_count(), m_blocks = (m + kBlockM - 1) / kBlockM, n_acc = gate ? 2 * n : n;
   const int64_t stages = (k_bytes + kStageKBytes - 1) / kStageKBytes, rows = m < kBlockM ? m : kBlockM;
   auto tiles = [&](int bn) { return m_blocks * ((n_acc + bn - 1) / bn); };
   auto stage_us = [](int bn) { return bn == 128 ? 0.235 : 0.38; };
@@ -1565,6 +1569,7 @@ static LaunchPlan launch_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogu
       best = {kSplitCluster, bn, (int)splits, (int)kps};
     }
   }
+  if (best.form == kSplitNone && best.block_n != sp.block_n && tiles(best.block_n) > gemm_sms()) best.block_n = sp.block_n;
   return best;
 }
 
@@ -1614,7 +1619,7 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     TF_LAUNCH_CHECK();
     return TF_OK;
   }
-  if (use_pair_kernel(p, lp, epilogue == TF_EPI_SILU_GATE ? 128 : 256)) {
+  if (!p.scatter_rows && use_pair_kernel(p.m, p.n, epilogue, lp)) {
     if (epilogue == TF_EPI_SILU_GATE) return launch_gemm_pair<FMT, TF_EPI_SILU_GATE>(ta, tb, p, stream);
     if (epilogue == TF_EPI_RESIDUAL) return launch_gemm_pair<FMT, TF_EPI_RESIDUAL>(ta, tb, p, stream);
     return launch_gemm_pair<FMT, TF_EPI_NONE>(ta, tb, p, stream);
@@ -1709,6 +1714,19 @@ static tf_status static_scratch_address(void** out) {
 int32_t tf_gemm_splits(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue) {
   if (m <= 0 || n <= 0 || k <= 0 || format < TF_FMT_MXFP8 || format > TF_FMT_NVFP4 || epilogue < TF_EPI_NONE || epilogue > TF_EPI_RESIDUAL) return 0;
   return split_plan(m, n, format == TF_FMT_MXFP8 ? k : k / 2, epilogue).splits;
+}
+
+tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue, int32_t* form) {
+  clear_error();
+  TF_CHECK_ARG(form != nullptr, "%s: null pointer", __func__);
+  TF_CHECK_ARG(m > 0 && n > 0 && k > 0 && format >= TF_FMT_MXFP8 && format <= TF_FMT_NVFP4 && epilogue >= TF_EPI_NONE && epilogue <= TF_EPI_RESIDUAL,
+               "%s: bad argument", __func__);
+  const int64_t k_bytes = format == TF_FMT_MXFP8 ? k : k / 2;
+  const LaunchPlan lp = launch_plan(m, n, k_bytes, epilogue, split_plan(m, n, k_bytes, epilogue));
+  form[0] = use_pair_kernel(m, n, epilogue, lp) ? kFormPair : lp.form;
+  form[1] = lp.block_n;
+  form[2] = lp.splits;
+  return TF_OK;
 }
 
 int64_t tf_gemm_static_scratch_bytes(void) { return kStaticScratchBytes; }

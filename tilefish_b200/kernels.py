@@ -9,7 +9,7 @@ reference checks a launch (python/src/tilefish/_launch.py:263-315, :433-500); fa
 from __future__ import annotations
 
 import ctypes
-from typing import Optional
+from typing import Optional, Tuple
 
 from . import _native as N
 from .errors import TilefishPreconditionError, TilefishRuntimeError
@@ -453,6 +453,14 @@ def gemm_blockscaled_scatter(a: BlockScaledTensor, b: BlockScaledTensor, out_ptr
 def gemm_splits(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> int:
     """How many K ranges the GEMM cuts this problem into (1: not split; more than 1 only for few rows)."""
     return int(N.load().tf_gemm_splits(m, n, k, FORMATS[fmt], EPILOGUES[epilogue]))
+
+
+def gemm_launch_form(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> Tuple[str, int, int]:
+    """How the GEMM launches this problem under the settings in force: ("tiles" | "planes" | "cluster" | "pair", accumulator columns of a
+    tile, K ranges)."""
+    form = (ctypes.c_int32 * 3)()
+    N.check(N.load().tf_gemm_launch_form(m, n, k, FORMATS[fmt], EPILOGUES[epilogue], form), "tf_gemm_launch_form")
+    return ("tiles", "planes", "cluster", "pair")[form[0]], form[1], form[2]
 
 
 class SplitKPartials:
