@@ -24,3 +24,21 @@ def test_shapes_that_leave_partial_sums_or_fit_the_static_scratch():
     assert lib.tf_gemm_splits(58, 8456, 7456, MXFP4, NONE) > 1  # tf_gemm_blockscaled_partials takes it
     assert lib.tf_gemm_splits(52, 7936, 3584, MXFP8, NONE) > 1  # so does the fused decode step of such a stack
     assert lib.tf_gemm_workspace_bytes(11, 38960, 24032, MXFP8, NONE) <= lib.tf_gemm_static_scratch_bytes()
+
+
+@pytest.fixture
+def margin():
+    lib = _native.load()
+    yield lambda sms: _native.check(lib.tf_set_sm_margin(sms), "tf_set_sm_margin")
+    _native.check(lib.tf_set_sm_margin(0), "tf_set_sm_margin")
+
+
+@pytest.mark.parametrize("fmt,m,n,k,epi", [("nvfp4", 2048, 14336, 8192, "silu_gate"), ("mxfp8", 8192, 6144, 2560, "none"), ("mxfp4", 4096, 8192, 14336, "residual")])
+def test_cta_pairs_are_left_beside_a_margin(margin, fmt, m, n, k, epi):
+    """A pair of CTAs needs two neighbouring SMs, which the kernel beside it need not leave whole."""
+    from tilefish_b200 import kernels as K
+
+    assert K.gemm_launch_form(m, n, k, fmt, epi) == ("pair", 256, 1)
+    for sms in (1, 16, 64):
+        margin(sms)
+        assert K.gemm_launch_form(m, n, k, fmt, epi) == ("tiles", 256, 1)

@@ -1311,8 +1311,9 @@ static tf_status make_operand_map(CUtensorMap* map, const void* base, int64_t ro
 
 // SMs the persistent GEMM leaves free (for a collective running beside it in another stream).
 static std::atomic<int> g_sm_margin{0};  // process-wide (tf_set_sm_margin); atomic so that a concurrent reader sees the old or the new value
+static int sm_margin() { return g_sm_margin.load(std::memory_order_relaxed); }
 static int gemm_sms() {
-  const int n = sm_count() - g_sm_margin.load(std::memory_order_relaxed);
+  const int n = sm_count() - sm_margin();
   return n < 2 ? 2 : n;
 }
 
@@ -1486,12 +1487,16 @@ static int two_cta_forced() {
 // Per wave of tiles the pair is 5-13 % faster than the one-CTA kernel (measured on B200, one-CTA -> pair: nvfp4 4096 x 8192 x 28672
 // 385 -> 336 us, 4096 x 28672 x 8192 + gate 713 -> 666, 4096 x 6144 x 2560 35.1 -> 33.2; mxfp8 8192 x 6144 x 2560 106 -> 98.8;
 // mxfp4 300 x 8192 x 4096 12.8 -> 12.1), but its row blocks are 256 high: it is left where that costs a tenth more waves.
+// Beside a margin it is left too: a pair needs two SMs of one TPC, and the kernel that the margin is for need not leave them whole. CTAs
+// of 200 KB that start beside a quantizer split 4 to 12 pairs; with 16 pairs split, nvfp4 2048 x 14336 x 8192 + gate takes 303 us on pairs and 199 on
+// single CTAs at margin 16 (342 and 217 at 32), since tiles are dealt out statically. With none split it is 184 and 203.
 static bool use_pair_kernel(int64_t m, int64_t n, int epilogue, const LaunchPlan& lp) {
   const int forced = two_cta_forced();
   const bool gate = epilogue == TF_EPI_SILU_GATE;
   if (forced == 0 || lp.form != kSplitNone || lp.block_n != 256 || m <= kBlockM || (gate ? 2 * n : n) < 256) return false;
   if (forced == 1) return true;
-  const int64_t sms = gemm_sms(), pairs = sms / 2, n_blocks = gate ? (n + 127) / 128 : (n + 255) / 256;
+  if (sm_margin() > 0) return false;
+  const int64_t sms = sm_count(), pairs = sms / 2, n_blocks = gate ? (n + 127) / 128 : (n + 255) / 256;
   const int64_t waves = ((m + kBlockM - 1) / kBlockM * n_blocks + sms - 1) / sms, pair_waves = ((m + 255) / 256 * n_blocks + pairs - 1) / pairs;
   return 10 * pair_waves <= 11 * waves;
 }
