@@ -77,10 +77,10 @@ TF_API tf_status tf_device_status(int32_t* status, int32_t* detail);
  * 0 restores the default. No counterpart in the reference (its GEMM is cuBLASLt's `sm_count_target`, python/src/tilefish/_cublaslt.py). */
 TF_API tf_status tf_set_sm_margin(int32_t sms);
 
-/* Programmatic dependent launch for all of this library's kernels (off by default: then only GEMMs of at most 256 rows and
- * row kernels of at most 4 rows use it; PROCESS-WIDE, as tf_set_sm_margin). On: the quantize, rmsnorm, GEMM and split-K
- * reduction kernels are launched so that each may be scheduled while the kernel before it on the stream is still
- * draining; each waits (griddepcontrol.wait) for that kernel to complete before its first access to global memory, so results
+/* Programmatic dependent launch (PROCESS-WIDE, as tf_set_sm_margin): 1 for all quantize, rmsnorm, GEMM and split-K reduction kernels, 0 for
+ * none, -1 (what is in force until the first call) for short ones, as long as the SM margin is 0: GEMMs of at most 256 rows (with one CTA per
+ * tile only if all tiles run at once), row kernels of at most 4 rows, the quantizer of tf_quantize_nvfp4_dynamic up to 2^24 elements. Such a kernel may be
+ * scheduled while the kernel before it on the stream is still draining; each waits (griddepcontrol.wait) for that kernel to complete before its first access to global memory, so results
  * are unchanged. It hides launch latency and kernel set-up in chains of short kernels (small M, decode, many GPUs). No
  * counterpart in the reference. */
 TF_API tf_status tf_set_programmatic_launch(int32_t enabled);
@@ -222,7 +222,7 @@ TF_API tf_status tf_gemm_blockscaled_partials(const void* a_codes, const void* a
 
 /* How tf_gemm_blockscaled launches a problem under the settings in force, for tests and profiles (no counterpart in the reference): form[0] = 0
  * one CTA per tile, 1 K ranges as planes of the workspace and a reduction launch, 2 K ranges over a cluster of CTAs, 3 a pair of CTAs per
- * 256 x 256 tile; form[1] = accumulator columns of a tile (of one CTA); form[2] = K ranges. */
+ * 256 x 256 tile; form[1] = accumulator columns of a tile (of one CTA); form[2] = K ranges; form[3] = 1 for a programmatic dependent. */
 TF_API tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue, int32_t* form);
 
 /* The GEMM with a scattered output: the tensor-parallel second GEMM (w_d split along K) whose epilogue delivers each row block of

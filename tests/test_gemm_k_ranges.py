@@ -38,7 +38,26 @@ def test_cta_pairs_are_left_beside_a_margin(margin, fmt, m, n, k, epi):
     """A pair of CTAs needs two neighbouring SMs, which the kernel beside it need not leave whole."""
     from tilefish_b200 import kernels as K
 
-    assert K.gemm_launch_form(m, n, k, fmt, epi) == ("pair", 256, 1)
+    assert K.gemm_launch_form(m, n, k, fmt, epi)[:3] == ("pair", 256, 1)
     for sms in (1, 16, 64):
         margin(sms)
-        assert K.gemm_launch_form(m, n, k, fmt, epi) == ("tiles", 256, 1)
+        assert K.gemm_launch_form(m, n, k, fmt, epi)[:3] == ("tiles", 256, 1)
+
+
+def test_programmatic_launch_can_be_switched_off_and_stays_off_beside_a_margin(margin):
+    """Waiting CTAs of a dependent GEMM would take the SMs that the margin leaves to another kernel."""
+    from tilefish_b200 import kernels as K
+
+    dependent = lambda m: K.gemm_launch_form(m, 6144, 2560, "mxfp8")[3]  # noqa: E731
+    try:
+        assert dependent(16) and not dependent(512)
+        margin(16)
+        assert not dependent(16)
+        K.set_programmatic_launch(True)
+        assert dependent(16) and dependent(512)
+        margin(0)
+        K.set_programmatic_launch(False)
+        assert not dependent(16)
+    finally:
+        K.set_programmatic_launch(None)
+    assert dependent(16)

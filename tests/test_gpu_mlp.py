@@ -174,7 +174,7 @@ def test_programmatic_launch_gives_the_same_bytes(fmt, m):
             torch.cuda.synchronize()
             assert torch.equal(y2, y0) and torch.equal(res2, res0)
     finally:
-        K.set_programmatic_launch(False)
+        K.set_programmatic_launch(None)
     assert _native.device_status() == (0, 0)
 
 

@@ -33,9 +33,12 @@ int sm_count() {
   return cached;
 }
 
-static std::atomic<int> g_programmatic_launch{0};  // process-wide (tf_set_programmatic_launch)
-bool programmatic_launch_enabled() { return g_programmatic_launch.load(std::memory_order_relaxed) != 0; }
-void set_programmatic_launch(bool on) { g_programmatic_launch.store(on ? 1 : 0, std::memory_order_relaxed); }
+static std::atomic<int> g_programmatic_launch{-1};  // process-wide (tf_set_programmatic_launch)
+bool dependent_launch(bool chain) {
+  const int setting = g_programmatic_launch.load(std::memory_order_relaxed);
+  return setting > 0 || (setting < 0 && chain && sm_margin() == 0);
+}
+void set_programmatic_launch(int setting) { g_programmatic_launch.store(setting, std::memory_order_relaxed); }
 
 }  // namespace tf
 
@@ -45,7 +48,7 @@ extern "C" {
 
 tf_status tf_set_programmatic_launch(int32_t enabled) {
   tf::clear_error();
-  tf::set_programmatic_launch(enabled != 0);
+  tf::set_programmatic_launch(enabled == -1 ? -1 : enabled != 0);
   return TF_OK;
 }
 

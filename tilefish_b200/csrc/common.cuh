@@ -39,14 +39,19 @@ tf_status scale_padding(void* scales, int32_t format, int64_t rows, int64_t k, i
 // Programmatic dependent launch (tf_set_programmatic_launch): a kernel launched through launch_dependent() may be scheduled
 // while the kernel before it on the stream is still draining, so that its launch latency and set-up overlap that tail. Every
 // kernel launched this way executes griddep_wait() before its first access to global memory, which blocks until the previous
-// kernel has completed and its writes are visible. Off: a plain stream-ordered launch, but for chains of short kernels (`chain`, see
-// chain_gemm_launch), where the overlap is worth more than it costs.
-bool programmatic_launch_enabled();
-void set_programmatic_launch(bool on);
+// kernel has completed and its writes are visible. Three settings: never, always, or (until the caller says otherwise) for chains of short
+// kernels only (`chain`, see chain_gemm_launch), and those only without an SM margin: a dependent GEMM's waiting CTAs would take the
+// SMs that the margin leaves to the kernel beside it.
+int sm_margin();
+bool dependent_launch(bool chain);
+void set_programmatic_launch(int setting);  // 0 never, 1 always, -1 the rule
 
 #ifdef __CUDACC__
-// Launched as programmatic dependents whatever the switch says: GEMMs of one wave and at most 256 rows, and the row kernels of at most
-// four rows. A GEMM's CTAs take a whole SM each, so starting early only hides their set-up. A row kernel's CTAs are small: started
+// The rule: GEMMs of at most 256 rows (one CTA per tile: of one wave), row kernels of at most four rows, and the nvfp4 quantizer behind its
+// own amax launch up to 16 M elements (launch_quantize). A GEMM's CTAs take a whole SM each, so starting early only hides their set-up: 200
+// GEMMs back to back on a full queue, plain -> dependent: mxfp8 1 x 2560 x 3072 8.2 -> 5.9 us, 128 x 6144 x 2560 11.6 -> 9.0, nvfp4
+// 64 x 8192 x 28672 36.7 -> 32.9; pairs in two waves mxfp4 256 x 16384 x 2048 + gate 20.5 -> 17.2, mxfp8 256 x 28672 x 2048 22.5 -> 20.6; one CTA per tile in
+// two waves nvfp4 64 x 28672 x 8192 + gate 52.2 -> 52.1, left plain. A row kernel's CTAs are small: started
 // early they all pile onto the few SMs that the GEMM in front leaves free and then share those (70B-shaped decode at 64 rows: its
 // rmsnorm launch went from 9.8 to 14.7 us; two blocks at 16 rows 184.6 us without, 190.4 with). Above 256 rows the waiting CTAs
 // take the registers that the rest of the row kernel in front needs (README block at 8192 rows 189.5 -> 196.2 us).
@@ -66,7 +71,7 @@ inline cudaError_t launch_dependent(bool chain, void (*kernel)(KArgs...), dim3 g
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = chain || programmatic_launch_enabled() ? 1 : 0;
+  cfg.numAttrs = dependent_launch(chain) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 #endif

@@ -1311,7 +1311,7 @@ static tf_status make_operand_map(CUtensorMap* map, const void* base, int64_t ro
 
 // SMs the persistent GEMM leaves free (for a collective running beside it in another stream).
 static std::atomic<int> g_sm_margin{0};  // process-wide (tf_set_sm_margin); atomic so that a concurrent reader sees the old or the new value
-static int sm_margin() { return g_sm_margin.load(std::memory_order_relaxed); }
+int sm_margin() { return g_sm_margin.load(std::memory_order_relaxed); }
 static int gemm_sms() {
   const int n = sm_count() - sm_margin();
   return n < 2 ? 2 : n;
@@ -1392,7 +1392,7 @@ static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmP
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = chain_gemm_launch(p.m) || programmatic_launch_enabled() ? 2 : 1;
+    cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m)) ? 2 : 1;
     TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
     return TF_OK;
   }
@@ -1468,7 +1468,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = chain_gemm_launch(p.m) || programmatic_launch_enabled() ? 2 : 1;
+  cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m)) ? 2 : 1;
   TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tsa, tsb, to, p));
   return TF_OK;
 }
@@ -1728,9 +1728,12 @@ tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, i
                "%s: bad argument", __func__);
   const int64_t k_bytes = format == TF_FMT_MXFP8 ? k : k / 2;
   const LaunchPlan lp = launch_plan(m, n, k_bytes, epilogue, split_plan(m, n, k_bytes, epilogue));
+  const int64_t n_acc = epilogue == TF_EPI_SILU_GATE ? 2 * n : n;
+  const int64_t tiles = (m + kBlockM - 1) / kBlockM * ((n_acc + lp.block_n - 1) / lp.block_n) * lp.splits;
   form[0] = use_pair_kernel(m, n, epilogue, lp) ? kFormPair : lp.form;
   form[1] = lp.block_n;
   form[2] = lp.splits;
+  form[3] = dependent_launch(chain_gemm_launch(m) && (form[0] >= kSplitCluster || tiles <= gemm_sms()));
   return TF_OK;
 }
 

@@ -327,10 +327,11 @@ def silu_gate(t, up=None, *, out=None, stream=None):
     return out
 
 
-def set_programmatic_launch(enabled: bool) -> None:
+def set_programmatic_launch(enabled: Optional[bool]) -> None:
     """Process-wide: launch this library's kernels as programmatic dependents (each may be scheduled while its predecessor on
-    the stream drains, and waits for it before touching memory). Same results; hides launch latency in chains of short kernels."""
-    N.check(N.load().tf_set_programmatic_launch(1 if enabled else 0), "tf_set_programmatic_launch")
+    the stream drains, and waits for it before touching memory). Same results; hides launch latency in chains of short kernels.
+    True: all of them; False: none; None (the state a process starts in): chains of short kernels, without an SM margin."""
+    N.check(N.load().tf_set_programmatic_launch(-1 if enabled is None else 1 if enabled else 0), "tf_set_programmatic_launch")
 
 
 def gemm_workspace_bytes(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> int:
@@ -455,12 +456,12 @@ def gemm_splits(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> int
     return int(N.load().tf_gemm_splits(m, n, k, FORMATS[fmt], EPILOGUES[epilogue]))
 
 
-def gemm_launch_form(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> Tuple[str, int, int]:
+def gemm_launch_form(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> Tuple[str, int, int, bool]:
     """How the GEMM launches this problem under the settings in force: ("tiles" | "planes" | "cluster" | "pair", accumulator columns of a
-    tile, K ranges)."""
-    form = (ctypes.c_int32 * 3)()
+    tile, K ranges, launched as a programmatic dependent)."""
+    form = (ctypes.c_int32 * 4)()
     N.check(N.load().tf_gemm_launch_form(m, n, k, FORMATS[fmt], EPILOGUES[epilogue], form), "tf_gemm_launch_form")
-    return ("tiles", "planes", "cluster", "pair")[form[0]], form[1], form[2]
+    return ("tiles", "planes", "cluster", "pair")[form[0]], form[1], form[2], bool(form[3])
 
 
 class SplitKPartials:
