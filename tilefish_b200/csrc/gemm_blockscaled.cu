@@ -27,6 +27,7 @@
 #include <atomic>
 #include <cstdlib>
 
+#include "ask_once.h"
 #include "async_copy.cuh"
 #include "quant_core.cuh"
 
@@ -1502,14 +1503,13 @@ static bool use_pair_kernel(int64_t m, int64_t n, int epilogue, const LaunchPlan
 }
 
 // How many clusters of `splits` GEMM CTAs (one CTA fills an SM) the current device runs at once: a cluster lives inside one GPC, so
-// this is less than SMs / splits (measured on B200: 47 clusters of 3 or fewer, where 48 would need 144 of the 148 SMs). Asked once.
+// this is less than SMs / splits (measured on B200: 47 clusters of 3 or fewer, where 48 would need 144 of the 148 SMs).
 static int cluster_capacity(int splits) {
   constexpr int kMaxDevices = 64;
-  static std::atomic<int> cached[kMaxDevices][kMaxClusterSplits + 1];  // 0: not asked yet; else capacity + 1
+  static std::atomic<int> cached[kMaxDevices][kMaxClusterSplits + 1];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-  int c = cached[dev][splits].load(std::memory_order_relaxed);
-  if (c == 0) {
+  return ask_once(cached[dev][splits], [splits]() -> int {
     using Cfg = TileCfg<TF_FMT_MXFP8, 128>;
     auto kernel = gemm_blockscaled_kernel<TF_FMT_MXFP8, 128, TF_EPI_NONE, kSplitCluster>;
     cudaLaunchConfig_t cfg = {};
@@ -1527,12 +1527,10 @@ static int cluster_capacity(int splits) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
-      n = 0;
+      return -1;
     }
-    c = n + 1;
-    cached[dev][splits].store(c, std::memory_order_relaxed);
-  }
-  return c - 1;
+    return n;
+  });
 }
 
 // The launch plan: `sp` as it stands, or 128-column tiles, or (kSplitCluster) each tile cut over a cluster of CTAs, whichever the model
