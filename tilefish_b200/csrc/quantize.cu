@@ -219,31 +219,19 @@ __global__ void __launch_bounds__(kStreamThreads) stream_amax_kernel(const uint8
   }
 }
 
-// Whether the streaming form serves this tensor: dense, and at least two chunks per SM.
-static bool use_stream(int64_t m, int64_t k, int64_t ldx) {
-  return (ldx == k || m == 1) && m * (k >> 4) >= 2 * (int64_t)sm_count() * kStreamChunkVecs;
-}
-
-// max |x| over the tensor as the f32 bit pattern of a bf16 magnitude: 256-bit loads, four in flight per thread.
-__global__ void __launch_bounds__(256) amax_bits_kernel(const uint8_t* __restrict__ x, int64_t m, int nvec, int64_t ldx,
-                                                        unsigned int* __restrict__ out_bits, unsigned int* __restrict__ partials) {
+// The amax of a dense tensor too small for the ring: 256-bit loads, four in flight per thread. Result as stream_amax_kernel's.
+__global__ void __launch_bounds__(256) amax_bits_kernel(const uint8_t* __restrict__ x, int64_t total, unsigned int* __restrict__ out_bits,
+                                                        unsigned int* __restrict__ partials) {
   griddep_launch_dependents();
   uint32_t acc = 0;  // two packed 16-bit maxima
-  const int64_t total = m * nvec;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const bool dense = ldx == (int64_t)nvec * 16;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
     uint32_t v[4][8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int64_t i = i0 + j * stride;
       if (i < total) {
-        int64_t off = i * 32;
-        if (!dense) {
-          const int64_t row = i / nvec;
-          off = (row * ldx + (i - row * nvec) * 16) * 2;
-        }
-        load_256(x + off, v[j]);
+        load_256(x + i * 32, v[j]);
       } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[j][e] = 0;
@@ -257,6 +245,35 @@ __global__ void __launch_bounds__(256) amax_bits_kernel(const uint8_t* __restric
   else if (threadIdx.x == 0 && mx) atomicMax(out_bits, mx << 16);
 }
 
+// The amax of rows with a stride (column slices), bound by HBM: the quantizer's walk over the rows. A flat index over the vectors costs a 64-bit
+// division for each. Flat index -> here, tf_nvfp4_global_scale of 65536 x 4096 out of rows of 8192 106.7 -> 82.8 us, 131072 x 1024 out of 2048 57.9 ->
+// 45.0, 2048 x 28672 out of 57344 31.0 -> 24.6, 1000 x 2080 out of 4160 8.2 -> 6.9.
+__global__ void __launch_bounds__(kQuantThreads) amax_rows_kernel(const uint8_t* __restrict__ x, int64_t m, int nvec, int64_t ldx,
+                                                                  unsigned int* __restrict__ out_bits, unsigned int* __restrict__ partials) {
+  griddep_launch_dependents();
+  uint32_t acc = 0;  // two packed 16-bit maxima
+  int begin, end;
+  row_segment(nvec, begin, end);
+  for (int64_t row0 = (int64_t)blockIdx.x * blockDim.y; row0 < m; row0 += (int64_t)gridDim.x * blockDim.y) {
+    const int64_t row = row0 + threadIdx.y;
+    const bool row_ok = row < m;
+    const uint8_t* xr = x + (row_ok ? row : 0) * ldx * 2;
+    for (int base = begin; base < end; base += kQuantUnroll * (int)blockDim.x) {
+      uint32_t v[kQuantUnroll][8];
+      bool has[kQuantUnroll];
+      load_round(xr, row_ok, base, nvec, v, has);
+#pragma unroll
+      for (int j = 0; j < kQuantUnroll; ++j) acc = amax16(v[j], acc);
+    }
+  }
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  const uint32_t mx = block_amax<kQuantThreads>(acc, tid);
+  if (tid == 0 && partials) partials[blockIdx.y * gridDim.x + blockIdx.x] = mx << 16;
+  else if (tid == 0 && mx) atomicMax(out_bits, mx << 16);
+}
+
+static void quantize_shape(int64_t m, int64_t k, int pad, int per_sm, dim3& grid, dim3& block);
+
 // nvfp4 without a given scale is two launches: an amax launch whose blocks leave their maxima, and the quantizer, which derives the scale
 // from them. Before: a memset, an amax launch with an atomic, a one-thread launch for the scale and the quantizer. Graphs of 12: 128 x
 // 4096 10.5 -> 5.7 us, 4096 x 2560 20.6 -> 14.1, 8192 x 4096 35.1 -> 30.0, 65536 x 4096 212 -> 194. One cooperative launch with a grid
@@ -268,7 +285,13 @@ static tf_status launch_amax(const char* fn, const void* x, int64_t m, int64_t k
                              cudaStream_t stream) {
   const uint8_t* xb = static_cast<const uint8_t*>(x);
   const int64_t total = m * (k >> 4);
-  if (use_stream(m, k, ldx)) {
+  if (ldx != k && m > 1) {
+    const int per_sm = kMaxAmaxBlocks / sm_count();
+    dim3 grid, block;
+    quantize_shape(m, k, 0, per_sm < kStreamCtasPerSm ? per_sm : kStreamCtasPerSm, grid, block);
+    *blocks = (int)(grid.x * grid.y);
+    amax_rows_kernel<<<grid, block, 0, stream>>>(xb, m, (int)(k >> 4), ldx, out_bits, partials);
+  } else if (total >= 2 * (int64_t)sm_count() * kStreamChunkVecs) {  // at least two chunks per SM
     int* status = device_status_words();
     if (!status) return fail(TF_ERR_CUDA, "%s: cannot locate the device status words", fn);
     static thread_local int configured_dev = -1;
@@ -287,7 +310,7 @@ static tf_status launch_amax(const char* fn, const void* x, int64_t m, int64_t k
   } else {
     const int64_t need = (total + 1023) / 1024;
     *blocks = (int)(need < kMaxAmaxBlocks ? need : kMaxAmaxBlocks);
-    amax_bits_kernel<<<*blocks, 256, 0, stream>>>(xb, m, (int)(k >> 4), ldx, out_bits, partials);
+    amax_bits_kernel<<<*blocks, 256, 0, stream>>>(xb, total, out_bits, partials);
   }
   TF_LAUNCH_CHECK();
   return TF_OK;
