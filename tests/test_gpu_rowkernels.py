@@ -61,11 +61,11 @@ def test_quantize_is_bit_exact(K, fmt, m, k):
 
 
 @pytest.mark.parametrize("fmt", FMTS)
-@pytest.mark.parametrize("m,k", [(300, 2048), (160, 2560), (100, 4128), (24, 28672), (297, 8192)])
+@pytest.mark.parametrize("m,k", [(300, 2048), (160, 2560), (100, 4128), (24, 28672), (297, 8192), (300, 4128), (1217, 1056)])
 def test_quantize_long_rows_streaming_form_is_bit_exact(K, fmt, m, k):
-    """Long rows: the mxfp8 quantizer and the nvfp4 amax pass stage rows of at least 2048 elements through a shared-memory ring
-    (bulk copies of 4 KB row chunks) once there are enough chunks to fill the GPU; the e2m1 quantizers keep the register form.
-    Full chunks, a ragged last chunk per row, many chunks per row, and a strided input."""
+    """The nvfp4 amax pass of a dense tensor of 1212416 elements or more (the last three shapes) goes through a shared-memory ring of flat
+    8 KB chunks, whose last one is short in two of them; smaller tensors and strided rows are read into registers. The quantizers: rows of
+    one to many rounds per thread, cut into segments where there are few, ragged ends, and a strided input."""
     x = O.outlier_input(m, k, seed=m + k)
     check_quant(K, x, fmt, "swizzled")
     wide = torch.zeros((m, k + 64), dtype=torch.bfloat16)
