@@ -165,8 +165,11 @@ def test_gemm_refusals(K):
 @pytest.mark.parametrize("m,n,k,epi", [(1, 2560, 8192, "none"), (16, 6144, 8192, "none"), (64, 1024, 8192, "none"), (32, 1536, 2560, "silu_gate"),
                                        (40, 512, 4096, "residual"), (130, 1024, 4096, "residual"), (200, 512, 8192, "silu_gate")])
 def test_gemm_small_m_takes_the_split_k_path(K, fmt, m, n, k, epi):
-    """Few output tiles and a long K: the problem is cut along K into an f32 workspace and reduced by a second kernel. Same
-    oracle, same bound; the partial sums are added in split order, so two runs give identical bytes."""
+    """Few output tiles and a long K: the problem is cut along K. The ranges meet in an f32 workspace that a second kernel reduces, or, where
+    their CTAs fit a cluster, in shared memory. Same oracle, same bound; the partial sums are added in split order, so two runs give
+    identical bytes. The workspace is asked for and checked either way."""
+    form = K.gemm_launch_form(m, n, k, fmt, epi)
+    assert form[0] == ("planes" if epi == "silu_gate" or form[2] > 8 else form[0]) and form[0] in ("planes", "cluster")
     assert K.gemm_workspace_bytes(m, n, k, fmt, epi) > 0, "this shape is meant to exercise split-K"
     rows_b = 2 * n if epi == "silu_gate" else n
     a, w = operands(m, rows_b, k, seed=m + n)
@@ -263,7 +266,7 @@ def test_a_wait_that_runs_out_is_reported_and_the_context_survives(K):
                                        (16, 1024, 4096, "none")])
 def test_gemm_quantized_output_equals_quantize_of_the_bf16_output(K, fmt, m, n, k, epi):
     """The epilogue's own MX quantization (one 32-element block per thread) against the quantizer kernel on the same bf16
-    result: codes and swizzled scale bytes (padding included) identical, with and without the bf16 copy, one-pass and split-K."""
+    result: codes and swizzled scale bytes (padding included) identical, with and without the bf16 copy, one-pass and K cut over a cluster."""
     rows_b = 2 * n if epi == "silu_gate" else n
     a, w = operands(m, rows_b, k, seed=m * 3 + n)
     qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)

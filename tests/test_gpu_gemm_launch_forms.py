@@ -21,7 +21,7 @@ def K():
 
 
 SHAPES = [(1, 2560, 3072), (33, 264, 4096), (128, 136, 2080), (129, 1000, 1024), (300, 1024, 4128), (257, 392, 8192), (700, 520, 2048), (1024, 1024, 512),
-          (200, 2048, 1024), (513, 4104, 288), (1100, 3104, 544)]
+          (200, 2048, 1024), (513, 4104, 288), (1100, 3104, 544), (100, 20512, 288), (300, 12512, 160)]
 
 
 @pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
@@ -38,12 +38,75 @@ def test_every_form_meets_the_oracle(K, fmt, m, n, k):
     assert bool((wide[:, n:] == -7.0).all()) and float(amax) == float(out.float().abs().max())
     r = res.cuda()
     again = K.gemm_blockscaled(qa, qb, epilogue="residual", residual=r)
+    assert float((again.cpu().float() - ref).abs().max()) <= TOL * float(ref.abs().max())
+    if K.gemm_launch_form(m, n, k, fmt)[2] == K.gemm_launch_form(m, n, k, fmt, "residual")[2]:  # the same K ranges, the same sums
+        assert torch.equal(again, out)
     assert torch.equal(again, K.gemm_blockscaled(qa, qb, epilogue="residual", residual=res.cuda())), "deterministic"
     assert torch.equal(r.cpu(), res + again.cpu().float())
     if fmt != "nvfp4" and n % 32 == 0:
         o, q = K.gemm_blockscaled(qa, qb, quantize_out=True)
         ref_q = K.quantize(o, fmt)
         assert torch.equal(q.codes, ref_q.codes) and torch.equal(q.scales, ref_q.scales)
+
+
+def test_the_shapes_above_take_every_form(K):
+    forms = {fmt: [K.gemm_launch_form(m, n, k, fmt, epi)[:2] for m, n, k in SHAPES for epi in ("none", "residual")] for fmt in ("mxfp8", "mxfp4", "nvfp4")}
+    for got in forms.values():
+        assert {("tiles", 128), ("tiles", 256), ("cluster", 128), ("pair", 256)} <= set(got)
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
+@pytest.mark.parametrize("m,n,k", [(2600, 3592, 544), (2600, 3624, 288)])
+def test_pairs_that_take_more_than_one_tile(K, fmt, m, n, k):
+    """165 tiles on 74 pairs: the second accumulator, its held columns and the staging boxes' reuse, with every epilogue, against the oracle."""
+    assert K.gemm_launch_form(m, n, k, fmt)[0] == K.gemm_launch_form(m, n, k, fmt, "residual")[0] == "pair"
+    a, w = O.randn((m, k), m, torch.bfloat16), O.randn((n, k), n, torch.bfloat16, scale=k**-0.5)
+    qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)
+    oa, ob = O.quantize(a, fmt), O.quantize(w, fmt)
+    ref = O.dequantize(oa[0], oa[1], fmt, oa[2]) @ O.dequantize(ob[0], ob[1], fmt, ob[2]).t()
+    res, amax = O.randn((m, n), 7), torch.zeros(1, device="cuda")
+    r = res.cuda()
+    wide = torch.full((m, n + 16), -7.0, dtype=torch.bfloat16, device="cuda")
+    out = K.gemm_blockscaled(qa, qb, epilogue="residual", residual=r, out=wide[:, :n], amax_out=amax)
+    assert float((out.cpu().float() - ref).abs().max()) <= TOL * float(ref.abs().max())
+    assert bool((wide[:, n:] == -7.0).all()) and float(amax) == float(out.float().abs().max())
+    assert torch.equal(r.cpu(), res + out.cpu().float())
+    assert torch.equal(K.gemm_blockscaled(qa, qb), out)
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
+def test_gated_pairs_that_take_more_than_one_tile(K, fmt):
+    m, f, k = 2600, 1920, 544
+    assert K.gemm_launch_form(m, f, k, fmt, "silu_gate")[0] == "pair"
+    a, w = O.randn((m, k), m, torch.bfloat16), O.randn((2 * f, k), f, torch.bfloat16, scale=k**-0.5)
+    qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)
+    oa, ob = O.quantize(a, fmt), O.quantize(w, fmt)
+    t = O.f32_to_bf16(O.dequantize(oa[0], oa[1], fmt, oa[2]) @ O.dequantize(ob[0], ob[1], fmt, ob[2]).t())
+    out = K.gemm_blockscaled(qa, qb, epilogue="silu_gate")
+    top = float(t.float().abs().max())
+    # the bound of the gate test below, and the unfused kernels on the same sums bit for bit
+    assert float((out.cpu().float() - O.silu_gate(t[:, :f], t[:, f:]).float()).abs().max()) <= 2 * TOL * top * (top + 1.0)
+    assert torch.equal(K.silu_gate(K.gemm_blockscaled(qa, qb)), out)
+    if fmt != "nvfp4":
+        o, q = K.gemm_blockscaled(qa, qb, epilogue="silu_gate", quantize_out=True)
+        ref = K.quantize(o, fmt)
+        assert torch.equal(o, out) and torch.equal(q.codes, ref.codes) and torch.equal(q.scales, ref.scales)
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4"])
+@pytest.mark.parametrize("m,n,k", [(40, 1056, 16384), (5, 288, 28672), (64, 8192, 28672)])
+def test_the_planes_reduction_quantizes_its_output(K, fmt, m, n, k):
+    """Planes and the reduction launch (more ranges than a cluster holds, or more tiles than clusters fit): the quantized copy and the
+    padding of its scales, over a buffer that held other bytes."""
+    assert K.gemm_launch_form(m, n, k, fmt)[0] == "planes"
+    qa = K.quantize(O.randn((m, k), m, torch.bfloat16).cuda(), fmt)
+    qb = K.quantize(O.randn((n, k), n, torch.bfloat16, scale=k**-0.5).cuda(), fmt)
+    dirty = K.BlockScaledTensor(fmt, (m, n), torch.empty((m, n // K.ELEMS_PER_BYTE[fmt]), dtype=torch.uint8, device="cuda"),
+                                torch.full((K.scale_bytes(fmt, m, n),), 0xA5, dtype=torch.uint8, device="cuda"))
+    out, q = K.gemm_blockscaled(qa, qb, q_out=dirty)
+    codes, scales, _ = O.quantize(out.cpu(), fmt)
+    assert torch.equal(out, K.gemm_blockscaled(qa, qb))
+    assert torch.equal(q.codes.cpu(), codes) and torch.equal(q.scales.cpu(), O.swizzle_scales(scales))
 
 
 @pytest.mark.parametrize("fmt", ["mxfp8", "nvfp4"])
