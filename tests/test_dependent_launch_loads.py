@@ -26,3 +26,9 @@ def test_nothing_a_predecessor_may_write_is_read_non_coherently(name):
     text = code(name)
     assert "ld.global.nc" not in text
     assert set(re.findall(r"__ldg\(([^)]*)\)", text)) <= {"w + v"}  # the norm weights
+
+
+def test_the_aligned_cluster_barrier_is_reached_by_whole_warps():
+    text = code("gemm_blockscaled.cu")
+    assert len(re.findall(r"barrier\.cluster\.(?:arrive|wait)", text)) == 2  # both in one place
+    assert re.search(r"void cluster_sync_all\(\) \{\s*__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.arrive", text)
