@@ -1487,9 +1487,9 @@ static int two_cta_forced() {
 }
 
 // Whether the 2-CTA kernel serves this problem (TF_GEMM_TWO_CTA in the environment: 0 never, 1 wherever it can, unset this rule).
-// Per wave of tiles the pair is 5-13 % faster than the one-CTA kernel (measured on B200, one-CTA -> pair: nvfp4 4096 x 8192 x 28672
-// 385 -> 336 us, 4096 x 28672 x 8192 + gate 713 -> 666, 4096 x 6144 x 2560 35.1 -> 33.2; mxfp8 8192 x 6144 x 2560 106 -> 98.8;
-// mxfp4 300 x 8192 x 4096 12.8 -> 12.1), but its row blocks are 256 high: it is left where that costs a tenth more waves.
+// Per wave of tiles the pair is 6-9 % faster than the one-CTA kernel (B200 after a second of load, one-CTA -> pair: nvfp4 4096 x 8192 x 28672
+// 434 -> 400 us, 4096 x 28672 x 8192 + gate 836 -> 779, 4096 x 6144 x 2560 41.2 -> 37.9; mxfp8 8192 x 6144 x 2560 125.4 -> 117.7; problems of one wave 0-8 %,
+// 14 of 15, mxfp8 512 x 3072 x 2560 + gate 14.1 -> 14.5), but its row blocks are 256 high: it is left where that costs a tenth more waves.
 // Beside a margin it is left too: a pair needs two SMs of one TPC, and the kernel that the margin is for need not leave them whole. CTAs
 // of 200 KB that start beside a quantizer split 4 to 12 pairs; with 16 pairs split, nvfp4 2048 x 14336 x 8192 + gate takes 303 us on pairs and 199 on
 // single CTAs at margin 16 (342 and 217 at 32), since tiles are dealt out statically. With none split it is 184 and 203.
@@ -1539,8 +1539,8 @@ static int cluster_capacity(int splits) {
 // below says is shortest. Microseconds beyond a launch's fixed 4.4, fitted to B200 measurements of graphs of 24 launches:
 //   a K stage takes 0.235 with 128-column tiles and 0.38 with 256 (bound by shared-memory reads and fills), a tile's epilogue 0.5 / 1.0;
 //   planes and a reduction launch 2.0 + 8 bytes per partial sum at 3 TB/s; a cluster 1.6 + its remote reads at 26.6 GB/s per SM.
-// before -> after: mxfp8 512 x 2560 x 3072 13.5 -> 11.2 us (128-column tiles), 128 x 2560 x 3072 12.4 -> 10.2 (4 ranges), 1 x 2560 x 3072
-// 7.3 -> 6.2 (6), 700 x 1024 x 16384 43.0 -> 23.2 (2), mxfp4 300 x 1024 x 8192 residual 27.0 -> 11.0 (3).
+// One form for all -> the plan: mxfp8 512 x 2560 x 3072 13.7 -> 10.9 us (128-column tiles), 128 x 2560 x 3072 12.3 -> 9.8 (4 ranges), 1 x 2560 x 3072
+// 7.8 -> 5.9 (6), 700 x 1024 x 16384 51.6 -> 23.8 (2), mxfp4 300 x 1024 x 8192 residual 27.7 -> 12.7 (5).
 // A problem with a planes plan keeps that plan's K ranges in every form, so that its result is the sum of the planes bit for bit.
 // The plan is made for the whole device, whatever margin is set (tf_set_sm_margin): K ranges are part of a result, so they may not depend on
 // it. Beside a margin a cluster launch takes the SMs it was planned for; the tile width, which no sum depends on, follows the free SMs.
