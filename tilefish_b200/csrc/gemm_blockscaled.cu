@@ -108,6 +108,7 @@ struct GemmParams {
   int q_pad;      // the scales have padding that this launch zeroes (by the epilogue warps, while they wait for the first tile)
   int a_gs_rows;  // 0: a has one global scale; else a_gs[row / a_gs_rows] (row blocks quantized separately, e.g. gathered from ranks)
   int a_box_bytes;  // bytes one A load brings per stage: 128 bytes x the rows of its box (fewer than 128 rows when M is small)
+  int early_stages;  // K stages of B that a CTA asks into L2 while it waits for the kernel in front (0: none), see prefetch_b_stage
   // Scattered output (tf_gemm_blockscaled_scatter): rows [i * scatter_rows, (i + 1) * scatter_rows) go to scatter_out[i], a
   // [scatter_rows, n] matrix with leading dimension ldo that may live in another GPU's memory (plain stores over NVLink).
   // scatter_rows is a multiple of 128, so a tile has one destination. 0: everything goes to `out`.
@@ -760,6 +761,37 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
   }
 }
 
+// ---- L2 prefetch of the weights ---------------------------------------------------------------------------------------------
+// A dependent of at most 128 rows streams its weights once, and HBM is idle while it waits: the row kernels between two GEMMs of a decode
+// step touch a few MB. So a waiting CTA asks its first stages of B and their scales into L2. Nothing is read here: the lines are coherent
+// with what the kernel in front may still write (it may be the one that quantizes these weights), and the loads behind griddep_wait()
+// read them as they would without. 70B-shaped NVFP4 blocks, us per captured step, plain -> dependent -> with this: 64 rows, 4 layers
+// 394.6 -> 389.2 -> 378.5; 16 rows, 2 layers 187.2 -> 185.1 -> 183.0; 128 rows, 2 layers 214.4 -> 212.0 -> 209.2; MXFP8 block 64 x 4096 x 8192
+// 41.1 -> 41.0 -> 39.6. More stages give the first of these up to 1 % and cost others as much (MXFP8 64 x 8192 x 14336 164.4 at 6, 168.1 at 24): the
+// SM's copy engine serves the prefetch before the loads (about 2.7 clocks per 128-byte row), which is also why prefetching ahead inside the main loop
+// or for other CTAs' tiles loses (53.4 against 50.6 us, 64 x 28672 x 8192 + gate; 2 to 3 us per layer).
+constexpr int kEarlyStages = 8;
+constexpr unsigned kEarlyStageNs = 300;  // pause between two stages: 36 KB per SM and pause is more than HBM brings
+__device__ __forceinline__ void l2_prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void l2_prefetch_bulk(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+template <int FMT, int BLOCK_N, int EPI>
+__device__ __forceinline__ void prefetch_b_stage(const GemmParams& p, const CUtensorMap* tma_b, int n_blk, int ks) {
+  constexpr int kST = TileCfg<FMT, BLOCK_N>::kST;
+  const int sf_tiles = min(p.sf_col_tiles - ks * kST, kST);
+#pragma unroll
+  for (int nb = 0; nb < TileCfg<FMT, BLOCK_N>::kNB; ++nb) {
+    const int row = (EPI == TF_EPI_SILU_GATE) ? nb * p.n + n_blk * 128 : n_blk * BLOCK_N + nb * 128;
+    if (row < p.n_rows_b) {
+      l2_prefetch_2d(tma_b, ks * kStageKBytes, row);
+      l2_prefetch_bulk(p.sfb + ((int64_t)(row >> 7) * p.sf_col_tiles + ks * kST) * 512, (uint32_t)sf_tiles * 512u);
+    }
+  }
+}
+
 // ---- the kernel ------------------------------------------------------------------------------------------------------------
 // SPLITK: kSplitNone; kSplitPlanes: every (tile, K range) is a unit of its own and leaves its accumulator in the workspace;
 // kSplitCluster: a cluster of `splits` CTAs per tile, launched with exactly one tile per cluster.
@@ -791,6 +823,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - smem_base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + (abort_slot - smem_base));
+  volatile int* started_flag = abort_flag + 1;  // the kernel in front has completed
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   griddep_launch_dependents();  // the next kernel on the stream may be scheduled; it waits for this one before touching memory
@@ -803,6 +836,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     mbar_init(bar_tmem_full, 1);
     mbar_init(bar_tmem_empty, 8);  // every epilogue warp, once it holds its share of the columns both accumulators cover
     *abort_flag = 0;
+    *started_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // whole warp: allocate tensor memory
@@ -813,6 +847,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  if (p.early_stages > 0 && warp == 10) {
+    // stage by stage until warp 0 is through its wait (not by a load warp, which must not be late for its own wait)
+    int left = p.early_stages;
+    for (int tile = blockIdx.x; tile < p.num_tiles && left > 0; tile += gridDim.x) {
+      const int split = SPLITK == kSplitPlanes ? tile / (p.m_blocks * p.n_blocks) : kCluster ? tile % p.splits : 0;
+      const int n_blk = (SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile) / p.m_blocks;
+      const int ks_end = min((split + 1) * p.k_stages_per_split, p.num_k_stages);
+      for (int ks = split * p.k_stages_per_split; ks < ks_end && left > 0; ++ks, --left) {
+        if (*started_flag) left = 0;
+        if (left > 0 && lane == 0) prefetch_b_stage<FMT, BLOCK_N, EPI>(p, &tma_b, n_blk, ks);
+        __syncwarp();
+        if (left > 0) __nanosleep(kEarlyStageNs);
+      }
+    }
+  }
   griddep_wait();  // barriers and tensor memory are set up; nothing of global memory was touched before the previous kernel is done
 
   if (warp == 0 || warp == 6) {
@@ -820,6 +869,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     // The whole warp runs the loops; lane 0 serves the A side, lane 1 + nb the 128-row half nb of the B tile, so that one
     // instruction per stage issues all of the warp's copies.
     const bool scales = warp == 6;
+    if (!scales && lane == 0) *started_flag = 1;
     const int nb = lane - 1;
     int stage = 0;
     uint32_t phase = 0;
@@ -1381,9 +1431,12 @@ static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmP
   constexpr int out_cols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;
   p.n_blocks = (p.n + out_cols - 1) / out_cols;
   p.num_tiles = p.m_blocks * p.n_blocks * p.splits;
+  const int grid = SPLITK == kSplitCluster || p.num_tiles < gemm_sms() ? p.num_tiles : gemm_sms();
+  const bool dependent = dependent_launch(chain_gemm_launch(p.m, p.num_tiles <= grid));
+  if (dependent && p.m <= kBlockM) p.early_stages = kEarlyStages;
   if (SPLITK == kSplitCluster) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.num_tiles);
+    cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     cfg.stream = stream;
@@ -1395,12 +1448,11 @@ static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmP
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m)) ? 2 : 1;
+    cfg.numAttrs = dependent ? 2 : 1;
     TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
     return TF_OK;
   }
-  const int grid = p.num_tiles < gemm_sms() ? p.num_tiles : gemm_sms();
-  TF_CUDA(launch_dependent(chain_gemm_launch(p.m) && p.num_tiles <= grid, kernel, dim3(grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, ta, tb, p));
+  TF_CUDA(launch_dependent(dependent, kernel, dim3(grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, ta, tb, p));
   return TF_OK;
 }
 
@@ -1471,7 +1523,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m)) ? 2 : 1;
+  cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m, true)) ? 2 : 1;
   TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tsa, tsb, to, p));
   return TF_OK;
 }
@@ -1733,7 +1785,7 @@ tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, i
   form[0] = use_pair_kernel(m, n, epilogue, lp) ? kFormPair : lp.form;
   form[1] = lp.block_n;
   form[2] = lp.splits;
-  form[3] = dependent_launch(chain_gemm_launch(m) && (form[0] >= kSplitCluster || tiles <= gemm_sms()));
+  form[3] = dependent_launch(chain_gemm_launch(m, form[0] >= kSplitCluster || tiles <= gemm_sms()));
   return TF_OK;
 }
 
@@ -1833,6 +1885,7 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
   p.q_pad = 0;
   p.a_gs_rows = (int)a_global_scale_rows;
   p.a_box_bytes = a_box_rows * kStageKBytes;
+  p.early_stages = 0;
   p.scatter_rows = 0;
   for (int i = 0; i < 8; ++i) p.scatter_out[i] = nullptr;
   const SplitPlan sp = split_plan(m, n, k_bytes, epilogue);
