@@ -765,11 +765,12 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
 // A dependent of at most 128 rows streams its weights once, and HBM is idle while it waits: the row kernels between two GEMMs of a decode
 // step touch a few MB. So a waiting CTA asks its first stages of B and their scales into L2. Nothing is read here: the lines are coherent
 // with what the kernel in front may still write (it may be the one that quantizes these weights), and the loads behind griddep_wait()
-// read them as they would without. 70B-shaped NVFP4 blocks, us per captured step, plain -> dependent -> with this: 64 rows, 4 layers
-// 394.6 -> 389.2 -> 378.5; 16 rows, 2 layers 187.2 -> 185.1 -> 183.0; 128 rows, 2 layers 214.4 -> 212.0 -> 209.2; MXFP8 block 64 x 4096 x 8192
-// 41.1 -> 41.0 -> 39.6. More stages give the first of these up to 1 % and cost others as much (MXFP8 64 x 8192 x 14336 164.4 at 6, 168.1 at 24): the
-// SM's copy engine serves the prefetch before the loads (about 2.7 clocks per 128-byte row), which is also why prefetching ahead inside the main loop
-// or for other CTAs' tiles loses (53.4 against 50.6 us, 64 x 28672 x 8192 + gate; 2 to 3 us per layer).
+// read them as they would without. 70B-shaped NVFP4 blocks under sustained load, us per captured step, plain -> dependent -> with this: 64 rows, 4 layers
+// 402 -> 396 -> 391.5; 16 rows, 2 layers 189.4 -> 187.2 -> 186.3; 128 rows, 2 layers 221.5 -> 219.3 -> 217.6; MXFP8 block 64 x 4096 x 8192 40.4 -> 40.0 -> 39.0;
+// MXFP4 1 x 4096 x 14336, 2 layers 68.6 -> 69.0 -> 67.7. More stages give the first of these up to 1 % and cost others as much (MXFP8 64 x 8192 x 14336
+// 174 at 8, 176 at 16): the SM's copy engine serves the prefetch before the loads (about 2.7 clocks per 128-byte row), which is also why
+// prefetching ahead inside the main loop or for other CTAs' tiles loses (64 x 28672 x 8192 + gate 50.6 -> 53.4 us; 2 to 3 us per layer).
+// It stands in the epilogue's branch: in front of the roles the same code cost every launch 0.2 us (68.6 -> 70.6 for the last of these).
 constexpr int kEarlyStages = 8;
 constexpr unsigned kEarlyStageNs = 300;  // pause between two stages: 36 KB per SM and pause is more than HBM brings
 __device__ __forceinline__ void l2_prefetch_2d(const CUtensorMap* map, int x, int y) {
@@ -847,27 +848,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  if (p.early_stages > 0 && warp == 10) {
-    // stage by stage until warp 0 is through its wait (not by a load warp, which must not be late for its own wait)
-    int left = p.early_stages;
-    for (int tile = blockIdx.x; tile < p.num_tiles && left > 0; tile += gridDim.x) {
-      const int split = SPLITK == kSplitPlanes ? tile / (p.m_blocks * p.n_blocks) : kCluster ? tile % p.splits : 0;
-      const int n_blk = (SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile) / p.m_blocks;
-      const int ks_end = min((split + 1) * p.k_stages_per_split, p.num_k_stages);
-      for (int ks = split * p.k_stages_per_split; ks < ks_end && left > 0; ++ks, --left) {
-        if (*started_flag) left = 0;
-        if (left > 0 && lane == 0) prefetch_b_stage<FMT, BLOCK_N, EPI>(p, &tma_b, n_blk, ks);
-        __syncwarp();
-        if (left > 0) __nanosleep(kEarlyStageNs);
-      }
-    }
-  }
-  griddep_wait();  // barriers and tensor memory are set up; nothing of global memory was touched before the previous kernel is done
+  // barriers and tensor memory are set up; no role touches global memory before its own griddep_wait()
 
   if (warp == 0 || warp == 6) {
     // ---------------- load warps: warp 0 the operand tiles (TMA), warp 6 the scale tiles (bulk copies) ----------------
     // The whole warp runs the loops; lane 0 serves the A side, lane 1 + nb the 128-row half nb of the B tile, so that one
     // instruction per stage issues all of the warp's copies.
+    griddep_wait();
     const bool scales = warp == 6;
     if (!scales && lane == 0) *started_flag = 1;
     const int nb = lane - 1;
@@ -923,6 +910,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     }
     __syncwarp();
   } else if (warp == 1) {
+    griddep_wait();
     // ---------------- MMA issuer ----------------
     // The whole warp runs the loops (so every value below is warp-uniform and lives in the uniform datapath); one elected lane
     // issues the tcgen05 instructions. A full stage is straight-line code: its descriptors differ from the stage's base by
@@ -1016,6 +1004,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
     }
   } else {
     // ---------------- epilogue (warps 2..5 = group 0, warps 7..10 = group 1; warp w reads lanes 32*(w%4) .. +31) ----------------
+    if (p.early_stages > 0 && warp == 10) {
+      // stage by stage until warp 0 is through its wait (not by a load warp, which must not be late for its own wait)
+      int left = p.early_stages;
+      for (int tile = blockIdx.x; tile < p.num_tiles && left > 0; tile += gridDim.x) {
+        const int split = SPLITK == kSplitPlanes ? tile / (p.m_blocks * p.n_blocks) : kCluster ? tile % p.splits : 0;
+        const int n_blk = (SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile) / p.m_blocks;
+        const int ks_end = min((split + 1) * p.k_stages_per_split, p.num_k_stages);
+        for (int ks = split * p.k_stages_per_split; ks < ks_end && left > 0; ++ks, --left) {
+          if (*started_flag) left = 0;
+          if (left > 0 && lane == 0) prefetch_b_stage<FMT, BLOCK_N, EPI>(p, &tma_b, n_blk, ks);
+          __syncwarp();
+          if (left > 0) __nanosleep(kEarlyStageNs);
+        }
+      }
+    }
+    griddep_wait();
     const int q = warp & 3;
     const int grp = warp >= 7 ? 1 : 0;
     const float alpha = (FMT == TF_FMT_NVFP4 && SPLITK == kSplitNone) ? __fmul_rn(load_f32(p.a_gs), load_f32(p.b_gs)) : 1.0f;
