@@ -1,0 +1,54 @@
+"""The quantizer's steps of eight rows x 256 columns at their edges: ragged rows and columns, rows with a stride, swizzled scales stored as words and
+as bytes (a scale pointer without 4-byte alignment), plain scales, and the round trip through the amax launch with two steps per warp. Codes
+and scales are defined bit for bit, so everything is compared exactly, and nothing around them may be written."""
+
+import pytest
+import torch
+
+from oracle import blockscaled as O
+
+pytestmark = pytest.mark.gpu
+FMTS = ["mxfp8", "mxfp4", "nvfp4"]
+
+
+@pytest.fixture(scope="module")
+def K():
+    from tilefish_b200 import kernels
+
+    kernels.require_cuda()
+    return kernels
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("layout", ["swizzled", "plain"])
+@pytest.mark.parametrize("m,k,offset", [(1, 32, 0), (2, 64, 1), (31, 288, 2), (33, 96, 4), (64, 256, 3), (97, 4128, 16), (127, 544, 0), (129, 224, 1), (257, 800, 4), (385, 2080, 0)])
+def test_against_the_oracle(K, fmt, layout, m, k, offset):
+    wide = O.randn((m, k + 48), m + k, torch.bfloat16)
+    wide[:, ::37] *= 100.0
+    x = wide[:, 16:16 + k]
+    codes, scales, gs = O.quantize(x.contiguous(), fmt)
+    scales = O.swizzle_scales(scales) if layout == "swizzled" else scales.reshape(-1)
+    n_codes, n_scales = codes.numel(), K.scale_bytes(fmt, m, k, layout)
+    codes_buf = torch.full((n_codes + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    scales_buf = torch.full((n_scales + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    out = K.BlockScaledTensor(fmt, (m, k), codes_buf[:n_codes].view(m, -1), scales_buf[offset:offset + n_scales],
+                              torch.empty(1, device="cuda") if fmt == "nvfp4" else None, layout)
+    q = K.quantize(wide.cuda()[:, 16:16 + k], fmt, layout=layout, out=out)
+    assert torch.equal(codes_buf[:n_codes].cpu().view_as(codes), codes)
+    assert torch.equal(scales_buf[offset:offset + n_scales].cpu(), scales.reshape(-1))
+    assert bool((codes_buf[n_codes:] == 0xA5).all()) and bool((scales_buf[:offset] == 0xA5).all()) and bool((scales_buf[offset + n_scales:] == 0xA5).all())
+    if fmt == "nvfp4":
+        assert q.global_scale.cpu().view(torch.int32).item() == gs.reshape(1).view(torch.int32).item()
+
+
+@pytest.mark.parametrize("m,k", [(2400, 4128), (4700, 2080), (9000, 8192), (1, 28672)])
+def test_the_scale_from_the_amax_launch(K, m, k):
+    """Blocks that take two steps (and the large case, where they start after the amax launch): the bytes of the same tensor with its scale given."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn((m, k), generator=g, device="cuda").bfloat16()
+    for scale in (1.0, 3.0e-3):
+        x.mul_(scale)
+        q = K.quantize(x, "nvfp4")
+        gs = (x.abs().max().float().cpu() / torch.tensor(2688.0)).reshape(1).cuda()  # divided on the host: one correctly rounded division
+        ref = K.quantize(x, "nvfp4", global_scale=gs)
+        assert torch.equal(q.global_scale, gs) and torch.equal(q.codes, ref.codes) and torch.equal(q.scales, ref.scales)

@@ -124,23 +124,6 @@ __device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs,
   }
 }
 
-// Stores the codes of 16 elements (vector index `vec` of 16-element vectors in row `row`) and the block's scale byte.
-template <int FMT>
-__device__ __forceinline__ void store_quantized16(uint8_t* __restrict__ codes_out, uint8_t* __restrict__ scales, int swizzled, int64_t row, int vec,
-                                                  int64_t k, const uint32_t (&codes)[4], uint32_t scale) {
-  if (FMT == TF_FMT_MXFP8) {
-    *reinterpret_cast<uint4*>(codes_out + row * k + (int64_t)vec * 16) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
-  } else {
-    *reinterpret_cast<uint2*>(codes_out + row * (k >> 1) + (int64_t)vec * 8) = make_uint2(codes[0], codes[1]);
-  }
-  if (FMT == TF_FMT_NVFP4 || (vec & 1) == 0) {
-    const int64_t cols = k / (FMT == TF_FMT_NVFP4 ? 16 : 32);
-    const int64_t c = (FMT == TF_FMT_NVFP4) ? vec : (vec >> 1);
-    const int64_t off = swizzled ? swizzled_scale_offset(row, c, (cols + 3) >> 2) : row * cols + c;
-    scales[off] = (uint8_t)scale;
-  }
-}
-
 // Zeroes the padding of a swizzled scale tensor: the rows past `rows` of the last row tile and the columns past `cols` of the last
 // column tile. Thread `first` of `stride` threads that share the work. The bytes are disjoint from the scales, so no ordering is
 // needed; a kernel that writes scales does this itself instead of a memset of the whole tensor in front of it (measured in captured

@@ -1,12 +1,8 @@
 // BlockScaled quantization row kernels (bf16 -> MXFP8 / MXFP4 / NVFP4) and the scale-layout helpers.
 //
-// HBM-bound: every thread moves four 256-bit vectors of 16 bf16 per step (coalesced: consecutive lanes, consecutive
-// vectors), block maxima are combined with at most one warp shuffle, codes leave as 16-byte (e4m3) or 8-byte (e2m1)
-// coalesced stores. Algorithmic bytes per element: 2 + 1 + 1/32 (mxfp8), 2 + 0.5 + 1/32 (mxfp4), 2 + 0.5 + 1/16 (nvfp4).
-// Four loads in flight per thread, two before, and a shared-memory ring fed by bulk copies for mxfp8 (graphs of 12 launches, ring or
-// two -> four): 65536 x 4096 mxfp8 135.2 -> 132.9 us (6.1 TB/s), mxfp4 111.7 -> 102.5 (6.6 TB/s), nvfp4 112.3 -> 104.2 (6.6 TB/s);
-// 8192 x 4096 nvfp4 17.9 -> 16.8; 16384 x 2080 mxfp8 37.5 -> 20.7. Eight loads, 64, 128 or 512 threads and streaming (evict-first)
-// stores were no better over that range.
+// HBM-bound: four 256-bit loads of 16 bf16 in flight per thread, block maxima combined with at most one warp shuffle, codes stored as 16 (e4m3)
+// or 8 bytes (e2m1) per thread, scales as whole sectors. Algorithmic bytes per element: 2 + 1 + 1/32 (mxfp8), 2 + 0.5 + 1/32 (mxfp4),
+// 2 + 0.5 + 1/16 (nvfp4).
 #include "async_copy.cuh"
 #include "quant_core.cuh"
 
@@ -15,7 +11,6 @@ namespace tf {
 constexpr int kQuantThreads = 256;
 constexpr int kQuantUnroll = 4;
 
-// Block = (TPR threads along the row) x (256 / TPR rows); rows are taken grid-stride.
 __device__ __forceinline__ void load_256(const void* p, uint32_t (&w)[8]) {
   asm volatile("ld.global.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
@@ -39,22 +34,6 @@ __device__ __forceinline__ void load_round(const uint8_t* __restrict__ xr, bool 
   }
 }
 
-// Quantizes and stores one round. All threads of the block call it with the same `base`, so the warp shuffle inside quantize_vec16
-// always sees whole warps; threads without data quantize zeros and store nothing. nvec is even and blockDim.x a power of two >= 2,
-// so the two lanes of one 32-element block have data together.
-template <int FMT>
-__device__ __forceinline__ void store_round(const uint32_t (&v)[kQuantUnroll][8], const bool (&has)[kQuantUnroll], int64_t row, int base, int nvec,
-                                            int64_t k, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int swizzled, float gs, float inv_t) {
-#pragma unroll
-  for (int j = 0; j < kQuantUnroll; ++j) {
-    if (base + j * (int)blockDim.x < nvec) {  // uniform over the block
-      uint32_t c[4], sc;
-      quantize_vec16<FMT>(v[j], gs, inv_t, c, sc);
-      if (has[j]) store_quantized16<FMT>(codes, scales, swizzled, row, base + threadIdx.x + j * (int)blockDim.x, k, c, sc);
-    }
-  }
-}
-
 // gridDim.y cuts the rows into segments of whole rounds (few, long rows: more CTAs than row blocks). The segment of this block.
 __device__ __forceinline__ void row_segment(int nvec, int& begin, int& end) {
   const int step = kQuantUnroll * (int)blockDim.x;
@@ -65,57 +44,125 @@ __device__ __forceinline__ void row_segment(int nvec, int& begin, int& end) {
 }
 
 // gs_ptr holds the nvfp4 global scale, or (gs_out != nullptr) the tensor's amax from which it is derived here: one value, or the
-// `n_partials` maxima that the blocks of an amax launch left (every block of this kernel takes their maximum again: at most 1024 words).
-// One thread = 16 consecutive bf16 (one 256-bit load); block = (TPR threads along the row) x (256 / TPR rows).
+// `n_partials` maxima that the blocks of an amax launch left (every block of a quantizer takes their maximum again: at most 1024 words).
+// All `threads` threads of the block call it.
+__device__ __forceinline__ float partials_max(const float* __restrict__ partials, int n, int tid, int threads) {
+  uint32_t mx = 0;  // non-negative floats order like their bits
+  for (int i = tid; i < n; i += threads) mx = max(mx, __float_as_uint(load_f32(partials + i)));
+  __shared__ uint32_t warp_max[kQuantThreads / 32];
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+  if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
+  __syncthreads();
+  for (int i = 0; i < threads / 32; ++i) mx = max(mx, warp_max[i]);
+  return __uint_as_float(mx);
+}
+
+// ---- the quantizer ------------------------------------------------------------------------------------------------------------
+// HBM-bound. A 32-byte sector of the swizzled scales holds 4 scales each of the rows r, r + 32, r + 64, r + 96 and of the rows behind them.
+// Where a warp walks along one row, every such sector is put together in L2 from eight 4-byte pieces of different warps, a store transaction
+// each (as many as the codes take, for nvfp4). Here a warp takes these eight rows together: in one step 16 vectors (256 elements) of each, half
+// a warp per row, four 256-bit loads in flight per thread. The scale bytes of a thread's four loads are one word; a 4 x 4 byte transpose
+// over the lanes that share a scale word (two shuffles) leaves each word in a lane of its own, and one store writes whole sectors,
+// the padding's zeros included.
+// One step per warp, so that the hardware deals the steps out: blocks that stay and walk keep every SM's loads and stores in phase. Graphs of 12,
+// rows per block with a persistent grid -> this: 65536 x 4096 mxfp8 133.5 -> 118.2 us (6.9 TB/s), mxfp4 102.8 -> 95.9 (7.1), nvfp4 105.9 -> 101.4 (6.8;
+// with its amax launch 195 -> 187); 4096 x 28672 59.2 -> 53.5, 48.4 -> 44.1, 50.9 -> 46.6; 8192 x 4096 18.5 -> 17.3, 16.4 -> 15.2, 17.5 -> 16.2; 1000 x 2720
+// 3.7 -> 2.9, 3.8 -> 2.9, 4.0 -> 3.2; 64 x 28672 3.4 -> 2.7, 3.4 -> 2.6, 3.8 -> 2.9; 1 x 4096 2.6 -> 1.7, 2.6 -> 1.6, 3.1 -> 1.9. The same steps with a
+// persistent grid took 137 us for the first (four rounds 121), 8-warp blocks 118 / 96 / 102.7.
+constexpr int kTileWarps = 4;  // of a block
+
+// Lane i of four (lanes `step` and 2 * step apart) holds bytes a_i[0..3]; returns a_0[i] | a_1[i] << 8 | a_2[i] << 16 | a_3[i] << 24.
+__device__ __forceinline__ uint32_t transpose_bytes(uint32_t a, int step, int i) {
+  uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, a, step);
+  a = __byte_perm(a, o, (i & 1) ? 0x3715 : 0x6240);
+  o = __shfl_xor_sync(0xFFFFFFFFu, a, 2 * step);
+  return __byte_perm(a, o, (i & 2) ? 0x3276 : 0x5410);
+}
+
+// A step is 16 vectors of eight rows; steps_per_unit = ceil(nvec / 16) steps along a row, `total` steps in all.
+// n_partials > 0: the kernel in front is this tensor's own amax launch. That one starts only when x is complete, so a warp's first step is
+// loaded while it still runs; and the last rows come first, which the amax launch read last and left in L2.
+// layout: kWordScales for swizzled scales that can be stored as words, else TF_SCALES_PLAIN or TF_SCALES_SWIZZLED, byte by byte.
+constexpr int kWordScales = 2;
 template <int FMT>
-__global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const uint8_t* __restrict__ x, int64_t m, int64_t k, int64_t ldx,
-                                                                      uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
-                                                                      int swizzled, int pad, const float* __restrict__ gs_ptr, float* __restrict__ gs_out,
-                                                                      int n_partials, int backwards) {
-  const int nvec = (int)(k >> 4);
+__global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(const uint8_t* __restrict__ x, int64_t m, int k, int64_t ldx, uint8_t* __restrict__ codes,
+                                                                          uint8_t* __restrict__ scales, int layout, int steps_per_unit, int total,
+                                                                          const float* __restrict__ gs_ptr, float* __restrict__ gs_out, int n_partials) {
+  constexpr bool kNv = FMT == TF_FMT_NVFP4;
+  constexpr int kCodeBytes = FMT == TF_FMT_MXFP8 ? 16 : 8;  // per vector
+  const int nvec = k >> 4, cols = kNv ? nvec : nvec >> 1, n_ct = (cols + 3) >> 2;
+  const int lane = threadIdx.x & 31, h = lane >> 4, q = lane & 15;
   griddep_launch_dependents();
-  griddep_wait();
-  const int cols = nvec / (FMT == TF_FMT_NVFP4 ? 1 : 2);
-  if (pad)
-    zero_scale_padding<false>(scales, m, cols,
-                              ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kQuantThreads + threadIdx.y * blockDim.x + threadIdx.x,
-                              (int64_t)gridDim.x * gridDim.y * kQuantThreads);
-  float gs = 0.0f;
-  if (FMT == TF_FMT_NVFP4 && n_partials > 0) {
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    uint32_t mx = 0;  // non-negative floats order like their bits
-    for (int i = tid; i < n_partials; i += kQuantThreads) mx = max(mx, __float_as_uint(load_f32(gs_ptr + i)));
-    __shared__ uint32_t warp_max[kQuantThreads / 32];
-    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
-    if ((tid & 31) == 0) warp_max[tid >> 5] = mx;
-    __syncthreads();
+  float gs = 0.0f, inv_t = 0.0f;
+  if (!kNv || n_partials == 0) {
+    griddep_wait();
+    if (kNv) gs = load_f32(gs_ptr);  // used behind the first loads
+  }
+  bool first = kNv;  // the first round, which every warp of the block runs: the scale is formed in it
+  for (int s0 = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));; s0 += (int)(gridDim.x * (blockDim.x >> 5))) {
+    const bool live = s0 < total;
+    if (!live && !first) break;
+    const int s = !live ? 0 : n_partials > 0 ? total - 1 - s0 : s0;
+    const int unit = s / steps_per_unit, c = s - unit * steps_per_unit;
+    const int rr = (unit & 15) * 2 + h;  // this half warp's place in a group of 32 rows
+    const int64_t row = (int64_t)(unit >> 4) * 128 + rr;
+    const int vec = c * 16 + q;
+    const uint8_t* xp = x + row * ldx * 2 + (int64_t)vec * 32;
+    uint32_t v[4][8];
+    bool has[4];  // j: row + 32 * j
 #pragma unroll
-    for (int i = 0; i < kQuantThreads / 32; ++i) mx = max(mx, warp_max[i]);
-    gs = __uint_as_float(mx);
-  } else if (FMT == TF_FMT_NVFP4) {
-    gs = load_f32(gs_ptr);
-  }
-  if (FMT == TF_FMT_NVFP4 && gs_out != nullptr) {
-    gs = __fdiv_rn(gs, 2688.0f);
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) gs_out[0] = gs;
-  }
-  const float inv_t = (FMT == TF_FMT_NVFP4 && gs != 0.0f) ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
-  const int64_t row_stride = (int64_t)gridDim.x * blockDim.y;
-  int begin, end;
-  row_segment(nvec, begin, end);
-  // backwards: the last rows first, which the amax launch in front read last and left in L2
-  const int64_t last = (m - 1) / blockDim.y * blockDim.y;
-  for (int64_t row_it = (int64_t)blockIdx.x * blockDim.y; row_it < m; row_it += row_stride) {
-    const int64_t row = (backwards ? last - row_it : row_it) + threadIdx.y;
-    const bool row_ok = row < m;
-    const uint8_t* xr = x + (row_ok ? row : 0) * ldx * 2;
-    for (int base = begin; base < end; base += kQuantUnroll * (int)blockDim.x) {
-      uint32_t v[kQuantUnroll][8];
-      bool has[kQuantUnroll];
-      load_round(xr, row_ok, base, nvec, v, has);
-      store_round<FMT>(v, has, row, base, nvec, k, codes, scales, swizzled, gs, inv_t);
+    for (int j = 0; j < 4; ++j) {
+      has[j] = live && row + 32 * j < m && vec < nvec;
+      if (has[j]) {
+        load_256(xp + 64 * j * ldx, v[j]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[j][e] = 0;
+      }
     }
-    if (pad && row_ok && blockIdx.y == 0 && threadIdx.x < 2) zero_row_padding(scales, row, cols, threadIdx.x);
+    if (kNv && first) {
+      if (n_partials > 0) {
+        griddep_wait();
+        gs = partials_max(gs_ptr, n_partials, threadIdx.x, blockDim.x);
+      }
+      if (gs_out != nullptr) {
+        gs = __fdiv_rn(gs, 2688.0f);
+        if (blockIdx.x == 0 && threadIdx.x == 0) gs_out[0] = gs;
+      }
+      inv_t = gs != 0.0f ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
+      first = false;
+      if (!live) break;
+    }
+    uint8_t* cp = codes + (row * nvec + vec) * kCodeBytes;
+    uint32_t word = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t cw[4], sc;
+      quantize_vec16<FMT>(v[j], gs, inv_t, cw, sc);
+      if (has[j]) {
+        word |= sc << (8 * j);
+        uint8_t* dst = cp + (int64_t)(32 * j) * nvec * kCodeBytes;
+        if (FMT == TF_FMT_MXFP8) *reinterpret_cast<uint4*>(dst) = make_uint4(cw[0], cw[1], cw[2], cw[3]);
+        else *reinterpret_cast<uint2*>(dst) = make_uint2(cw[0], cw[1]);
+      }
+    }
+    // four scales of one row are four lanes (nvfp4) or four pairs of lanes; lane (pair) i of them gets the word of load i
+    const int i = (kNv ? q : q >> 1) & 3;
+    word = transpose_bytes(word, kNv ? 1 : 2, i);
+    const int ct = kNv ? c * 4 + (q >> 2) : c * 2 + (q >> 3);
+    if (ct < n_ct && (kNv || (q & 1) == 0)) {
+      uint8_t* dst = scales + ((int64_t)(unit >> 4) * n_ct + ct) * 512 + rr * 16 + i * 4;
+      if (layout == kWordScales) {
+        *reinterpret_cast<uint32_t*>(dst) = word;
+      } else {
+        const int64_t r = row + 32 * i;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          if (layout == TF_SCALES_SWIZZLED) dst[b] = (uint8_t)(word >> (8 * b));
+          else if (r < m && ct * 4 + b < cols) scales[r * cols + ct * 4 + b] = (uint8_t)(word >> (8 * b));
+        }
+      }
+    }
   }
 }
 
@@ -272,7 +319,7 @@ __global__ void __launch_bounds__(kQuantThreads) amax_rows_kernel(const uint8_t*
   else if (tid == 0 && mx) atomicMax(out_bits, mx << 16);
 }
 
-static void quantize_shape(int64_t m, int64_t k, int pad, int per_sm, dim3& grid, dim3& block);
+static void rows_shape(int64_t m, int64_t k, int per_sm, dim3& grid, dim3& block);
 
 // nvfp4 without a given scale is two launches: an amax launch whose blocks leave their maxima, and the quantizer, which derives the scale
 // from them. Before: a memset, an amax launch with an atomic, a one-thread launch for the scale and the quantizer. Graphs of 12: 128 x
@@ -288,7 +335,7 @@ static tf_status launch_amax(const char* fn, const void* x, int64_t m, int64_t k
   if (ldx != k && m > 1) {
     const int per_sm = kMaxAmaxBlocks / sm_count();
     dim3 grid, block;
-    quantize_shape(m, k, 0, per_sm < kStreamCtasPerSm ? per_sm : kStreamCtasPerSm, grid, block);
+    rows_shape(m, k, per_sm < kStreamCtasPerSm ? per_sm : kStreamCtasPerSm, grid, block);
     *blocks = (int)(grid.x * grid.y);
     amax_rows_kernel<<<grid, block, 0, stream>>>(xb, m, (int)(k >> 4), ldx, out_bits, partials);
   } else if (total >= 2 * (int64_t)sm_count() * kStreamChunkVecs) {  // at least two chunks per SM
@@ -354,8 +401,8 @@ static tf_status check_quant_args(const char* fn, const void* x, int64_t m, int6
   return TF_OK;
 }
 
-// Block and grid of the register form: a power of two of threads along the row, at most `per_sm` blocks per SM.
-static void quantize_shape(int64_t m, int64_t k, int pad, int per_sm, dim3& grid, dim3& block) {
+// Block and grid of amax_rows_kernel: a power of two of threads along the row, at most `per_sm` blocks per SM.
+static void rows_shape(int64_t m, int64_t k, int per_sm, dim3& grid, dim3& block) {
   int tpr = 2;
   while (tpr < kQuantThreads && tpr * kQuantUnroll < (k >> 4)) tpr <<= 1;
   const int rpb = kQuantThreads / tpr;
@@ -368,7 +415,6 @@ static void quantize_shape(int64_t m, int64_t k, int pad, int per_sm, dim3& grid
     if (want * blocks_needed > cap) want = cap / blocks_needed;
     grid.y = (unsigned)(want < 1 ? 1 : want < rounds ? want : rounds);
   }
-  if (pad && grid.x * grid.y < kPadBlocks) grid.x = kPadBlocks;
 }
 
 template <int FMT>
@@ -378,16 +424,19 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   if (st != TF_OK) return st;
   if (FMT == TF_FMT_NVFP4 && !gs) return fail(TF_ERR_INVALID_ARGUMENT, "%s: nvfp4 needs a global scale", fn);
   if (m == 0) return TF_OK;
-  int pad = 0;
-  st = scale_padding(scales, FMT, m, k, layout, stream, &pad);
-  if (st != TF_OK) return st;
-  dim3 grid, block;
-  quantize_shape(m, k, pad, 8, grid, block);
-  // After its own amax launch (n_partials > 0) a quantizer of at most 16 M elements starts as that launch's dependent (128 x 4096 6.3 ->
-  // 5.7 us, 4096 x 2560 14.4 -> 14.1); beyond that its waiting blocks cost the amax launch more (8192 x 4096 30.0 -> 31.6 us).
-  TF_CUDA(launch_dependent((n_partials > 0 && m * k <= (int64_t)1 << 24) || chain_rows_launch(m), quantize_rows_kernel<FMT>, grid, block, 0, stream, static_cast<const uint8_t*>(x), m, k,
-                           ldx, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), (int)(layout == TF_SCALES_SWIZZLED), pad, gs, gs_out,
-                           n_partials, (int)(n_partials > 0)));
+  const int64_t steps_per_unit = ((k >> 4) + 15) / 16, total = (m + 127) / 128 * 16 * steps_per_unit;
+  if (total > INT32_MAX) return fail(TF_ERR_UNSUPPORTED, "%s: m=%lld x k=%lld is too large", fn, (long long)m, (long long)k);
+  int64_t warps = (total + sm_count() - 1) / sm_count();  // few steps: narrower blocks, so that every SM gets some
+  if (warps > kTileWarps) warps = kTileWarps;
+  // Behind an amax launch every block takes the maximum of its words: two steps for each (65536 x 4096 with the amax launch 195.5 -> 187 us).
+  // Up to 16 M elements the blocks start as that launch's dependents (128 x 4096 4.5 -> 4.0 us, 2048 x 4096 9.6 -> 8.3); beyond that their
+  // waiting costs the amax launch more (8192 x 4096 29.9 -> 33.0).
+  const int64_t rounds = n_partials > 0 && total > 32 * (int64_t)sm_count() ? 2 : 1;
+  const bool dependent = (n_partials > 0 && m * k <= (int64_t)1 << 24) || chain_rows_launch(m);
+  const int words = layout == TF_SCALES_SWIZZLED && reinterpret_cast<uintptr_t>(scales) % 4 == 0;
+  TF_CUDA(launch_dependent(dependent, quantize_tiles_kernel<FMT>, dim3((unsigned)((total + warps * rounds - 1) / (warps * rounds))), dim3((unsigned)warps * 32), 0, stream,
+                           static_cast<const uint8_t*>(x), m, (int)k, ldx, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales),
+                           (int)(words ? kWordScales : layout), (int)steps_per_unit, (int)total, gs, gs_out, n_partials));
   return TF_OK;
 }
 
