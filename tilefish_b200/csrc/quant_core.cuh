@@ -131,9 +131,9 @@ __device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs,
 // row padding is 16 contiguous bytes (the four row groups of one tile row), so a tensor of one row and 2560 columns takes two stores
 // per thread of a single block. `scales` is 16-byte aligned.
 constexpr unsigned kPadBlocks = 8;  // a launch that pads has at least this many blocks to share the work
-// COLUMNS = false leaves the columns to zero_row_padding, called where a row's scales are stored: the row kernels pass tens of megabytes
-// through L2 before they come to the later rows, whose sectors a sweep at the start would leave half written for that long (rmsnorm with an mxfp4 copy, 16026 x 1504: 61.2 us with
-// the sweep, 54.2 without, 57.2 with the memset).
+// COLUMNS = false: the columns are written with the row's scales (store_quantized_words): the rmsnorm kernel passes tens of megabytes
+// through L2 before it comes to the later rows, whose sectors a sweep at the start would leave half written for that long (with an mxfp4 copy,
+// 16026 x 1504: 61.2 us with the sweep, 54.2 with the columns behind each row, 57.2 with the memset).
 template <bool COLUMNS = true>
 __device__ __forceinline__ void zero_scale_padding(uint8_t* __restrict__ scales, int64_t rows, int64_t cols, int64_t first, int64_t stride) {
   const int64_t n_ct = (cols + 3) >> 2;
@@ -157,10 +157,38 @@ __device__ __forceinline__ void zero_scale_padding(uint8_t* __restrict__ scales,
   }
 }
 
-// The padding columns of one row (at most three), by two threads of those that store the row: t is 0 or 1.
-__device__ __forceinline__ void zero_row_padding(uint8_t* __restrict__ scales, int64_t row, int cols, int t) {
-  const int n_ct = (cols + 3) >> 2;
-  for (int c = cols + t; c < n_ct * 4; c += 2) scales[swizzled_scale_offset(row, c, n_ct)] = 0;
+// Four scales of row `row`, columns col .. col + 3 (col a multiple of 4), as the bytes of `word`. WORDS: swizzled scales that can be stored as words; else
+// byte by byte in either layout (a template: the short row kernels run from a cold instruction cache, and the branches over the byte
+// stores cost the README block at 1 and 512 rows 0.3 and 0.6 us). real: the row is one of the tensor's (the swizzled layout has more).
+template <bool WORDS>
+__device__ __forceinline__ void store_scale_word(uint8_t* __restrict__ scales, int layout, int64_t row, int col, int cols, int n_ct, bool real, uint32_t word) {
+  if (WORDS) {
+    *reinterpret_cast<uint32_t*>(scales + swizzled_scale_offset(row, col, n_ct)) = word;
+    return;
+  }
+  uint8_t* dst = scales + (layout == TF_SCALES_PLAIN ? row * cols + col : swizzled_scale_offset(row, col, n_ct));
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+    if (layout == TF_SCALES_SWIZZLED || (real && col + b < cols)) dst[b] = (uint8_t)(word >> (8 * b));
+}
+inline bool scales_as_words(const void* scales, int layout) { return layout == TF_SCALES_SWIZZLED && reinterpret_cast<uintptr_t>(scales) % 4 == 0; }
+
+// One thread's codes of 8 elements (vector `vec` of row `row`), and the scales of a row's column tile as one word of the swizzled layout, the zeros of
+// its padding columns included. All 32 lanes call it together, with consecutive vectors from a multiple of 32 on; `has`: this lane has data.
+template <int FMT, bool WORDS>
+__device__ __forceinline__ void store_quantized_words(uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int layout, bool has, int64_t row, int vec, int d,
+                                                      uint32_t c0, uint32_t c1, uint32_t scale) {
+  constexpr int kLanes = (FMT == TF_FMT_NVFP4) ? 2 : 4;  // of one block
+  uint32_t word = has ? scale << (8 * ((vec / kLanes) & 3)) : 0u;
+  word |= __shfl_xor_sync(0xFFFFFFFFu, word, kLanes);
+  word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2 * kLanes);
+  if (!has) return;
+  if (FMT == TF_FMT_MXFP8) *reinterpret_cast<uint2*>(codes + row * d + (int64_t)vec * 8) = make_uint2(c0, c1);
+  else *reinterpret_cast<uint32_t*>(codes + row * (d >> 1) + (int64_t)vec * 4) = c0;
+  if ((vec & (4 * kLanes - 1)) == 0) {
+    const int cols = (d >> 3) / kLanes, col = vec / kLanes;
+    store_scale_word<WORDS>(scales, layout, row, col, cols, (cols + 3) >> 2, true, word);
+  }
 }
 
 // Stores one thread's codes (8 elements starting at element column `col` of row `row`) and, from the first lane of each

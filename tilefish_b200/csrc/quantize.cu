@@ -82,9 +82,7 @@ __device__ __forceinline__ uint32_t transpose_bytes(uint32_t a, int step, int i)
 // A step is 16 vectors of eight rows; steps_per_unit = ceil(nvec / 16) steps along a row, `total` steps in all.
 // n_partials > 0: the kernel in front is this tensor's own amax launch. That one starts only when x is complete, so a warp's first step is
 // loaded while it still runs; and the last rows come first, which the amax launch read last and left in L2.
-// layout: kWordScales for swizzled scales that can be stored as words, else TF_SCALES_PLAIN or TF_SCALES_SWIZZLED, byte by byte.
-constexpr int kWordScales = 2;
-template <int FMT>
+template <int FMT, bool WORDS>
 __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(const uint8_t* __restrict__ x, int64_t m, int k, int64_t ldx, uint8_t* __restrict__ codes,
                                                                           uint8_t* __restrict__ scales, int layout, int steps_per_unit, int total,
                                                                           const float* __restrict__ gs_ptr, float* __restrict__ gs_out, int n_partials) {
@@ -150,19 +148,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
     const int i = (kNv ? q : q >> 1) & 3;
     word = transpose_bytes(word, kNv ? 1 : 2, i);
     const int ct = kNv ? c * 4 + (q >> 2) : c * 2 + (q >> 3);
-    if (ct < n_ct && (kNv || (q & 1) == 0)) {
-      uint8_t* dst = scales + ((int64_t)(unit >> 4) * n_ct + ct) * 512 + rr * 16 + i * 4;
-      if (layout == kWordScales) {
-        *reinterpret_cast<uint32_t*>(dst) = word;
-      } else {
-        const int64_t r = row + 32 * i;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          if (layout == TF_SCALES_SWIZZLED) dst[b] = (uint8_t)(word >> (8 * b));
-          else if (r < m && ct * 4 + b < cols) scales[r * cols + ct * 4 + b] = (uint8_t)(word >> (8 * b));
-        }
-      }
-    }
+    if (ct < n_ct && (kNv || (q & 1) == 0)) store_scale_word<WORDS>(scales, layout, row + 32 * i, ct * 4, cols, n_ct, row + 32 * i < m, word);
   }
 }
 
@@ -433,10 +419,10 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   // waiting costs the amax launch more (8192 x 4096 29.9 -> 33.0).
   const int64_t rounds = n_partials > 0 && total > 32 * (int64_t)sm_count() ? 2 : 1;
   const bool dependent = (n_partials > 0 && m * k <= (int64_t)1 << 24) || chain_rows_launch(m);
-  const int words = layout == TF_SCALES_SWIZZLED && reinterpret_cast<uintptr_t>(scales) % 4 == 0;
-  TF_CUDA(launch_dependent(dependent, quantize_tiles_kernel<FMT>, dim3((unsigned)((total + warps * rounds - 1) / (warps * rounds))), dim3((unsigned)warps * 32), 0, stream,
-                           static_cast<const uint8_t*>(x), m, (int)k, ldx, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales),
-                           (int)(words ? kWordScales : layout), (int)steps_per_unit, (int)total, gs, gs_out, n_partials));
+  auto kernel = scales_as_words(scales, layout) ? quantize_tiles_kernel<FMT, true> : quantize_tiles_kernel<FMT, false>;
+  TF_CUDA(launch_dependent(dependent, kernel, dim3((unsigned)((total + warps * rounds - 1) / (warps * rounds))), dim3((unsigned)warps * 32), 0, stream,
+                           static_cast<const uint8_t*>(x), m, (int)k, ldx, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), layout,
+                           (int)steps_per_unit, (int)total, gs, gs_out, n_partials));
   return TF_OK;
 }
 

@@ -4,18 +4,20 @@
 //   out = bf16(r * rstd * f32(w))   rstd = rsqrt(sum(r*r) * f32(1/D) + eps); the only rounding point is the bf16 cast
 //
 // HBM-bound: 12 bytes per element (2 read x, 4 read + 4 write residual, 2 write out), plus the quantized copy when asked
-// for. One block per row (grid-stride), 128-bit loads, the row's r values stay in registers between the reduction and the
+// for. One or two rows per block, 128-bit loads, the row's r values stay in registers between the reduction and the
 // normalisation, warp-shuffle + shared-memory block reduction.
 #include "async_copy.cuh"
 #include "quant_core.cuh"
 
 namespace tf {
 
-template <int VPT, int QFMT>  // VPT: 8-element vectors per thread; QFMT: -1 none, else TF_FMT_*
-__global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* __restrict__ x, float4* __restrict__ residual,
+// VPT: 8-element vectors per thread; QFMT: -1 none, else TF_FMT_*; WORDS: the scales leave as words (scales_as_words).
+// Registers for four blocks of 512 threads per SM (three with two vectors per thread: 16384 x 8192 247 us with two blocks, 234.8 = 6.86 TB/s with three).
+template <int VPT, int QFMT, bool WORDS>
+__global__ void __launch_bounds__(512, VPT == 1 ? 4 : VPT == 2 ? 3 : 0) residual_add_rmsnorm_kernel(const uint4* __restrict__ x, float4* __restrict__ residual,
                                                                    const uint4* __restrict__ w, uint4* __restrict__ out, int64_t m, int d,
                                                                    float eps, float inv_d, uint8_t* __restrict__ q_codes,
-                                                                   uint8_t* __restrict__ q_scales, int q_swizzled, int q_pad,
+                                                                   uint8_t* __restrict__ q_scales, int q_layout, int q_pad,
                                                                    const float* __restrict__ q_gs_ptr, unsigned int* __restrict__ out_amax) {
   __shared__ float warp_sums[16];
   __shared__ unsigned int warp_amax[16];
@@ -27,7 +29,7 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
   griddep_wait();
   const float gs = (QFMT == TF_FMT_NVFP4) ? load_f32(q_gs_ptr) : 0.0f;
   const float inv_t = (QFMT == TF_FMT_NVFP4 && gs != 0.0f) ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
-  if (QFMT >= 0 && q_pad)
+  if (QFMT >= 0 && q_pad)  // rows; the columns go with the words
     zero_scale_padding<false>(q_scales, m, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), (int64_t)blockIdx.x * nthreads + tid, (int64_t)gridDim.x * nthreads);
 
   for (int64_t row = blockIdx.x; row < m; row += gridDim.x) {
@@ -88,11 +90,10 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
         if (i * nthreads < nvec) {
           uint32_t c0, c1, sc;
           quantize_vec8<(QFMT < 0 ? 0 : QFMT)>(o, gs, inv_t, c0, c1, sc);
-          if (has) store_quantized<(QFMT < 0 ? 0 : QFMT)>(q_codes, q_scales, q_swizzled, row, v, d, c0, c1, sc);
+          store_quantized_words<(QFMT < 0 ? 0 : QFMT), WORDS>(q_codes, q_scales, q_layout, has, row, v, d, c0, c1, sc);
         }
       }
     }
-    if (QFMT >= 0 && q_pad && tid < 2) zero_row_padding(q_scales, row, d / (QFMT == TF_FMT_NVFP4 ? 16 : 32), tid);
     __syncthreads();  // warp_sums / row_rstd are reused by the next row
   }
   if (out_amax) {  // one atomic per block
@@ -108,13 +109,16 @@ __global__ void __launch_bounds__(512) residual_add_rmsnorm_kernel(const uint4* 
 
 template <int VPT>
 static void launch_vpt(int qfmt, dim3 grid, dim3 block, cudaStream_t s, const uint4* x, float4* res, const uint4* w, uint4* out, int64_t m, int d,
-                       float eps, float inv_d, uint8_t* qc, uint8_t* qs, int qsw, int qpad, const float* qgs, unsigned int* amax) {
+                       float eps, float inv_d, uint8_t* qc, uint8_t* qs, int qlayout, int qpad, const float* qgs, unsigned int* amax) {
+  const bool words = scales_as_words(qs, qlayout);
+  auto kernel = residual_add_rmsnorm_kernel<VPT, -1, true>;
   switch (qfmt) {
-    case TF_FMT_MXFP8: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
-    case TF_FMT_MXFP4: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
-    case TF_FMT_NVFP4: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
-    default: launch_dependent(chain_rows_launch(m), residual_add_rmsnorm_kernel<VPT, -1>, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qsw, qpad, qgs, amax); break;
+    case TF_FMT_MXFP8: kernel = words ? residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8, true> : residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP8, false>; break;
+    case TF_FMT_MXFP4: kernel = words ? residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4, true> : residual_add_rmsnorm_kernel<VPT, TF_FMT_MXFP4, false>; break;
+    case TF_FMT_NVFP4: kernel = words ? residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4, true> : residual_add_rmsnorm_kernel<VPT, TF_FMT_NVFP4, false>; break;
+    default: break;
   }
+  launch_dependent(chain_rows_launch(m), kernel, grid, block, 0, s, x, res, w, out, m, d, eps, inv_d, qc, qs, qlayout, qpad, qgs, amax);
 }
 
 
@@ -311,8 +315,13 @@ extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, cons
   vpt = vpt <= 1 ? 1 : vpt <= 2 ? 2 : vpt <= 4 ? 4 : 8;
   int threads = (nvec + vpt - 1) / vpt;
   threads = (threads + 31) / 32 * 32;
-  const int64_t cap = (int64_t)sm_count() * (2048 / threads);
-  dim3 grid((unsigned)(m < cap ? m : cap)), block(threads);
+  // A block per row once the rows exceed what is resident: the hardware deals the rows out, while blocks that stay and walk keep every SM's loads and
+  // stores in phase. Two rows where a block is short against its launch: less than 2 K columns, or only the quantized copy to write (up to
+  // 4 K). Persistent -> this, graphs of 12: 8192 x 2560 42.3 -> 39.2 us, with an mxfp8 copy 48.4 -> 45.1; 10000 x 4064 79.7 -> 73.0 (6.7 TB/s); 4096 x 8192
+  // with an mxfp8 copy 85 -> 71; two rows: 16000 x 512 18.1 -> 17.2 (one row 18.0), mxfp4 copy alone 10000 x 4064 71.6 -> 71.7 (75.3).
+  const int64_t resident = (int64_t)sm_count() * (2048 / threads);
+  const int64_t rows_per_block = m > resident && (threads < 256 || (!out && vpt == 1)) ? 2 : 1;
+  dim3 grid((unsigned)((m + rows_per_block - 1) / rows_per_block)), block(threads);
   if (pad && grid.x < kPadBlocks) grid.x = kPadBlocks;  // one to seven rows: blocks without a row share the padding (0.6 us at one row)
   const float inv_d = 1.0f / (float)d;  // correctly rounded f32 reciprocal of D (IEEE division on the host)
   const uint4* xp = static_cast<const uint4*>(x);
@@ -321,12 +330,11 @@ extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, cons
   uint4* op = static_cast<uint4*>(out);
   uint8_t* qc = static_cast<uint8_t*>(q_codes);
   uint8_t* qs = static_cast<uint8_t*>(q_scales);
-  const int qsw = q_layout == TF_SCALES_SWIZZLED;
   switch (vpt) {
-    case 1: launch_vpt<1>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
-    case 2: launch_vpt<2>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
-    case 4: launch_vpt<4>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
-    default: launch_vpt<8>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, qsw, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    case 1: launch_vpt<1>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, q_layout, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    case 2: launch_vpt<2>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, q_layout, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    case 4: launch_vpt<4>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, q_layout, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
+    default: launch_vpt<8>(q_format, grid, block, stream, xp, rp, wp, op, m, (int)d, eps, inv_d, qc, qs, q_layout, pad, q_global_scale, reinterpret_cast<unsigned int*>(out_amax)); break;
   }
   TF_LAUNCH_CHECK();
   return TF_OK;
