@@ -1125,6 +1125,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
   constexpr int kST = PC::kST;
   constexpr int kNB = 2;
   constexpr int kOutCols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;
+  // The load warps take the stages in turn where the epilogue's arithmetic competes with them for issue slots: two stages' time for five copies
+  // instead of one for two or three (mxfp8 8192 x 3072 x 2560 + gate 98.0 -> 95.5 us, hot 116.4 -> 112.8; nvfp4 4096 x 28672 x 8192 + gate 672.9 -> 665.4). Without
+  // the gate a tile's first stage comes later for it (mxfp4 300 x 8192 x 4096 12.3 -> 12.55, mxfp8 1024 x 4096 x 4096 residual 22.0 -> 22.65).
+  constexpr bool kTurns = EPI == TF_EPI_SILU_GATE;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -1148,7 +1152,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(bar_full + 8 * s, 4);   // one arrive.expect_tx from each load warp of each CTA (used in the leader only)
+      mbar_init(bar_full + 8 * s, kTurns ? 2 : 4);  // an arrive.expect_tx of each load warp that serves the stage, from both CTAs (used in the leader only)
       mbar_init(bar_empty + 8 * s, 1);  // the leader's commit arrives in both CTAs
     }
     mbar_init(bar_tmem_full, 1);
@@ -1169,40 +1173,45 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
 
   if (warp == 0 || warp == 6) {
     // ---------------- load warps (each CTA loads its own halves; completion is counted on the leader's barrier) ----------------
-    // warp 0: lane 0 the A rows, lane 1 the B rows of this CTA. warp 6: lane 0 the A scales, lanes 1-2 the scales of the two B
-    // halves, through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows past the end read as
+    // Lane 0 loads the A rows, lane 1 the B rows of this CTA, lane 2 the A scales, lanes 3-4 the scales of the two B halves (warp 0 the operands
+    // and warp 6 the scales of every stage, or with kTurns both in turn), the scales through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows past the end read as
     // zero), because only the tensor form of the copy may signal the peer's barrier.
-    const bool scales = warp == 6;
-    int stage = 0;
+    constexpr int kStep = kTurns ? 2 : 1;
+    const int turn = kTurns && warp == 6 ? 1 : 0;
+    const bool sf = lane >= 2;
+    const int half = lane < 2 ? (int)rank : (lane == 4 ? 1 : 0);  // the B half of a lane that serves B
+    const bool serves_a = lane == 0 || lane == 2;
+    const CUtensorMap* my_map = lane == 0 ? &tma_a : lane == 1 ? &tma_b : lane == 2 ? &tma_sfa : &tma_sfb;
+    const uint32_t my_dst = lane == 0 ? smem_a : lane == 1 ? smem_b : lane == 2 ? smem_sfa : smem_sfb + (uint32_t)half * kST * 512;
+    const uint32_t my_stage_bytes = lane < 2 ? kAStageBytes : lane == 2 ? PC::kSfaStageBytes : PC::kSfbStageBytes;
+    int stage = turn, ks0 = turn;
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = pair; tile < p.num_tiles && ok; tile += num_pairs) {
       const int m_blk = tile % p.m_blocks, n_blk = tile / p.m_blocks;
       const int a_row = m_blk * 256 + (int)rank * 128;
-      const int half = scales ? (lane == 2 ? 1 : 0) : (int)rank;  // the B half a lane other than 0 serves
       const int b_row = (EPI == TF_EPI_SILU_GATE) ? half * p.n + n_blk * 128 : n_blk * BLOCK_N + half * 128;
-      const int my_row = lane == 0 ? a_row : b_row;
-      const bool mine = lane == 0 ? a_row < p.m : (lane <= (scales ? 2 : 1) && b_row < p.n_rows_b);
-      const uint32_t copies = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine));
-      const CUtensorMap* my_map = scales ? (lane == 0 ? &tma_sfa : &tma_sfb) : (lane == 0 ? &tma_a : &tma_b);
-      const uint32_t my_dst = scales ? (lane == 0 ? smem_sfa : smem_sfb + (uint32_t)half * kST * 512) : (lane == 0 ? smem_a : smem_b);
-      const uint32_t my_stage_bytes = scales ? (lane == 0 ? PC::kSfaStageBytes : PC::kSfbStageBytes) : kAStageBytes;
-      const uint32_t tx = copies * (scales ? (uint32_t)kST * 512u : (uint32_t)kAStageBytes);
-      const int y_base = scales ? (my_row >> 7) * p.sf_col_tiles : my_row;
-      for (int ks = 0; ks < p.num_k_stages; ++ks) {
+      const int my_row = serves_a ? a_row : b_row;
+      const bool mine = lane < 5 && (kTurns || sf == (warp == 6)) && (serves_a ? a_row < p.m : b_row < p.n_rows_b);
+      const uint32_t tx = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && !sf)) * kAStageBytes + (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && sf)) * (kST * 512u);
+      const int y_base = sf ? (my_row >> 7) * p.sf_col_tiles : my_row;
+      int ks = ks0;
+      for (; ks < p.num_k_stages; ks += kStep) {
         ok = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, 1);
         ok = __all_sync(0xFFFFFFFFu, ok);
         if (!ok) break;
         const uint32_t full = mapa_shared(bar_full + 8 * stage, 0);  // the leader's barrier
         if (lane == 0) mbar_expect_tx_cluster(full, tx);
         __syncwarp();
-        if (mine) tma_load_2d_pair(my_dst + stage * my_stage_bytes, my_map, scales ? 0 : ks * kStageKBytes, scales ? y_base + ks * kST : y_base, full);
+        if (mine) tma_load_2d_pair(my_dst + stage * my_stage_bytes, my_map, sf ? 0 : ks * kStageKBytes, sf ? y_base + ks * kST : y_base, full);
         __syncwarp();
-        if (++stage == kStages) {
-          stage = 0;
+        stage += kStep;
+        if (stage >= kStages) {
+          stage -= kStages;
           phase ^= 1;
         }
       }
+      ks0 = ks - p.num_k_stages;
     }
     if (!ok && lane == 0) {
       const unsigned long long t0 = globaltimer_ns();
