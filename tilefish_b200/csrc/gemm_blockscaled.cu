@@ -385,36 +385,32 @@ __device__ __forceinline__ constexpr bool chunk_is_mine(int c) {
 }
 
 // residual += f32(staged bf16) for one warp's box of 32 rows x 64 columns, whose first row and column are row0 and col0. A half-warp
-// takes one row's 64 columns, 256 contiguous bytes, four loads in flight per thread (eight spill: 25 us on the first shape below). Taken
-// straight from the accumulator layout (a thread owns a row) every access of a warp touched 32 lines. Before -> after: mxfp4 1000 x 3000 x
-// 2720 23.2 -> 16.5 us, 787 x 7536 x 1696 37.1 -> 23.9, nvfp4 4096 x 4096 x 4096 81 -> 56, mxfp8 8192 x 2560 x 3072 120 -> 76.
-constexpr int kResidualLoads = 4;
+// takes one row's 64 columns, 256 contiguous bytes, and all 16 loads of a thread are in flight at once, 64 KB per SM: with four (16 KB per SM) a
+// 256 x 256 tile whose residual is in HBM took 24000 clocks, twice its 20 K stages. Taken straight from the accumulator layout (a thread
+// owns a row) every access of a warp would touch 32 lines.
+constexpr int kResidualLoads = 16;
 __device__ __forceinline__ void residual_add_box(const GemmParams& p, uint32_t box, int lane, int row0, int col0) {
   const int half = lane >> 4, c4 = lane & 15, col = col0 + c4 * 4;
   if (col >= p.n) return;  // n is a multiple of 8: the four columns are inside together
   float4* at = reinterpret_cast<float4*>(p.residual + (int64_t)(row0 + half) * p.n + col);
   const int step = p.n >> 1;  // float4 units of two rows
   const int rows = p.m - row0 - half;
-#pragma unroll 1
-  for (int b = 0; b < 16; b += kResidualLoads) {
-    float4 r[kResidualLoads];
+  float4 r[kResidualLoads];
 #pragma unroll
-    for (int i = 0; i < kResidualLoads; ++i)
-      if ((b + i) * 2 < rows) r[i] = at[i * step];
+  for (int i = 0; i < kResidualLoads; ++i)
+    if (i * 2 < rows) r[i] = at[(int64_t)i * step];
 #pragma unroll
-    for (int i = 0; i < kResidualLoads; ++i) {
-      const int rr = (b + i) * 2 + half;
-      if ((b + i) * 2 < rows) {
-        uint32_t w0, w1;
-        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1) : "r"(box + rr * 128 + (((c4 >> 1) ^ (rr & 7)) << 4) + (c4 & 1) * 8));
-        r[i].x = __fadd_rn(r[i].x, bf16lo_to_f32(w0));
-        r[i].y = __fadd_rn(r[i].y, bf16hi_to_f32(w0));
-        r[i].z = __fadd_rn(r[i].z, bf16lo_to_f32(w1));
-        r[i].w = __fadd_rn(r[i].w, bf16hi_to_f32(w1));
-        at[i * step] = r[i];
-      }
+  for (int i = 0; i < kResidualLoads; ++i) {
+    const int rr = i * 2 + half;
+    if (i * 2 < rows) {
+      uint32_t w0, w1;
+      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1) : "r"(box + rr * 128 + (((c4 >> 1) ^ (rr & 7)) << 4) + (c4 & 1) * 8));
+      r[i].x = __fadd_rn(r[i].x, bf16lo_to_f32(w0));
+      r[i].y = __fadd_rn(r[i].y, bf16hi_to_f32(w0));
+      r[i].z = __fadd_rn(r[i].z, bf16lo_to_f32(w1));
+      r[i].w = __fadd_rn(r[i].w, bf16hi_to_f32(w1));
+      at[(int64_t)i * step] = r[i];
     }
-    at += kResidualLoads * step;
   }
 }
 
@@ -446,21 +442,6 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
     if (PAIR) mbar_arrive_cluster(bar_release);
     else mbar_arrive(bar_release);
   }
-  // with a residual the held columns become their bf16 outputs right away: half the registers, which the residual's loads need (the plain
-  // epilogue has them to spare and is 1.5 % faster without: nvfp4 4096 x 6144 x 2560 32.2 against 32.7 us)
-  constexpr bool kHold = EPI == TF_EPI_RESIDUAL;
-  uint32_t held[kOv > 0 ? kOv : 1][16];
-  if (kHold) {
-#pragma unroll
-    for (int i = 0; i < kOv; ++i) {
-      if (chunk_is_mine<GRP, EPI, BLOCK_N>(kOvFirst + i)) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          held[i][j] = pack_bf16x2(__fmul_rn(__uint_as_float(ov[i][2 * j]), alpha), __fmul_rn(__uint_as_float(ov[i][2 * j + 1]), alpha));
-      }
-    }
-  }
-
 #pragma unroll
   for (int c = 0; c < kOutCols / 32; ++c) {
     if (!chunk_is_mine<GRP, EPI, BLOCK_N>(c)) continue;
@@ -468,13 +449,8 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
     const bool v_in_regs = kOv > 0 && c >= kOvFirst && c < kOvFirst + kOv;
     if (v_in_regs) {
       const int h = (c - kOvFirst) < 0 ? 0 : ((c - kOvFirst) >= kOv ? 0 : (c - kOvFirst));
-      if (!kHold) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = ov[h][j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) packed[j] = held[h][j];
-      }
+      for (int j = 0; j < 32; ++j) v[j] = ov[h][j];
     } else {
       tc_ld32(t_acc + c * 32, v);
     }
@@ -498,7 +474,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
         const float hi = __fmul_rn(silu_f32(bf16hi_to_f32(g2)), bf16hi_to_f32(u2));
         packed[j] = pack_bf16x2(lo, hi);
       }
-    } else if (!v_in_regs || !kHold) {
+    } else {
       if (!v_in_regs) tc_wait_ld();
 #pragma unroll
       for (int j = 0; j < 16; ++j)
@@ -524,11 +500,48 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
       // a box that starts inside the matrix is clipped at its edges; one that starts outside is not stored
       if (lane == 0 && row < p.m && col0 + (c - 1) * 32 < p.n) tma_store_2d(tma_out, stage_smem, col0 + (c - 1) * 32, row);
       if (lane == 0) bulk_commit();
-      if (EPI == TF_EPI_RESIDUAL) {
-        residual_add_box(p, stage_smem, lane, row - lane, col0 + (c - 1) * 32);
-        __syncwarp();  // every lane has read the box before the next chunk is staged in it
-      }
     }
+  }
+}
+
+// The pair kernel's epilogue with a residual, one pair of chunks (64 columns) after the other: staged as bf16, stored, and added into the residual
+// with nothing held in registers but the residual's loads. The columns shared with the other accumulator (chunks 5-7 of accumulator 0, 0-2 of
+// accumulator 1) lie in a group's first pair here, so they need not be held either. Four loads in flight and held columns -> this (graphs of 10):
+// mxfp4 787 x 7536 x 1696 23.4 -> 19.8 us, 1000 x 3000 x 2720 16.6 -> 15.4; nvfp4 4096 x 4096 x 4096 56.5 -> 51.0, 8192 x 8192 x 1024 178.6 -> 163.6; mxfp8
+// 8192 x 2560 x 3072 75.9 -> 70.5, 1024 x 4096 x 4096 22.0 -> 21.7. Both pairs staged at once in two boxes cost mxfp8 its fifth ring stage (78.6).
+template <int FMT>
+__device__ __forceinline__ void epilogue_tile_residual(const GemmParams& p, uint32_t t_acc, int buf, int grp, uint32_t bar_release, int lane, int row, int col0,
+                                                       float alpha, uint32_t& amax2, const CUtensorMap* tma_out, uint32_t stage_smem) {
+  static_assert(TileCfg<FMT, 256>::kOverlapChunks == 3, "the order of the pairs");
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i) {
+    const int c0 = grp * 2 + (buf == i ? 4 : 0);  // a group's pairs are chunks 2 grp and 2 grp + 4
+    if (lane == 0) bulk_wait_read();              // the box is free once the previous store has read it
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t v[32], packed[16];
+      tc_ld32(t_acc + (c0 + h) * 32, v);
+      tc_wait_ld();
+      if (i == 0 && h == 1) {  // the next tile's MMAs may start
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(bar_release);
+      }
+#pragma unroll
+      for (int e = 0; e < 16; ++e)
+        packed[e] = pack_bf16x2(__fmul_rn(__uint_as_float(v[2 * e]), alpha), __fmul_rn(__uint_as_float(v[2 * e + 1]), alpha));
+      store_chunk<TF_EPI_RESIDUAL, FMT, false>(p, packed, row, col0 + (c0 + h) * 32, amax2);
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        sts_128(stage_smem + (uint32_t)lane * 128u + ((uint32_t)((h * 4 + g) ^ (lane & 7)) << 4), packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0 && row < p.m && col0 + c0 * 32 < p.n) tma_store_2d(tma_out, stage_smem, col0 + c0 * 32, row);
+    if (lane == 0) bulk_commit();
+    residual_add_box(p, stage_smem, lane, row - lane, col0 + c0 * 32);
+    __syncwarp();  // every lane has read the box before the next pair is staged in it
   }
 }
 
@@ -1317,7 +1330,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const int col0 = n_blk * kOutCols;
       const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(load_f32(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), load_f32(p.b_gs)) : alpha;
-      if (acc_buf == 0) {
+      if (EPI == TF_EPI_RESIDUAL) {
+        epilogue_tile_residual<FMT>(p, t_row + acc_buf * Cfg::kAccStride, (int)acc_buf, grp, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+      } else if (acc_buf == 0) {
         if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 0, 0, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
         else epilogue_tile<FMT, BLOCK_N, EPI, 0, 1, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
       } else {
