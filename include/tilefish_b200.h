@@ -209,6 +209,16 @@ TF_API tf_status tf_gemm_blockscaled_static(const void* a_codes, const void* a_s
                                      const void* b_scales, const float* b_global_scale, void* out, int64_t ldo, int64_t m, int64_t n,
                                      int64_t k, int32_t format, int32_t epilogue, void* epilogue_arg, float* out_amax, void* stream);
 
+/* The library gemm's usual call in one: `x` (bf16 [m, k], row stride ldx, as tf_quantize_*) is quantized in `format` into the scratch and multiplied,
+ * exactly as tf_quantize_mxfp8 / _mxfp4 / _nvfp4 / _nvfp4_from_amax / _nvfp4_dynamic followed by tf_gemm_blockscaled.
+ *   x_global_scale, x_amax   nvfp4: the activation's global scale or its amax (device f32, one of the two), or NULL and NULL to compute it
+ *   scratch                  tf_gemm_bf16_scratch_bytes() bytes, 256-byte aligned, whose content does not matter
+ * Every refusal comes before anything is enqueued. The other arguments are tf_gemm_blockscaled's. */
+TF_API int64_t tf_gemm_bf16_scratch_bytes(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue);
+TF_API tf_status tf_gemm_bf16(const void* x, int64_t ldx, const float* x_global_scale, const float* x_amax, const void* b_codes, const void* b_scales,
+                              const float* b_global_scale, void* out, int64_t ldo, int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue,
+                              void* epilogue_arg, float* out_amax, void* scratch, int64_t scratch_bytes, void* stream);
+
 /* The first pass of a split-K problem only (epilogue TF_EPI_NONE): the f32 partial sums stay in the workspace as `*splits` planes
  * [splits][m][n] for a consumer that sums them itself (tf_rmsnorm_quantize_rows: the few-rows step between two blocks, where a separate
  * reduction launch costs as much as the arithmetic). No counterpart in the reference. Shapes that are not split along K

@@ -1846,7 +1846,7 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
                             const void* b_scales, const float* b_global_scale, void* out, int64_t ldo, int64_t m, int64_t n, int64_t k, int32_t format,
                             int32_t epilogue, void* epilogue_arg, float* out_amax, void* q_codes, void* q_scales, int64_t a_global_scale_rows,
                             void* workspace, int64_t workspace_bytes, const uint64_t* scatter_ptrs, int32_t owners, int64_t rows_per_owner,
-                            void* stream_, int32_t* partial_splits = nullptr) {
+                            void* stream_, int32_t* partial_splits = nullptr, bool check_only = false) {
   cudaStream_t stream = (cudaStream_t)stream_;
   TF_CHECK_ARG(format >= TF_FMT_MXFP8 && format <= TF_FMT_NVFP4, "%s: unknown format %d", fn, format);
   TF_CHECK_ARG(epilogue >= TF_EPI_NONE && epilogue <= TF_EPI_RESIDUAL, "%s: unknown epilogue %d", fn, epilogue);
@@ -1875,6 +1875,7 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
   TF_CHECK_ALIGNED(b_scales, 16, "b_scales");
   if (out) TF_CHECK_ALIGNED(out, 16, "out");
   if (epilogue == TF_EPI_RESIDUAL) TF_CHECK_ALIGNED(epilogue_arg, 16, "residual");
+  if (check_only) return TF_OK;  // tf_gemm_bf16, which has sized the workspace itself
 
   const int64_t k_bytes = (format == TF_FMT_MXFP8) ? k : k / 2;
   const int64_t n_rows_b = (epilogue == TF_EPI_SILU_GATE) ? 2 * n : n;
@@ -1959,6 +1960,61 @@ tf_status tf_gemm_blockscaled(const void* a_codes, const void* a_scales, const f
   clear_error();
   return gemm_entry(__func__, a_codes, a_scales, a_global_scale, b_codes, b_scales, b_global_scale, out, ldo, m, n, k, format, epilogue, epilogue_arg,
                     out_amax, q_codes, q_scales, a_global_scale_rows, workspace, workspace_bytes, nullptr, 0, 0, stream);
+}
+
+namespace {
+// The scratch of tf_gemm_bf16: byte offsets of the quantized activation's parts and of the split-K workspace.
+struct Bf16Scratch {
+  int64_t scales, global_scale, partials, workspace, total;
+};
+Bf16Scratch bf16_scratch(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue) {
+  auto align = [](int64_t b) { return (b + 255) / 256 * 256; };
+  Bf16Scratch s;
+  s.scales = align(m * (format == TF_FMT_MXFP8 ? k : k / 2));
+  s.global_scale = s.scales + align(tf_scale_bytes(format, m, k, TF_SCALES_SWIZZLED));
+  s.partials = s.global_scale + (format == TF_FMT_NVFP4 ? 256 : 0);
+  s.workspace = s.partials + (format == TF_FMT_NVFP4 ? align(tf_quantize_nvfp4_dynamic_scratch_bytes()) : 0);
+  s.total = s.workspace + tf_gemm_workspace_bytes(m, n, k, format, epilogue);
+  return s;
+}
+}  // namespace
+
+int64_t tf_gemm_bf16_scratch_bytes(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue) {
+  if (m <= 0 || n <= 0 || k <= 0 || k % 32 || format < TF_FMT_MXFP8 || format > TF_FMT_NVFP4 || epilogue < TF_EPI_NONE || epilogue > TF_EPI_RESIDUAL) return 0;
+  return bf16_scratch(m, n, k, format, epilogue).total;
+}
+
+tf_status tf_gemm_bf16(const void* x, int64_t ldx, const float* x_global_scale, const float* x_amax, const void* b_codes, const void* b_scales,
+                       const float* b_global_scale, void* out, int64_t ldo, int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue,
+                       void* epilogue_arg, float* out_amax, void* scratch, int64_t scratch_bytes, void* stream) {
+  clear_error();
+  TF_CHECK_ARG(m >= 0 && n > 0 && k > 0 && format >= TF_FMT_MXFP8 && format <= TF_FMT_NVFP4 && epilogue >= TF_EPI_NONE && epilogue <= TF_EPI_RESIDUAL, "%s: bad argument", __func__);
+  if (m == 0) return TF_OK;
+  if (k % 32 != 0) return fail(TF_ERR_UNSUPPORTED, "%s: k=%lld is not a multiple of 32", __func__, (long long)k);
+  TF_CHECK_ARG(!(x_global_scale && x_amax), "%s: x_global_scale and x_amax exclude each other", __func__);
+  const Bf16Scratch at = bf16_scratch(m, n, k, format, epilogue);
+  if (!scratch || scratch_bytes < at.total) return fail(TF_ERR_WORKSPACE, "%s: needs %lld bytes of scratch (tf_gemm_bf16_scratch_bytes)", __func__, (long long)at.total);
+  TF_CHECK_ALIGNED(scratch, 256, "scratch");
+  uint8_t* base = static_cast<uint8_t*>(scratch);
+  float* own_scale = reinterpret_cast<float*>(base + at.global_scale);
+  const float* a_gs = format != TF_FMT_NVFP4 ? nullptr : x_global_scale ? x_global_scale : own_scale;
+  tf_status st = TF_OK;
+  for (int pass = 0; pass < 2; ++pass) {  // first what the multiplication refuses, then the quantization, then the multiplication
+    st = gemm_entry(__func__, base, base + at.scales, a_gs, b_codes, b_scales, b_global_scale, out, ldo, m, n, k, format, epilogue, epilogue_arg, out_amax, nullptr, nullptr, 0,
+                    base + at.workspace, at.total - at.workspace, nullptr, 0, 0, stream, nullptr, pass == 0);
+    if (st != TF_OK || pass == 1) return st;
+    switch (format) {
+      case TF_FMT_MXFP8: st = tf_quantize_mxfp8(x, m, k, ldx, base, base + at.scales, TF_SCALES_SWIZZLED, stream); break;
+      case TF_FMT_MXFP4: st = tf_quantize_mxfp4(x, m, k, ldx, base, base + at.scales, TF_SCALES_SWIZZLED, stream); break;
+      default:
+        st = x_global_scale ? tf_quantize_nvfp4(x, m, k, ldx, base, base + at.scales, TF_SCALES_SWIZZLED, x_global_scale, stream)
+             : x_amax       ? tf_quantize_nvfp4_from_amax(x, m, k, ldx, base, base + at.scales, TF_SCALES_SWIZZLED, x_amax, own_scale, stream)
+                            : tf_quantize_nvfp4_dynamic(x, m, k, ldx, base, base + at.scales, TF_SCALES_SWIZZLED, own_scale,
+                                                        reinterpret_cast<float*>(base + at.partials), stream);
+    }
+    if (st != TF_OK) return st;
+  }
+  return st;
 }
 
 tf_status tf_gemm_blockscaled_partials(const void* a_codes, const void* a_scales, const float* a_global_scale, const void* b_codes, const void* b_scales,

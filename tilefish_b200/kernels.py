@@ -9,6 +9,7 @@ reference checks a launch (python/src/tilefish/_launch.py:263-315, :433-500); fa
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Tuple
 
 from . import _native as N
@@ -64,6 +65,11 @@ def _check_failed(t, name: str, dtype, rank: Optional[int], device, align: int) 
 def _dense(t, name: str) -> None:
     if not t.is_contiguous():
         _pre(False, f"{name}: must be contiguous (strides {tuple(t.stride())})", "contiguous", name)
+
+
+def _empty_rows(m: int, n: int, dtype, device):
+    """``torch.empty((m, n))`` by its strides: two thirds of the call's time."""
+    return _torch().empty_strided((m, n), (n, 1), dtype=dtype, device=device)
 
 
 def _stream(stream) -> int:
@@ -149,6 +155,24 @@ def nvfp4_global_scale(x, *, out=None, stream=None):
     return out
 
 
+def _quantizer_source(x):
+    """The checks of a tensor to quantize: (m, k, its row stride, the row stride for the kernels, its address)."""
+    _check(x, "x", _torch().bfloat16, 2)
+    m, k = x.shape
+    ld, inner = x.stride()
+    _pre(inner == 1 and (m <= 1 or (ld >= k and ld % 16 == 0)), "x: rows must be dense with a row stride that is a multiple of 16", "contiguous", "x")
+    if k % 32 != 0 or k <= 0:
+        _pre(False, f"x: K={k} is not a multiple of 32", "divisible", "x")
+    xp = x.data_ptr()
+    _pre(m == 0 or xp % 32 == 0, "x: the data pointer is not 32-byte aligned (the quantizer uses 256-bit loads)", "pointer_alignment", "x")
+    return m, k, ld, ld if m > 1 else k, xp
+
+
+@functools.lru_cache(maxsize=1)
+def _dynamic_scratch_bytes() -> int:
+    return int(N.load().tf_quantize_nvfp4_dynamic_scratch_bytes())
+
+
 def quantize(x, fmt: str, *, layout: str = "swizzled", global_scale=None, amax=None, out: Optional[BlockScaledTensor] = None,
              stream=None) -> BlockScaledTensor:
     """BlockScaled quantization of a bf16 [M, K] tensor along K.
@@ -161,22 +185,14 @@ def quantize(x, fmt: str, *, layout: str = "swizzled", global_scale=None, amax=N
         _pre(False, f"unknown block-scaled format {fmt!r}", "dtype", "fmt")
     if layout != "swizzled" and layout != "plain":
         _pre(False, f"unknown scale layout {layout!r}", "argument", "layout")
-    _check(x, "x", torch.bfloat16, 2)
-    m, k = x.shape
-    ld, inner = x.stride()
-    _pre(inner == 1 and (m <= 1 or (ld >= k and ld % 16 == 0)), "x: rows must be dense with a row stride that is a multiple of 16", "contiguous", "x")
-    if k % 32 != 0 or k <= 0:
-        _pre(False, f"x: K={k} is not a multiple of 32", "divisible", "x")
-    xp = x.data_ptr()
-    _pre(m == 0 or xp % 32 == 0, "x: the data pointer is not 32-byte aligned (the quantizer uses 256-bit loads)", "pointer_alignment", "x")
-    ldx = ld if m > 1 else k
+    m, k, ld, ldx, xp = _quantizer_source(x)
     lay = N.SCALES_SWIZZLED if layout == "swizzled" else N.SCALES_PLAIN
     if out is not None:  # preallocated result (a plan's arena): same format, shape and layout
         if out.fmt != fmt or out.shape != (m, k) or out.layout != layout:
             _pre(False, f"out: expected a {fmt} {layout} tensor of shape {(m, k)}", "shape", "out")
         codes, scales = out.codes, out.scales
     else:
-        codes = torch.empty((m, k // ELEMS_PER_BYTE[fmt]), dtype=torch.uint8, device=x.device)
+        codes = _empty_rows(m, k // ELEMS_PER_BYTE[fmt], torch.uint8, x.device)
         scales = torch.empty(_swizzled_bytes(fmt, m, k) if layout == "swizzled" else m * (k // BLOCK[fmt]), dtype=torch.uint8, device=x.device)
     s = _stream(stream)
     lib = N.load()
@@ -194,7 +210,7 @@ def quantize(x, fmt: str, *, layout: str = "swizzled", global_scale=None, amax=N
     elif fmt == "nvfp4" and global_scale is None:
         _pre(ld % 16 == 0, "x: rows must be dense, K and the row stride multiples of 16", "contiguous", "x")
         gs = out.global_scale if out is not None and out.global_scale is not None else torch.empty(1, dtype=torch.float32, device=x.device)
-        scratch = torch.empty(lib.tf_quantize_nvfp4_dynamic_scratch_bytes(), dtype=torch.uint8, device=x.device)
+        scratch = torch.empty(_dynamic_scratch_bytes(), dtype=torch.uint8, device=x.device)
         N.check(lib.tf_quantize_nvfp4_dynamic(xp, m, k, ldx, codes.data_ptr(), scales.data_ptr(), lay, gs.data_ptr(), scratch.data_ptr(), s),
                 "tf_quantize_nvfp4_dynamic")
     elif fmt == "nvfp4":
@@ -251,7 +267,7 @@ def residual_add_rmsnorm(x, residual, w, eps: float = 1e-6, *, out=None, quantiz
         _pre(False, f"x: D={d} is not a multiple of 8", "divisible", "x")
     if want_bf16:
         if out is None:
-            out = torch.empty((m, d), dtype=torch.bfloat16, device=x.device)
+            out = _empty_rows(m, d, torch.bfloat16, x.device)
         else:
             _check(out, "out", torch.bfloat16, 2, x.device)
             _dense(out, "out")
@@ -270,7 +286,7 @@ def residual_add_rmsnorm(x, residual, w, eps: float = 1e-6, *, out=None, quantiz
             _pre(q_out.fmt == quantize_to and q_out.shape == (m, d) and q_out.layout == "swizzled", "q_out: wrong format or shape", "shape", "q_out")
             codes, scales = q_out.codes, q_out.scales
         else:
-            codes = torch.empty((m, d // ELEMS_PER_BYTE[quantize_to]), dtype=torch.uint8, device=x.device)
+            codes = _empty_rows(m, d // ELEMS_PER_BYTE[quantize_to], torch.uint8, x.device)
             scales = torch.empty(_swizzled_bytes(quantize_to, m, d), dtype=torch.uint8, device=x.device)
         if quantize_to == "nvfp4":
             _pre(q_global_scale is not None, "nvfp4 output needs q_global_scale (a float32 [1] device tensor)", "argument", "q_global_scale")
@@ -334,8 +350,38 @@ def set_programmatic_launch(enabled: Optional[bool]) -> None:
     N.check(N.load().tf_set_programmatic_launch(-1 if enabled is None else 1 if enabled else 0), "tf_set_programmatic_launch")
 
 
+@functools.lru_cache(maxsize=1024)
+def _scratch_bytes(device: int, entry: str, m: int, n: int, k: int, fmt_id: int, epi_id: int) -> int:
+    """What the library's size query ``entry`` says: a function of the sizes and of the device's SM count alone."""
+    return int(getattr(N.load(), entry)(m, n, k, fmt_id, epi_id))
+
+
 def gemm_workspace_bytes(m: int, n: int, k: int, fmt: str, epilogue: str = "none") -> int:
     return int(N.load().tf_gemm_workspace_bytes(m, n, k, FORMATS[fmt], EPILOGUES[epilogue]))
+
+
+def _check_gemm_out(out, m: int, n: int, device) -> None:
+    _check(out, "out", _torch().bfloat16, 2, device)
+    _pre(tuple(out.shape) == (m, n) and out.stride(1) == 1 and (m <= 1 or out.stride(0) % 8 == 0), "out: wrong shape or strides", "shape", "out")
+
+
+def _residual_ptr(residual, m: int, n: int, device) -> int:
+    _pre(residual is not None, "epilogue='residual' needs the f32 residual", "argument", "residual")
+    _check(residual, "residual", _torch().float32, 2, device)
+    _dense(residual, "residual")
+    _pre(tuple(residual.shape) == (m, n), "residual: wrong shape", "shape", "residual")
+    return residual.data_ptr()
+
+
+def _gemm_rows(epilogue: str, nb: int) -> int:
+    """Output columns for ``nb`` rows of b."""
+    if epilogue not in EPILOGUES:
+        _pre(False, f"unknown epilogue {epilogue!r}", "argument", "epilogue")
+    if epilogue != "silu_gate":
+        return nb
+    if nb % 256 != 0:
+        _pre(False, f"silu_gate: b has {nb} rows; each half must be a multiple of 128", "divisible", "b")
+    return nb // 2
 
 
 def gemm_blockscaled(a: BlockScaledTensor, b: BlockScaledTensor, *, epilogue: str = "none", out=None, residual=None, amax_out=None,
@@ -353,15 +399,11 @@ def gemm_blockscaled(a: BlockScaledTensor, b: BlockScaledTensor, *, epilogue: st
     if a.fmt != b.fmt:
         _pre(False, f"a is {a.fmt} but b is {b.fmt}: block-scaled formats must match exactly", "dtype", "b")
     _pre(a.layout == "swizzled" and b.layout == "swizzled", "the GEMM consumes swizzled scales", "contiguous")
-    if epilogue not in EPILOGUES:
-        _pre(False, f"unknown epilogue {epilogue!r}", "argument", "epilogue")
     m, k = a.shape
     nb, kb = b.shape
     if k != kb:
         _pre(False, f"K differs: a is {a.shape}, b is {b.shape}", "shape", "b")
-    n = nb // 2 if epilogue == "silu_gate" else nb
-    if epilogue == "silu_gate" and nb % 256 != 0:
-        _pre(False, f"silu_gate: b has {nb} rows; each half must be a multiple of 128", "divisible", "b")
+    n = _gemm_rows(epilogue, nb)
     device = a.device
     _pre(device == b.device, "a and b are on different devices", "device", "b")
     for t, nm in ((a.codes, "a.codes"), (b.codes, "b.codes"), (a.scales, "a.scales"), (b.scales, "b.scales")):
@@ -385,20 +427,13 @@ def gemm_blockscaled(a: BlockScaledTensor, b: BlockScaledTensor, *, epilogue: st
     if not want_bf16:
         out = None
     elif out is None:
-        out = torch.empty((m, n), dtype=torch.bfloat16, device=device)
+        out = _empty_rows(m, n, torch.bfloat16, device)
     else:
-        _check(out, "out", torch.bfloat16, 2, a.device)
-        _pre(tuple(out.shape) == (m, n) and out.stride(1) == 1 and (m <= 1 or out.stride(0) % 8 == 0), "out: wrong shape or strides", "shape", "out")
+        _check_gemm_out(out, m, n, device)
     ldo = out.stride(0) if (out is not None and m > 1) else n
-    res_ptr = None
-    if epilogue == "residual":
-        _pre(residual is not None, "epilogue='residual' needs the f32 residual", "argument", "residual")
-        _check(residual, "residual", torch.float32, 2, a.device)
-        _dense(residual, "residual")
-        _pre(tuple(residual.shape) == (m, n), "residual: wrong shape", "shape", "residual")
-        res_ptr = residual.data_ptr()
+    res_ptr = _residual_ptr(residual, m, n, device) if epilogue == "residual" else None
     lib, fmt_id, epi_id = N.load(), FORMATS[a.fmt], EPILOGUES[epilogue]
-    need = lib.tf_gemm_workspace_bytes(m, n, k, fmt_id, epi_id)
+    need = _scratch_bytes(torch._C._cuda_getDevice(), "tf_gemm_workspace_bytes", m, n, k, fmt_id, epi_id) if m > 0 else 0
     ws_ptr, ws_bytes = None, 0
     if need > 0:
         if workspace is None:
@@ -559,9 +594,51 @@ def rmsnorm_quantize_rows(x, residual, w, eps: float, fmt: str, q_out: BlockScal
 def gemm(a, b: BlockScaledTensor, *, epilogue: str = "none", out=None, residual=None, a_global_scale=None, a_amax=None, amax_out=None,
          stream=None):
     """The library ``gemm``: ``a`` is bf16 [M, K] (quantized on the fly in b's format) or already a BlockScaledTensor."""
-    if not isinstance(a, BlockScaledTensor):
-        a = quantize(a, b.fmt, global_scale=a_global_scale, amax=a_amax, stream=stream)
-    return gemm_blockscaled(a, b, epilogue=epilogue, out=out, residual=residual, amax_out=amax_out, stream=stream)
+    torch = _torch()
+    if not isinstance(a, torch.Tensor) or not isinstance(b, BlockScaledTensor) or b.layout != "swizzled" or a.dim() != 2 or a.shape[0] == 0:
+        if not isinstance(a, BlockScaledTensor):
+            a = quantize(a, b.fmt, global_scale=a_global_scale, amax=a_amax, stream=stream)
+        return gemm_blockscaled(a, b, epilogue=epilogue, out=out, residual=residual, amax_out=amax_out, stream=stream)
+    # One native call and one scratch tensor for both steps. With a call and tensors for each (codes, scales, global scale, its scratch, workspace)
+    # 16 x 6144 x 2560 mxfp8 took 28.4 us of Python and launches, now 17.6.
+    m, k, ld, ldx, xp = _quantizer_source(a)
+    device, fmt = a.device, b.fmt
+    nb, kb = b.shape
+    if k != kb:
+        _pre(False, f"K differs: a is {(m, k)}, b is {b.shape}", "shape", "b")
+    n = _gemm_rows(epilogue, nb)
+    codes, scales, gs, agp, amp, bgp = b.codes, b.scales, b.global_scale, None, None, None
+    _check(codes, "b.codes", torch.uint8, None, device)
+    _check(scales, "b.scales", torch.uint8, None, device)
+    _dense(codes, "b.codes")
+    _dense(scales, "b.scales")
+    if fmt == "nvfp4":
+        _pre(gs is not None, "nvfp4 operands need their global scales", "argument")
+        bgp = gs.data_ptr()
+        if a_amax is not None:
+            _check(a_amax, "amax", torch.float32, None, device, align=4)
+            _pre(a_amax.numel() == 1 and a_global_scale is None, "amax: expected one element and no global_scale", "shape", "amax")
+            amp = a_amax.data_ptr()
+        elif a_global_scale is not None:
+            _check(a_global_scale, "global_scale", torch.float32, None, device, align=4)
+            _pre(a_global_scale.numel() == 1, "global_scale: expected one element", "shape", "global_scale")
+            agp = a_global_scale.data_ptr()
+        else:
+            _pre(ld % 16 == 0, "x: rows must be dense, K and the row stride multiples of 16", "contiguous", "x")
+    if out is None:
+        out = _empty_rows(m, n, torch.bfloat16, device)
+    else:
+        _check_gemm_out(out, m, n, device)
+    fmt_id, epi_id = FORMATS[fmt], EPILOGUES[epilogue]
+    need = _scratch_bytes(torch._C._cuda_getDevice(), "tf_gemm_bf16_scratch_bytes", m, n, k, fmt_id, epi_id)
+    scratch = torch.empty(need, dtype=torch.uint8, device=device)
+    N.check(
+        N.load().tf_gemm_bf16(xp, ldx, agp, amp, codes.data_ptr(), scales.data_ptr(), bgp, out.data_ptr(), out.stride(0) if m > 1 else n, m, n, k, fmt_id, epi_id,
+                              _residual_ptr(residual, m, n, device) if epilogue == "residual" else None, _amax_ptr(amax_out, device), scratch.data_ptr(), need,
+                              _stream(stream)),
+        "tf_gemm_bf16",
+    )
+    return out
 
 
 def require_cuda() -> None:
