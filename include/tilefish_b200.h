@@ -232,7 +232,7 @@ TF_API tf_status tf_gemm_blockscaled_partials(const void* a_codes, const void* a
 
 /* How tf_gemm_blockscaled launches a problem under the settings in force, for tests and profiles (no counterpart in the reference): form[0] = 0
  * one CTA per tile, 1 K ranges as planes of the workspace and a reduction launch, 2 K ranges over a cluster of CTAs, 3 a pair of CTAs per
- * 256 x 256 tile; form[1] = accumulator columns of a tile (of one CTA); form[2] = K ranges; form[3] = 1 for a programmatic dependent. */
+ * 256 x 256 or 256 x 192 tile; form[1] = accumulator columns of a tile; form[2] = K ranges; form[3] = 1 for a programmatic dependent. */
 TF_API tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, int32_t epilogue, int32_t* form);
 
 /* The GEMM with a scattered output: the tensor-parallel second GEMM (w_d split along K) whose epilogue delivers each row block of

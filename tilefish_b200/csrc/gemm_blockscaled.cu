@@ -504,26 +504,25 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t t_ac
   }
 }
 
-// The pair kernel's epilogue with a residual, one pair of chunks (64 columns) after the other: staged as bf16, stored, and added into the residual
-// with nothing held in registers but the residual's loads. The columns shared with the other accumulator (chunks 5-7 of accumulator 0, 0-2 of
-// accumulator 1) lie in a group's first pair here, so they need not be held either. Four loads in flight and held columns -> this (graphs of 10):
+// The pair kernel's epilogue one pair of chunks (64 columns) after the other: `count` pairs from chunk c0 on, c_step chunks apart; staged as bf16,
+// stored, and (residual) added with nothing held in registers but the residual's loads. The accumulator is released behind pair `release_at`: the last
+// one where tiles have accumulators of their own (192 columns), the first one with 256 columns. There the columns shared with the other accumulator (chunks 5-7 of accumulator 0, 0-2 of
+// accumulator 1) lie in a group's first pair, so they need not be held either. Residual, four loads in flight and held columns -> this (graphs of 10):
 // mxfp4 787 x 7536 x 1696 23.4 -> 19.8 us, 1000 x 3000 x 2720 16.6 -> 15.4; nvfp4 4096 x 4096 x 4096 56.5 -> 51.0, 8192 x 8192 x 1024 178.6 -> 163.6; mxfp8
 // 8192 x 2560 x 3072 75.9 -> 70.5, 1024 x 4096 x 4096 22.0 -> 21.7. Both pairs staged at once in two boxes cost mxfp8 its fifth ring stage (78.6).
-template <int FMT>
-__device__ __forceinline__ void epilogue_tile_residual(const GemmParams& p, uint32_t t_acc, int buf, int grp, uint32_t bar_release, int lane, int row, int col0,
-                                                       float alpha, uint32_t& amax2, const CUtensorMap* tma_out, uint32_t stage_smem) {
-  static_assert(TileCfg<FMT, 256>::kOverlapChunks == 3, "the order of the pairs");
+template <int FMT, int EPI>
+__device__ __forceinline__ void epilogue_pairs(const GemmParams& p, uint32_t t_acc, int c0, int c_step, int count, int release_at, uint32_t bar_release, int lane,
+                                               int row, int col0, float alpha, uint32_t& amax2, const CUtensorMap* tma_out, uint32_t stage_smem) {
 #pragma unroll 1
-  for (int i = 0; i < 2; ++i) {
-    const int c0 = grp * 2 + (buf == i ? 4 : 0);  // a group's pairs are chunks 2 grp and 2 grp + 4
-    if (lane == 0) bulk_wait_read();              // the box is free once the previous store has read it
+  for (int i = 0; i < count; ++i, c0 += c_step) {
+    if (lane == 0) bulk_wait_read();  // the box is free once the previous store has read it
     __syncwarp();
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       uint32_t v[32], packed[16];
       tc_ld32(t_acc + (c0 + h) * 32, v);
       tc_wait_ld();
-      if (i == 0 && h == 1) {  // the next tile's MMAs may start
+      if (i == release_at && h == 1) {  // the accumulator (or what the next tile's shares of it) is read
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(bar_release);
@@ -531,17 +530,23 @@ __device__ __forceinline__ void epilogue_tile_residual(const GemmParams& p, uint
 #pragma unroll
       for (int e = 0; e < 16; ++e)
         packed[e] = pack_bf16x2(__fmul_rn(__uint_as_float(v[2 * e]), alpha), __fmul_rn(__uint_as_float(v[2 * e + 1]), alpha));
-      store_chunk<TF_EPI_RESIDUAL, FMT, false>(p, packed, row, col0 + (c0 + h) * 32, amax2);
+      store_chunk<EPI, FMT, false>(p, packed, row, col0 + (c0 + h) * 32, amax2);
+      if (p.out) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
-        sts_128(stage_smem + (uint32_t)lane * 128u + ((uint32_t)((h * 4 + g) ^ (lane & 7)) << 4), packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
+        for (int g = 0; g < 4; ++g)
+          sts_128(stage_smem + (uint32_t)lane * 128u + ((uint32_t)((h * 4 + g) ^ (lane & 7)) << 4), packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
+      }
     }
+    if (!p.out) continue;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
+    // a box that starts inside the matrix is clipped at its edges; one that starts outside is not stored
     if (lane == 0 && row < p.m && col0 + c0 * 32 < p.n) tma_store_2d(tma_out, stage_smem, col0 + c0 * 32, row);
     if (lane == 0) bulk_commit();
-    residual_add_box(p, stage_smem, lane, row - lane, col0 + c0 * 32);
-    __syncwarp();  // every lane has read the box before the next pair is staged in it
+    if (EPI == TF_EPI_RESIDUAL) {
+      residual_add_box(p, stage_smem, lane, row - lane, col0 + c0 * 32);
+      __syncwarp();  // every lane has read the box before the next pair is staged in it
+    }
   }
 }
 
@@ -1100,8 +1105,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
 }
 
 // ---- the 2-CTA kernel ------------------------------------------------------------------------------------------------------
-// Two CTAs of a cluster (a pair of SMs) compute one 256 x 256 tile with tcgen05.mma.cta_group::2: CTA r of the pair holds rows
-// [128 r, 128 r + 128) of the A tile and of the B tile in its own shared memory and the accumulator of its 128 rows in its own
+// Two CTAs of a cluster (a pair of SMs) compute one 256 x 256 tile (or 256 x 192, see pair_width) with tcgen05.mma.cta_group::2: CTA r of the pair holds
+// rows [128 r, 128 r + 128) of the A tile and half r of the B tile in its own shared memory and the accumulator of its 128 rows in its own
 // tensor memory. Per stage each SM fills 256 operand rows instead of the 384 that bound the one-CTA kernel (38 KB instead of 54
 // for nvfp4). Each CTA loads its own halves with plain (non-multicast) TMA; the scale tiles of all 256 B rows are loaded by
 // both CTAs (4 KB per stage). The warp roles are the one-CTA kernel's: operand loads (warp 0) and scale loads (warp 6), one
@@ -1110,10 +1115,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
 // peer's load and epilogue warps signal the leader through cluster-mapped mbarrier addresses. The bf16 outputs are staged in
 // shared memory (a 4 KB box per epilogue warp) and leave as TMA stores: whole 128-byte lines instead of 32 partial lines per
 // warp instruction. Same bounded waits and teardown as the one-CTA kernel, plus a cluster barrier at both ends.
-template <int FMT>
+template <int FMT, int BLOCK_N>
 struct PairCfg {
+  static_assert(BLOCK_N == 256 || BLOCK_N == 192, "tile widths of the pair");
   static constexpr int kST = FmtTraits<FMT>::kSfTiles;
-  static constexpr int kBHalfBytes = 128 * kStageKBytes;
+  static constexpr int kBHalfBytes = BLOCK_N / 2 * kStageKBytes;
   static constexpr int kSfaStageBytes = kST * 512;
   static constexpr int kSfbStageBytes = kST * 512 * 2;
   static constexpr int kStageBytes = kAStageBytes + kBHalfBytes + kSfaStageBytes + kSfbStageBytes;
@@ -1122,18 +1128,23 @@ struct PairCfg {
   static constexpr int kOutStageBytes = 8 * kOutBoxBytes;
   static constexpr int kStagesRaw = (kSmemLimit - 1024 - kBarrierBytes - kOutStageBytes) / kStageBytes;
   static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
+  // Tensor memory of each CTA (128 lanes): 256 columns as the one-CTA kernel's; two accumulators of 192 and the scales fit without overlap
+  static constexpr int kAccStride = BLOCK_N == 256 ? TileCfg<FMT, 256>::kAccStride : BLOCK_N;
+  static constexpr int kAccBars = BLOCK_N == 256 ? 1 : 2;  // full and empty barriers: one pair for both accumulators, or one each
+  static constexpr int kTmemSfSet = kST * 12;              // the A scales and those of two 128-row tiles of B
+  static constexpr int kTmemSfa = kAccStride + BLOCK_N, kTmemSfb = kTmemSfa + kST * 4;
+  static_assert(kTmemSfa + 2 * kTmemSfSet <= 512, "tensor memory budget");
   static constexpr int kSmemBytes = kStages * kStageBytes + kOutStageBytes + kBarrierBytes + 1024;
 };
 
-template <int FMT, int EPI>
+template <int FMT, int EPI, int BLOCK_N>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                                  const __grid_constant__ CUtensorMap tma_b,
                                                                                  const __grid_constant__ CUtensorMap tma_sfa,
                                                                                  const __grid_constant__ CUtensorMap tma_sfb,
                                                                                  const __grid_constant__ CUtensorMap tma_out, const GemmParams p) {
-  constexpr int BLOCK_N = 256;
-  using Cfg = TileCfg<FMT, BLOCK_N>;  // tensor-memory layout (per CTA: 128 lanes x 256 columns) is the one-CTA kernel's
-  using PC = PairCfg<FMT>;
+  static_assert(EPI != TF_EPI_SILU_GATE || BLOCK_N == 256, "the SiLU-gate epilogue pairs a 128-column gate tile with its up tile");
+  using PC = PairCfg<FMT, BLOCK_N>;
   constexpr int kStages = PC::kStages;
   constexpr int kST = PC::kST;
   constexpr int kNB = 2;
@@ -1151,8 +1162,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
   const uint32_t smem_sfa = smem_out + PC::kOutStageBytes;
   const uint32_t smem_sfb = smem_sfa + kStages * PC::kSfaStageBytes;
   const uint32_t bars = smem_sfb + kStages * PC::kSfbStageBytes;
-  const uint32_t bar_full = bars, bar_empty = bars + 8 * kStages, bar_tmem_full = bars + 16 * kStages, bar_tmem_empty = bar_tmem_full + 8;
-  const uint32_t tmem_slot = bar_tmem_empty + 8;
+  const uint32_t bar_full = bars, bar_empty = bars + 8 * kStages, bar_tmem_full = bars + 16 * kStages,
+                 bar_tmem_empty = bar_tmem_full + 8 * PC::kAccBars;
+  const uint32_t tmem_slot = bar_tmem_empty + 8 * PC::kAccBars;
   const uint32_t abort_slot = tmem_slot + 4;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_gen + (tmem_slot - smem_base));
@@ -1168,13 +1180,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
       mbar_init(bar_full + 8 * s, kTurns ? 2 : 4);  // an arrive.expect_tx of each load warp that serves the stage, from both CTAs (used in the leader only)
       mbar_init(bar_empty + 8 * s, 1);  // the leader's commit arrives in both CTAs
     }
-    mbar_init(bar_tmem_full, 1);
-    mbar_init(bar_tmem_empty, 16);  // 8 epilogue warps of each CTA (used in the leader only)
+    for (int i = 0; i < PC::kAccBars; ++i) {
+      mbar_init(bar_tmem_full + 8 * i, 1);
+      mbar_init(bar_tmem_empty + 8 * i, 16);  // 8 epilogue warps of each CTA (used in the leader only)
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // the same warp of both CTAs allocates the pair's tensor memory
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"((uint32_t)Cfg::kTmemCols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -1196,17 +1210,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
     const bool serves_a = lane == 0 || lane == 2;
     const CUtensorMap* my_map = lane == 0 ? &tma_a : lane == 1 ? &tma_b : lane == 2 ? &tma_sfa : &tma_sfb;
     const uint32_t my_dst = lane == 0 ? smem_a : lane == 1 ? smem_b : lane == 2 ? smem_sfa : smem_sfb + (uint32_t)half * kST * 512;
-    const uint32_t my_stage_bytes = lane < 2 ? kAStageBytes : lane == 2 ? PC::kSfaStageBytes : PC::kSfbStageBytes;
+    const uint32_t my_stage_bytes = lane == 0 ? kAStageBytes : lane == 1 ? PC::kBHalfBytes : lane == 2 ? PC::kSfaStageBytes : PC::kSfbStageBytes;
     int stage = turn, ks0 = turn;
     uint32_t phase = 0;
     bool ok = true;
     for (int tile = pair; tile < p.num_tiles && ok; tile += num_pairs) {
       const int m_blk = tile % p.m_blocks, n_blk = tile / p.m_blocks;
       const int a_row = m_blk * 256 + (int)rank * 128;
-      const int b_row = (EPI == TF_EPI_SILU_GATE) ? half * p.n + n_blk * 128 : n_blk * BLOCK_N + half * 128;
+      // first B row of the lane's half, or (scales) of its 128-row tile: a 192-column tile starts in the middle of one or at its edge
+      const int b_row = (EPI == TF_EPI_SILU_GATE) ? half * p.n + n_blk * 128
+                        : BLOCK_N == 256 || !sf   ? n_blk * BLOCK_N + half * (BLOCK_N / 2)
+                                                  : ((n_blk * BLOCK_N) & ~127) + half * 128;
       const int my_row = serves_a ? a_row : b_row;
       const bool mine = lane < 5 && (kTurns || sf == (warp == 6)) && (serves_a ? a_row < p.m : b_row < p.n_rows_b);
-      const uint32_t tx = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && !sf)) * kAStageBytes + (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && sf)) * (kST * 512u);
+      const uint32_t tx = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && lane == 0)) * kAStageBytes +
+                          (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && lane == 1)) * PC::kBHalfBytes +
+                          (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && sf)) * (kST * 512u);
       const int y_base = sf ? (my_row >> 7) * p.sf_col_tiles : my_row;
       int ks = ks0;
       for (; ks < p.num_k_stages; ks += kStep) {
@@ -1243,19 +1262,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
       uint32_t phase = 0, tile_phase = 0, sf_buf = 0, acc_buf = 0;
       bool ok = true;
       for (int tile = pair; tile < p.num_tiles && ok; tile += num_pairs) {
-        ok = mbar_wait(bar_tmem_empty, tile_phase ^ 1, abort_flag, 2);
+        const uint32_t acc_bar = PC::kAccBars == 1 ? 0u : 8 * acc_buf;
+        ok = mbar_wait(bar_tmem_empty + acc_bar, tile_phase ^ 1, abort_flag, 2);
         ok = __all_sync(0xFFFFFFFFu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t tmem_acc = tmem_base + acc_buf * Cfg::kAccStride;
-        acc_buf ^= 1;
+        const uint32_t tmem_acc = tmem_base + acc_buf * PC::kAccStride;
+        const uint32_t sfb_shift = BLOCK_N == 256 ? 0u : (uint32_t)(tile / p.m_blocks & 1) * 2u;  // odd 192-column tiles start 64 rows into their scales
         for (int ks = 0; ks < p.num_k_stages; ++ks) {
           ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, 3);
           ok = __all_sync(0xFFFFFFFFu, ok);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t tmem_sfa = tmem_base + Cfg::kTmemSfa + sf_buf * Cfg::kTmemSfSet;
-          const uint32_t tmem_sfb = tmem_base + Cfg::kTmemSfb + sf_buf * Cfg::kTmemSfSet;
+          const uint32_t tmem_sfa = tmem_base + PC::kTmemSfa + sf_buf * PC::kTmemSfSet;
+          const uint32_t tmem_sfb = tmem_base + PC::kTmemSfb + sf_buf * PC::kTmemSfSet;
           sf_buf ^= 1;
           const uint32_t sfa_lo = ((smem_sfa + stage * PC::kSfaStageBytes) & 0x3FFFFu) >> 4;
           const uint32_t sfb_lo = ((smem_sfb + stage * PC::kSfbStageBytes) & 0x3FFFFu) >> 4;
@@ -1277,7 +1297,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
                 const int t = (FMT == TF_FMT_MXFP8) ? 0 : (FMT == TF_FMT_MXFP4) ? (j >> 1) : j;
                 const uint32_t sf_id = (FMT == TF_FMT_MXFP8) ? (uint32_t)j : (FMT == TF_FMT_MXFP4) ? (uint32_t)((j & 1) * 2) : 0u;
                 tc_mma_pair<FMT>(tmem_acc, make_desc(a_lo + j * 2, kDescHiSw128), make_desc(b_lo + j * 2, kDescHiSw128),
-                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4, j > 0 ? 1u : first);
+                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4 + sfb_shift, j > 0 ? 1u : first);
               }
             } else {  // last, ragged stage: fewer scale tiles, fewer MMAs
               const int sf_tiles = sf_left > kST ? kST : sf_left;
@@ -1291,7 +1311,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
                 const int t = (FMT == TF_FMT_MXFP8) ? 0 : (FMT == TF_FMT_MXFP4) ? (j >> 1) : j;
                 const uint32_t sf_id = (FMT == TF_FMT_MXFP8) ? (uint32_t)j : (FMT == TF_FMT_MXFP4) ? (uint32_t)((j & 1) * 2) : 0u;
                 tc_mma_pair<FMT>(tmem_acc, make_desc(a_lo + j * 2, kDescHiSw128), make_desc(b_lo + j * 2, kDescHiSw128),
-                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4, j > 0 ? 1u : first);
+                                 idesc_base | (sf_id << 4) | (sf_id << 29), tmem_sfa + t * 4, tmem_sfb + t * kNB * 4 + sfb_shift, j > 0 ? 1u : first);
               }
             }
             tc_commit_pair(bar_empty + 8 * stage);  // frees the stage in both CTAs
@@ -1303,9 +1323,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
           }
         }
         if (!ok) break;
-        if (elected) tc_commit_pair(bar_tmem_full);  // both CTAs' epilogues may read their accumulator halves
+        if (elected) tc_commit_pair(bar_tmem_full + acc_bar);  // both CTAs' epilogues may read their accumulator halves
         __syncwarp();
-        tile_phase ^= 1;
+        if (PC::kAccBars == 1 || acc_buf) tile_phase ^= 1;
+        acc_buf ^= 1;
       }
     }
     __syncwarp();
@@ -1322,7 +1343,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
       zero_scale_padding(p.q_scales, p.m, p.n >> 5, (int64_t)blockIdx.x * 256 + (grp * 4 + q) * 32 + lane, (int64_t)gridDim.x * 256);
     for (int tile = pair; tile < p.num_tiles; tile += num_pairs) {
       const int m_blk = tile % p.m_blocks, n_blk = tile / p.m_blocks;
-      bool ok = mbar_wait(bar_tmem_full, tile_phase, abort_flag, 4);
+      const uint32_t acc_bar = PC::kAccBars == 1 ? 0u : 8 * acc_buf;
+      bool ok = mbar_wait(bar_tmem_full + acc_bar, tile_phase, abort_flag, 4);
       ok = __all_sync(0xFFFFFFFFu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -1330,17 +1352,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const int col0 = n_blk * kOutCols;
       const float alpha_t = (FMT == TF_FMT_NVFP4 && p.a_gs_rows > 0) ? __fmul_rn(load_f32(p.a_gs + min(row, p.m - 1) / p.a_gs_rows), load_f32(p.b_gs)) : alpha;
-      if (EPI == TF_EPI_RESIDUAL) {
-        epilogue_tile_residual<FMT>(p, t_row + acc_buf * Cfg::kAccStride, (int)acc_buf, grp, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+      const uint32_t t_acc = t_row + acc_buf * PC::kAccStride;
+      if (BLOCK_N == 192) {  // three pairs: a group takes one and two of them in turn
+        const int first = grp == 0 ? 0 : acc_buf == 0 ? 2 : 1, count = (int)acc_buf == grp ? 2 : 1;
+        epilogue_pairs<FMT, EPI>(p, t_acc, first * 2, 2, count, count - 1, release + acc_bar, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+      } else if (EPI == TF_EPI_RESIDUAL) {
+        epilogue_pairs<FMT, EPI>(p, t_acc, grp * 2 + (acc_buf == 0 ? 4 : 0), acc_buf == 0 ? -4 : 4, 2, 0, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
       } else if (acc_buf == 0) {
-        if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 0, 0, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
-        else epilogue_tile<FMT, BLOCK_N, EPI, 0, 1, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+        if (grp == 0) epilogue_tile<FMT, 256, EPI, 0, 0, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+        else epilogue_tile<FMT, 256, EPI, 0, 1, true>(p, t_row, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
       } else {
-        if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 1, 0, true>(p, t_row + Cfg::kAccStride, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
-        else epilogue_tile<FMT, BLOCK_N, EPI, 1, 1, true>(p, t_row + Cfg::kAccStride, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+        if (grp == 0) epilogue_tile<FMT, 256, EPI, 1, 0, true>(p, t_acc, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
+        else epilogue_tile<FMT, 256, EPI, 1, 1, true>(p, t_acc, release, lane, row, col0, alpha_t, amax2, &tma_out, stage_smem);
       }
+      if (PC::kAccBars == 1 || acc_buf) tile_phase ^= 1;
       acc_buf ^= 1;
-      tile_phase ^= 1;
     }
     if (lane == 0) bulk_wait_all();  // the stores have read their boxes and are written
     __syncwarp();
@@ -1357,7 +1383,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
   cluster_sync_all();
   if (warp == 1) {
     __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)Cfg::kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
   }
 }
 
@@ -1512,9 +1538,9 @@ static tf_status make_output_map(CUtensorMap* map, const GemmParams& p) {
   return TF_OK;
 }
 
-template <int FMT, int EPI>
+template <int FMT, int EPI, int BLOCK_N>
 static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
-  using PC = PairCfg<FMT>;
+  using PC = PairCfg<FMT, BLOCK_N>;
   CUtensorMap tsa, tsb, to = {};
   if (p.out) {
     const tf_status so = make_output_map(&to, p);
@@ -1524,7 +1550,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   if (st != TF_OK) return st;
   st = make_scale_map(&tsb, p.sfb, (int64_t)p.sfb_row_tiles * p.sf_col_tiles, PC::kST);
   if (st != TF_OK) return st;
-  auto kernel = gemm_blockscaled_pair_kernel<FMT, EPI>;
+  auto kernel = gemm_blockscaled_pair_kernel<FMT, EPI, BLOCK_N>;
   static thread_local int configured_dev = -1;
   int dev = 0;
   TF_CUDA(cudaGetDevice(&dev));
@@ -1532,7 +1558,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
     TF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PC::kSmemBytes));
     configured_dev = dev;
   }
-  constexpr int out_cols = (EPI == TF_EPI_SILU_GATE) ? 128 : 256;
+  constexpr int out_cols = (EPI == TF_EPI_SILU_GATE) ? 128 : BLOCK_N;
   p.m_blocks = (p.m + 255) / 256;
   p.n_blocks = (p.n + out_cols - 1) / out_cols;
   p.num_tiles = p.m_blocks * p.n_blocks;
@@ -1582,6 +1608,17 @@ static bool use_pair_kernel(int64_t m, int64_t n, int epilogue, const LaunchPlan
   const int64_t sms = sm_count(), pairs = sms / 2, n_blocks = gate ? (n + 127) / 128 : (n + 255) / 256;
   const int64_t waves = ((m + kBlockM - 1) / kBlockM * n_blocks + sms - 1) / sms, pair_waves = ((m + 255) / 256 * n_blocks + pairs - 1) / pairs;
   return 10 * pair_waves <= 11 * waves;
+}
+
+// The tile width of a pair. 192 columns take 0.79 of the time of 256 per K stage, not 0.75 (shared memory: 256 rows of operands are read for fewer
+// columns), and lose 5 to 9 % over many waves (mxfp8 8192 x 6144 x 2560 96 -> 101 us), but fill a wave that 256 leave part empty: one wave either way
+// mxfp8 512 x 6144 x 2560 13.4 -> 12.3, mxfp4 1000 x 3000 x 2720 residual 15.3 -> 14.3; six waves or seven nvfp4 4096 x 6144 x 2560 33.8 -> 33.8. Microseconds
+// fitted to those; the gate pairs 128 + 128 columns.
+static int pair_width(int64_t m, int64_t n, int64_t stages, int epilogue) {
+  if (epilogue == TF_EPI_SILU_GATE) return 256;
+  const int64_t pairs = gemm_sms() / 2, m_blocks = (m + 255) / 256;
+  auto waves = [&](int64_t bn) { return (double)((m_blocks * ((n + bn - 1) / bn) + pairs - 1) / pairs); };
+  return waves(192) * (0.33 * (double)stages + 0.95) < 0.97 * waves(256) * (0.414 * (double)stages + 0.85) ? 192 : 256;
 }
 
 // How many clusters of `splits` GEMM CTAs (one CTA fills an SM) the current device runs at once: a cluster lives inside one GPC, so
@@ -1659,7 +1696,7 @@ static LaunchPlan launch_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogu
 }
 
 template <int FMT>
-static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int epilogue, const LaunchPlan& lp, cudaStream_t stream,
+static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int epilogue, const LaunchPlan& lp, int pair_n, cudaStream_t stream,
                                bool partials_only = false) {
   if (lp.form == kSplitCluster) {
     if (epilogue == TF_EPI_SILU_GATE) return launch_gemm<FMT, 256, TF_EPI_SILU_GATE, kSplitCluster>(ta, tb, p, stream);
@@ -1704,10 +1741,12 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     TF_LAUNCH_CHECK();
     return TF_OK;
   }
-  if (!p.scatter_rows && use_pair_kernel(p.m, p.n, epilogue, lp)) {
-    if (epilogue == TF_EPI_SILU_GATE) return launch_gemm_pair<FMT, TF_EPI_SILU_GATE>(ta, tb, p, stream);
-    if (epilogue == TF_EPI_RESIDUAL) return launch_gemm_pair<FMT, TF_EPI_RESIDUAL>(ta, tb, p, stream);
-    return launch_gemm_pair<FMT, TF_EPI_NONE>(ta, tb, p, stream);
+  if (pair_n == 192)
+    return epilogue == TF_EPI_RESIDUAL ? launch_gemm_pair<FMT, TF_EPI_RESIDUAL, 192>(ta, tb, p, stream) : launch_gemm_pair<FMT, TF_EPI_NONE, 192>(ta, tb, p, stream);
+  if (pair_n == 256) {
+    if (epilogue == TF_EPI_SILU_GATE) return launch_gemm_pair<FMT, TF_EPI_SILU_GATE, 256>(ta, tb, p, stream);
+    if (epilogue == TF_EPI_RESIDUAL) return launch_gemm_pair<FMT, TF_EPI_RESIDUAL, 256>(ta, tb, p, stream);
+    return launch_gemm_pair<FMT, TF_EPI_NONE, 256>(ta, tb, p, stream);
   }
   if (epilogue == TF_EPI_SILU_GATE) return launch_gemm<FMT, 256, TF_EPI_SILU_GATE, kSplitNone>(ta, tb, p, stream);
   if (epilogue == TF_EPI_RESIDUAL)
@@ -1811,7 +1850,7 @@ tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, i
   const int64_t n_acc = epilogue == TF_EPI_SILU_GATE ? 2 * n : n;
   const int64_t tiles = (m + kBlockM - 1) / kBlockM * ((n_acc + lp.block_n - 1) / lp.block_n) * lp.splits;
   form[0] = use_pair_kernel(m, n, epilogue, lp) ? kFormPair : lp.form;
-  form[1] = lp.block_n;
+  form[1] = form[0] == kFormPair ? pair_width(m, n, (k_bytes + kStageKBytes - 1) / kStageKBytes, epilogue) : lp.block_n;
   form[2] = lp.splits;
   form[3] = dependent_launch(chain_gemm_launch(m, form[0] >= kSplitCluster || tiles <= gemm_sms()));
   return TF_OK;
@@ -1887,8 +1926,6 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
   const int a_box_rows = m >= kBlockM ? kBlockM : (int)((m + 15) / 16 * 16);
   tf_status st = make_operand_map(&ta, a_codes, m, k_bytes, a_box_rows);
   if (st != TF_OK) return st;
-  st = make_operand_map(&tb, b_codes, n_rows_b, k_bytes);
-  if (st != TF_OK) return st;
 
   GemmParams p;
   p.m = (int)m;
@@ -1930,6 +1967,9 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
     if (sp.splits <= 1) return fail(TF_ERR_UNSUPPORTED, "%s: this shape is not split along K (tf_gemm_splits == 1): there are no partial sums to leave", fn);
     *partial_splits = sp.splits;
   }
+  const int pair_n = !scatter_ptrs && !partial_splits && use_pair_kernel(m, n, epilogue, lp) ? pair_width(m, n, p.num_k_stages, epilogue) : 0;
+  st = make_operand_map(&tb, b_codes, n_rows_b, k_bytes, pair_n == 192 ? 96 : kBlockM);
+  if (st != TF_OK) return st;
   p.splits = lp.splits;
   p.k_stages_per_split = lp.k_stages_per_split;
   p.ws = static_cast<float*>(workspace);
@@ -1945,9 +1985,9 @@ static tf_status gemm_entry(const char* fn, const void* a_codes, const void* a_s
     if (st != TF_OK) return st;
   }
   switch (format) {
-    case TF_FMT_MXFP8: return dispatch_gemm<TF_FMT_MXFP8>(ta, tb, p, epilogue, lp, stream, partial_splits != nullptr);
-    case TF_FMT_MXFP4: return dispatch_gemm<TF_FMT_MXFP4>(ta, tb, p, epilogue, lp, stream, partial_splits != nullptr);
-    default: return dispatch_gemm<TF_FMT_NVFP4>(ta, tb, p, epilogue, lp, stream, partial_splits != nullptr);
+    case TF_FMT_MXFP8: return dispatch_gemm<TF_FMT_MXFP8>(ta, tb, p, epilogue, lp, pair_n, stream, partial_splits != nullptr);
+    case TF_FMT_MXFP4: return dispatch_gemm<TF_FMT_MXFP4>(ta, tb, p, epilogue, lp, pair_n, stream, partial_splits != nullptr);
+    default: return dispatch_gemm<TF_FMT_NVFP4>(ta, tb, p, epilogue, lp, pair_n, stream, partial_splits != nullptr);
   }
 }
 
