@@ -47,7 +47,7 @@ bool dependent_launch(bool chain);
 void set_programmatic_launch(int setting);  // 0 never, 1 always, -1 the rule
 
 #ifdef __CUDACC__
-// The rule: GEMMs of at most 256 rows (above 128 and with one CTA per tile: of one wave), row kernels of at most four rows, and the nvfp4 quantizer behind its
+// The rule: GEMMs of at most 256 rows (above 128 and with one CTA per tile: of one wave), gated GEMMs of CTA pairs in one wave up to 1024 rows, row kernels of at most four rows, and the nvfp4 quantizer behind its
 // own amax launch up to 16 M elements (launch_quantize). A GEMM's CTAs take a whole SM each, so starting early only hides their set-up: 200
 // GEMMs back to back on a full queue, plain -> dependent: mxfp8 1 x 2560 x 3072 8.2 -> 5.9 us, 128 x 6144 x 2560 11.6 -> 9.0, nvfp4
 // 64 x 8192 x 28672 36.7 -> 32.9; pairs in two waves mxfp4 256 x 16384 x 2048 + gate 20.5 -> 17.2, mxfp8 256 x 28672 x 2048 22.5 -> 20.6; one CTA per tile in
@@ -55,9 +55,15 @@ void set_programmatic_launch(int setting);  // 0 never, 1 always, -1 the rule
 // early they all pile onto the few SMs that the GEMM in front leaves free and then share those (70B-shaped decode at 64 rows: its
 // rmsnorm launch went from 9.8 to 14.7 us; two blocks at 16 rows 184.6 us without, 190.4 with). Above 256 rows the waiting CTAs
 // take the registers that the rest of the row kernel in front needs (README block at 8192 rows 189.5 -> 196.2 us).
+// The gated pairs stand behind a row kernel whose blocks all fit beside them: mxfp8 block 2560 x 3072 at 300 / 384 / 512 / 700 rows 32.8 / 32.7 / 33.2 / 36.7 -> 31.8 / 31.3 / 32.6 /
+// 34.8 us, nvfp4 2048 x 4096 at 512 32.6 -> 31.6; the second GEMM as a dependent too gives back half of it (32.7 / 32.5 / 33.9 / 35.4).
 // Captured graphs, before -> after: README block at one row 20.5 -> 18.4 us, 70B-shaped decode at 64 rows 402 -> 389, two
 // 4096 x 8192 blocks at 200 rows 93 -> 85.
-inline bool chain_gemm_launch(int64_t rows, bool one_wave) { return rows <= 128 || (rows <= 256 && one_wave); }
+enum class GemmKind { kOneCta, kPair, kGatedPair };
+inline bool chain_gemm_launch(int64_t rows, bool one_wave, GemmKind kind) {
+  if (rows <= 256) return rows <= 128 || one_wave || kind != GemmKind::kOneCta;
+  return rows <= 1024 && one_wave && kind == GemmKind::kGatedPair;
+}
 inline bool chain_rows_launch(int64_t rows) { return rows <= 4; }
 
 template <typename... KArgs, typename... Args>

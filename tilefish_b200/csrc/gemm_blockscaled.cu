@@ -1523,7 +1523,7 @@ static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmP
   p.n_blocks = (p.n + out_cols - 1) / out_cols;
   p.num_tiles = p.m_blocks * p.n_blocks * p.splits;
   const int grid = SPLITK == kSplitCluster || p.num_tiles < gemm_sms() ? p.num_tiles : gemm_sms();
-  const bool dependent = dependent_launch(chain_gemm_launch(p.m, p.num_tiles <= grid));
+  const bool dependent = dependent_launch(chain_gemm_launch(p.m, p.num_tiles <= grid, GemmKind::kOneCta));
   if (dependent && p.m <= kBlockM) p.early_stages = kEarlyStages;
   if (SPLITK == kSplitCluster) {
     cudaLaunchConfig_t cfg = {};
@@ -1614,7 +1614,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m, true)) ? 2 : 1;
+  cfg.numAttrs = dependent_launch(chain_gemm_launch(p.m, p.num_tiles <= pairs, EPI == TF_EPI_SILU_GATE ? GemmKind::kGatedPair : GemmKind::kPair)) ? 2 : 1;
   TF_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tsa, tsb, to, p));
   return TF_OK;
 }
@@ -1884,12 +1884,15 @@ tf_status tf_gemm_launch_form(int64_t m, int64_t n, int64_t k, int32_t format, i
                "%s: bad argument", __func__);
   const int64_t k_bytes = format == TF_FMT_MXFP8 ? k : k / 2;
   const LaunchPlan lp = launch_plan(m, n, k_bytes, epilogue, split_plan(m, n, k_bytes, epilogue));
-  const int64_t n_acc = epilogue == TF_EPI_SILU_GATE ? 2 * n : n;
-  const int64_t tiles = (m + kBlockM - 1) / kBlockM * ((n_acc + lp.block_n - 1) / lp.block_n) * lp.splits;
+  const bool gate = epilogue == TF_EPI_SILU_GATE;
+  const int64_t n_acc = gate ? 2 * n : n;
   form[0] = use_pair_kernel(m, n, epilogue, lp) ? kFormPair : lp.form;
   form[1] = form[0] == kFormPair ? pair_width(m, n, (k_bytes + kStageKBytes - 1) / kStageKBytes, epilogue) : lp.block_n;
   form[2] = lp.splits;
-  form[3] = dependent_launch(chain_gemm_launch(m, form[0] >= kSplitCluster || tiles <= gemm_sms()));
+  const bool pair = form[0] == kFormPair;
+  const int64_t tiles = (m + (pair ? 255 : 127)) / (pair ? 256 : 128) * ((n_acc + form[1] - 1) / form[1]) * lp.splits;
+  form[3] = dependent_launch(chain_gemm_launch(m, form[0] == kSplitCluster || tiles <= gemm_sms() / (pair ? 2 : 1),
+                                               !pair ? GemmKind::kOneCta : gate ? GemmKind::kGatedPair : GemmKind::kPair));
   return TF_OK;
 }
 
