@@ -52,3 +52,18 @@ def test_the_scale_from_the_amax_launch(K, m, k):
         gs = (x.abs().max().float().cpu() / torch.tensor(2688.0)).reshape(1).cuda()  # divided on the host: one correctly rounded division
         ref = K.quantize(x, "nvfp4", global_scale=gs)
         assert torch.equal(q.global_scale, gs) and torch.equal(q.codes, ref.codes) and torch.equal(q.scales, ref.scales)
+
+
+@pytest.mark.parametrize("gs", [0.0, -0.01, 0.003, 1e-30, 1e-38, 1e30, 3e37])
+def test_nvfp4_block_scales_at_the_ends_of_their_range(K, gs):
+    """Blocks of zeros, signed zeros, subnormal, huge and mixed values under global scales that underflow, saturate or are negative: the reciprocals come
+    from a table over the scale bytes, and a product of zero is a block of zero codes whatever its signs."""
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn((160, 288), generator=g).bfloat16()
+    for i, v in enumerate((0.0, -0.0, 9.2e-41, -1e-38, 3.3e38, -3.3e38, 1e-20, 448.0 * 6)):
+        x[i::16, :144] = v
+    x[8::16] *= 1e30
+    x[9::16] *= 1e-30
+    codes, scales, _ = O.quantize(x, "nvfp4", torch.tensor([gs]))
+    q = K.quantize(x.cuda(), "nvfp4", global_scale=torch.tensor([gs]).cuda())
+    assert torch.equal(q.scales.cpu(), O.swizzle_scales(scales)) and torch.equal(q.codes.cpu(), codes)

@@ -69,11 +69,24 @@ __device__ __forceinline__ void quantize_vec8(const uint4& v, float gs, float in
   }
 }
 
+// nvfp4: the reciprocal of a block scale, 1 / (f32(s8) * gs), or kZeroBlock where that product is zero (no reciprocal has these bits: a NaN result is canonical).
+constexpr uint32_t kZeroBlock = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t nvfp4_inverse(uint32_t s8, float gs) {
+  const float d = __fmul_rn(e4m3_to_f32(s8), gs);
+  return d == 0.0f ? kZeroBlock : __float_as_uint(__frcp_rn(d));
+}
+// (a.lo * b, a.hi * b) of the two bf16 of `w`, as two f32.
+__device__ __forceinline__ void mul_bf16_pair(uint32_t w, float b, float& lo, float& hi) {
+  asm("{ .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %4};\n mul.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x; }"
+      : "=f"(lo), "=f"(hi)
+      : "f"(bf16lo_to_f32(w)), "f"(bf16hi_to_f32(w)), "f"(b));
+}
+
 // 16 consecutive bf16 values per thread (one 256-bit load): half the shuffles, scale arithmetic and address arithmetic per element
 // of the 8-value form. A block of 32 is two adjacent lanes; an nvfp4 block of 16 is the thread's own. Same arithmetic, same bytes.
-// codes: 4 words (e4m3) or 2 words (e2m1).
+// codes: 4 words (e4m3) or 2 words (e2m1). nvfp4: gs, inv_t = 1 / (6 * gs), and where there is one the table of nvfp4_inverse for gs.
 template <int FMT>
-__device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs, float inv_t, uint32_t (&codes)[4], uint32_t& scale) {
+__device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs, float inv_t, uint32_t (&codes)[4], uint32_t& scale, const uint32_t* inverses = nullptr) {
   const uint32_t k = 0x7FFF7FFFu;
   uint32_t t0 = __vimax3_u16x2(w[0] & k, w[1] & k, w[2] & k);
   uint32_t t1 = __vimax3_u16x2(w[3] & k, w[4] & k, w[5] & k);
@@ -86,19 +99,15 @@ __device__ __forceinline__ void quantize_vec16(const uint32_t (&w)[8], float gs,
     const float amax = __uint_as_float(m << 16);
     uint32_t s8 = 0;
     if (gs != 0.0f && m != 0) s8 = cvt_e4m3x2(__fmul_rn(amax, inv_t), 0.0f) & 0xFFu;
-    const float d = __fmul_rn(e4m3_to_f32(s8), gs);
-    const bool zero = (d == 0.0f);
-    const float inv = zero ? 0.0f : __frcp_rn(d);
+    const uint32_t bits = inverses ? inverses[s8 & 127u] : nvfp4_inverse(s8, gs);
+    const float inv = __uint_as_float(bits);
     scale = s8;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       float f[8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f[2 * j] = __fmul_rn(bf16lo_to_f32(w[4 * h + j]), inv);
-        f[2 * j + 1] = __fmul_rn(bf16hi_to_f32(w[4 * h + j]), inv);
-      }
-      codes[h] = zero ? 0u : cvt_e2m1x8(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
+      for (int j = 0; j < 4; ++j) mul_bf16_pair(w[4 * h + j], inv, f[2 * j], f[2 * j + 1]);
+      codes[h] = bits == kZeroBlock ? 0u : cvt_e2m1x8(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
     }
     codes[2] = codes[3] = 0;
     return;

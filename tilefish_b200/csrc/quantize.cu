@@ -69,6 +69,9 @@ __device__ __forceinline__ float partials_max(const float* __restrict__ partials
 // with its amax launch 195 -> 187); 4096 x 28672 59.2 -> 53.5, 48.4 -> 44.1, 50.9 -> 46.6; 8192 x 4096 18.5 -> 17.3, 16.4 -> 15.2, 17.5 -> 16.2; 1000 x 2720
 // 3.7 -> 2.9, 3.8 -> 2.9, 4.0 -> 3.2; 64 x 28672 3.4 -> 2.7, 3.4 -> 2.6, 3.8 -> 2.9; 1 x 4096 2.6 -> 1.7, 2.6 -> 1.6, 3.1 -> 1.9. The same steps with a
 // persistent grid took 137 us for the first (four rounds 121), 8-warp blocks 118 / 96 / 102.7.
+// nvfp4 is bound by its instructions where x is in L2 (8192 x 4096: 169 per 16 elements, 65 % of the issue slots): each block keeps the reciprocals of all
+// block scales in a table, multiplies pairs, and loads without branches. Without -> with: 65536 x 4096 103.5 -> 100.5 us, with the amax launch 188.9 -> 185.7; 8192 x 4096
+// 16.3 -> 15.8, 31.0 -> 29.6; 4096 x 28672 47.7 -> 46.0; 4096 x 4096 in L2 7.8 -> 7.2.
 constexpr int kTileWarps = 4;  // of a block
 
 // Lane i of four (lanes `step` and 2 * step apart) holds bytes a_i[0..3]; returns a_0[i] | a_1[i] << 8 | a_2[i] << 16 | a_3[i] << 24.
@@ -90,6 +93,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
   constexpr int kCodeBytes = FMT == TF_FMT_MXFP8 ? 16 : 8;  // per vector
   const int nvec = k >> 4, cols = kNv ? nvec : nvec >> 1, n_ct = (cols + 3) >> 2;
   const int lane = threadIdx.x & 31, h = lane >> 4, q = lane & 15;
+  __shared__ uint32_t inverses[kNv ? 128 : 1];
   griddep_launch_dependents();
   float gs = 0.0f, inv_t = 0.0f;
   if (!kNv || n_partials == 0) {
@@ -111,12 +115,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       has[j] = live && row + 32 * j < m && vec < nvec;
-      if (has[j]) {
-        load_256(xp + 64 * j * ldx, v[j]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[j][e] = 0;
-      }
+      load_256(has[j] ? xp + 64 * j * ldx : x, v[j]);  // a load without data is read from the tensor's start and not used
     }
     if (kNv && first) {
       if (n_partials > 0) {
@@ -128,6 +127,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
         if (blockIdx.x == 0 && threadIdx.x == 0) gs_out[0] = gs;
       }
       inv_t = gs != 0.0f ? __frcp_rn(__fmul_rn(6.0f, gs)) : 0.0f;
+      // a block's scale byte has the sign of gs, its other seven bits are the index
+      for (int i = threadIdx.x; i < 128; i += blockDim.x) inverses[i] = nvfp4_inverse(gs < 0.0f ? i | 0x80 : i, gs);
+      __syncthreads();
       first = false;
       if (!live) break;
     }
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       uint32_t cw[4], sc;
-      quantize_vec16<FMT>(v[j], gs, inv_t, cw, sc);
+      quantize_vec16<FMT>(v[j], gs, inv_t, cw, sc, inverses);
       if (has[j]) {
         word |= sc << (8 * j);
         uint8_t* dst = cp + (int64_t)(32 * j) * nvec * kCodeBytes;
