@@ -78,10 +78,11 @@ TF_API tf_status tf_device_status(int32_t* status, int32_t* detail);
 TF_API tf_status tf_set_sm_margin(int32_t sms);
 
 /* Programmatic dependent launch (PROCESS-WIDE, as tf_set_sm_margin): 1 for all quantize, rmsnorm, GEMM and split-K reduction kernels, 0 for
- * none, -1 (what is in force until the first call) for short ones, as long as the SM margin is 0: GEMMs of at most 256 rows (with one CTA per
- * tile only if all tiles run at once), row kernels of at most 4 rows, the quantizer of tf_quantize_nvfp4_dynamic up to 2^24 elements. Such a kernel may be
- * scheduled while the kernel before it on the stream is still draining; each waits (griddepcontrol.wait) for that kernel to complete before its first access to global memory, so results
- * are unchanged. It hides launch latency and kernel set-up in chains of short kernels (small M, decode, many GPUs). No
+ * none, -1 (what is in force until the first call) for short ones, as long as the SM margin is 0: GEMMs of at most 128 rows, of at most 256 rows as CTA
+ * pairs or with all tiles at once, gated CTA pairs of one wave up to 1024 rows, row kernels of at most 4 rows, the quantizer of tf_quantize_nvfp4_dynamic
+ * up to 2^24 elements. Such a kernel may be scheduled while the kernel before it on the stream is still draining; each waits (griddepcontrol.wait) for that
+ * kernel to complete before it reads or writes anything that kernel may write or read, so results are unchanged (a GEMM asks weights into L2
+ * before that, and the quantizer loads the tensor that its own amax launch in front reads). It hides launch latency and kernel set-up in chains of short kernels (small M, decode, many GPUs). No
  * counterpart in the reference. */
 TF_API tf_status tf_set_programmatic_launch(int32_t enabled);
 

@@ -12,9 +12,10 @@
 namespace tf {
 
 // VPT: 8-element vectors per thread; QFMT: -1 none, else TF_FMT_*; WORDS: the scales leave as words (scales_as_words).
-// Registers for four blocks of 512 threads per SM (three with two vectors per thread: 16384 x 8192 247 us with two blocks, 234.8 = 6.86 TB/s with three).
+// Registers for four, three and two blocks of 512 threads per SM with one, two and four vectors per thread: 16384 x 8192 247 us with two blocks, 234.8 (6.86 TB/s) with
+// three; with an mxfp8 copy 4096 x 16384 191 us with one block, 144 with two.
 template <int VPT, int QFMT, bool WORDS>
-__global__ void __launch_bounds__(512, VPT == 1 ? 4 : VPT == 2 ? 3 : 0) residual_add_rmsnorm_kernel(const uint4* __restrict__ x, float4* __restrict__ residual,
+__global__ void __launch_bounds__(512, VPT == 1 ? 4 : VPT == 2 ? 3 : VPT == 4 ? 2 : 1) residual_add_rmsnorm_kernel(const uint4* __restrict__ x, float4* __restrict__ residual,
                                                                    const uint4* __restrict__ w, uint4* __restrict__ out, int64_t m, int d,
                                                                    float eps, float inv_d, uint8_t* __restrict__ q_codes,
                                                                    uint8_t* __restrict__ q_scales, int q_layout, int q_pad,
