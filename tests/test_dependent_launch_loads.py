@@ -32,3 +32,10 @@ def test_the_aligned_cluster_barrier_is_reached_by_whole_warps():
     text = code("gemm_blockscaled.cu")
     assert len(re.findall(r"barrier\.cluster\.(?:arrive|wait)", text)) == 2  # both in one place
     assert re.search(r"void cluster_sync_all\(\) \{\s*__syncwarp\(\);\s*asm volatile\(\"barrier\.cluster\.arrive", text)
+
+
+def test_a_flag_of_another_warp_is_read_by_vote():
+    """Lanes that branch on what each of them reads of a word another warp is storing may leave a loop of warp operations at different turns."""
+    reads = re.findall(r"^.*\*started_flag\b(?! = ).*$", code("gemm_blockscaled.cu"), re.M)
+    reads = [r.strip() for r in reads if "volatile" not in r]
+    assert reads == ["if (__any_sync(0xFFFFFFFFu, *started_flag)) left = 0;"]

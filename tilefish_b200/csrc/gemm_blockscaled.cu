@@ -1087,13 +1087,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
         const int n_blk = (SPLITK == kSplitPlanes ? tile % (p.m_blocks * p.n_blocks) : kCluster ? tile / p.splits : tile) / p.m_blocks;
         const int ks_end = min((split + 1) * p.k_stages_per_split, p.num_k_stages);
         for (int ks = split * p.k_stages_per_split; ks < ks_end && left > 0; ++ks, --left) {
-          if (*started_flag) left = 0;
+          if (__any_sync(0xFFFFFFFFu, *started_flag)) left = 0;  // one answer for the warp: warp 0 may be storing it just now
           if (left > 0 && lane == 0) prefetch_b_stage<FMT, BLOCK_N, EPI>(p, &tma_b, n_blk, ks);
           __syncwarp();
           if (left > 0) __nanosleep(kEarlyStageNs);
         }
       }
     }
+    __syncwarp();
     griddep_wait();
     const int q = warp & 3;
     const int grp = warp >= 7 ? 1 : 0;
