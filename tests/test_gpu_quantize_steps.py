@@ -21,7 +21,10 @@ def K():
 
 @pytest.mark.parametrize("fmt", FMTS)
 @pytest.mark.parametrize("layout", ["swizzled", "plain"])
-@pytest.mark.parametrize("m,k,offset", [(1, 32, 0), (2, 64, 1), (31, 288, 2), (33, 96, 4), (64, 256, 3), (97, 4128, 16), (127, 544, 0), (129, 224, 1), (257, 800, 4), (385, 2080, 0)])
+@pytest.mark.parametrize("m,k,offset", [(1, 32, 0), (2, 64, 1), (31, 288, 2), (33, 96, 4), (64, 256, 3), (97, 4128, 16), (127, 544, 0), (129, 224, 1), (257, 800, 4), (385, 2080, 0),
+                                        # rows of fewer than 256 columns: two and four lanes, one to four steps
+                                        (300, 32, 4), (65, 32, 3), (1025, 64, 0), (17, 64, 2), (300, 96, 0), (129, 128, 4), (40, 128, 1), (300, 160, 0), (33, 160, 2), (127, 192, 4), (1, 224, 0),
+                                        (5000, 224, 0)])
 def test_against_the_oracle(K, fmt, layout, m, k, offset):
     wide = O.randn((m, k + 48), m + k, torch.bfloat16)
     wide[:, ::37] *= 100.0
@@ -67,3 +70,26 @@ def test_nvfp4_block_scales_at_the_ends_of_their_range(K, gs):
     codes, scales, _ = O.quantize(x, "nvfp4", torch.tensor([gs]))
     q = K.quantize(x.cuda(), "nvfp4", global_scale=torch.tensor([gs]).cuda())
     assert torch.equal(q.scales.cpu(), O.swizzle_scales(scales)) and torch.equal(q.codes.cpu(), codes)
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+def test_narrow_rows_take_no_longer_than_wide_ones(K, fmt):
+    """The same number of elements in rows of 32 to 192 columns and of 256: a step is bound by its instructions, so lanes without data
+    show (the ratio was 1.4 at 192 columns, 6 at 32)."""
+    def time(k):
+        x = torch.zeros((196608 * 256 // k, k), dtype=torch.bfloat16, device="cuda")
+        gs = torch.ones(1, device="cuda") if fmt == "nvfp4" else None
+        q = K.quantize(x, fmt, global_scale=gs)
+        times = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                K.quantize(x, fmt, global_scale=gs, out=q)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[2:])
+
+    wide = time(256)
+    assert max(time(32), time(64), time(96), time(128)) <= 2.0 * wide and time(192) <= 1.5 * wide

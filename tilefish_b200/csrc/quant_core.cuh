@@ -166,19 +166,23 @@ __device__ __forceinline__ void zero_scale_padding(uint8_t* __restrict__ scales,
   }
 }
 
-// Four scales of row `row`, columns col .. col + 3 (col a multiple of 4), as the bytes of `word`. WORDS: swizzled scales that can be stored as words; else
-// byte by byte in either layout (a template: the short row kernels run from a cold instruction cache, and the branches over the byte
-// stores cost the README block at 1 and 512 rows 0.3 and 0.6 us). real: the row is one of the tensor's (the swizzled layout has more).
+// Scales of row `row` as the bytes of `word`: columns col .. col + 3 (col a multiple of 4), or with `pair` col and col + 1 (col even). WORDS: swizzled
+// scales that can be stored as words; else byte by byte in either layout (a template: the short row kernels run from a cold instruction
+// cache, and the branches over the byte stores cost the README block at 1 and 512 rows 0.3 and 0.6 us). real: the row is one of the tensor's
+// (the swizzled layout has more).
 template <bool WORDS>
-__device__ __forceinline__ void store_scale_word(uint8_t* __restrict__ scales, int layout, int64_t row, int col, int cols, int n_ct, bool real, uint32_t word) {
+__device__ __forceinline__ void store_scale_word(uint8_t* __restrict__ scales, int layout, int64_t row, int col, int cols, int n_ct, bool real, uint32_t word,
+                                                 bool pair = false) {
   if (WORDS) {
-    *reinterpret_cast<uint32_t*>(scales + swizzled_scale_offset(row, col, n_ct)) = word;
+    uint8_t* dst = scales + swizzled_scale_offset(row, col, n_ct);
+    if (pair) *reinterpret_cast<uint16_t*>(dst) = (uint16_t)word;
+    else *reinterpret_cast<uint32_t*>(dst) = word;
     return;
   }
   uint8_t* dst = scales + (layout == TF_SCALES_PLAIN ? row * cols + col : swizzled_scale_offset(row, col, n_ct));
 #pragma unroll
   for (int b = 0; b < 4; ++b)
-    if (layout == TF_SCALES_SWIZZLED || (real && col + b < cols)) dst[b] = (uint8_t)(word >> (8 * b));
+    if ((b < 2 || !pair) && (layout == TF_SCALES_SWIZZLED || (real && col + b < cols))) dst[b] = (uint8_t)(word >> (8 * b));
 }
 inline bool scales_as_words(const void* scales, int layout) { return layout == TF_SCALES_SWIZZLED && reinterpret_cast<uintptr_t>(scales) % 4 == 0; }
 

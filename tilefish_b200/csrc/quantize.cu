@@ -63,7 +63,7 @@ __device__ __forceinline__ float partials_max(const float* __restrict__ partials
 // each (as many as the codes take, for nvfp4). Here a warp takes these eight rows together: in one step 16 vectors (256 elements) of each, half
 // a warp per row, four 256-bit loads in flight per thread. The scale bytes of a thread's four loads are one word; a 4 x 4 byte transpose
 // over the lanes that share a scale word (two shuffles) leaves each word in a lane of its own, and one store writes whole sectors,
-// the padding's zeros included.
+// the padding's zeros included. Rows of fewer than 256 columns get four lanes or two, and a warp more of them (quantize_lanes).
 // One step per warp, so that the hardware deals the steps out: blocks that stay and walk keep every SM's loads and stores in phase. Graphs of 12,
 // rows per block with a persistent grid -> this: 65536 x 4096 mxfp8 133.5 -> 118.2 us (6.9 TB/s), mxfp4 102.8 -> 95.9 (7.1), nvfp4 105.9 -> 101.4 (6.8;
 // with its amax launch 195 -> 187); 4096 x 28672 59.2 -> 53.5, 48.4 -> 44.1, 50.9 -> 46.6; 8192 x 4096 18.5 -> 17.3, 16.4 -> 15.2, 17.5 -> 16.2; 1000 x 2720
@@ -82,17 +82,18 @@ __device__ __forceinline__ uint32_t transpose_bytes(uint32_t a, int step, int i)
   return __byte_perm(a, o, (i & 2) ? 0x3276 : 0x5410);
 }
 
-// A step is 16 vectors of eight rows; steps_per_unit = ceil(nvec / 16) steps along a row, `total` steps in all.
+// A step is LANES vectors of 128 / LANES rows (16 of eight); steps_per_unit = ceil(nvec / LANES) steps along a row, `total` steps in all.
 // n_partials > 0: the kernel in front is this tensor's own amax launch. That one starts only when x is complete, so a warp's first step is
 // loaded while it still runs; and the last rows come first, which the amax launch read last and left in L2.
-template <int FMT, bool WORDS>
+template <int FMT, bool WORDS, int LANES>
 __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(const uint8_t* __restrict__ x, int64_t m, int k, int64_t ldx, uint8_t* __restrict__ codes,
                                                                           uint8_t* __restrict__ scales, int layout, int steps_per_unit, int total,
                                                                           const float* __restrict__ gs_ptr, float* __restrict__ gs_out, int n_partials) {
   constexpr bool kNv = FMT == TF_FMT_NVFP4;
   constexpr int kCodeBytes = FMT == TF_FMT_MXFP8 ? 16 : 8;  // per vector
   const int nvec = k >> 4, cols = kNv ? nvec : nvec >> 1, n_ct = (cols + 3) >> 2;
-  const int lane = threadIdx.x & 31, h = lane >> 4, q = lane & 15;
+  constexpr int kBlockLanes = kNv ? 1 : 2;                  // lanes that hold one block's elements
+  const int lane = threadIdx.x & 31, h = lane / LANES, q = lane % LANES;
   __shared__ uint32_t inverses[kNv ? 128 : 1];
   griddep_launch_dependents();
   float gs = 0.0f, inv_t = 0.0f;
@@ -106,9 +107,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
     if (!live && !first) break;
     const int s = !live ? 0 : n_partials > 0 ? total - 1 - s0 : s0;
     const int unit = s / steps_per_unit, c = s - unit * steps_per_unit;
-    const int rr = (unit & 15) * 2 + h;  // this half warp's place in a group of 32 rows
-    const int64_t row = (int64_t)(unit >> 4) * 128 + rr;
-    const int vec = c * 16 + q;
+    const int rr = unit % LANES * (32 / LANES) + h;  // these lanes' place in a group of 32 rows
+    const int64_t row = (int64_t)(unit / LANES) * 128 + rr;
+    const int vec = c * LANES + q;
     const uint8_t* xp = x + row * ldx * 2 + (int64_t)vec * 32;
     uint32_t v[4][8];
     bool has[4];  // j: row + 32 * j
@@ -146,11 +147,23 @@ __global__ void __launch_bounds__(kTileWarps * 32, 8) quantize_tiles_kernel(cons
         else *reinterpret_cast<uint2*>(dst) = make_uint2(cw[0], cw[1]);
       }
     }
-    // four scales of one row are four lanes (nvfp4) or four pairs of lanes; lane (pair) i of them gets the word of load i
-    const int i = (kNv ? q : q >> 1) & 3;
-    word = transpose_bytes(word, kNv ? 1 : 2, i);
-    const int ct = kNv ? c * 4 + (q >> 2) : c * 2 + (q >> 3);
-    if (ct < n_ct && (kNv || (q & 1) == 0)) store_scale_word<WORDS>(scales, layout, row + 32 * i, ct * 4, cols, n_ct, row + 32 * i < m, word);
+    if (LANES >= 4 * kBlockLanes) {
+      // four scales of one row are four lanes (nvfp4) or four pairs of lanes; lane (pair) i of them gets the word of load i
+      const int i = q / kBlockLanes & 3;
+      word = transpose_bytes(word, kBlockLanes, i);
+      const int ct = vec / (4 * kBlockLanes);
+      if (ct < n_ct && q % kBlockLanes == 0) store_scale_word<WORDS>(scales, layout, row + 32 * i, ct * 4, cols, n_ct, row + 32 * i < m, word);
+    } else {
+      // two scales of a row (one with mx and two lanes), in the lower and upper lanes; lane i gets the pair of load i (and of load i + 2 where there
+      // are two lanes). The last step's pair is a word with the zeros behind it, if it starts one.
+      const uint32_t other = LANES > kBlockLanes ? __shfl_xor_sync(0xFFFFFFFFu, word, LANES / 2) : 0u;
+      const bool upper = LANES > kBlockLanes && q >= LANES / 2;
+      const uint32_t lo = upper ? other : word, hi = upper ? word : other;
+      const bool pair = LANES == 4 && ((c & 1) || (c + 1) * LANES < nvec);
+#pragma unroll
+      for (int i = q; i < 4; i += LANES)
+        store_scale_word<WORDS>(scales, layout, row + 32 * i, c * 2, cols, n_ct, row + 32 * i < m, (lo >> (8 * i) & 255u) | (hi >> (8 * i) & 255u) << 8, pair);
+    }
   }
 }
 
@@ -405,6 +418,19 @@ static void rows_shape(int64_t m, int64_t k, int per_sm, dim3& grid, dim3& block
   }
 }
 
+// Lanes per row of the quantizer. A step is bound by its instructions and costs the same whatever its lanes hold: below 256 columns, rows of 16 lanes took
+// up to four times as long as a walk with two threads per row. 16 lanes -> 4 (2 at 32 columns; the walk), us, mxfp8 / mxfp4 / nvfp4: 1048576 x 32
+// 112.9 -> 17.6 (27.8) / 112.3 -> 15.3 (28.3) / 112.0 -> 15.4 (28.3); 524288 x 64 60.4 -> 17.7 (20.3) / 59.0 -> 15.3 (19.8) / 59.1 -> 15.6 (20.4);
+// 200001 x 96 25.9 -> 12.7 (12.8) / 25.0 -> 11.5 (12.0) / 25.2 -> 12.4 (13.2); 65536 x 192 11.6 -> 8.1 (9.6) / 10.8 -> 6.2 (8.0) / 11.1 -> 7.3 (8.7);
+// 65536 x 224 11.7 -> 9.8 (10.9) / 11.1 -> 8.0 (9.9) / 11.3 -> 8.9 (10.9). Eight lanes are no better at 128 columns and took 15.9 us for 200001 x 96 mxfp8. At 256
+// columns and above 16 lanes beat the walk everywhere (65536 x 288 13.2 (13.9) / 12.4 (13.6) / 13.8 (14.4)).
+static int quantize_lanes(int64_t nvec) { return nvec >= 16 ? 16 : nvec == 2 ? 2 : 4; }
+
+template <int FMT, bool WORDS>
+static auto tiles_kernel(int lanes) {
+  return lanes == 16 ? quantize_tiles_kernel<FMT, WORDS, 16> : lanes == 4 ? quantize_tiles_kernel<FMT, WORDS, 4> : quantize_tiles_kernel<FMT, WORDS, 2>;
+}
+
 template <int FMT>
 static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64_t k, int64_t ldx, void* codes, void* scales, int layout,
                                  const float* gs, cudaStream_t stream, float* gs_out = nullptr, int n_partials = 0) {
@@ -412,7 +438,8 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   if (st != TF_OK) return st;
   if (FMT == TF_FMT_NVFP4 && !gs) return fail(TF_ERR_INVALID_ARGUMENT, "%s: nvfp4 needs a global scale", fn);
   if (m == 0) return TF_OK;
-  const int64_t steps_per_unit = ((k >> 4) + 15) / 16, total = (m + 127) / 128 * 16 * steps_per_unit;
+  const int lanes = quantize_lanes(k >> 4);
+  const int64_t steps_per_unit = ((k >> 4) + lanes - 1) / lanes, total = (m + 127) / 128 * lanes * steps_per_unit;
   if (total > INT32_MAX) return fail(TF_ERR_UNSUPPORTED, "%s: m=%lld x k=%lld is too large", fn, (long long)m, (long long)k);
   int64_t warps = (total + sm_count() - 1) / sm_count();  // few steps: narrower blocks, so that every SM gets some
   if (warps > kTileWarps) warps = kTileWarps;
@@ -421,7 +448,7 @@ static tf_status launch_quantize(const char* fn, const void* x, int64_t m, int64
   // waiting costs the amax launch more (8192 x 4096 29.9 -> 33.0).
   const int64_t rounds = n_partials > 0 && total > 32 * (int64_t)sm_count() ? 2 : 1;
   const bool dependent = (n_partials > 0 && m * k <= (int64_t)1 << 24) || chain_rows_launch(m);
-  auto kernel = scales_as_words(scales, layout) ? quantize_tiles_kernel<FMT, true> : quantize_tiles_kernel<FMT, false>;
+  auto kernel = scales_as_words(scales, layout) ? tiles_kernel<FMT, true>(lanes) : tiles_kernel<FMT, false>(lanes);
   TF_CUDA(launch_dependent(dependent, kernel, dim3((unsigned)((total + warps * rounds - 1) / (warps * rounds))), dim3((unsigned)warps * 32), 0, stream,
                            static_cast<const uint8_t*>(x), m, (int)k, ldx, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales), layout,
                            (int)steps_per_unit, (int)total, gs, gs_out, n_partials));
