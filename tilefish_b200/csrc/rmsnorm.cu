@@ -4,7 +4,7 @@
 //   out = bf16(r * rstd * f32(w))   rstd = rsqrt(sum(r*r) * f32(1/D) + eps); the only rounding point is the bf16 cast
 //
 // HBM-bound: 12 bytes per element (2 read x, 4 read + 4 write residual, 2 write out), plus the quantized copy when asked
-// for. One or two rows per block, 128-bit loads, the row's r values stay in registers between the reduction and the
+// for. A block takes whole rows (rows_grid), 128-bit loads, the row's r values stay in registers between the reduction and the
 // normalisation, warp-shuffle + shared-memory block reduction.
 #include "async_copy.cuh"
 #include "quant_core.cuh"
@@ -282,6 +282,31 @@ static void launch_rows_vpt(int qfmt, dim3 grid, dim3 block, cudaStream_t s, con
 
 using namespace tf;
 
+// The grid of residual_add_rmsnorm_kernel: blocks that walk over the rows, or blocks of one to four rows that the hardware deals out: those keep
+// SMs out of step, where walking blocks keep every SM's loads and stores in phase, but each costs its start. Graphs of 12, walking -> dealt out: 8192 x
+// 2560 44.0 -> 39.0 us, with an mxfp8 copy 49.0 -> 44.6; 10000 x 4064 82.6 -> 73.0 (6.7 TB/s); 4096 x 8192 with an mxfp8 copy 85 -> 70; 65536 x 512
+// 72.0 -> 61.7, one row per block 68.7.
+// They walk where dealing out loses:
+//   rows of at most 320 columns. The GPU starts about one block per ns, and a block of two such rows has less to do: 1048576 x 64 285 -> 539 us, 65536 x
+//   256 33.6 -> 35.9, 20000 x 288 13.5 -> 14.2;
+//   few rounds of rows, where every SM's share is even anyway: 651 x 4096 6.1 -> 7.0, 976 x 2560 with the maximum 7.0 -> 8.2, 1509 x 2560 with
+//   an mxfp8 copy 9.5 -> 9.8. Three rounds of what is resident (2.5 with more than one vector per thread), eight where only a copy is written: 2000 x
+//   2560 10.7 -> 12.1, 4000 x 2560 19.9 -> 20.8;
+//   rows beyond 16384 columns (2048 x 32768 157.0 -> 158.8), and beyond 8192 with the maximum (4096 x 16384 126.8 -> 128.2).
+// With the maximum every block has one atomic on the same word, which takes one at about 2 ns: four short rows per block (65536 x 512 73.5 walking,
+// 80.7 with two rows, 64.9 with four; 65536 x 384 56.1, 62.3, 50.3).
+static unsigned rows_grid(int64_t m, int d, int vpt, int threads, bool out, bool amax) {
+  const auto blocks = [&](int threads_per_sm) { return (int64_t)sm_count() * (threads_per_sm / threads < 32 ? threads_per_sm / threads : 32); };
+  const int64_t resident = blocks(vpt == 1 ? 2048 : vpt == 2 ? 1536 : vpt == 4 ? 1024 : 512);  // the kernel's launch bounds
+  const int64_t half_rounds = vpt > 1 ? 5 : out ? 6 : 16;
+  if (d <= 320 || vpt == 8 || (vpt == 4 && amax) || 2 * m <= half_rounds * resident) {
+    const int64_t walkers = blocks(2048);
+    return (unsigned)(m < walkers ? m : walkers);
+  }
+  const int64_t rows = amax && threads < 128 && m > 8 * resident ? 4 : threads < 256 || (!out && vpt == 1) ? 2 : 1;
+  return (unsigned)((m + rows - 1) / rows);
+}
+
 extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, const void* w, void* out, int64_t m, int64_t d, float eps,
                                              int32_t q_format, void* q_codes, void* q_scales, int32_t q_layout, const float* q_global_scale,
                                              float* out_amax, void* stream_) {
@@ -316,13 +341,7 @@ extern "C" tf_status tf_residual_add_rmsnorm(const void* x, void* residual, cons
   vpt = vpt <= 1 ? 1 : vpt <= 2 ? 2 : vpt <= 4 ? 4 : 8;
   int threads = (nvec + vpt - 1) / vpt;
   threads = (threads + 31) / 32 * 32;
-  // A block per row once the rows exceed what is resident: the hardware deals the rows out, while blocks that stay and walk keep every SM's loads and
-  // stores in phase. Two rows where a block is short against its launch: less than 2 K columns, or only the quantized copy to write (up to
-  // 4 K). Persistent -> this, graphs of 12: 8192 x 2560 42.3 -> 39.2 us, with an mxfp8 copy 48.4 -> 45.1; 10000 x 4064 79.7 -> 73.0 (6.7 TB/s); 4096 x 8192
-  // with an mxfp8 copy 85 -> 71; two rows: 16000 x 512 18.1 -> 17.2 (one row 18.0), mxfp4 copy alone 10000 x 4064 71.6 -> 71.7 (75.3).
-  const int64_t resident = (int64_t)sm_count() * (2048 / threads);
-  const int64_t rows_per_block = m > resident && (threads < 256 || (!out && vpt == 1)) ? 2 : 1;
-  dim3 grid((unsigned)((m + rows_per_block - 1) / rows_per_block)), block(threads);
+  dim3 grid(rows_grid(m, (int)d, vpt, threads, out != nullptr, out_amax != nullptr)), block(threads);
   if (pad && grid.x < kPadBlocks) grid.x = kPadBlocks;  // one to seven rows: blocks without a row share the padding (0.6 us at one row)
   const float inv_d = 1.0f / (float)d;  // correctly rounded f32 reciprocal of D (IEEE division on the host)
   const uint4* xp = static_cast<const uint4*>(x);
