@@ -75,6 +75,25 @@ def test_pairs_that_take_more_than_one_tile(K, fmt, m, n, k):
 
 
 @pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
+@pytest.mark.parametrize("m,n,k,tiles", [(16, 38400, 544, 300), (100, 38392, 1056, 300), (40000, 128, 288, 313), (39937, 120, 544, 313)])
+def test_residual_tiles_of_128_columns_more_than_one_per_cta(K, fmt, m, n, k, tiles):
+    """300 and 313 tiles on 148 CTAs: the staging boxes are filled again while the next tile's sums are formed, in one ring stage fewer."""
+    form = K.gemm_launch_form(m, n, k, fmt, "residual")
+    assert form[:3] == ("tiles", 128, 1) and -(-m // 128) * -(-n // 128) == tiles
+    a, w = O.randn((m, k), m, torch.bfloat16), O.randn((n, k), n, torch.bfloat16, scale=k**-0.5)
+    qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)
+    oa, ob = O.quantize(a, fmt), O.quantize(w, fmt)
+    ref = O.dequantize(oa[0], oa[1], fmt, oa[2]) @ O.dequantize(ob[0], ob[1], fmt, ob[2]).t()
+    res, amax = O.randn((m, n), 7), torch.zeros(1, device="cuda")
+    r = res.cuda()
+    wide = torch.full((m, n + 16), -7.0, dtype=torch.bfloat16, device="cuda")
+    out = K.gemm_blockscaled(qa, qb, epilogue="residual", residual=r, out=wide[:, :n], amax_out=amax)
+    assert float((out.cpu().float() - ref).abs().max()) <= TOL * float(ref.abs().max())
+    assert bool((wide[:, n:] == -7.0).all()) and float(amax) == float(out.float().abs().max())
+    assert torch.equal(r.cpu(), res + out.cpu().float())
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
 def test_gated_pairs_that_take_more_than_one_tile(K, fmt):
     m, f, k = 2600, 1920, 544
     assert K.gemm_launch_form(m, f, k, fmt, "silu_gate")[0] == "pair"
