@@ -94,8 +94,9 @@ def test_residual_tiles_of_128_columns_more_than_one_per_cta(K, fmt, m, n, k, ti
 
 
 @pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
-def test_gated_pairs_that_take_more_than_one_tile(K, fmt):
-    m, f, k = 2600, 1920, 544
+@pytest.mark.parametrize("k_bytes", [544, 1920, 2048, 2080])  # 5, 15, 16 and 17 stages: from 16 on the load warps take them in turn
+def test_gated_pairs_that_take_more_than_one_tile(K, fmt, k_bytes):
+    m, f, k = 2600, 1920, k_bytes if fmt == "mxfp8" else 2 * k_bytes
     assert K.gemm_launch_form(m, f, k, fmt, "silu_gate")[0] == "pair"
     a, w = O.randn((m, k), m, torch.bfloat16), O.randn((2 * f, k), f, torch.bfloat16, scale=k**-0.5)
     qa, qb = K.quantize(a.cuda(), fmt), K.quantize(w.cuda(), fmt)

@@ -1197,7 +1197,8 @@ struct PairCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + kOutStageBytes + kBarrierBytes + 1024;
 };
 
-template <int FMT, int EPI, int BLOCK_N>
+// TURNS: each load warp loads all of every second stage, instead of warp 0 the operands and warp 6 the scales of every stage (see pair_turns).
+template <int FMT, int EPI, int BLOCK_N, bool TURNS>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                                  const __grid_constant__ CUtensorMap tma_b,
                                                                                  const __grid_constant__ CUtensorMap tma_sfa,
@@ -1209,11 +1210,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
   constexpr int kST = PC::kST;
   constexpr int kNB = 2;
   constexpr int kOutCols = (EPI == TF_EPI_SILU_GATE) ? BLOCK_N / 2 : BLOCK_N;
-  // The load warps take the stages in turn where the epilogue's arithmetic competes with them for issue slots: two stages' time for five copies
-  // instead of one for two or three (mxfp8 8192 x 3072 x 2560 + gate 98.0 -> 95.5 us, hot 116.4 -> 112.8; nvfp4 4096 x 28672 x 8192 + gate 672.9 -> 665.4). Without
-  // the gate a tile's first stage comes later for it (mxfp4 300 x 8192 x 4096 12.3 -> 12.55, mxfp8 1024 x 4096 x 4096 residual 22.0 -> 22.65).
-  constexpr bool kTurns = EPI == TF_EPI_SILU_GATE;
-
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t smem_a = smem_base;
@@ -1237,7 +1233,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(bar_full + 8 * s, kTurns ? 2 : 4);  // an arrive.expect_tx of each load warp that serves the stage, from both CTAs (used in the leader only)
+      mbar_init(bar_full + 8 * s, TURNS ? 2 : 4);  // an arrive.expect_tx of each load warp that serves the stage, from both CTAs (used in the leader only)
       mbar_init(bar_empty + 8 * s, 1);  // the leader's commit arrives in both CTAs
     }
     for (int i = 0; i < PC::kAccBars; ++i) {
@@ -1260,11 +1256,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
 
   if (warp == 0 || warp == 6) {
     // ---------------- load warps (each CTA loads its own halves; completion is counted on the leader's barrier) ----------------
-    // Lane 0 loads the A rows, lane 1 the B rows of this CTA, lane 2 the A scales, lanes 3-4 the scales of the two B halves (warp 0 the operands
-    // and warp 6 the scales of every stage, or with kTurns both in turn), the scales through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows past the end read as
+    // Lane 0 loads the A rows, lane 1 the B rows of this CTA, lane 2 the A scales, lanes 3-4 the scales of the two B halves, those
+    // through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows past the end read as
     // zero), because only the tensor form of the copy may signal the peer's barrier.
-    constexpr int kStep = kTurns ? 2 : 1;
-    const int turn = kTurns && warp == 6 ? 1 : 0;
+    constexpr int kStep = TURNS ? 2 : 1;
+    const int turn = TURNS && warp == 6 ? 1 : 0;
     const bool sf = lane >= 2;
     const int half = lane < 2 ? (int)rank : (lane == 4 ? 1 : 0);  // the B half of a lane that serves B
     const bool serves_a = lane == 0 || lane == 2;
@@ -1282,7 +1278,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
                         : BLOCK_N == 256 || !sf   ? n_blk * BLOCK_N + half * (BLOCK_N / 2)
                                                   : ((n_blk * BLOCK_N) & ~127) + half * 128;
       const int my_row = serves_a ? a_row : b_row;
-      const bool mine = lane < 5 && (kTurns || sf == (warp == 6)) && (serves_a ? a_row < p.m : b_row < p.n_rows_b);
+      const bool mine = lane < 5 && (TURNS || sf == (warp == 6)) && (serves_a ? a_row < p.m : b_row < p.n_rows_b);
       const uint32_t tx = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && lane == 0)) * kAStageBytes +
                           (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && lane == 1)) * PC::kBHalfBytes +
                           (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && sf)) * (kST * 512u);
@@ -1598,7 +1594,7 @@ static tf_status make_output_map(CUtensorMap* map, const GemmParams& p) {
   return TF_OK;
 }
 
-template <int FMT, int EPI, int BLOCK_N>
+template <int FMT, int EPI, int BLOCK_N, bool TURNS = false>
 static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
   using PC = PairCfg<FMT, BLOCK_N>;
   CUtensorMap tsa, tsb, to = {};
@@ -1610,7 +1606,7 @@ static tf_status launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, 
   if (st != TF_OK) return st;
   st = make_scale_map(&tsb, p.sfb, (int64_t)p.sfb_row_tiles * p.sf_col_tiles, PC::kST);
   if (st != TF_OK) return st;
-  auto kernel = gemm_blockscaled_pair_kernel<FMT, EPI, BLOCK_N>;
+  auto kernel = gemm_blockscaled_pair_kernel<FMT, EPI, BLOCK_N, TURNS>;
   static thread_local int configured_dev = -1;
   int dev = 0;
   TF_CUDA(cudaGetDevice(&dev));
@@ -1679,6 +1675,17 @@ static int pair_width(int64_t m, int64_t n, int64_t stages, int epilogue) {
   const int64_t pairs = gemm_sms() / 2, m_blocks = (m + 255) / 256;
   auto waves = [&](int64_t bn) { return (double)((m_blocks * ((n + bn - 1) / bn) + pairs - 1) / pairs); };
   return waves(192) * (0.33 * (double)stages + 0.95) < 0.97 * waves(256) * (0.414 * (double)stages + 0.85) ? 192 : 256;
+}
+
+// Whether the load warps of a gated pair take the stages in turn. The gate's arithmetic, which runs beside the next tile's stages, competes with them for
+// issue slots: in turn they have two stages' time for five copies instead of one for two or three. It needs a next tile, and a tile's first
+// stage comes later for it. Split by kind -> in turn, cold, us: mxfp8 8192 x 3072 with K 512 / 1024 / 1536 / 2560 / 4096 60.2 / 65.4 / 69.1 / 98.2 / 145.1
+// -> 60.7 / 65.6 / 68.9 / 96.0 / 142.7; mxfp4 4096 x 4096 with K 1024 / 3072 / 5120 / 8192 38.7 / 47.4 / 66.9 / 96.1 -> 39.3 / 48.1 / 65.4 / 94.1; nvfp4 2048 x
+// 8192 with K 2048 / 5120 42.7 / 67.9 -> 43.3 / 66.8; one tile per pair mxfp8 1024 x 2304 x 2560 14.7 -> 14.9, 512 x 3072 x 2560 14.3 -> 14.6. Without
+// the gate it costs (mxfp4 300 x 8192 x 4096 12.3 -> 12.55, mxfp8 1024 x 4096 x 4096 residual 22.0 -> 22.65).
+static bool pair_turns(const GemmParams& p) {
+  const int64_t tiles = (int64_t)((p.m + 255) / 256) * ((p.n + 127) / 128);
+  return p.num_k_stages >= 16 && tiles > gemm_sms() / 2;
 }
 
 // How many clusters of `splits` GEMM CTAs (one CTA fills an SM) the current device runs at once: a cluster lives inside one GPC, so
@@ -1804,7 +1811,8 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
   if (pair_n == 192)
     return epilogue == TF_EPI_RESIDUAL ? launch_gemm_pair<FMT, TF_EPI_RESIDUAL, 192>(ta, tb, p, stream) : launch_gemm_pair<FMT, TF_EPI_NONE, 192>(ta, tb, p, stream);
   if (pair_n == 256) {
-    if (epilogue == TF_EPI_SILU_GATE) return launch_gemm_pair<FMT, TF_EPI_SILU_GATE, 256>(ta, tb, p, stream);
+    if (epilogue == TF_EPI_SILU_GATE)
+      return pair_turns(p) ? launch_gemm_pair<FMT, TF_EPI_SILU_GATE, 256, true>(ta, tb, p, stream) : launch_gemm_pair<FMT, TF_EPI_SILU_GATE, 256>(ta, tb, p, stream);
     if (epilogue == TF_EPI_RESIDUAL) return launch_gemm_pair<FMT, TF_EPI_RESIDUAL, 256>(ta, tb, p, stream);
     return launch_gemm_pair<FMT, TF_EPI_NONE, 256>(ta, tb, p, stream);
   }
