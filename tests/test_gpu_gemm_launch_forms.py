@@ -75,7 +75,8 @@ def test_pairs_that_take_more_than_one_tile(K, fmt, m, n, k):
 
 
 @pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "nvfp4"])
-@pytest.mark.parametrize("m,n,k,tiles", [(16, 38400, 544, 300), (100, 38392, 1056, 300), (40000, 128, 288, 313), (39937, 120, 544, 313)])
+@pytest.mark.parametrize("m,n,k,tiles", [(16, 38400, 544, 300), (100, 38392, 1056, 300), (40000, 128, 288, 313), (39937, 120, 544, 313), (40000, 32, 544, 313),
+                                         (40000, 24, 544, 313), (39937, 8, 1056, 313)])  # up to 24 columns: from the accumulator, no boxes
 def test_residual_tiles_of_128_columns_more_than_one_per_cta(K, fmt, m, n, k, tiles):
     """300 and 313 tiles on 148 CTAs: the staging boxes are filled again while the next tile's sums are formed, in one ring stage fewer."""
     form = K.gemm_launch_form(m, n, k, fmt, "residual")

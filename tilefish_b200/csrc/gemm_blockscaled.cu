@@ -889,13 +889,14 @@ __device__ __forceinline__ void prefetch_b_stage(const GemmParams& p, const CUte
 constexpr int kSplitNone = 0, kSplitPlanes = 1, kSplitCluster = 2;
 constexpr int kFormPair = 3;  // what tf_gemm_launch_form calls the CTA pair
 constexpr int kMaxClusterSplits = 8;  // the portable cluster size
-template <int FMT, int BLOCK_N, int EPI, int SPLITK>
+// BOXES (128-column tiles with a residual): a 4 KB staging box per epilogue warp in place of a ring stage, see epilogue_residual_128.
+template <int FMT, int BLOCK_N, int EPI, int SPLITK, bool BOXES = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                             const __grid_constant__ CUtensorMap tma_b, const GemmParams p) {
   using Cfg = TileCfg<FMT, BLOCK_N>;
-  constexpr bool kBoxes = EPI == TF_EPI_RESIDUAL && SPLITK == kSplitNone && BLOCK_N == 128;  // a 4 KB staging box per epilogue warp in place of a stage
-  constexpr int kBoxBytes = kBoxes ? 8 * 4096 : 0;
-  constexpr int kStages = Cfg::kStages - (kBoxes ? 1 : 0);
+  static_assert(!BOXES || (EPI == TF_EPI_RESIDUAL && SPLITK == kSplitNone && BLOCK_N == 128), "staging boxes");
+  constexpr int kBoxBytes = BOXES ? 8 * 4096 : 0;
+  constexpr int kStages = Cfg::kStages - (BOXES ? 1 : 0);
   static_assert(kBoxBytes <= (Cfg::kStages - kStages) * Cfg::kStageBytes, "the boxes take a stage's place");
   constexpr int kNB = Cfg::kNB;
   constexpr int kST = Cfg::kST;
@@ -1149,7 +1150,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
           if (grp == 0) epilogue_partial<FMT, BLOCK_N, 1, 0>(p, t_row + Cfg::kAccStride, bar_tmem_empty, lane, row, col0, ws_row);
           else epilogue_partial<FMT, BLOCK_N, 1, 1>(p, t_row + Cfg::kAccStride, bar_tmem_empty, lane, row, col0, ws_row);
         }
-      } else if (kBoxes) {
+      } else if (BOXES) {
         epilogue_residual_128<FMT>(p, t_row + acc_buf * Cfg::kAccStride, grp, bar_tmem_empty, lane, row, col0, alpha_t, amax2, smem_boxes + (uint32_t)(grp * 4 + q) * 4096u);
       } else if (acc_buf == 0) {
         if (grp == 0) epilogue_tile<FMT, BLOCK_N, EPI, 0, 0>(p, t_row, bar_tmem_empty, lane, row, col0, alpha_t, amax2);
@@ -1546,10 +1547,10 @@ static SplitPlan split_plan(int64_t m, int64_t n, int64_t k_bytes, int epilogue)
   return sp;
 }
 
-template <int FMT, int BLOCK_N, int EPI, int SPLITK>
+template <int FMT, int BLOCK_N, int EPI, int SPLITK, bool BOXES = false>
 static tf_status launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
   using Cfg = TileCfg<FMT, BLOCK_N>;
-  auto kernel = gemm_blockscaled_kernel<FMT, BLOCK_N, EPI, SPLITK>;
+  auto kernel = gemm_blockscaled_kernel<FMT, BLOCK_N, EPI, SPLITK, BOXES>;
   static thread_local int configured_dev = -1;
   int dev = 0;
   TF_CUDA(cudaGetDevice(&dev));
@@ -1836,8 +1837,12 @@ static tf_status dispatch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, Gem
     return launch_gemm_pair<FMT, TF_EPI_NONE, 256>(ta, tb, p, stream);
   }
   if (epilogue == TF_EPI_SILU_GATE) return launch_gemm<FMT, 256, TF_EPI_SILU_GATE, kSplitNone>(ta, tb, p, stream);
-  if (epilogue == TF_EPI_RESIDUAL)
-    return lp.block_n == 256 ? launch_gemm<FMT, 256, TF_EPI_RESIDUAL, kSplitNone>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_RESIDUAL, kSplitNone>(ta, tb, p, stream);
+  if (epilogue == TF_EPI_RESIDUAL) {
+    if (lp.block_n == 256) return launch_gemm<FMT, 256, TF_EPI_RESIDUAL, kSplitNone>(ta, tb, p, stream);
+    // Up to 24 columns a staged row is 6 lanes of 16, and the ring keeps its stage: staged -> from the accumulator, mxfp8 33507 x 8 x 14112 129.7 -> 120.4 us,
+    // x 24 84.7 -> 82.9, 64959 x 16 x 2048 42.3 -> 40.2, nvfp4 11355 x 8 x 1696 8.4 -> 7.8; at 32 columns 42.3 -> 43.9 and 8.7 -> 9.9.
+    return p.n > 24 ? launch_gemm<FMT, 128, TF_EPI_RESIDUAL, kSplitNone, true>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_RESIDUAL, kSplitNone>(ta, tb, p, stream);
+  }
   return lp.block_n == 256 ? launch_gemm<FMT, 256, TF_EPI_NONE, kSplitNone>(ta, tb, p, stream) : launch_gemm<FMT, 128, TF_EPI_NONE, kSplitNone>(ta, tb, p, stream);
 }
 
