@@ -855,13 +855,14 @@ __device__ __forceinline__ void cluster_reduce(const GemmParams& p, uint32_t dum
 // A dependent of at most 128 rows streams its weights once, and HBM is idle while it waits: the row kernels between two GEMMs of a decode
 // step touch a few MB. So a waiting CTA asks its first stages of B and their scales into L2. Nothing is read here: the lines are coherent
 // with what the kernel in front may still write (it may be the one that quantizes these weights), and the loads behind griddep_wait()
-// read them as they would without. 70B-shaped NVFP4 blocks under sustained load, us per captured step, plain -> dependent -> with this: 64 rows, 4 layers
-// 402 -> 396 -> 391.5; 16 rows, 2 layers 189.4 -> 187.2 -> 186.3; 128 rows, 2 layers 221.5 -> 219.3 -> 217.6; MXFP8 block 64 x 4096 x 8192 40.4 -> 40.0 -> 39.0;
-// MXFP4 1 x 4096 x 14336, 2 layers 68.6 -> 69.0 -> 67.7. More stages give the first of these up to 1 % and cost others as much (MXFP8 64 x 8192 x 14336
-// 174 at 8, 176 at 16): the SM's copy engine serves the prefetch before the loads (about 2.7 clocks per 128-byte row), which is also why
-// prefetching ahead inside the main loop or for other CTAs' tiles loses (64 x 28672 x 8192 + gate 50.6 -> 53.4 us; 2 to 3 us per layer).
-// It stands in the epilogue's branch: in front of the roles the same code cost every launch 0.2 us (68.6 -> 70.6 for the last of these).
-constexpr int kEarlyStages = 8;
+// read them as they would without. Captured stacks, us per step, dependents without -> with this: 70B-shaped NVFP4 blocks 64 rows, 4 layers 382.7 ->
+// 378.6, 128 rows, 2 layers 209.0 -> 207.8; MXFP8 64 x 4096 x 8192, 4 layers 146.5 -> 142.5, 8 x 2560 x 3072, 6 layers 105.8 -> 100.7; MXFP4 1 x 4096 x 14336,
+// 3 layers 103.3 -> 101.4. Eight stages give the first 376.2 and the fourth 99.4, but behind a GEMM that streams weights of its own they take
+// HBM from its last CTAs: nvfp4 8 x 26240 x 5984 back to back over cold weights 19.4 without, 19.5 with four, 20.4 with eight, mxfp4 3 x 20096 x 4096
+// 13.1 / 13.1 / 13.6 (mxfp8 2 x 34432 x 608 9.5 / 8.9 / 8.9). The SM's copy engine serves the prefetch before the loads (about 2.7
+// clocks per 128-byte row), so prefetching ahead inside the main loop or for other CTAs' tiles loses too (64 x 28672 x 8192 + gate 50.6 -> 53.4 us;
+// 2 to 3 us per layer). It stands in the epilogue's branch: in front of the roles the same code cost every launch 0.2 us.
+constexpr int kEarlyStages = 4;
 constexpr unsigned kEarlyStageNs = 300;  // pause between two stages: 36 KB per SM and pause is more than HBM brings
 __device__ __forceinline__ void l2_prefetch_2d(const CUtensorMap* map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
