@@ -38,25 +38,33 @@ tf_status scale_padding(void* scales, int32_t format, int64_t rows, int64_t k, i
 
 // Programmatic dependent launch (tf_set_programmatic_launch): a kernel launched through launch_dependent() may be scheduled
 // while the kernel before it on the stream is still draining, so that its launch latency and set-up overlap that tail. Every
-// kernel launched this way executes griddep_wait() before its first access to global memory, which blocks until the previous
-// kernel has completed and its writes are visible. Three settings: never, always, or (until the caller says otherwise) for chains of short
-// kernels only (`chain`, see chain_gemm_launch), and those only without an SM margin: a dependent GEMM's waiting CTAs would take the
-// SMs that the margin leaves to the kernel beside it.
+// thread of such a kernel executes griddep_wait() before it reads or writes anything that the kernel in front may write or read; the wait
+// ends when that kernel has completed and its writes are visible. Two things happen before it: a GEMM asks weights into L2
+// (prefetch_b_stage: nothing is read), and the nvfp4 quantizer loads the tensor that its own amax launch in front only reads
+// (quantize_tiles_kernel: that launch is a plain one, so the tensor is complete).
+// Three settings: never, always, or (until the caller says otherwise) for chains of short kernels only (`chain`, see chain_gemm_launch),
+// and those only without an SM margin: a dependent GEMM's waiting CTAs would take the SMs that the margin leaves to the kernel beside it.
 int sm_margin();
 bool dependent_launch(bool chain);
 void set_programmatic_launch(int setting);  // 0 never, 1 always, -1 the rule
 
 #ifdef __CUDACC__
-// The rule: GEMMs of at most 256 rows (above 128 and with one CTA per tile: of one wave), gated GEMMs of CTA pairs in one wave up to 1024 rows, row kernels of at most four rows, and the nvfp4 quantizer behind its
-// own amax launch up to 16 M elements (launch_quantize). A GEMM's CTAs take a whole SM each, so starting early only hides their set-up: 200
-// GEMMs back to back on a full queue, plain -> dependent: mxfp8 1 x 2560 x 3072 8.2 -> 5.9 us, 128 x 6144 x 2560 11.6 -> 9.0, nvfp4
-// 64 x 8192 x 28672 36.7 -> 32.9; pairs in two waves mxfp4 256 x 16384 x 2048 + gate 20.5 -> 17.2, mxfp8 256 x 28672 x 2048 22.5 -> 20.6; one CTA per tile in
-// two waves nvfp4 64 x 28672 x 8192 + gate 52.2 -> 52.1 back to back, where it gains behind a row kernel instead (prefetch_b_stage). A row kernel's CTAs are small: started
-// early they all pile onto the few SMs that the GEMM in front leaves free and then share those (70B-shaped decode at 64 rows: its
-// rmsnorm launch went from 9.8 to 14.7 us; two blocks at 16 rows 184.6 us without, 190.4 with). Above 256 rows the waiting CTAs
-// take the registers that the rest of the row kernel in front needs (README block at 8192 rows 189.5 -> 196.2 us).
-// The gated pairs stand behind a row kernel whose blocks all fit beside them: mxfp8 block 2560 x 3072 at 300 / 384 / 512 / 700 rows 32.8 / 32.7 / 33.2 / 36.7 -> 31.8 / 31.3 / 32.6 /
-// 34.8 us, nvfp4 2048 x 4096 at 512 32.6 -> 31.6; the second GEMM as a dependent too gives back half of it (32.7 / 32.5 / 33.9 / 35.4).
+// The rule: GEMMs of at most 256 rows (above 128 and with one CTA per tile: of one wave), gated GEMMs of CTA pairs in one wave up to 1024
+// rows, row kernels of at most four rows, and the nvfp4 quantizer behind its own amax launch up to 16 M elements (launch_quantize).
+// A GEMM's CTAs take a whole SM each, so starting early only hides their set-up: 200 GEMMs back to back on a full queue, plain ->
+// dependent: mxfp8 1 x 2560 x 3072 8.2 -> 5.9 us, 128 x 6144 x 2560 11.6 -> 9.0, nvfp4 64 x 8192 x 28672 36.7 -> 32.9; pairs in two
+// waves mxfp4 256 x 16384 x 2048 + gate 20.5 -> 17.2, mxfp8 256 x 28672 x 2048 22.5 -> 20.6; one CTA per tile in two waves nvfp4
+// 64 x 28672 x 8192 + gate 52.2 -> 52.1 back to back, where it gains behind a row kernel instead (prefetch_b_stage).
+// A row kernel's CTAs are small: started early they all pile onto the few SMs that the GEMM in front leaves free and then share those
+// (70B-shaped decode at 64 rows: its rmsnorm launch went from 9.8 to 14.7 us; two blocks at 16 rows 184.6 us without, 190.4 with).
+// Above 256 rows the waiting CTAs take the registers that the rest of the row kernel in front needs (README block at 8192 rows
+// 189.5 -> 196.2 us). Gated pairs of one wave stand behind a row kernel of at most 1024 rows, which fits beside them. Graphs of 12 chains,
+// 15 shapes of 300 to 1024 rows, 1024 to 16384 columns and 2048 to 4608 gate columns in each format, plain -> dependent: behind rmsnorm
+// (and a quantizer and second GEMM) mxfp8 512 x 2560 x 3072 33.1 -> 31.8 us, 700 x 2560 x 3072 40.6 -> 39.0, 1024 x 8192 x 2304 76.9 -> 75.8,
+// nvfp4 1024 x 4096 x 2304 38.1 -> 36.5; behind a quantizer alone mxfp8 512 x 8192 x 4608 36.9 -> 35.5, mxfp4 1024 x 2560 x 2304 15.3 ->
+// 14.2, nvfp4 300 x 4096 x 4096 16.4 -> 16.0. All between 0.93 and 1.01 of the time; 300 x 1024 x 2048 is the one that gains nothing. Only
+// behind one another do 48 tiles of long K lose (512 x 3072 x 8192 mxfp8 30.3 -> 31.4, 1024 x 2304 x 8192 33.6 -> 32.5). The second GEMM
+// of a block as a dependent too gives back half of the gain.
 // Captured graphs, before -> after: README block at one row 20.5 -> 18.4 us, 70B-shaped decode at 64 rows 402 -> 389, two
 // 4096 x 8192 blocks at 200 rows 93 -> 85.
 enum class GemmKind { kOneCta, kPair, kGatedPair };

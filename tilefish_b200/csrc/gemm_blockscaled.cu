@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_kernel(const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  // barriers and tensor memory are set up; no role touches global memory before its own griddep_wait()
+  // barriers and tensor memory are set up; every role waits (griddep_wait) before it reads or writes global memory
 
   if (warp == 0 || warp == 6) {
     // ---------------- load warps: warp 0 the operand tiles (TMA), warp 6 the scale tiles (bulk copies) ----------------
