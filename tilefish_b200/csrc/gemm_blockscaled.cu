@@ -1277,17 +1277,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
 
   if (warp == 0 || warp == 6) {
     // ---------------- load warps (each CTA loads its own halves; completion is counted on the leader's barrier) ----------------
-    // Lane 0 loads the A rows, lane 1 the B rows of this CTA, lane 2 the A scales, lanes 3-4 the scales of the two B halves, those
-    // through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is always kST tiles, rows past the end read as
-    // zero), because only the tensor form of the copy may signal the peer's barrier.
+    // Role 0 loads the A rows, role 1 the B rows of this CTA, role 2 the A scales, roles 3-4 the scales of the two B halves: lanes 0-4 of both
+    // warps with TURNS, else lanes 0-1 of warp 0 and 0-2 of warp 6 (on lanes 2-4 the scales came 1 to 2 % later for short K: mxfp8
+    // 6933 x 128 x 736 + gate 9.03 -> 9.17 us). The scales go through tensor maps too ([tiles, 512 bytes] as 128 x u32 rows; a box is
+    // always kST tiles, rows past the end read as zero), because only the tensor form of the copy may signal the peer's barrier.
     constexpr int kStep = TURNS ? 2 : 1;
     const int turn = TURNS && warp == 6 ? 1 : 0;
-    const bool sf = lane >= 2;
-    const int half = lane < 2 ? (int)rank : (lane == 4 ? 1 : 0);  // the B half of a lane that serves B
-    const bool serves_a = lane == 0 || lane == 2;
-    const CUtensorMap* my_map = lane == 0 ? &tma_a : lane == 1 ? &tma_b : lane == 2 ? &tma_sfa : &tma_sfb;
-    const uint32_t my_dst = lane == 0 ? smem_a : lane == 1 ? smem_b : lane == 2 ? smem_sfa : smem_sfb + (uint32_t)half * kST * 512;
-    const uint32_t my_stage_bytes = lane == 0 ? kAStageBytes : lane == 1 ? PC::kBHalfBytes : lane == 2 ? PC::kSfaStageBytes : PC::kSfbStageBytes;
+    const int role = TURNS || warp == 0 ? lane : lane + 2;
+    const bool sf = role >= 2;
+    const int half = role < 2 ? (int)rank : (role == 4 ? 1 : 0);  // the B half of a role that serves B
+    const bool serves_a = role == 0 || role == 2;
+    const CUtensorMap* my_map = role == 0 ? &tma_a : role == 1 ? &tma_b : role == 2 ? &tma_sfa : &tma_sfb;
+    const uint32_t my_dst = role == 0 ? smem_a : role == 1 ? smem_b : role == 2 ? smem_sfa : smem_sfb + (uint32_t)half * kST * 512;
+    const uint32_t my_stage_bytes = role == 0 ? kAStageBytes : role == 1 ? PC::kBHalfBytes : role == 2 ? PC::kSfaStageBytes : PC::kSfbStageBytes;
     int stage = turn, ks0 = turn;
     uint32_t phase = 0;
     bool ok = true;
@@ -1299,10 +1301,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_blockscaled_pair_kernel(
                         : BLOCK_N == 256 || !sf   ? n_blk * BLOCK_N + half * (BLOCK_N / 2)
                                                   : ((n_blk * BLOCK_N) & ~127) + half * 128;
       const int my_row = serves_a ? a_row : b_row;
-      const bool mine = lane < 5 && (TURNS || sf == (warp == 6)) && (serves_a ? a_row < p.m : b_row < p.n_rows_b);
-      const uint32_t tx = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && lane == 0)) * kAStageBytes +
-                          (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && lane == 1)) * PC::kBHalfBytes +
-                          (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, mine && sf)) * (kST * 512u);
+      const bool mine = role < (TURNS || warp == 6 ? 5 : 2) && (serves_a ? a_row < p.m : b_row < p.n_rows_b);
+      const uint32_t copies = __ballot_sync(0xFFFFFFFFu, mine) << (TURNS || warp == 0 ? 0 : 2);  // a bit per role
+      const uint32_t tx = (copies & 1u) * kAStageBytes + (copies >> 1 & 1u) * PC::kBHalfBytes + (uint32_t)__popc(copies >> 2) * (kST * 512u);
       const int y_base = sf ? (my_row >> 7) * p.sf_col_tiles : my_row;
       int ks = ks0;
       for (; ks < p.num_k_stages; ks += kStep) {
