@@ -92,4 +92,4 @@ def test_narrow_rows_take_no_longer_than_wide_ones(K, fmt):
         return min(times[2:])
 
     wide = time(256)
-    assert max(time(32), time(64), time(96), time(128)) <= 2.0 * wide and time(192) <= 1.5 * wide
+    assert max(time(32), time(64), time(96), time(128)) <= 2.0 * wide and time(192) <= 1.25 * wide
